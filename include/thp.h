@@ -196,8 +196,9 @@ int thp_batch_destroy(thp_batch* b);
  * energy.  The torques need the frame atoms given to thp_set_frames (kept
  * when thp_set_rpole later replaces the multipoles).  THP_E_STATE without
  * frames or without a solve since the last position / multipole change.
- * Gradients accumulate in 64-bit fixed point (2^-34 kcal/mol/A) in both
- * precisions, so the order of the per-atom additions does not matter. */
+ * Gradients accumulate in 64-bit fixed point (2^-34 kcal/mol/A, in the FP64
+ * form with a second word for the remainders), so the order of the per-atom
+ * additions does not matter. */
 int thp_get_gradient(thp_ctx* ctx, double* dep, double* ep);
 /* same gradient into device memory d_dep [n][3], enqueued on the context's
  * stream without a host synchronisation */

@@ -126,7 +126,7 @@ struct Ctx {
   float* d_muf = nullptr;         // [n][8] FP32 sorted dipoles for the mixed gradient pass
   int2* d_vinfo = nullptr;
   // vdW pair list (vlistcell): full list within vdwcut + lbuffer of the
-  // reduced sites, slot-major [s*npad + i], rebuilt after a re-sort or when an
+  // reduced sites, at pair_slot(maxvnb/8, i, s), rebuilt after a re-sort or when an
   // atom has moved lbuffer/2 since the positions it was built from
   int maxvnb = 0;
   int* d_vnb = nullptr;
@@ -140,7 +140,7 @@ struct Ctx {
   double* d_em = nullptr;         // their total (d_empart + blocks), made on first use
   double4* d_pos_built = nullptr; // positions at the last list build
 
-  // full neighbor list within ewaldcut+lbuffer (slot-major: nb[s*npad+i])
+  // full neighbor list within ewaldcut+lbuffer (entry s of atom i at pair_slot(maxpr/8, i, s))
   int maxnb = 0;
   int* d_nnb = nullptr;
   int* d_nb = nullptr;
@@ -204,7 +204,7 @@ struct Ctx {
 
   // polarization gradient (allocated on first use)
   double* d_fphirec = nullptr;    // [n][20] permanent-multipole potential, fractional
-  unsigned long long* d_depfix = nullptr;  // [n][3] 64-bit fixed-point gradient, sorted
+  unsigned long long* d_depfix = nullptr;  // [n][3] 64-bit fixed-point gradient, sorted (FP64 form: then the low words)
   double* d_trq = nullptr;        // [n][3] reciprocal-space torque
   // virial of the polarization gradient (thp_set_virial): partial sums on
   // the device, and the last gradient call's totals: the reference's terms

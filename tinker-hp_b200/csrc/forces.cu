@@ -10,7 +10,7 @@
 //     at every site for the torques;
 //   * self torque (epolar1.f:190-206), and torque (torque.f:6-390) for the
 //     Z-then-X and Bisector frames.
-// One thread owns atom i over the full neighbor list (each pair is evaluated
+// Eight lanes own atom i over its interacting pairs (each pair is evaluated
 // from both ends, the i-side terms only).  The three torques of a site are
 // summed before one torque distribution.  Gradients are accumulated in 64-bit
 // fixed point with 2^-34 kcal/mol/A resolution, so the order in which threads
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kBlock) k_force_recip(int n, PmeGeom g, const 
                                                         const double* __restrict__ fphirec,
                                                         const double* __restrict__ mu, const double* __restrict__ rp,
                                                         double* __restrict__ trq_out,
-                                                        unsigned long long* __restrict__ dep,
+                                                        FixAcc dep,
                                                         double* __restrict__ vpart) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double vs[6] = {0, 0, 0, 0, 0, 0};
@@ -131,9 +131,9 @@ __global__ void __launch_bounds__(kBlock) k_force_recip(int n, PmeGeom g, const 
   f1 = 0.5 * (double)g.n1 * f1;
   f2 = 0.5 * (double)g.n2 * f2;
   f3 = 0.5 * (double)g.n3 * f3;
-  fix_add(dep + 3 * i + 0, g.recip[0] * f1);
-  fix_add(dep + 3 * i + 1, g.recip[1] * f2);
-  fix_add(dep + 3 * i + 2, g.recip[2] * f3);
+  dep.add(3 * i + 0, g.recip[0] * f1);
+  dep.add(3 * i + 1, g.recip[1] * f2);
+  dep.add(3 * i + 2, g.recip[2] * f3);
   // cphidprec = fphi_to_cphi(fphidprec/2), torque on the permanent moments
   double cp[10];
   cp[0] = 0.5 * FS[1];
@@ -250,362 +250,289 @@ struct EwC {
   double a, f1, f2, f3, f4;  // 2 a^2 powers / (sqrt(pi) a) of dampewald order 9
 };
 
-// epreal1c pair terms seen from atom i over its full list, the self torque,
-// and the torque distribution of the summed torque of site i.
+// The radial functions of one pair (each with electric/2 folded in):
+// Ewald-damped e_l and bare rr_l of l = 3, 5, 7, 9, and the Thole factors
+// l3, l5, l7 with their derivatives q_l = (dl_l/dr) / r.
+template <typename T>
+struct PairRadial {
+  T e3, e5, e7, e9, rr3, rr5, rr7, rr9;
+  T l3, l5, l7, q3, q5, q7;
+};
+
+// Interaction of the permanent moments of sites i and k with the induced
+// dipoles u at i and v at k under one scale factor s (epolar1.f:1700-2170):
+//   W = F3 (ck u.r - ci v.r + u.dk + v.di)
+//     + F5 (2 v.Qi r - 2 u.Qk r - u.r dk.r - v.r di.r) + F7 (u.r qk - v.r qi)
+// with r = x_k - x_i, F_l = e_l - (1 - s l_l) rr_l, qk = r.Qk r.  Adds dW/dr to
+// frc (the F's own derivatives are -D_l r with D_l = e_{l+2} -
+// (1 - s l_l) rr_{l+2} - s q_l rr_l), and the field and field gradient of v at i
+// to uf and duf (:2230-2260).  The reference expands the second-derivative
+// tensors of each moment; gathering the terms by F_l first gives the same
+// sums in about a quarter of the operations.
+template <typename T>
+__device__ __forceinline__ void perm_terms(const PairRadial<T>& p, T s, const T (&r)[3], const T (&u)[3],
+                                           const T (&v)[3], T ur, T vr, T ci, const T (&di)[3], const T (&Qi)[6],
+                                           T ck, const T (&dk)[3], const T (&Qk)[6], const T (&qi)[3],
+                                           const T (&qk)[3], T dir, T dkr, T qir, T qkr, T (&frc)[3], T (&uf)[3],
+                                           T (&duf)[6]) {
+  const T n3 = T(1) - s * p.l3, n5 = T(1) - s * p.l5, n7 = T(1) - s * p.l7;
+  const T F3 = p.e3 - n3 * p.rr3, F5 = p.e5 - n5 * p.rr5, F7 = p.e7 - n7 * p.rr7;
+  const T D3 = p.e5 - n3 * p.rr5 - s * p.q3 * p.rr3;
+  const T D5 = p.e7 - n5 * p.rr7 - s * p.q5 * p.rr5;
+  const T D7 = p.e9 - n7 * p.rr9 - s * p.q7 * p.rr7;
+  const T A3 = ck * ur - ci * vr + (u[0] * dk[0] + u[1] * dk[1] + u[2] * dk[2]) +
+               (v[0] * di[0] + v[1] * di[1] + v[2] * di[2]);
+  const T A5 = T(2) * ((v[0] * qi[0] + v[1] * qi[1] + v[2] * qi[2]) - (u[0] * qk[0] + u[1] * qk[1] + u[2] * qk[2])) -
+               ur * dkr - vr * dir;
+  const T A7 = ur * qkr - vr * qir;
+  const T rad = D3 * A3 + D5 * A5 + D7 * A7;
+  const T cu = F3 * ck - F5 * dkr + F7 * qkr, cv = -F3 * ci - F5 * dir - F7 * qir;
+  const T cdk = -F5 * ur, cdi = -F5 * vr, cqk = T(2) * F7 * ur, cqi = T(-2) * F7 * vr, c2 = T(2) * F5;
+  // Q = xx xy xz yy yz zz
+  const T Qkux = Qk[0] * u[0] + Qk[1] * u[1] + Qk[2] * u[2], Qivx = Qi[0] * v[0] + Qi[1] * v[1] + Qi[2] * v[2];
+  const T Qkuy = Qk[1] * u[0] + Qk[3] * u[1] + Qk[4] * u[2], Qivy = Qi[1] * v[0] + Qi[3] * v[1] + Qi[4] * v[2];
+  const T Qkuz = Qk[2] * u[0] + Qk[4] * u[1] + Qk[5] * u[2], Qivz = Qi[2] * v[0] + Qi[4] * v[1] + Qi[5] * v[2];
+  frc[0] += cu * u[0] + cv * v[0] + cdk * dk[0] + cdi * di[0] + cqk * qk[0] + cqi * qi[0] + c2 * (Qivx - Qkux) -
+            rad * r[0];
+  frc[1] += cu * u[1] + cv * v[1] + cdk * dk[1] + cdi * di[1] + cqk * qk[1] + cqi * qi[1] + c2 * (Qivy - Qkuy) -
+            rad * r[1];
+  frc[2] += cu * u[2] + cv * v[2] + cdk * dk[2] + cdi * di[2] + cqk * qk[2] + cqi * qi[2] + c2 * (Qivz - Qkuz) -
+            rad * r[2];
+  const T w5 = F5 * vr, w7 = F7 * vr;
+  uf[0] += F3 * v[0] - w5 * r[0];
+  uf[1] += F3 * v[1] - w5 * r[1];
+  uf[2] += F3 * v[2] - w5 * r[2];
+  const T tx = c2 * v[0] - w7 * r[0], ty = c2 * v[1] - w7 * r[1], tz = c2 * v[2] - w7 * r[2];
+  duf[0] += r[0] * tx;
+  duf[1] += r[0] * ty + r[1] * tx;
+  duf[2] += r[1] * ty;
+  duf[3] += r[0] * tz + r[2] * tx;
+  duf[4] += r[1] * tz + r[2] * ty;
+  duf[5] += r[2] * tz;
+}
+
+// epreal1c pair terms seen from atom i over its interacting pairs, the self
+// torque, and the torque distribution of the summed torque of site i.
 // resident blocks of the mixed gradient pass the register budget is cut for
 #ifndef THP_FORCE_MINB
 #define THP_FORCE_MINB 4
 #endif
 
-// lanes per site of the real-space gradient pass (1 or 8)
-#ifndef THP_FORCE_LPA
-#define THP_FORCE_LPA 8
-#endif
+// special partners of a site held in registers (a longer list is searched
+// past those)
+constexpr int kSpCache = 4;
 
+// A warp takes four consecutive (cell-sorted) sites, eight lanes each; the
+// partners come from the pair stream of the solve whose dipoles are
+// differentiated (the pairs within ewaldcut at these positions, 32 consecutive
+// entries per warp step), lane j of a site taking its slots j, j+8, ...  The
+// lanes' sums are combined in a fixed shuffle tree and the first lane of the
+// site finishes it.  The pass is bound by the pair arithmetic.
 // VIR: each block also writes to vpart[block][12] the sum of its sites' pair
 // virials (epolar1.f:2326-2342, half from each end of a pair) and the
 // frame-atom virial of their real-space torques (:2460-2486) in 0..5, and
 // the frame-atom virial of their reciprocal and self torques, which the
 // reference does not add, in 6..11.
-// LPA: lanes per atom.  1: one thread per site over its whole list; 8: a
-// warp takes four consecutive (cell-sorted) sites, eight lanes each, lane j
-// taking list entries j, j+8, ...; the lanes' sums are combined in a fixed
-// shuffle tree and the first lane of the site finishes it.
-template <bool MIXED, bool VIR, int LPA>
+template <bool MIXED, bool VIR>
 __global__ void __launch_bounds__(kBlock, MIXED ? THP_FORCE_MINB : 1) k_force_real(
-    int n, int npad, Box box, double off2, EwC ew, const double4* __restrict__ pos,
+    int n, Box box, EwC ew, const double4* __restrict__ pos,
     const typename std::conditional<MIXED, float, double>::type* __restrict__ mrec, const double* __restrict__ mu,
     const float* __restrict__ erec, const float* __restrict__ muf, const int* __restrict__ perm,
     const int* __restrict__ sp_off, const int* __restrict__ sp_ks, const double* __restrict__ sp_s,
-    const int* __restrict__ nnb, const int* __restrict__ nb, int maxnb, const int* __restrict__ frs,
-    const double* __restrict__ trq_recip, unsigned long long* __restrict__ dep, double* __restrict__ vpart) {
+    const int* __restrict__ npr, const int* __restrict__ pk, int cap8, const int* __restrict__ frs,
+    const double* __restrict__ trq_recip, FixAcc dep, double* __restrict__ vpart) {
   using T = typename std::conditional<MIXED, float, double>::type;
-  static_assert(LPA == 1 || LPA == 8, "one or eight lanes per site");
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i0 = LPA == 1 ? t : t >> 3, jl = LPA == 1 ? 0 : t & 7;
+  const int i0 = t >> 3, jl = t & 7;
   const bool live = i0 < n;
-  if (LPA == 1 && !live && !VIR) return;
   const int i = live ? i0 : n - 1;  // a valid site for the loads of idle lanes
   double vout[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   {
   const double4 pi4 = pos[i];
   // mixed form: partners from the 64-B FP32 site record (wrapped position,
   // 1/pdamp, thole, multipoles) and the FP32 dipole record, imaged in FP32
-  float xi = 0.f, yi = 0.f, zi = 0.f;
+  float xi = 0.f, yi = 0.f, zi = 0.f, ipdi = 0.f;
   if constexpr (MIXED) {
     xi = erec[(size_t)i * 16 + 0];
     yi = erec[(size_t)i * 16 + 1];
     zi = erec[(size_t)i * 16 + 2];
+    ipdi = erec[(size_t)i * 16 + 3];
   }
   const float bxf = (float)box.l[0], byf = (float)box.l[1], bzf = (float)box.l[2];
   const float hxf = 0.5f * bxf, hyf = 0.5f * byf, hzf = 0.5f * bzf;
-  const float off2f = (float)off2;
   const T* ri = mrec + (size_t)i * 12;
-  const T pti = (T)ri[0], ci = (T)ri[1], dix = (T)ri[2], diy = (T)ri[3], diz = (T)ri[4];
-  const T qixx = (T)ri[5], qixy = (T)ri[6], qixz = (T)ri[7], qiyy = (T)ri[8], qiyz = (T)ri[9], qizz = (T)ri[10];
+  const T pti = ri[0], ci = ri[1];
+  const T di[3] = {ri[2], ri[3], ri[4]};
+  const T Qi[6] = {ri[5], ri[6], ri[7], ri[8], ri[9], ri[10]};
   const double* mi = mu + (size_t)i * 6;
-  const T uix = (T)mi[0], uiy = (T)mi[1], uiz = (T)mi[2], uixp = (T)mi[3], uiyp = (T)mi[4], uizp = (T)mi[5];
-  const T pdi = (T)pi4.w;
+  const T ud[3] = {(T)mi[0], (T)mi[1], (T)mi[2]}, up[3] = {(T)mi[3], (T)mi[4], (T)mi[5]};
   const int io = perm[i];
   const int s0 = sp_off[io], s1 = sp_off[io + 1];
+  int spk[kSpCache];
+#pragma unroll
+  for (int q = 0; q < kSpCache; ++q) spk[q] = s0 + q < s1 ? __ldg(sp_ks + s0 + q) : -1;
   const T f = (T)(0.5 * kElectric);
   double gx = 0.0, gy = 0.0, gz = 0.0;
   T uf[3] = {0, 0, 0}, duf[6] = {0, 0, 0, 0, 0, 0};
   T vp[6] = {0, 0, 0, 0, 0, 0};  // pair virial, half of each pair's
-  const int nn = live ? min(nnb[i], maxnb) : 0;
+  const int nn = live ? npr[i] : 0;
+  const int* __restrict__ row = pk + pair_slot(cap8, i, jl);  // slot s: 4 (s - j) entries on
+  int knext = jl < nn ? __ldg(row) : i;  // partners fetched one step ahead of their records
 #pragma unroll 1
-  for (int s = jl; s < nn; s += LPA) {
-    const int k = __ldg(nb + (size_t)s * npad + i);
-    T xr, yr, zr, r2, pdk;
-    T ptk, ck, dkx, dky, dkz, qkxx, qkxy, qkxz, qkyy, qkyz, qkzz;
-    T ukx, uky, ukz, ukxp, ukyp, ukzp;
+  for (int s = jl; s < nn; s += 8) {
+    const int k = knext;
+    if (s + 8 < nn) knext = __ldg(row + 4 * (size_t)(s + 8 - jl));
+    T r[3], r2, pdk, ptk, ck, dk[3], Qk[6], vd[3], vq[3];
     if constexpr (MIXED) {
-      float v[16];
-      ld_rec8(erec + (size_t)k * 16, *reinterpret_cast<float(*)[8]>(&v[0]));
-      float x = v[0] - xi, y = v[1] - yi, z = v[2] - zi;
-      x = fabsf(x) > hxf ? x - copysignf(bxf, x) : x;
-      y = fabsf(y) > hyf ? y - copysignf(byf, y) : y;
-      z = fabsf(z) > hzf ? z - copysignf(bzf, z) : z;
-      const float rf2 = x * x + y * y + z * z;
-      if (rf2 > off2f) continue;
-      ld_rec8(erec + (size_t)k * 16 + 8, *reinterpret_cast<float(*)[8]>(&v[8]));
-      float u[8];
-      ld_rec8(muf + (size_t)k * 8, u);
-      xr = x;
-      yr = y;
-      zr = z;
-      r2 = rf2;
-      pdk = v[3] != 0.f ? 1.f / v[3] : 0.f;
-      ptk = v[4];
-      ck = v[5];
-      dkx = v[6];
-      dky = v[7];
-      dkz = v[8];
-      qkxx = v[9];
-      qkxy = v[10];
-      qkxz = v[11];
-      qkyy = v[12];
-      qkyz = v[13];
-      qkzz = v[14];
-      ukx = u[0];
-      uky = u[1];
-      ukz = u[2];
-      ukxp = u[3];
-      ukyp = u[4];
-      ukzp = u[5];
+      float w[16], m[8];
+      ld_rec8(erec + (size_t)k * 16, *reinterpret_cast<float(*)[8]>(&w[0]));
+      ld_rec8(erec + (size_t)k * 16 + 8, *reinterpret_cast<float(*)[8]>(&w[8]));
+      ld_rec8(muf + (size_t)k * 8, m);
+      float x = w[0] - xi, y = w[1] - yi, z = w[2] - zi;
+      r[0] = fabsf(x) > hxf ? x - copysignf(bxf, x) : x;
+      r[1] = fabsf(y) > hyf ? y - copysignf(byf, y) : y;
+      r[2] = fabsf(z) > hzf ? z - copysignf(bzf, z) : z;
+      r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+      pdk = w[3];
+      ptk = w[4];
+      ck = w[5];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        dk[q] = w[6 + q];
+        vd[q] = m[q];
+        vq[q] = m[3 + q];
+      }
+#pragma unroll
+      for (int q = 0; q < 6; ++q) Qk[q] = w[9 + q];
     } else {
       const double4 pk4 = pos[k];
-      double xrd = pk4.x - pi4.x, yrd = pk4.y - pi4.y, zrd = pk4.z - pi4.z;
-      image3(box, xrd, yrd, zrd);
-      const double r2d = r2_exact(xrd, yrd, zrd);
-      if (r2d > off2) continue;
-      xr = (T)xrd;
-      yr = (T)yrd;
-      zr = (T)zrd;
-      r2 = (T)r2d;
-      pdk = (T)pk4.w;
-      const T* rk = mrec + (size_t)k * 12;
-      ptk = (T)rk[0];
-      ck = (T)rk[1];
-      dkx = (T)rk[2];
-      dky = (T)rk[3];
-      dkz = (T)rk[4];
-      qkxx = (T)rk[5];
-      qkxy = (T)rk[6];
-      qkxz = (T)rk[7];
-      qkyy = (T)rk[8];
-      qkyz = (T)rk[9];
-      qkzz = (T)rk[10];
-      const double* mk = mu + (size_t)k * 6;
-      ukx = (T)mk[0];
-      uky = (T)mk[1];
-      ukz = (T)mk[2];
-      ukxp = (T)mk[3];
-      ukyp = (T)mk[4];
-      ukzp = (T)mk[5];
+      r[0] = pk4.x - pi4.x;
+      r[1] = pk4.y - pi4.y;
+      r[2] = pk4.z - pi4.z;
+      image3(box, r[0], r[1], r[2]);
+      r2 = r2_exact(r[0], r[1], r[2]);
+      pdk = pk4.w;
+      const double2* rk = reinterpret_cast<const double2*>(mrec + (size_t)k * 12);
+      const double2 a0 = __ldg(rk), a1 = __ldg(rk + 1), a2 = __ldg(rk + 2), a3 = __ldg(rk + 3), a4 = __ldg(rk + 4),
+                    a5 = __ldg(rk + 5);
+      ptk = a0.x;
+      ck = a0.y;
+      dk[0] = a1.x; dk[1] = a1.y; dk[2] = a2.x;
+      Qk[0] = a2.y; Qk[1] = a3.x; Qk[2] = a3.y; Qk[3] = a4.x; Qk[4] = a4.y; Qk[5] = a5.x;
+      const double2* mk = reinterpret_cast<const double2*>(mu + (size_t)k * 6);
+      const double2 b0 = __ldg(mk), b1 = __ldg(mk + 1), b2 = __ldg(mk + 2);
+      vd[0] = b0.x; vd[1] = b0.y; vd[2] = b1.x;
+      vq[0] = b1.y; vq[1] = b2.x; vq[2] = b2.y;
     }
     T ds = 1, ps = 1, us = 1;
-    for (int q = s0; q < s1; ++q)
-      if (__ldg(sp_ks + q) == k) {
-        ds = (T)sp_s[3 * q];
-        ps = (T)sp_s[3 * q + 1];
-        us = (T)sp_s[3 * q + 2];
-        break;
-      }
-    // the mixed form: one rsqrt, then products in place of the divisions
-    T r, rinv, r2inv;
-    if constexpr (MIXED) {
+    int sq = -1;
+#pragma unroll
+    for (int q = 0; q < kSpCache; ++q)
+      if (spk[q] == k) sq = s0 + q;
+    if (sq < 0 && s1 - s0 > kSpCache)
+      for (int q = s0 + kSpCache; q < s1; ++q)
+        if (__ldg(sp_ks + q) == k) {
+          sq = q;
+          break;
+        }
+    if (sq >= 0) {
+      ds = (T)sp_s[3 * sq];
+      ps = (T)sp_s[3 * sq + 1];
+      us = (T)sp_s[3 * sq + 2];
+    }
+    // dampewald(9) (damping.f:17-55) and the bare terms: one reciprocal root,
+    // then products
+    T rinv;
+    if constexpr (MIXED)
       rinv = rsqrtf(r2);
-      r = r2 * rinv;
-      r2inv = rinv * rinv;
-    } else {
-      r = sqrt(r2);
-      rinv = T(1) / r;
-      r2inv = T(1) / r2;
-    }
-    const T dir = dix * xr + diy * yr + diz * zr;
-    const T qix = qixx * xr + qixy * yr + qixz * zr, qiy = qixy * xr + qiyy * yr + qiyz * zr,
-            qiz = qixz * xr + qiyz * yr + qizz * zr;
-    const T qir = qix * xr + qiy * yr + qiz * zr;
-    const T dkr = dkx * xr + dky * yr + dkz * zr;
-    const T qkx = qkxx * xr + qkxy * yr + qkxz * zr, qky = qkxy * xr + qkyy * yr + qkyz * zr,
-            qkz = qkxz * xr + qkyz * yr + qkzz * zr;
-    const T qkr = qkx * xr + qky * yr + qkz * zr;
-    const T uir = uix * xr + uiy * yr + uiz * zr, uirp = uixp * xr + uiyp * yr + uizp * zr;
-    const T ukr = ukx * xr + uky * yr + ukz * zr, ukrp = ukxp * xr + ukyp * yr + ukzp * zr;
-    T rr1, rr3, rr5, rr7, rr9, b0, b1, b2, b3, b4;
-    // dampewald(9, r, r2, f) (damping.f:17-55)
-    const T ra = (T)ew.a * r;
+    else
+      rinv = T(1) / sqrt(r2);
+    const T rr = r2 * rinv, r2inv = rinv * rinv;
+    PairRadial<T> p;
+    const T ra = (T)ew.a * rr;
     const T ex = exp(-ra * ra);
-    if constexpr (MIXED) {
-      rr1 = f * rinv;
-      rr3 = rr1 * r2inv;
-      rr5 = T(3) * rr3 * r2inv;
-      rr7 = T(5) * rr5 * r2inv;
-      rr9 = T(7) * rr7 * r2inv;
-      b0 = erfc(ra) * rinv;
-      b1 = (b0 + (T)ew.f1 * ex) * r2inv;
-      b2 = (T(3) * b1 + (T)ew.f2 * ex) * r2inv;
-      b3 = (T(5) * b2 + (T)ew.f3 * ex) * r2inv;
-      b4 = (T(7) * b3 + (T)ew.f4 * ex) * r2inv;
-    } else {
-      rr1 = f / r;
-      rr3 = rr1 / r2;
-      rr5 = T(3) * rr3 / r2;
-      rr7 = T(5) * rr5 / r2;
-      rr9 = T(7) * rr7 / r2;
-      b0 = erfc(ra) / r;
-      b1 = (b0 + (T)ew.f1 * ex) / r2;
-      b2 = (T(3) * b1 + (T)ew.f2 * ex) / r2;
-      b3 = (T(5) * b2 + (T)ew.f3 * ex) / r2;
-      b4 = (T(7) * b3 + (T)ew.f4 * ex) / r2;
-    }
-    const T e3 = f * b1, e5 = f * b2, e7 = f * b3, e9 = f * b4;
+    const T b0 = erfc(ra) * rinv;
+    const T b1 = (b0 + (T)ew.f1 * ex) * r2inv;
+    const T b2 = (T(3) * b1 + (T)ew.f2 * ex) * r2inv;
+    const T b3 = (T(5) * b2 + (T)ew.f3 * ex) * r2inv;
+    const T b4 = (T(7) * b3 + (T)ew.f4 * ex) * r2inv;
+    p.e3 = f * b1;
+    p.e5 = f * b2;
+    p.e7 = f * b3;
+    p.e9 = f * b4;
+    p.rr3 = f * rinv * r2inv;
+    p.rr5 = T(3) * p.rr3 * r2inv;
+    p.rr7 = T(5) * p.rr5 * r2inv;
+    p.rr9 = T(7) * p.rr7 * r2inv;
     // Thole factors and their r-derivatives (epolar1.f:1620-1660)
-    T sc3 = 1, sc5 = 1, sc7 = 1, rc3[3] = {0, 0, 0}, rc5[3] = {0, 0, 0}, rc7[3] = {0, 0, 0};
-    T l3d = 1, l5d = 1, l7d = 1;  // damptholed order 7 for the energy-field (same values)
-    T damp = pdi * pdk;
+    p.l3 = p.l5 = p.l7 = T(1);
+    p.q3 = p.q5 = p.q7 = T(0);
     T pg = min(pti, ptk);
     if (pg == T(0)) pg = max(pti, ptk);
-    if (damp != T(0) && pg != T(0)) {
-      const T t = MIXED ? r * (T(1) / damp) : r / damp;
-      damp = pg * (t * t * t);
+    const T pd = MIXED ? (T)ipdi * pdk : (T)pi4.w * pdk;  // mixed: the product of the reciprocals
+    if (pd != T(0) && pg != T(0)) {
+      const T tt = MIXED ? rr * pd : rr / pd;
+      const T damp = pg * (tt * tt * tt);
       if (damp < T(50)) {
         const T ed = exp(-damp);
-        sc3 = T(1) - ed;
-        sc5 = T(1) - (T(1) + damp) * ed;
-        sc7 = T(1) - (T(1) + damp + T(0.6) * damp * damp) * ed;
-        const T temp3 = MIXED ? T(3) * damp * ed * r2inv : T(3) * damp * ed / r2, temp5 = damp,
-                temp7 = T(-0.2) + T(0.6) * damp;
-        rc3[0] = xr * temp3;
-        rc3[1] = yr * temp3;
-        rc3[2] = zr * temp3;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          rc5[j] = rc3[j] * temp5;
-          rc7[j] = rc5[j] * temp7;
-        }
-        l3d = sc3;
-        l5d = sc5;
-        l7d = sc7;
+        p.l3 = T(1) - ed;
+        p.l5 = T(1) - (T(1) + damp) * ed;
+        p.l7 = T(1) - (T(1) + damp + T(0.6) * damp * damp) * ed;
+        p.q3 = T(3) * damp * ed * r2inv;
+        p.q5 = p.q3 * damp;
+        p.q7 = p.q5 * (T(-0.2) + T(0.6) * damp);
       }
     }
-    (void)l3d;
-    (void)l5d;
-    (void)l7d;
-    const T psc3 = T(1) - sc3 * ps, psc5 = T(1) - sc5 * ps, psc7 = T(1) - sc7 * ps;
-    const T dsc3 = T(1) - sc3 * ds, dsc5 = T(1) - sc5 * ds, dsc7 = T(1) - sc7 * ds;
-    const T usc3 = T(1) - sc3 * us, usc5 = T(1) - sc5 * us;
-    const T psr3 = e3 - psc3 * rr3, psr5 = e5 - psc5 * rr5, psr7 = e7 - psc7 * rr7;
-    const T dsr3 = e3 - dsc3 * rr3, dsr5 = e5 - dsc5 * rr5, dsr7 = e7 - dsc7 * rr7;
-    const T usr5 = e5 - usc5 * rr5;
-    // induced field and gradient at i (ufld, dufld)
+    const T dir = di[0] * r[0] + di[1] * r[1] + di[2] * r[2], dkr = dk[0] * r[0] + dk[1] * r[1] + dk[2] * r[2];
+    const T qi[3] = {Qi[0] * r[0] + Qi[1] * r[1] + Qi[2] * r[2], Qi[1] * r[0] + Qi[3] * r[1] + Qi[4] * r[2],
+                     Qi[2] * r[0] + Qi[4] * r[1] + Qi[5] * r[2]};
+    const T qk[3] = {Qk[0] * r[0] + Qk[1] * r[1] + Qk[2] * r[2], Qk[1] * r[0] + Qk[3] * r[1] + Qk[4] * r[2],
+                     Qk[2] * r[0] + Qk[4] * r[1] + Qk[5] * r[2]};
+    const T qir = qi[0] * r[0] + qi[1] * r[1] + qi[2] * r[2], qkr = qk[0] * r[0] + qk[1] * r[1] + qk[2] * r[2];
+    const T uir = ud[0] * r[0] + ud[1] * r[1] + ud[2] * r[2], uirp = up[0] * r[0] + up[1] * r[1] + up[2] * r[2];
+    const T ukr = vd[0] * r[0] + vd[1] * r[1] + vd[2] * r[2], ukrp = vq[0] * r[0] + vq[1] * r[1] + vq[2] * r[2];
+    // mutual part (uscale): F3 (ud_i.up_k + ud_k.up_i) - F5 (products along r)
+    T frc[3];
     {
-      const T tix3 = psr3 * ukx + dsr3 * ukxp, tiy3 = psr3 * uky + dsr3 * ukyp, tiz3 = psr3 * ukz + dsr3 * ukzp;
-      const T tuir3 = -psr5 * ukr - dsr5 * ukrp;
-      uf[0] += tix3 + xr * tuir3;
-      uf[1] += tiy3 + yr * tuir3;
-      uf[2] += tiz3 + zr * tuir3;
-      const T tix5 = T(2) * (psr5 * ukx + dsr5 * ukxp), tiy5 = T(2) * (psr5 * uky + dsr5 * ukyp),
-              tiz5 = T(2) * (psr5 * ukz + dsr5 * ukzp);
-      const T tuir = -psr7 * ukr - dsr7 * ukrp;
-      duf[0] += xr * tix5 + xr * xr * tuir;
-      duf[1] += xr * tiy5 + yr * tix5 + T(2) * xr * yr * tuir;
-      duf[2] += yr * tiy5 + yr * yr * tuir;
-      duf[3] += xr * tiz5 + zr * tix5 + T(2) * xr * zr * tuir;
-      duf[4] += yr * tiz5 + zr * tiy5 + T(2) * yr * zr * tuir;
-      duf[5] += zr * tiz5 + zr * zr * tuir;
-    }
-    // permanent-field gradient parts (d with uinp, p with uind)
-    T frc[3] = {0, 0, 0};
+      const T n3 = T(1) - us * p.l3, n5 = T(1) - us * p.l5;
+      const T F5 = p.e5 - n5 * p.rr5;
+      const T D3 = p.e5 - n3 * p.rr5 - us * p.q3 * p.rr3, D5 = p.e7 - n5 * p.rr7 - us * p.q5 * p.rr5;
+      const T A3 = (ud[0] * vq[0] + ud[1] * vq[1] + ud[2] * vq[2]) + (vd[0] * up[0] + vd[1] * up[1] + vd[2] * up[2]);
+      const T rad = D3 * A3 - D5 * (uir * ukrp + ukr * uirp);
 #pragma unroll
-    for (int part = 0; part < 2; ++part) {
-      const T s3 = part ? psc3 : dsc3, s5 = part ? psc5 : dsc5, s7 = part ? psc7 : dsc7;
-      const T sr3 = part ? psr3 : dsr3, sr5 = part ? psr5 : dsr5, sr7 = part ? psr7 : dsr7;
-      const T sc = part ? ps : ds;
-      const T vkx = part ? ukx : ukxp, vky = part ? uky : ukyp, vkz = part ? ukz : ukzp;
-      const T vix = part ? uix : uixp, viy = part ? uiy : uiyp, viz = part ? uiz : uizp;
-      const T term1 = e5 - s3 * rr5, term2 = e7 - s5 * rr7, e9s = e9 - s7 * rr9;
-      const T x3[3] = {rc3[0] * sc, rc3[1] * sc, rc3[2] * sc};
-      const T x5[3] = {rc5[0] * sc, rc5[1] * sc, rc5[2] * sc};
-      const T x7[3] = {rc7[0] * sc, rc7[1] * sc, rc7[2] * sc};
-      T term3 = -sr3 + term1 * xr * xr - rr3 * xr * x3[0];
-      T term4 = rr3 * x3[0] - term1 * xr - sr5 * xr;
-      T term5 = term2 * xr * xr - sr5 - rr5 * xr * x5[0];
-      T term6 = e9s * xr * xr - e7 - rr7 * xr * x7[0];
-      T term7 = rr5 * x5[0] - T(2) * e7 * xr + (s5 + T(1.5) * s7) * rr7 * xr;
-      const T tixx = ci * term3 + dix * term4 + dir * term5 + T(2) * sr5 * qixx + (qiy * yr + qiz * zr) * s7 * rr7 +
-                     T(2) * qix * term7 + qir * term6;
-      const T tkxx = ck * term3 - dkx * term4 - dkr * term5 + T(2) * sr5 * qkxx + (qky * yr + qkz * zr) * s7 * rr7 +
-                     T(2) * qkx * term7 + qkr * term6;
-      term3 = -sr3 + term1 * yr * yr - rr3 * yr * x3[1];
-      term4 = rr3 * x3[1] - term1 * yr - sr5 * yr;
-      term5 = term2 * yr * yr - sr5 - rr5 * yr * x5[1];
-      term6 = e9s * yr * yr - e7 - rr7 * yr * x7[1];
-      term7 = rr5 * x5[1] - T(2) * e7 * yr + (s5 + T(1.5) * s7) * rr7 * yr;
-      const T tiyy = ci * term3 + diy * term4 + dir * term5 + T(2) * sr5 * qiyy + (qix * xr + qiz * zr) * s7 * rr7 +
-                     T(2) * qiy * term7 + qir * term6;
-      const T tkyy = ck * term3 - dky * term4 - dkr * term5 + T(2) * sr5 * qkyy + (qkx * xr + qkz * zr) * s7 * rr7 +
-                     T(2) * qky * term7 + qkr * term6;
-      term3 = -sr3 + term1 * zr * zr - rr3 * zr * x3[2];
-      term4 = rr3 * x3[2] - term1 * zr - sr5 * zr;
-      term5 = term2 * zr * zr - sr5 - rr5 * zr * x5[2];
-      term6 = e9s * zr * zr - e7 - rr7 * zr * x7[2];
-      term7 = rr5 * x5[2] - T(2) * e7 * zr + (s5 + T(1.5) * s7) * rr7 * zr;
-      const T tizz = ci * term3 + diz * term4 + dir * term5 + T(2) * sr5 * qizz + (qix * xr + qiy * yr) * s7 * rr7 +
-                     T(2) * qiz * term7 + qir * term6;
-      const T tkzz = ck * term3 - dkz * term4 - dkr * term5 + T(2) * sr5 * qkzz + (qkx * xr + qky * yr) * s7 * rr7 +
-                     T(2) * qkz * term7 + qkr * term6;
-      term3 = term1 * xr * yr - rr3 * yr * x3[0];
-      term4 = rr3 * x3[0] - term1 * xr;
-      term5 = term2 * xr * yr - rr5 * yr * x5[0];
-      term6 = e9s * xr * yr - rr7 * yr * x7[0];
-      term7 = rr5 * x5[0] - term2 * xr;
-      const T tixy = ci * term3 - sr5 * dix * yr + diy * term4 + dir * term5 + T(2) * sr5 * qixy -
-                     T(2) * sr7 * yr * qix + T(2) * qiy * term7 + qir * term6;
-      const T tkxy = ck * term3 + sr5 * dkx * yr - dky * term4 - dkr * term5 + T(2) * sr5 * qkxy -
-                     T(2) * sr7 * yr * qkx + T(2) * qky * term7 + qkr * term6;
-      term3 = term1 * xr * zr - rr3 * zr * x3[0];
-      term5 = term2 * xr * zr - rr5 * zr * x5[0];
-      term6 = e9s * xr * zr - rr7 * zr * x7[0];
-      const T tixz = ci * term3 - sr5 * dix * zr + diz * term4 + dir * term5 + T(2) * sr5 * qixz -
-                     T(2) * sr7 * zr * qix + T(2) * qiz * term7 + qir * term6;
-      const T tkxz = ck * term3 + sr5 * dkx * zr - dkz * term4 - dkr * term5 + T(2) * sr5 * qkxz -
-                     T(2) * sr7 * zr * qkx + T(2) * qkz * term7 + qkr * term6;
-      term3 = term1 * yr * zr - rr3 * zr * x3[1];
-      term4 = rr3 * x3[1] - term1 * yr;
-      term5 = term2 * yr * zr - rr5 * zr * x5[1];
-      term6 = e9s * yr * zr - rr7 * zr * x7[1];
-      term7 = rr5 * x5[1] - term2 * yr;
-      const T tiyz = ci * term3 - sr5 * diy * zr + diz * term4 + dir * term5 + T(2) * sr5 * qiyz -
-                     T(2) * sr7 * zr * qiy + T(2) * qiz * term7 + qir * term6;
-      const T tkyz = ck * term3 + sr5 * dky * zr - dkz * term4 - dkr * term5 + T(2) * sr5 * qkyz -
-                     T(2) * sr7 * zr * qky + T(2) * qkz * term7 + qkr * term6;
-      frc[0] += tixx * vkx + tixy * vky + tixz * vkz - tkxx * vix - tkxy * viy - tkxz * viz;
-      frc[1] += tixy * vkx + tiyy * vky + tiyz * vkz - tkxy * vix - tkyy * viy - tkyz * viz;
-      frc[2] += tixz * vkx + tiyz * vky + tizz * vkz - tkxz * vix - tkyz * viy - tkzz * viz;
+      for (int q = 0; q < 3; ++q)
+        frc[q] = -F5 * (ukrp * ud[q] + uir * vq[q] + uirp * vd[q] + ukr * up[q]) - rad * r[q];
     }
-    // mutual part (uscale)
+    // permanent moments with the induced dipoles: the p dipoles under dscale
+    // and the d dipoles under pscale, in one go when the two scales agree
+    // (every pair but the few special pairs where they differ)
     {
-      const T term1 = e5 - usc3 * rr5, term2 = e7 - usc5 * rr7, term3 = usr5 + term1;
-      T term4 = rr3 * us;
-      T term5 = -xr * term3 + rc3[0] * term4;
-      T term6 = -usr5 + xr * xr * term2 - rr5 * xr * rc5[0] * us;
-      const T tixx = uix * term5 + uir * term6, tkxx = ukx * term5 + ukr * term6;
-      term5 = -yr * term3 + rc3[1] * term4;
-      term6 = -usr5 + yr * yr * term2 - rr5 * yr * rc5[1] * us;
-      const T tiyy = uiy * term5 + uir * term6, tkyy = uky * term5 + ukr * term6;
-      term5 = -zr * term3 + rc3[2] * term4;
-      term6 = -usr5 + zr * zr * term2 - rr5 * zr * rc5[2] * us;
-      const T tizz = uiz * term5 + uir * term6, tkzz = ukz * term5 + ukr * term6;
-      term4 = -usr5 * yr;
-      term5 = -xr * term1 + rr3 * rc3[0] * us;
-      term6 = xr * yr * term2 - rr5 * yr * rc5[0] * us;
-      const T tixy = uix * term4 + uiy * term5 + uir * term6, tkxy = ukx * term4 + uky * term5 + ukr * term6;
-      term4 = -usr5 * zr;
-      term6 = xr * zr * term2 - rr5 * zr * rc5[0] * us;
-      const T tixz = uix * term4 + uiz * term5 + uir * term6, tkxz = ukx * term4 + ukz * term5 + ukr * term6;
-      term5 = -yr * term1 + rr3 * rc3[1] * us;
-      term6 = yr * zr * term2 - rr5 * zr * rc5[1] * us;
-      const T tiyz = uiy * term4 + uiz * term5 + uir * term6, tkyz = uky * term4 + ukz * term5 + ukr * term6;
-      frc[0] += tixx * ukxp + tixy * ukyp + tixz * ukzp + tkxx * uixp + tkxy * uiyp + tkxz * uizp;
-      frc[1] += tixy * ukxp + tiyy * ukyp + tiyz * ukzp + tkxy * uixp + tkyy * uiyp + tkyz * uizp;
-      frc[2] += tixz * ukxp + tiyz * ukyp + tizz * ukzp + tkxz * uixp + tkyz * uiyp + tkzz * uizp;
+      const bool both = ds == ps;
+      T u[3], v[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        u[q] = both ? ud[q] + up[q] : up[q];
+        v[q] = both ? vd[q] + vq[q] : vq[q];
+      }
+      perm_terms<T>(p, ds, r, u, v, both ? uir + uirp : uirp, both ? ukr + ukrp : ukrp, ci, di, Qi, ck, dk, Qk, qi, qk,
+                    dir, dkr, qir, qkr, frc, uf, duf);
+      if (!both)
+        perm_terms<T>(p, ps, r, ud, vd, uir, ukr, ci, di, Qi, ck, dk, Qk, qi, qk, dir, dkr, qir, qkr, frc, uf, duf);
     }
     gx -= (double)frc[0];
     gy -= (double)frc[1];
     gz -= (double)frc[2];
     if (VIR) {
       const T h = T(0.5);
-      vp[0] += h * (xr * frc[0]);
-      vp[1] += h * (T(0.5) * (yr * frc[0] + xr * frc[1]));
-      vp[2] += h * (T(0.5) * (zr * frc[0] + xr * frc[2]));
-      vp[3] += h * (yr * frc[1]);
-      vp[4] += h * (T(0.5) * (zr * frc[1] + yr * frc[2]));
-      vp[5] += h * (zr * frc[2]);
+      vp[0] += h * (r[0] * frc[0]);
+      vp[1] += h * (T(0.5) * (r[1] * frc[0] + r[0] * frc[1]));
+      vp[2] += h * (T(0.5) * (r[2] * frc[0] + r[0] * frc[2]));
+      vp[3] += h * (r[1] * frc[1]);
+      vp[4] += h * (T(0.5) * (r[2] * frc[1] + r[1] * frc[2]));
+      vp[5] += h * (r[2] * frc[2]);
     }
   }
-  if (LPA == 8) {
+  {
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) {
       gx += __shfl_xor_sync(0xffffffffu, gx, o);
@@ -621,21 +548,21 @@ __global__ void __launch_bounds__(kBlock, MIXED ? THP_FORCE_MINB : 1) k_force_re
     }
   }
   if (live && jl == 0) {
-  fix_add(dep + 3 * i + 0, gx);
-  fix_add(dep + 3 * i + 1, gy);
-  fix_add(dep + 3 * i + 2, gz);
+  dep.add(3 * i + 0, gx);
+  dep.add(3 * i + 1, gy);
+  dep.add(3 * i + 2, gz);
   // torques: real-space induced field (epolar1.f:2427-2470) + reciprocal + self
   const double* u6 = mu + (size_t)i * 6;
   const double sterm = (4.0 / 3.0) * kElectric * ew.a * ew.a * ew.a / kSqrtPi;
   const double hx = 0.5 * (u6[0] + u6[3]), hy = 0.5 * (u6[1] + u6[4]), hz = 0.5 * (u6[2] + u6[5]);
   const double rdx = (double)ri[2], rdy = (double)ri[3], rdz = (double)ri[4];
   double tep[3];
-  tep[0] = (double)(diz * uf[1] - diy * uf[2] + qixz * duf[1] - qixy * duf[3] + T(2) * qiyz * (duf[2] - duf[5]) +
-                    (qizz - qiyy) * duf[4]);
-  tep[1] = (double)(dix * uf[2] - diz * uf[0] - qiyz * duf[1] + qixy * duf[4] + T(2) * qixz * (duf[5] - duf[0]) +
-                    (qixx - qizz) * duf[3]);
-  tep[2] = (double)(diy * uf[0] - dix * uf[1] + qiyz * duf[3] - qixz * duf[4] + T(2) * qixy * (duf[0] - duf[2]) +
-                    (qiyy - qixx) * duf[1]);
+  tep[0] = (double)(di[2] * uf[1] - di[1] * uf[2] + Qi[2] * duf[1] - Qi[1] * duf[3] +
+                    T(2) * Qi[4] * (duf[2] - duf[5]) + (Qi[5] - Qi[3]) * duf[4]);
+  tep[1] = (double)(di[0] * uf[2] - di[2] * uf[0] - Qi[4] * duf[1] + Qi[1] * duf[4] +
+                    T(2) * Qi[2] * (duf[5] - duf[0]) + (Qi[0] - Qi[5]) * duf[3]);
+  tep[2] = (double)(di[1] * uf[0] - di[0] * uf[1] + Qi[4] * duf[3] - Qi[2] * duf[4] +
+                    T(2) * Qi[1] * (duf[0] - duf[2]) + (Qi[3] - Qi[0]) * duf[1]);
   const int iz = frs[3 * i], ix = frs[3 * i + 1], axt = frs[3 * i + 2];
   if (VIR) {
 #pragma unroll
@@ -659,9 +586,9 @@ __global__ void __launch_bounds__(kBlock, MIXED ? THP_FORCE_MINB : 1) k_force_re
       }
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
-        fix_add(dep + 3 * iz + j, du[j] + dux[j]);
-        fix_add(dep + 3 * ix + j, dv[j] + dvx[j]);
-        fix_add(dep + 3 * i + j, -(du[j] + dux[j]) - (dv[j] + dvx[j]));
+        dep.add(3 * iz + j, du[j] + dux[j]);
+        dep.add(3 * ix + j, dv[j] + dvx[j]);
+        dep.add(3 * i + j, -(du[j] + dux[j]) - (dv[j] + dvx[j]));
       }
     }
   } else {
@@ -713,7 +640,7 @@ static int alloc_once(Ctx& c, P** p, size_t count, const char* what) {
 
 // fphirec [n][20] (unscaled) of the convolved permanent-multipole grid
 int launch_fphi_mpole20(Ctx& c) {
-  int st = alloc_once(c, &c.d_fphirec, 20 * (size_t)c.n, "alloc fphirec");
+  int st = alloc_once(c, &c.d_fphirec, 20 * c.cap_n, "alloc fphirec");
   if (st) return st;
   const int nb = (c.n + kBlock - 1) / kBlock;
   PmeGeom g = pme_geom(c);
@@ -727,17 +654,26 @@ int launch_fphi_mpole20(Ctx& c) {
 
 // sorted frame atoms of every site into d_frs
 int launch_frames_sorted(Ctx& c) {
-  int st = alloc_once(c, &c.d_frs, 3 * (size_t)c.n, "alloc frames");
+  int st = alloc_once(c, &c.d_frs, 3 * c.cap_n, "alloc frames");
   if (st) return st;
   const int nb = (c.n + kBlock - 1) / kBlock;
   k_frames_sorted<<<nb, kBlock, 0, c.stream>>>(c.n, c.d_perm, c.d_iperm, c.d_frames, c.d_frs);
   return cuda_status(cudaGetLastError(), &c, "frames");
 }
 
+// the fixed-point gradient sums (d_depfix) to zero, allocated on first use
+int zero_gradient(Ctx& c) {
+  const size_t words = c.mixed ? 3 : 6;
+  int st = alloc_once(c, &c.d_depfix, words * c.cap_n, "alloc gradient");
+  if (st) return st;
+  return cuda_status(cudaMemsetAsync(c.d_depfix, 0, sizeof(unsigned long long) * words * c.n, c.stream), &c,
+                     "zero gradient");
+}
+
 // fixed-point gradient (sorted) -> dE/dx [n][3] in original order
-int launch_gradient_out(Ctx& c, const unsigned long long* dep, double* d_out) {
+int launch_gradient_out(Ctx& c, double* d_out) {
   const int nb = (c.n + kBlock - 1) / kBlock;
-  k_dep_out<<<nb, kBlock, 0, c.stream>>>(c.n, c.d_perm, dep, d_out);
+  k_dep_out<<<nb, kBlock, 0, c.stream>>>(c.n, c.d_perm, fix_acc(c.d_depfix, c.n, c.mixed), d_out);
   return cuda_status(cudaGetLastError(), &c, "gradient out");
 }
 
@@ -778,20 +714,16 @@ int launch_forces(Ctx& c, double* d_out) {
   int st;
   const int nb = (c.n + kBlock - 1) / kBlock;
   if (!c.have_axes) return THP_E_STATE;
-  const size_t n = c.n;
-  if ((st = alloc_once(c, &c.d_fphirec, 20 * n, "alloc fphirec"))) return st;
-  if ((st = alloc_once(c, &c.d_depfix, 3 * n, "alloc gradient"))) return st;
-  if ((st = alloc_once(c, &c.d_trq, 3 * n, "alloc torque"))) return st;
-  if ((st = alloc_once(c, &c.d_frs, 3 * n, "alloc frames"))) return st;
+  if ((st = alloc_once(c, &c.d_fphirec, 20 * c.cap_n, "alloc fphirec"))) return st;
+  if ((st = zero_gradient(c))) return st;
+  if ((st = alloc_once(c, &c.d_trq, 3 * c.cap_n, "alloc torque"))) return st;
+  if ((st = alloc_once(c, &c.d_frs, 3 * c.cap_n, "alloc frames"))) return st;
   const bool vir = c.want_virial;
   const int nk = 2 * kspace_virial_blocks();
   double *kpart = nullptr, *rpart = nullptr, *epart = nullptr;
-  // the real-space pass: eight lanes per site (blocks of 16 sites)
-  const int nbr = THP_FORCE_LPA == 8 ? (c.n + 15) / 16 : nb;
+  const int nbr = (c.n + 15) / 16;  // the real-space pass: eight lanes per site, blocks of 16 sites
   if (vir && (st = virial_scratch(c, nb, nbr, &kpart, &rpart, &epart))) return st;
-  unsigned long long* dep = c.d_depfix;
-  if ((st = cuda_status(cudaMemsetAsync(dep, 0, sizeof(unsigned long long) * 3 * n, c.stream), &c, "zero gradient")))
-    return st;
+  const FixAcc dep = fix_acc(c.d_depfix, c.n, c.mixed);
   k_frames_sorted<<<nb, kBlock, 0, c.stream>>>(c.n, c.d_perm, c.d_iperm, c.d_frames, c.d_frs);
   PmeGeom g = pme_geom(c);
   // permanent-multipole potential, 20 derivatives per site (and the
@@ -800,7 +732,6 @@ int launch_forces(Ctx& c, double* d_out) {
   if ((st = launch_fphi_mpole20(c))) return st;
   // dipole grid of uind (Re) / uinp (Im), convolved
   if ((st = launch_pme_dipole(c, c.d_mu, nullptr, 0))) return st;
-#define THP_RECIP_ARGS c.n, g, c.d_pos, c.d_grid, c.d_fphirec, c.d_mu, c.d_rpole, c.d_trq, dep, rpart
   if (c.mixed && vir)
     k_force_recip<float, true><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_grid,
                                                             c.d_fphirec, c.d_mu, c.d_rpole, c.d_trq, dep, rpart);
@@ -813,7 +744,6 @@ int launch_forces(Ctx& c, double* d_out) {
   else
     k_force_recip<double, false><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_grid,
                                                               c.d_fphirec, c.d_mu, c.d_rpole, c.d_trq, dep, rpart);
-#undef THP_RECIP_ARGS
   if ((st = cuda_status(cudaGetLastError(), &c, "force recip"))) return st;
   // (rpole + uinp) x (rpole + uind) k-space virial: the grid is free again
   if (vir && (st = launch_pair_grid_virial(c, kpart + (size_t)kspace_virial_blocks() * 6))) return st;
@@ -829,36 +759,33 @@ int launch_forces(Ctx& c, double* d_out) {
   ew.f3 = afac;
   afac *= aesq2;
   ew.f4 = afac;
-  const double off2 = c.cfg.ewaldcut * c.cfg.ewaldcut;
   if (c.mixed) {
-    if ((st = alloc_once(c, &c.d_muf, 8 * n, "alloc dipoles f32"))) return st;
+    if ((st = alloc_once(c, &c.d_muf, 8 * c.cap_n, "alloc dipoles f32"))) return st;
     k_mu_f32<<<nb, kBlock, 0, c.stream>>>(c.n, c.d_mu, c.d_muf);
     if ((st = cuda_status(cudaGetLastError(), &c, "dipoles f32"))) return st;
   }
-#define THP_FORCE_ARGS                                                                                      \
-  c.n, c.npad, c.box, off2, ew, c.d_pos, MREC, c.d_mu, c.d_erec, c.d_muf, c.d_perm, c.d_sp_off, c.d_sp_ks, \
-      c.d_sp_s, c.d_nnb, c.d_nb, c.maxnb, c.d_frs, c.d_trq, dep, epart
-  constexpr int LPA = THP_FORCE_LPA;
+#define THP_FORCE_ARGS                                                                                            \
+  c.n, c.box, ew, c.d_pos, MREC, c.d_mu, c.d_erec, c.d_muf, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_s, c.d_npr, c.d_pk, \
+      c.maxpr / 8, c.d_frs, c.d_trq, dep, epart
   if (c.mixed) {
 #define MREC c.d_mrecf
     if (vir)
-      k_force_real<true, true, LPA><<<nbr, kBlock, 0, c.stream>>>(THP_FORCE_ARGS);
+      k_force_real<true, true><<<nbr, kBlock, 0, c.stream>>>(THP_FORCE_ARGS);
     else
-      k_force_real<true, false, LPA><<<nbr, kBlock, 0, c.stream>>>(THP_FORCE_ARGS);
+      k_force_real<true, false><<<nbr, kBlock, 0, c.stream>>>(THP_FORCE_ARGS);
 #undef MREC
   } else {
 #define MREC c.d_mrec
     if (vir)
-      k_force_real<false, true, LPA><<<nbr, kBlock, 0, c.stream>>>(THP_FORCE_ARGS);
+      k_force_real<false, true><<<nbr, kBlock, 0, c.stream>>>(THP_FORCE_ARGS);
     else
-      k_force_real<false, false, LPA><<<nbr, kBlock, 0, c.stream>>>(THP_FORCE_ARGS);
+      k_force_real<false, false><<<nbr, kBlock, 0, c.stream>>>(THP_FORCE_ARGS);
 #undef MREC
   }
 #undef THP_FORCE_ARGS
   if ((st = cuda_status(cudaGetLastError(), &c, "force real"))) return st;
   if (vir && (st = virial_total(c, nk, nb, nbr, kpart, rpart, epart, c.h_vir))) return st;
-  k_dep_out<<<nb, kBlock, 0, c.stream>>>(c.n, c.d_perm, dep, d_out);
-  return cuda_status(cudaGetLastError(), &c, "force out");
+  return launch_gradient_out(c, d_out);
 }
 
 }  // namespace thp

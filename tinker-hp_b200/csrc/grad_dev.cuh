@@ -7,11 +7,27 @@
 namespace thp {
 namespace {
 
-constexpr double kFix = 17179869184.0;  // 2^34
+constexpr double kFix = 17179869184.0;     // 2^34
+constexpr double kFixLow = 4294967296.0;   // 2^32
 
-__device__ __forceinline__ void fix_add(unsigned long long* a, double v) {
-  atomicAdd(a, (unsigned long long)(long long)llrint(v * kFix));
-}
+// Order-independent gradient sums: 64-bit fixed point in units of 2^-34
+// kcal/mol/A, and in the FP64 form (lo not null) the remainder of every addend
+// in units of 2^-66 in a second word.  Without it an addend whose 1e-15 noise
+// (the order of the PME spread's atomics) straddles a rounding boundary moves
+// the sum by a whole 2^-34.
+struct FixAcc {
+  unsigned long long* hi;
+  unsigned long long* lo;
+  __device__ __forceinline__ void add(int q, double v) const {
+    const double x = v * kFix;
+    const long long h = llrint(x);
+    atomicAdd(hi + q, (unsigned long long)h);
+    if (lo) atomicAdd(lo + q, (unsigned long long)llrint((x - (double)h) * kFixLow));
+  }
+};
+
+// the accumulators of n sites: dep holds 3 n words, 6 n in the FP64 form
+inline FixAcc fix_acc(unsigned long long* dep, int n, bool mixed) { return FixAcc{dep, mixed ? nullptr : dep + 3 * (size_t)n}; }
 
 // torque.f:6-390, Z-then-X (axt 1) and Bisector (axt 2); site ib, z atom ia,
 // x atom ic: the derivatives du (z atom) and dv (x atom) of the energy of
@@ -59,14 +75,14 @@ __device__ __forceinline__ void torque_frame(const double4* __restrict__ pos, in
 
 // adds d(energy)/d(coordinates) of the torque trq on site ib
 __device__ void torque_dist(const double4* __restrict__ pos, int ib, int ia, int ic, int axt, const double trq[3],
-                            unsigned long long* __restrict__ dep) {
+                            const FixAcc& dep) {
   double du[3], dv[3];
   torque_frame(pos, ib, ia, ic, axt, trq, du, dv);
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
-    fix_add(dep + 3 * ia + j, du[j]);
-    fix_add(dep + 3 * ic + j, dv[j]);
-    fix_add(dep + 3 * ib + j, -du[j] - dv[j]);
+    dep.add(3 * ia + j, du[j]);
+    dep.add(3 * ic + j, dv[j]);
+    dep.add(3 * ib + j, -du[j] - dv[j]);
   }
 }
 
@@ -96,13 +112,17 @@ __global__ void k_frames_sorted(int n, const int* __restrict__ perm, const int* 
   frs[3 * s + 2] = frames[3 * o + 2];
 }
 
-__global__ void k_dep_out(int n, const int* __restrict__ perm, const unsigned long long* __restrict__ dep,
-                          double* __restrict__ out) {
+__global__ void k_dep_out(int n, const int* __restrict__ perm, FixAcc dep, double* __restrict__ out) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const int o = perm[s];
 #pragma unroll
-  for (int j = 0; j < 3; ++j) out[3 * (size_t)o + j] = (double)(long long)dep[3 * (size_t)s + j] / kFix;
+  for (int j = 0; j < 3; ++j) {
+    const size_t q = 3 * (size_t)s + j;
+    double v = (double)(long long)dep.hi[q];
+    if (dep.lo) v += (double)(long long)dep.lo[q] / kFixLow;
+    out[3 * (size_t)o + j] = v / kFix;
+  }
 }
 
 // per-block energy partial (warp shuffles, then the warps in order)

@@ -6,7 +6,7 @@
 namespace thp {
 
 // nblist.cu
-int launch_sort_atoms(Ctx& c);          // cell sort, permutation, sorted copies
+int launch_sort_atoms(Ctx& c, bool carry = true);  // cell sort and permutation; the last dipoles and E0 follow
 int launch_gather_sorted(Ctx& c);       // positions/params/rpole into sorted order
 int launch_build_list(Ctx& c);
 int launch_build_list_on(Ctx& c, cudaStream_t s);          // full list within ewaldcut + lbuffer
@@ -49,7 +49,8 @@ int virial_total(Ctx& c, int nk, int nr, int ne, const double* kpart, const doub
                  double* h_out);
 int launch_fphi_mpole20(Ctx& c);          // fphirec [n][20] of the convolved multipole grid
 int launch_frames_sorted(Ctx& c);         // frame atoms in sorted numbering (d_frs)
-int launch_gradient_out(Ctx& c, const unsigned long long* dep, double* d_out);  // fixed point -> original order
+int zero_gradient(Ctx& c);                        // the fixed-point gradient sums
+int launch_gradient_out(Ctx& c, double* d_out);  // fixed point -> original order
 // permanent-multipole energy into d_em and dE/dx [n][3] (original order) into
 // d_out, for the current sorted positions, multipoles and list
 int launch_empole(Ctx& c, double* d_out);
@@ -57,8 +58,9 @@ int launch_empole(Ctx& c, double* d_out);
 // order) into d_out, for the current sorted positions and cell sort
 int launch_ehal(Ctx& c, double* d_out);
 int launch_vdw_list(Ctx& c);  // reduced sites, and the vdW list when it is stale
-// reference-format half list (k > i, original numbering) of a slot-major list
-int launch_export_pairs(Ctx& c, const int* nnb, const int* nb, int maxnb, int maxelst, int* d_nelst, int* d_elst);
+// reference-format half list (k > i, original numbering) of a full list in the pair stream's layout
+int launch_export_pairs(Ctx& c, const int* nnb, const int* nb, int maxnb, int cap8, int maxelst, int* d_nelst,
+                        int* d_elst);
 
 // sites.cu
 int launch_grid_uind_sites(Ctx& c, int nsites, const int* d_site, const double* d_fuind, const double* d_fuinp,

@@ -12,7 +12,7 @@
 //     factors;
 //   * the Ewald self energy (empole1.f:134-160);
 //   * torque (torque.f:6-390) of each site's summed torque.
-// One thread owns site i over the full neighbor list: each pair is evaluated
+// Eight lanes own site i over the full neighbor list: each pair is evaluated
 // from both ends, and each end keeps its own force, torque and half of the
 // pair energy (the reference's Newton's-third-law half-list loop gives the
 // same sums).  Gradients are accumulated in 64-bit fixed point, the energy
@@ -167,26 +167,37 @@ __device__ __forceinline__ void mpole_pair(U xr, U yr, U zr, U r2, U scalek, con
   e_acc += 0.5 * (double)e;
 }
 
+// special partners of a site held in registers (a longer list is searched
+// past those)
+constexpr int kSpCache = 4;
+
 // Pairs outside the 1-2..1-5 lists, in the form's precision over the list:
 // force and torque of site i, half of each pair energy (partials per block).
 // The FP64 form reads the sorted positions and the FP64 multipole records
 // and tests the cutoff in FP64; the mixed form reads one 64-B record per
 // partner (wrapped position and multipoles, FP32) and images and tests in
 // FP32, as its direct-field pass does.
+// A warp takes four consecutive (cell-sorted) sites, eight lanes each: lane j
+// takes list entries j, j+8, ..., and the lanes' sums are combined in a fixed
+// shuffle tree.  With one thread per site a 4,000-atom system had 33 blocks,
+// each a chain of 177 dependent gathers.
 // VIR: each block also writes the sum of its sites' pair virial halves and
 // the frame-atom virial of their pair torques (6 values) to vpart.
 template <bool MIXED, bool VIR>
 __global__ void __launch_bounds__(kBlock, MIXED ? THP_EMPOLE_MINB : 4) k_empole_pairs(
-    int n, int npad, Box box, double off2, EwM ew, const double4* __restrict__ pos, const double* __restrict__ mrec,
+    int n, int cap8, Box box, double off2, EwM ew, const double4* __restrict__ pos, const double* __restrict__ mrec,
     const float* __restrict__ erec, const int* __restrict__ perm, const int* __restrict__ sp_off,
     const int* __restrict__ sp_ks, const int* __restrict__ sp_c, const int* __restrict__ nnb,
-    const int* __restrict__ nb, int maxnb, const int* __restrict__ frs, unsigned long long* __restrict__ dem,
+    const int* __restrict__ nb, int maxnb, const int* __restrict__ frs, FixAcc dem,
     double* __restrict__ epart, double* __restrict__ vpart) {
   using T = typename std::conditional<MIXED, float, double>::type;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, jl = threadIdx.x & 7;
+  const bool live = i0 < n;
+  const int i = live ? i0 : n - 1;  // a valid site for the loads of idle lanes
   double eacc = 0.0;
   double v6[6] = {0, 0, 0, 0, 0, 0};
-  if (i < n) {
+  double g3[3] = {0.0, 0.0, 0.0}, t3[3] = {0.0, 0.0, 0.0};
+  {
     T mi[10];
     double4 pi4 = make_double4(0.0, 0.0, 0.0, 0.0);
     float xi = 0.f, yi = 0.f, zi = 0.f;
@@ -209,13 +220,18 @@ __global__ void __launch_bounds__(kBlock, MIXED ? THP_EMPOLE_MINB : 4) k_empole_
     const float off2f = (float)off2;
     const int io = perm[i];
     const int s0 = sp_off[io], s1 = sp_off[io + 1];
-    double g3[3] = {0.0, 0.0, 0.0}, t3[3] = {0.0, 0.0, 0.0};
-    const int nn = min(nnb[i], maxnb);
-    int knext = nn > 0 ? __ldg(nb + i) : 0;  // list entries fetched one pair ahead
+    // the scaled partners (class 0..3; the per-site kernel takes those pairs)
+    int spk[kSpCache];
+#pragma unroll
+    for (int q = 0; q < kSpCache; ++q)
+      spk[q] = s0 + q < s1 && __ldg(sp_c + s0 + q) < 4 ? __ldg(sp_ks + s0 + q) : -1;
+    const int nn = live ? min(nnb[i], maxnb) : 0;
+    const int* __restrict__ row = nb + pair_slot(cap8, i, jl);  // entry s: 4 (s - j) on
+    int knext = jl < nn ? __ldg(row) : i;  // list entries fetched one step ahead
 #pragma unroll 1
-    for (int s = 0; s < nn; ++s) {
+    for (int s = jl; s < nn; s += 8) {
       const int k = knext;
-      if (s + 1 < nn) knext = __ldg(nb + (size_t)(s + 1) * npad + i);
+      if (s + 8 < nn) knext = __ldg(row + 4 * (size_t)(s + 8 - jl));
       T xr, yr, zr, r2;
       T mk[10];
       if constexpr (MIXED) {
@@ -243,21 +259,36 @@ __global__ void __launch_bounds__(kBlock, MIXED ? THP_EMPOLE_MINB : 4) k_empole_
         yr = yrd;
         zr = zrd;
         r2 = r2d;
-#pragma unroll
-        for (int q = 0; q < 10; ++q) mk[q] = mrec[(size_t)k * 12 + 1 + q];
+        const double2* rk = reinterpret_cast<const double2*>(mrec + (size_t)k * 12);
+        const double2 a0 = __ldg(rk), a1 = __ldg(rk + 1), a2 = __ldg(rk + 2), a3 = __ldg(rk + 3), a4 = __ldg(rk + 4),
+                      a5 = __ldg(rk + 5);
+        mk[0] = a0.y; mk[1] = a1.x; mk[2] = a1.y; mk[3] = a2.x; mk[4] = a2.y;
+        mk[5] = a3.x; mk[6] = a3.y; mk[7] = a4.x; mk[8] = a4.y; mk[9] = a5.x;
       }
       bool scaled = false;
-      for (int q = s0; q < s1; ++q)
-        if (__ldg(sp_ks + q) == k) {
-          scaled = __ldg(sp_c + q) < 4;
-          break;
-        }
+#pragma unroll
+      for (int q = 0; q < kSpCache; ++q) scaled |= spk[q] == k;
+      if (!scaled && s1 - s0 > kSpCache)
+        for (int q = s0 + kSpCache; q < s1; ++q)
+          if (__ldg(sp_ks + q) == k) {
+            scaled = __ldg(sp_c + q) < 4;
+            break;
+          }
       if (scaled) continue;
       mpole_pair<T>(xr, yr, zr, r2, T(0), mi, mk, ew, eacc, g3, t3, VIR ? v6 : nullptr);
     }
-    fix_add(dem + 3 * i + 0, g3[0]);
-    fix_add(dem + 3 * i + 1, g3[1]);
-    fix_add(dem + 3 * i + 2, g3[2]);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      g3[q] += __shfl_xor_sync(0xffffffffu, g3[q], o);
+      t3[q] += __shfl_xor_sync(0xffffffffu, t3[q], o);
+    }
+  if (live && jl == 0) {
+    dem.add(3 * i + 0, g3[0]);
+    dem.add(3 * i + 1, g3[1]);
+    dem.add(3 * i + 2, g3[2]);
     const int iz = frs[3 * i], ix = frs[3 * i + 1], axt = frs[3 * i + 2];
     if (axt == 1 || axt == 2) {
       if (VIR) {
@@ -266,9 +297,9 @@ __global__ void __launch_bounds__(kBlock, MIXED ? THP_EMPOLE_MINB : 4) k_empole_
         frame_virial(pos, i, iz, ix, du, dv, v6);  // empole1.f:1466-1497
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-          fix_add(dem + 3 * iz + j, du[j]);
-          fix_add(dem + 3 * ix + j, dv[j]);
-          fix_add(dem + 3 * i + j, -du[j] - dv[j]);
+          dem.add(3 * iz + j, du[j]);
+          dem.add(3 * ix + j, dv[j]);
+          dem.add(3 * i + j, -du[j] - dv[j]);
         }
       } else {
         torque_dist(pos, i, iz, ix, axt, t3, dem);
@@ -296,7 +327,7 @@ __global__ void __launch_bounds__(kBlock) k_empole_site(
     int n, Box box, double off2, EwM ew, MScale ms, PmeGeom g, const double4* __restrict__ pos,
     const double* __restrict__ rp, const int* __restrict__ perm, const int* __restrict__ sp_off,
     const int* __restrict__ sp_ks, const int* __restrict__ sp_c, const double* __restrict__ fphirec,
-    const int* __restrict__ frs, unsigned long long* __restrict__ dem, double* __restrict__ epart,
+    const int* __restrict__ frs, FixAcc dem, double* __restrict__ epart,
     double* __restrict__ vpart) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double eacc = 0.0;
@@ -386,9 +417,9 @@ __global__ void __launch_bounds__(kBlock) k_empole_site(
     const double qii = 2.0 * (r[5] * r[5] + r[6] * r[6] + r[8] * r[8]) + r[4] * r[4] + r[7] * r[7] + r[9] * r[9];
     const double eself = fterm * (cm[0] * cm[0] + term * (dii / 3.0 + 2.0 * term * qii / 5.0));
     eacc += 0.5 * erec + eself;
-    fix_add(dem + 3 * i + 0, gx);
-    fix_add(dem + 3 * i + 1, gy);
-    fix_add(dem + 3 * i + 2, gz);
+    dem.add(3 * i + 0, gx);
+    dem.add(3 * i + 1, gy);
+    dem.add(3 * i + 2, gz);
     const int iz = frs[3 * i], ix = frs[3 * i + 1], axt = frs[3 * i + 2];
     if ((axt == 1 || axt == 2) && VIR) {
       // the scaled pairs' torque (real space) and the reciprocal torque apart
@@ -399,9 +430,9 @@ __global__ void __launch_bounds__(kBlock) k_empole_site(
       frame_virial(pos, i, iz, ix, dux, dvx, *reinterpret_cast<double(*)[6]>(&v12[6]));
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
-        fix_add(dem + 3 * iz + j, du[j] + dux[j]);
-        fix_add(dem + 3 * ix + j, dv[j] + dvx[j]);
-        fix_add(dem + 3 * i + j, -(du[j] + dux[j]) - (dv[j] + dvx[j]));
+        dem.add(3 * iz + j, du[j] + dux[j]);
+        dem.add(3 * ix + j, dv[j] + dvx[j]);
+        dem.add(3 * i + j, -(du[j] + dux[j]) - (dv[j] + dvx[j]));
       }
     } else if (axt == 1 || axt == 2) {
       const double tt[3] = {tx + trq[0], ty + trq[1], tz + trq[2]};
@@ -432,18 +463,16 @@ int alloc_once(Ctx& c, P** p, size_t count, const char* what) {
 int launch_empole(Ctx& c, double* d_out) {
   int st;
   if (!c.have_axes) return THP_E_STATE;
-  const size_t n = c.n;
   const int nb = (c.n + kBlock - 1) / kBlock;
-  if ((st = alloc_once(c, &c.d_depfix, 3 * n, "alloc gradient"))) return st;
-  if ((st = alloc_once(c, &c.d_empart, 2 * (size_t)nb + 1, "alloc mpole partials"))) return st;
-  c.d_em = c.d_empart + 2 * nb;
-  unsigned long long* dem = c.d_depfix;
-  if ((st = cuda_status(cudaMemsetAsync(dem, 0, sizeof(unsigned long long) * 3 * n, c.stream), &c, "zero dem")))
-    return st;
+  const int nbp = (c.n + 15) / 16;  // the pair pass: eight lanes per site, blocks of 16 sites
+  if ((st = zero_gradient(c))) return st;
+  if ((st = alloc_once(c, &c.d_empart, c.cap_n / 8 + 8, "alloc mpole partials"))) return st;
+  c.d_em = c.d_empart + nbp + nb;
+  const FixAcc dem = fix_acc(c.d_depfix, c.n, c.mixed);
   if ((st = launch_frames_sorted(c))) return st;
   const bool vir = c.want_virial;
   double *kpart = nullptr, *rpart = nullptr, *spart = nullptr;
-  if (vir && (st = virial_scratch(c, nb, nb, &kpart, &rpart, &spart))) return st;
+  if (vir && (st = virial_scratch(c, nbp, nb, &kpart, &rpart, &spart))) return st;
   // the convolved multipole grid (and emrecip1's scalar sum over the
   // reciprocal lattice, empole1.f:560-598)
   if ((st = vir ? launch_mpole_grid_virial(c, kpart, 1.0) : launch_mpole_grid(c))) return st;
@@ -462,32 +491,37 @@ int launch_empole(Ctx& c, double* d_out) {
   ms.v[4] = 1.0;
   const double off2 = c.cfg.ewaldcut * c.cfg.ewaldcut;
   const PmeGeom g = pme_geom(c);
+  // the partners: the pairs within ewaldcut that a field pass at these
+  // positions left in the pair stream, else the list (same layout)
+  const int* npart = c.have_coef ? c.d_npr : c.d_nnb;
+  const int* part = c.have_coef ? c.d_pk : c.d_nb;
+  const int maxpart = c.have_coef ? c.maxpr : c.maxnb;
 #define THP_EMPOLE_ARGS                                                                                          \
-  c.n, c.npad, c.box, off2, ew, c.d_pos, c.d_mrec, c.d_erec, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_c, c.d_nnb, c.d_nb, \
-      c.maxnb, c.d_frs, dem, c.d_empart, rpart
+  c.n, c.maxpr / 8, c.box, off2, ew, c.d_pos, c.d_mrec, c.d_erec, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_c, npart, part, \
+      maxpart, c.d_frs, dem, c.d_empart, rpart
   if (c.mixed && vir)
-    k_empole_pairs<true, true><<<nb, kBlock, 0, c.stream>>>(THP_EMPOLE_ARGS);
+    k_empole_pairs<true, true><<<nbp, kBlock, 0, c.stream>>>(THP_EMPOLE_ARGS);
   else if (c.mixed)
-    k_empole_pairs<true, false><<<nb, kBlock, 0, c.stream>>>(THP_EMPOLE_ARGS);
+    k_empole_pairs<true, false><<<nbp, kBlock, 0, c.stream>>>(THP_EMPOLE_ARGS);
   else if (vir)
-    k_empole_pairs<false, true><<<nb, kBlock, 0, c.stream>>>(THP_EMPOLE_ARGS);
+    k_empole_pairs<false, true><<<nbp, kBlock, 0, c.stream>>>(THP_EMPOLE_ARGS);
   else
-    k_empole_pairs<false, false><<<nb, kBlock, 0, c.stream>>>(THP_EMPOLE_ARGS);
+    k_empole_pairs<false, false><<<nbp, kBlock, 0, c.stream>>>(THP_EMPOLE_ARGS);
 #undef THP_EMPOLE_ARGS
   if ((st = cuda_status(cudaGetLastError(), &c, "empole pairs"))) return st;
 #define THP_SITE_ARGS                                                                                              \
   c.n, c.box, off2, ew, ms, g, c.d_pos, c.d_rpole, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_c, c.d_fphirec, c.d_frs, \
-      dem, c.d_empart + nb, spart
+      dem, c.d_empart + nbp, spart
   if (vir)
     k_empole_site<true><<<nb, kBlock, 0, c.stream>>>(THP_SITE_ARGS);
   else
     k_empole_site<false><<<nb, kBlock, 0, c.stream>>>(THP_SITE_ARGS);
 #undef THP_SITE_ARGS
   if ((st = cuda_status(cudaGetLastError(), &c, "empole"))) return st;
-  k_sum_partials<<<1, 256, 0, c.stream>>>(2 * nb, c.d_empart, c.d_em);
+  k_sum_partials<<<1, 256, 0, c.stream>>>(nbp + nb, c.d_empart, c.d_em);
   if ((st = cuda_status(cudaGetLastError(), &c, "empole energy"))) return st;
-  if (vir && (st = virial_total(c, kspace_virial_blocks(), nb, nb, kpart, rpart, spart, c.h_mvir))) return st;
-  return launch_gradient_out(c, dem, d_out);
+  if (vir && (st = virial_total(c, kspace_virial_blocks(), nbp, nb, kpart, rpart, spart, c.h_mvir))) return st;
+  return launch_gradient_out(c, d_out);
 }
 
 }  // namespace thp

@@ -5,11 +5,13 @@
 // evaluated as (xi-xk) imaged by image.f:122-138 and summed unfused, so the
 // set is bit-identical to the reference's.  The device layout differs: atoms
 // are counting-sorted into cells of edge >= (ewaldcut+lbuffer)/2 and the list
-// is a FULL list (both directions), slot-major nb[s*npad + i] so that a warp
-// of consecutive atoms reads one coalesced row per slot.
+// is a FULL list (both directions) in the pair stream's layout (pair_slot): a
+// warp working on four consecutive atoms reads 32 consecutive entries a step.
 #include <algorithm>
 
 #include "kernels.h"
+#include "pme_dev.cuh"
+#include "realspace_dev.cuh"
 
 namespace thp {
 
@@ -17,11 +19,7 @@ namespace {
 
 constexpr int kBlock = 256;
 
-__global__ void k_cell_count(int n, Box box, int ncx, int ncy, int ncz, const double* __restrict__ xyz,
-                             int* __restrict__ atom_cell, int* __restrict__ cell_count) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double x = xyz[i], y = xyz[n + i], z = xyz[2 * n + i];
+__device__ __forceinline__ int cell_of(const Box& box, int ncx, int ncy, int ncz, double x, double y, double z) {
   image3(box, x, y, z);  // build_cell_list images the absolute coordinates
   int nc[3] = {ncx, ncy, ncz};
   double v[3] = {x, y, z};
@@ -32,7 +30,14 @@ __global__ void k_cell_count(int n, Box box, int ncx, int ncy, int ncz, const do
     int q = (int)floor(f * nc[d]);
     c[d] = q < 0 ? 0 : (q >= nc[d] ? nc[d] - 1 : q);
   }
-  int cell = (c[2] * ncy + c[1]) * ncx + c[0];
+  return (c[2] * ncy + c[1]) * ncx + c[0];
+}
+
+__global__ void k_cell_count(int n, Box box, int ncx, int ncy, int ncz, const double* __restrict__ xyz,
+                             int* __restrict__ atom_cell, int* __restrict__ cell_count) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int cell = cell_of(box, ncx, ncy, ncz, xyz[i], xyz[n + i], xyz[2 * n + i]);
   atom_cell[i] = cell;
   atomicAdd(&cell_count[cell], 1);
 }
@@ -140,6 +145,80 @@ __global__ void k_cell_sort(int ncell, const int* __restrict__ cell_start, const
     iperm[perm[b + a]] = b + a;
     scell[b + a] = c;
   }
+}
+
+// The whole cell sort of a small system in one block: cells, counts, scan,
+// fill and the order inside each cell in shared memory, then the special
+// partners in the new numbering.  The seven launches of the general form take
+// about 3 us each whatever the size; one block keeps up with them to
+// kSortSmallAtoms atoms.
+constexpr int kSortSmallAtoms = 8192, kSortSmallCells = 4096;
+constexpr size_t kSortSmallSmem =
+    sizeof(int) * (kSortSmallAtoms + 2 * kSortSmallCells) + sizeof(unsigned short) * kSortSmallAtoms;
+
+__global__ void __launch_bounds__(1024) k_sort_small(int n, Box box, int ncx, int ncy, int ncz, int nsp,
+                                                      const double* __restrict__ xyz, int* __restrict__ cell_start,
+                                                      int* __restrict__ cell_count, int* __restrict__ perm,
+                                                      int* __restrict__ iperm, int* __restrict__ scell,
+                                                      const int* __restrict__ sp_k, int* __restrict__ sp_ks) {
+  extern __shared__ int sort_smem[];
+  int* sperm = sort_smem;
+  int* count = sperm + kSortSmallAtoms;
+  int* next = count + kSortSmallCells;
+  unsigned short* scid = reinterpret_cast<unsigned short*>(next + kSortSmallCells);
+  __shared__ int s_warp[32];
+  const int t = threadIdx.x, ncell = ncx * ncy * ncz;
+  for (int c = t; c < kSortSmallCells; c += 1024) count[c] = 0;
+  __syncthreads();
+  for (int i = t; i < n; i += 1024) {
+    const int c = cell_of(box, ncx, ncy, ncz, xyz[i], xyz[n + i], xyz[2 * n + i]);
+    scid[i] = (unsigned short)c;
+    atomicAdd(&count[c], 1);
+  }
+  __syncthreads();
+  int v[4], sum = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    v[q] = count[4 * t + q];
+    sum += v[q];
+  }
+  int total;
+  int run = block_excl_scan_1024(sum, s_warp, &total);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int c = 4 * t + q;
+    next[c] = run;
+    if (c < ncell) {
+      cell_start[c] = run;
+      cell_count[c] = v[q];
+    }
+    run += v[q];
+  }
+  __syncthreads();
+  for (int i = t; i < n; i += 1024) sperm[atomicAdd(&next[scid[i]], 1)] = i;
+  __syncthreads();
+  // ascending original index inside each cell
+  for (int c = t; c < ncell; c += 1024) {
+    const int m = count[c], b = next[c] - m;
+    for (int a = 1; a < m; ++a) {
+      const int w = sperm[b + a];
+      int q = a - 1;
+      while (q >= 0 && sperm[b + q] > w) {
+        sperm[b + q + 1] = sperm[b + q];
+        --q;
+      }
+      sperm[b + q + 1] = w;
+    }
+  }
+  __syncthreads();
+  for (int s = t; s < n; s += 1024) {
+    const int o = sperm[s];
+    perm[s] = o;
+    iperm[o] = s;
+    scell[s] = scid[o];
+  }
+  __syncthreads();
+  for (int q = t; q < nsp; q += 1024) sp_ks[q] = iperm[sp_k[q]];
 }
 
 __global__ void k_gather_sorted(int n, Box box, const int* __restrict__ perm, const double* __restrict__ xyz,
@@ -304,7 +383,7 @@ struct ListTest {
 };
 
 // The list row of atom i, its candidates read from global memory.
-__device__ __forceinline__ void list_row_global(int i, int npad, const ListTest& lt, int ncx, int ncy, int ncz,
+__device__ __forceinline__ void list_row_global(int i, int cap8, const ListTest& lt, int ncx, int ncy, int ncz,
                                                 const double4* __restrict__ pos, const float4* __restrict__ posf,
                                                 const int* __restrict__ scell, const int* __restrict__ cell_start,
                                                 const int* __restrict__ cell_count, int maxnb,
@@ -317,6 +396,7 @@ __device__ __forceinline__ void list_row_global(int i, int npad, const ListTest&
   int a0, a1, b0, b1;
   row_ranges(cx, ncx, a0, a1, b0, b1);
   const int my = min(ncy, 5), mz = min(ncz, 5);
+  int* __restrict__ row = nb + pair_slot(cap8, i, 0);  // entry s: row[s + 3 (s & ~7)]
   int cnt = 0;
   for (int qz = 0; qz < mz; ++qz) {
     const int z = axis_cells(cz, ncz, qz);
@@ -333,7 +413,7 @@ __device__ __forceinline__ void list_row_global(int i, int npad, const ListTest&
         for (int k = k0; k < k1; ++k) {
           if (k == i) continue;
           if (lt.take(pi, fi, k, pos, posf)) {
-            if (cnt < maxnb) nb[(size_t)cnt * npad + i] = k;
+            if (cnt < maxnb) row[cnt + 3 * (cnt & ~7)] = k;
             ++cnt;
           }
         }
@@ -351,7 +431,7 @@ __device__ __forceinline__ void list_row_global(int i, int npad, const ListTest&
 // fi - shift - fk with no per-candidate image.  The screen's error bound is
 // the same (two roundings per coordinate); the exact FP64 test still images
 // each undecided pair itself.
-__device__ __forceinline__ void list_row_shifted(int i, int npad, const ListTest& lt, int ncx, int ncy, int ncz,
+__device__ __forceinline__ void list_row_shifted(int i, int cap8, const ListTest& lt, int ncx, int ncy, int ncz,
                                                  const double4* __restrict__ pos, const float4* __restrict__ posf,
                                                  const int* __restrict__ scell, const int* __restrict__ cell_start,
                                                  const int* __restrict__ cell_count, int maxnb,
@@ -365,6 +445,7 @@ __device__ __forceinline__ void list_row_shifted(int i, int npad, const ListTest
   row_ranges(cx, ncx, a0, a1, b0, b1);
   // part b lies past the lower face (cx - 2 < 0) or the upper one
   const float fxb = cx < 2 ? fi.x + lt.bx : fi.x - lt.bx;
+  int* __restrict__ row = nb + pair_slot(cap8, i, 0);  // entry s: row[s + 3 (s & ~7)]
   int cnt = 0;
   for (int qz = 0; qz < 5; ++qz) {
     const int zr = cz + qz - 2;
@@ -396,7 +477,7 @@ __device__ __forceinline__ void list_row_shifted(int i, int npad, const ListTest
             const float r2f = dx * dx + dy * dy + dz * dz;
             if (r2f > lt.hi || k == i) continue;
             if (r2f >= lt.lo && !lt.exact(pi, k, pos)) continue;
-            if (cnt < maxnb) nb[(size_t)cnt * npad + i] = k;
+            if (cnt < maxnb) row[cnt + 3 * (cnt & ~7)] = k;
             ++cnt;
           }
         }
@@ -407,7 +488,7 @@ __device__ __forceinline__ void list_row_shifted(int i, int npad, const ListTest
   if (cnt > maxnb) atomicOr(flags, DEV_LIST_OVERFLOW);
 }
 
-__global__ void __launch_bounds__(128, THP_LIST_MINB) k_build_list_shifted(int n, int npad, ListTest lt, int ncx,
+__global__ void __launch_bounds__(128, THP_LIST_MINB) k_build_list_shifted(int n, int cap8, ListTest lt, int ncx,
                                                     int ncy, int ncz, const double4* __restrict__ pos,
                                                     const float4* __restrict__ posf, const int* __restrict__ scell,
                                                     const int* __restrict__ cell_start,
@@ -416,10 +497,10 @@ __global__ void __launch_bounds__(128, THP_LIST_MINB) k_build_list_shifted(int n
                                                     int* __restrict__ flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  list_row_shifted(i, npad, lt, ncx, ncy, ncz, pos, posf, scell, cell_start, cell_count, maxnb, nnb, nb, flags);
+  list_row_shifted(i, cap8, lt, ncx, ncy, ncz, pos, posf, scell, cell_start, cell_count, maxnb, nnb, nb, flags);
 }
 
-__global__ void __launch_bounds__(128, THP_LIST_MINB) k_build_list(int n, int npad, ListTest lt, int ncx,
+__global__ void __launch_bounds__(128, THP_LIST_MINB) k_build_list(int n, int cap8, ListTest lt, int ncx,
                                                     int ncy, int ncz, const double4* __restrict__ pos,
                                                     const float4* __restrict__ posf, const int* __restrict__ scell,
                                                     const int* __restrict__ cell_start,
@@ -428,7 +509,7 @@ __global__ void __launch_bounds__(128, THP_LIST_MINB) k_build_list(int n, int np
                                                     int* __restrict__ flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  list_row_global(i, npad, lt, ncx, ncy, ncz, pos, posf, scell, cell_start, cell_count, maxnb, nnb, nb, flags);
+  list_row_global(i, cap8, lt, ncx, ncy, ncz, pos, posf, scell, cell_start, cell_count, maxnb, nnb, nb, flags);
 }
 
 // The same list with one warp per atom: the lanes test 32 consecutive
@@ -439,7 +520,7 @@ __global__ void __launch_bounds__(128, THP_LIST_MINB) k_build_list(int n, int np
 // one chunk ahead of its tests, so a warp waits on far fewer dependent
 // loads.  Small systems, where the +-2 cell window spans most of the box and
 // few atoms leave most of the GPU idle, use it.
-__global__ void __launch_bounds__(128) k_build_list_warp(int n, int npad, ListTest lt, int ncx, int ncy, int ncz,
+__global__ void __launch_bounds__(128) k_build_list_warp(int n, int cap8, ListTest lt, int ncx, int ncy, int ncz,
                                                         const double4* __restrict__ pos,
                                                         const float4* __restrict__ posf,
                                                         const int* __restrict__ scell,
@@ -495,6 +576,7 @@ __global__ void __launch_bounds__(128) k_build_list_warp(int n, int npad, ListTe
     return (lt.prefilter && k < k1) ? __ldg(posf + k) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
   float4 fcur = q < nrow ? load(kb, ke) : make_float4(0.f, 0.f, 0.f, 0.f);
+  int* __restrict__ row = nb + pair_slot(cap8, i, 0);  // entry s: row[s + 3 (s & ~7)]
   int cnt = 0;
   while (q < nrow) {
     const int ck = kb, ce = ke;
@@ -514,7 +596,7 @@ __global__ void __launch_bounds__(128) k_build_list_warp(int n, int npad, ListTe
     const unsigned ball = __ballot_sync(0xffffffffu, t);
     if (t) {
       const int slot = cnt + __popc(ball & ((1u << lane) - 1u));
-      if (slot < maxnb) nb[(size_t)slot * npad + i] = k;
+      if (slot < maxnb) row[slot + 3 * (slot & ~7)] = k;
     }
     cnt += __popc(ball);
   }
@@ -525,7 +607,7 @@ __global__ void __launch_bounds__(128) k_build_list_warp(int n, int npad, ListTe
 }
 
 // reference-format half list: row perm[i], partners with larger original index
-__global__ void k_export(int n, int npad, int maxnb, const int* __restrict__ perm, const int* __restrict__ nnb,
+__global__ void k_export(int n, int cap8, int maxnb, const int* __restrict__ perm, const int* __restrict__ nnb,
                          const int* __restrict__ nb, int maxelst, int* __restrict__ nelst, int* __restrict__ elst,
                          int* __restrict__ flags) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -533,7 +615,7 @@ __global__ void k_export(int n, int npad, int maxnb, const int* __restrict__ per
   int io = perm[i];
   int m = min(nnb[i], maxnb), c = 0;
   for (int s = 0; s < m; ++s) {
-    int ko = perm[nb[(size_t)s * npad + i]];
+    int ko = perm[nb[pair_slot(cap8, i, s)]];
     if (ko > io) {
       if (c < maxelst) elst[(size_t)io * maxelst + c] = ko;
       ++c;
@@ -616,15 +698,17 @@ __global__ void k_max_disp(int n, const double4* __restrict__ pos, const double4
 
 }  // namespace
 
-int launch_sort_atoms(Ctx& c) {
+// carry: the last dipoles and E0 follow their atoms into the new order (a warm
+// start reads them; a solve from the direct guess overwrites both)
+int launch_sort_atoms(Ctx& c, bool carry) {
   const int n = c.n;
   ++c.sort_epoch;  // sorted numbering changes: lists in it are stale
   const int nb = (n + kBlock - 1) / kBlock;
   cudaStream_t s = c.stream;
   // the last dipoles (warm start) follow their atoms into the new order; the
   // CG residual buffer is free between solves and holds them meanwhile
-  const bool keep_mu = c.have_perm && c.have_dipoles;
-  const bool keep_ef = c.have_perm && c.have_ef_prev;  // so does the last E0 (d_zr is free too)
+  const bool keep_mu = carry && c.have_perm && c.have_dipoles;
+  const bool keep_ef = carry && c.have_perm && c.have_ef_prev;  // so does the last E0 (d_zr is free too)
   if (keep_mu) {
     int st = launch_to_orig6(c, c.d_mu, c.d_res, 2);
     if (st) return st;
@@ -634,6 +718,18 @@ int launch_sort_atoms(Ctx& c) {
     if (st) return st;
   }
   if (!c.have_perm) c.have_ef_prev = false;
+  const int m = (int)c.sp_k.size();
+  if (n <= kSortSmallAtoms && c.ncell <= kSortSmallCells) {
+    static std::atomic<unsigned long long> limit_set{0};
+    smem_limit_once(k_sort_small, kSortSmallSmem, limit_set);
+    k_sort_small<<<1, 1024, kSortSmallSmem, s>>>(n, c.box, c.nc[0], c.nc[1], c.nc[2], m, c.d_xyz_orig, c.d_cell_start,
+                                                 c.d_cell_count, c.d_perm, c.d_iperm, c.d_scell, c.d_sp_k, c.d_sp_ks);
+    c.have_perm = true;
+    int st = cuda_status(cudaGetLastError(), &c, "sort atoms");
+    if (!st && keep_mu) st = launch_to_sorted6(c, c.d_res, c.d_mu, 2);
+    if (!st && keep_ef) st = launch_to_sorted6(c, c.d_zr, c.d_ef_prev, 2);
+    return st;
+  }
   cudaMemsetAsync(c.d_cell_count, 0, sizeof(int) * c.ncell, s);
   cudaMemsetAsync(c.d_cell_fill, 0, sizeof(int) * c.ncell, s);
   k_cell_count<<<nb, kBlock, 0, s>>>(n, c.box, c.nc[0], c.nc[1], c.nc[2], c.d_xyz_orig, c.d_atom_cell,
@@ -653,7 +749,6 @@ int launch_sort_atoms(Ctx& c) {
   k_cell_sort<<<(c.ncell + kBlock - 1) / kBlock, kBlock, 0, s>>>(c.ncell, c.d_cell_start, c.d_cell_count,
                                                                  c.d_perm, c.d_iperm, c.d_scell);
   c.have_perm = true;
-  const int m = (int)c.sp_k.size();
   if (m > 0) k_sp_to_sorted<<<(m + 255) / 256, 256, 0, s>>>(m, c.d_iperm, c.d_sp_k, c.d_sp_ks);
   int st = cuda_status(cudaGetLastError(), &c, "sort atoms");
   if (!st && keep_mu) st = launch_to_sorted6(c, c.d_res, c.d_mu, 2);
@@ -700,16 +795,17 @@ int launch_build_list_on(Ctx& c, cudaStream_t s) {
   lt.hx = 0.5f * lt.bx;
   lt.hy = 0.5f * lt.by;
   lt.hz = 0.5f * lt.bz;
+  const int cap8 = c.maxpr / 8;
   if (n < THP_LIST_WARP_ATOMS)
-    k_build_list_warp<<<(n + 3) / 4, 128, 0, s>>>(n, c.npad, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos, c.d_posf,
+    k_build_list_warp<<<(n + 3) / 4, 128, 0, s>>>(n, cap8, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos, c.d_posf,
                                                   c.d_scell, c.d_cell_start, c.d_cell_count, c.maxnb, c.d_nnb,
                                                   c.d_nb, c.d_flags);
   else if (THP_LIST_SHIFTED && prefilter && c.nc[0] >= 7 && c.nc[1] >= 7 && c.nc[2] >= 7)
-    k_build_list_shifted<<<(n + 127) / 128, 128, 0, s>>>(n, c.npad, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos,
+    k_build_list_shifted<<<(n + 127) / 128, 128, 0, s>>>(n, cap8, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos,
                                                          c.d_posf, c.d_scell, c.d_cell_start, c.d_cell_count,
                                                          c.maxnb, c.d_nnb, c.d_nb, c.d_flags);
   else
-    k_build_list<<<(n + 127) / 128, 128, 0, s>>>(n, c.npad, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos, c.d_posf,
+    k_build_list<<<(n + 127) / 128, 128, 0, s>>>(n, cap8, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos, c.d_posf,
                                                  c.d_scell, c.d_cell_start, c.d_cell_count, c.maxnb, c.d_nnb,
                                                  c.d_nb, c.d_flags);
   cudaMemcpyAsync(c.d_pos_built, c.d_pos, sizeof(double4) * n, cudaMemcpyDeviceToDevice, s);
@@ -717,12 +813,13 @@ int launch_build_list_on(Ctx& c, cudaStream_t s) {
 }
 
 int launch_export_list(Ctx& c, int maxelst, int* d_nelst, int* d_elst) {
-  return launch_export_pairs(c, c.d_nnb, c.d_nb, c.maxnb, maxelst, d_nelst, d_elst);
+  return launch_export_pairs(c, c.d_nnb, c.d_nb, c.maxnb, c.maxpr / 8, maxelst, d_nelst, d_elst);
 }
 
-int launch_export_pairs(Ctx& c, const int* nnb, const int* nb, int maxnb, int maxelst, int* d_nelst, int* d_elst) {
+int launch_export_pairs(Ctx& c, const int* nnb, const int* nb, int maxnb, int cap8, int maxelst, int* d_nelst,
+                        int* d_elst) {
   const int n = c.n;
-  k_export<<<(n + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(n, c.npad, maxnb, c.d_perm, nnb, nb, maxelst, d_nelst,
+  k_export<<<(n + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(n, cap8, maxnb, c.d_perm, nnb, nb, maxelst, d_nelst,
                                                                d_elst, c.d_flags);
   return cuda_status(cudaGetLastError(), &c, "export list");
 }

@@ -53,56 +53,65 @@ struct Rec64 {  // FP64 record: thole, q, d(3), Q(6)
 // (ranked by lane), so each warp step writes into the group's current block:
 // a handful of sectors, not one partial sector per atom.  An atom's field is
 // the sum of its lanes' partial sums, combined in a fixed tree.
+// LPA lanes per atom: 8, or a whole warp (32) per atom in small systems, whose
+// groups of four leave most of the GPU idle behind chains of 22 steps.
+template <int LPA>
 struct GroupLane {
-  int a, j, i, is;  // atom of the group, lane of the atom, atom index, a valid index for short last groups
+  int a, j, i, is;  // atom of the warp, lane of the atom, atom index, a valid index for short last groups
   bool live;
   __device__ __forceinline__ GroupLane(int g, int lane, int n) {
-    a = lane >> 3;
-    j = lane & 7;
-    i = 4 * g + a;
+    a = lane / LPA;
+    j = lane % LPA;
+    i = (32 / LPA) * g + a;
     live = i < n;
-    is = live ? i : 4 * g;
+    is = live ? i : (32 / LPA) * g;
   }
 };
+
+// entry s of a list or pair-stream row whose entry 0 is at `row`
+__device__ __forceinline__ size_t row_entry(size_t row, int s) { return row + ((size_t)(s >> 3) << 5) + (s & 7); }
 
 // After one step: the accepted pair of this lane (take) goes to slot
 // cnt + (accepted lanes of the atom before it); cnt advances by the atom's
 // accepted count.  Returns the slot (or -1).
+template <int LPA>
 __device__ __forceinline__ int step_slot(bool take, int a, int j, int& cnt) {
   const unsigned ball = __ballot_sync(kFullMask, take);
-  const unsigned mine = (ball >> (8 * a)) & 0xffu;
+  const unsigned mine = LPA == 32 ? ball : (ball >> (LPA * a)) & ((1u << (LPA & 31)) - 1u);
   const int slot = take ? cnt + __popc(mine & ((1u << j) - 1u)) : -1;
   cnt += __popc(mine);
   return slot;
 }
 
 // FP64 pass (the FP64 form): exact r^2 test and FP64 pair terms.
-template <bool FIELD>
+template <bool FIELD, int LPA>
 __global__ void __launch_bounds__(kFieldBlock, THP_EFLD0_MINB) k_efld0_coef(
-    int n, int npad, Box box, double cut2, EwaldConst ew, const double4* __restrict__ pos,
+    int n, Box box, double cut2, EwaldConst ew, const double4* __restrict__ pos,
     const double* __restrict__ mrec, const int* __restrict__ perm, const int* __restrict__ sp_off,
     const int* __restrict__ sp_ks, const double* __restrict__ sp_s, const int* __restrict__ nnb,
     const int* __restrict__ nb, int maxnb, int* __restrict__ npr, int* __restrict__ pk_out,
     double2* __restrict__ pcc, int cap8, double* __restrict__ ef, int* __restrict__ flags) {
   const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (4 * g >= n) return;
-  const GroupLane L(g, threadIdx.x & 31, n);
+  if ((32 / LPA) * g >= n) return;
+  const GroupLane<LPA> L(g, threadIdx.x & 31, n);
   const int maxpr = 8 * cap8;
   const double4 pi = pos[L.is];
   const double thi = mrec[(size_t)L.is * 12];
   const int io = perm[L.is];
   const int s0 = sp_off[io], s1 = sp_off[io + 1];
   const int nn = L.live ? min(nnb[L.is], maxnb) : 0;
-  int mb = max(nn, __shfl_xor_sync(kFullMask, nn, 8));
-  mb = max(mb, __shfl_xor_sync(kFullMask, mb, 16));
+  int mb = nn;
+#pragma unroll
+  for (int o = LPA; o < 32; o <<= 1) mb = max(mb, __shfl_xor_sync(kFullMask, mb, o));
+  const size_t row = pair_slot(cap8, L.is, 0);
   double e[6] = {0, 0, 0, 0, 0, 0};
   int cnt = 0;
   // list entries one step ahead of their gathers (the list streams from DRAM)
-  int knext = L.j < nn ? __ldg(nb + (size_t)L.j * npad + L.is) : L.is;
+  int knext = L.j < nn ? __ldg(nb + row_entry(row, L.j)) : L.is;
 #pragma unroll 1
-  for (int s = L.j; s - L.j < mb; s += 8) {
+  for (int s = L.j; s - L.j < mb; s += LPA) {
     const int k = knext;
-    knext = s + 8 < nn ? __ldg(nb + (size_t)(s + 8) * npad + L.is) : L.is;
+    knext = s + LPA < nn ? __ldg(nb + row_entry(row, s + LPA)) : L.is;
     const double4 pk4 = pos[k];
     Rec64 r_k;
     r_k.load(mrec, k);
@@ -177,14 +186,14 @@ __global__ void __launch_bounds__(kFieldBlock, THP_EFLD0_MINB) k_efld0_coef(
       c3 = bn1 - (1.0 - us * l3) * rr3;
       c5 = bn2 - (1.0 - us * l5) * rr5;
     }
-    const int slot = step_slot(take, L.a, L.j, cnt);
+    const int slot = step_slot<LPA>(take, L.a, L.j, cnt);
     if (slot >= 0 && slot < maxpr) {
-      const size_t q = pair_slot(cap8, L.i, slot);
+      const size_t q = row_entry(row, slot);
       pk_out[q] = k;
       pcc[q] = make_double2(c3, c5);
     }
   }
-  if (FIELD) lane8_sum<6>(e);
+  if (FIELD) lanes_sum<LPA, 6>(e);
   if (!L.live) return;
   if (L.j == 0) {
     npr[L.i] = min(cnt, maxpr);
@@ -208,16 +217,16 @@ __global__ void __launch_bounds__(kFieldBlock, THP_EFLD0_MINB) k_efld0_coef(
 // The FP32 coefficients written for the CG rows follow the same formulas.
 constexpr int kSpCache = 4;
 
-template <bool FIELD>
+template <bool FIELD, int LPA>
 __global__ void __launch_bounds__(kFieldBlock, THP_EFLD0_MINB) k_efld0_coef32(
-    int n, int npad, float bx, float by, float bz, float cut2, EwaldConst ew, const float* __restrict__ erec,
+    int n, float bx, float by, float bz, float cut2, EwaldConst ew, const float* __restrict__ erec,
     const int* __restrict__ perm, const int* __restrict__ sp_off, const int* __restrict__ sp_ks,
     const double* __restrict__ sp_s, const int* __restrict__ nnb, const int* __restrict__ nb, int maxnb,
     int* __restrict__ npr, int* __restrict__ pk_out, float2* __restrict__ pcc, int cap8,
     double* __restrict__ ef, int* __restrict__ flags) {
   const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (4 * g >= n) return;
-  const GroupLane L(g, threadIdx.x & 31, n);
+  if ((32 / LPA) * g >= n) return;
+  const GroupLane<LPA> L(g, threadIdx.x & 31, n);
   const int maxpr = 8 * cap8;
   const float4 pi = *reinterpret_cast<const float4*>(erec + (size_t)L.is * 16);
   const float thi = erec[(size_t)L.is * 16 + 4];
@@ -230,17 +239,19 @@ __global__ void __launch_bounds__(kFieldBlock, THP_EFLD0_MINB) k_efld0_coef32(
   const float hx = 0.5f * bx, hy = 0.5f * by, hz = 0.5f * bz;
   const float ea = (float)ew.a, af1 = (float)ew.afac1, af2 = (float)ew.afac2, af3 = (float)ew.afac3;
   const int nn = L.live ? min(nnb[L.is], maxnb) : 0;
-  int mb = max(nn, __shfl_xor_sync(kFullMask, nn, 8));
-  mb = max(mb, __shfl_xor_sync(kFullMask, mb, 16));
+  int mb = nn;
+#pragma unroll
+  for (int o = LPA; o < 32; o <<= 1) mb = max(mb, __shfl_xor_sync(kFullMask, mb, o));
+  const size_t row = pair_slot(cap8, L.is, 0);
   double e[6] = {0, 0, 0, 0, 0, 0};
   int cnt = 0;
   // list entries one step ahead: the list streams from DRAM, and its load
   // would otherwise sit in front of every step's record gathers
-  int knext = L.j < nn ? __ldg(nb + (size_t)L.j * npad + L.is) : L.is;
+  int knext = L.j < nn ? __ldg(nb + row_entry(row, L.j)) : L.is;
 #pragma unroll 1
-  for (int s = L.j; s - L.j < mb; s += 8) {
+  for (int s = L.j; s - L.j < mb; s += LPA) {
     const int k = knext;
-    knext = s + 8 < nn ? __ldg(nb + (size_t)(s + 8) * npad + L.is) : L.is;
+    knext = s + LPA < nn ? __ldg(nb + row_entry(row, s + LPA)) : L.is;
     float v[16];
     ld_rec8(erec + (size_t)k * 16, *reinterpret_cast<float(*)[8]>(&v[0]));
     ld_rec8(erec + (size_t)k * 16 + 8, *reinterpret_cast<float(*)[8]>(&v[8]));
@@ -331,14 +342,14 @@ __global__ void __launch_bounds__(kFieldBlock, THP_EFLD0_MINB) k_efld0_coef32(
       c3 = bn1 - (1.f - us * l3) * rr3;
       c5 = bn2 - (1.f - us * l5) * rr5;
     }
-    const int slot = step_slot(take, L.a, L.j, cnt);
+    const int slot = step_slot<LPA>(take, L.a, L.j, cnt);
     if (slot >= 0 && slot < maxpr) {
-      const size_t o = pair_slot(cap8, L.i, slot);
+      const size_t o = row_entry(row, slot);
       pk_out[o] = k;
       pcc[o] = make_float2(c3, c5);
     }
   }
-  if (FIELD) lane8_sum<6>(e);
+  if (FIELD) lanes_sum<LPA, 6>(e);
   if (!L.live) return;
   if (L.j == 0) {
     npr[L.i] = min(cnt, maxpr);
@@ -439,31 +450,44 @@ int group_blocks(int n, int block) { return (((n + 3) / 4) * 32 + block - 1) / b
 
 int launch_efld0_coef(Ctx& c, bool with_field) { return launch_efld0_coef_on(c, with_field, c.stream); }
 
-int launch_efld0_coef_on(Ctx& c, bool with_field, cudaStream_t s) {
-  const int nb = group_blocks(c.n, kFieldBlock);
+// systems below this many atoms take a warp per atom in the field passes
+#ifndef THP_EFLD0_WARP_ATOMS
+#define THP_EFLD0_WARP_ATOMS 8000
+#endif
+
+template <int LPA>
+static void launch_field_pass(Ctx& c, bool with_field, cudaStream_t s) {
+  const int nb = (int)(((c.n + 32 / LPA - 1) / (32 / LPA) * 32 + kFieldBlock - 1) / kFieldBlock);
   const double cut2 = c.cfg.ewaldcut * c.cfg.ewaldcut;
   EwaldConst ew = ewald_const(c.cfg.aewald);
   const int cap8 = c.maxpr / 8;
   if (c.mixed) {
     const float bx = (float)c.box.l[0], by = (float)c.box.l[1], bz = (float)c.box.l[2];
-#define THP_EFLD0_ARGS32                                                                                        \
-  c.n, c.npad, bx, by, bz, (float)cut2, ew, c.d_erec, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_s, c.d_nnb, c.d_nb, \
-      c.maxnb, c.d_npr, c.d_pk, (float2*)c.d_pcc, cap8, c.d_ef, c.d_flags
+#define THP_EFLD0_ARGS32                                                                                           \
+  c.n, bx, by, bz, (float)cut2, ew, c.d_erec, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_s, c.d_nnb, c.d_nb, c.maxnb, \
+      c.d_npr, c.d_pk, (float2*)c.d_pcc, cap8, c.d_ef, c.d_flags
     if (with_field)
-      k_efld0_coef32<true><<<nb, kFieldBlock, 0, s>>>(THP_EFLD0_ARGS32);
+      k_efld0_coef32<true, LPA><<<nb, kFieldBlock, 0, s>>>(THP_EFLD0_ARGS32);
     else
-      k_efld0_coef32<false><<<nb, kFieldBlock, 0, s>>>(THP_EFLD0_ARGS32);
+      k_efld0_coef32<false, LPA><<<nb, kFieldBlock, 0, s>>>(THP_EFLD0_ARGS32);
 #undef THP_EFLD0_ARGS32
   } else {
-#define THP_EFLD0_ARGS                                                                                          \
-  c.n, c.npad, c.box, cut2, ew, c.d_pos, c.d_mrec, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_s, c.d_nnb, c.d_nb,   \
-      c.maxnb, c.d_npr, c.d_pk, (double2*)c.d_pcc, cap8, c.d_ef, c.d_flags
+#define THP_EFLD0_ARGS                                                                                               \
+  c.n, c.box, cut2, ew, c.d_pos, c.d_mrec, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_s, c.d_nnb, c.d_nb, c.maxnb,      \
+      c.d_npr, c.d_pk, (double2*)c.d_pcc, cap8, c.d_ef, c.d_flags
     if (with_field)
-      k_efld0_coef<true><<<nb, kFieldBlock, 0, s>>>(THP_EFLD0_ARGS);
+      k_efld0_coef<true, LPA><<<nb, kFieldBlock, 0, s>>>(THP_EFLD0_ARGS);
     else
-      k_efld0_coef<false><<<nb, kFieldBlock, 0, s>>>(THP_EFLD0_ARGS);
+      k_efld0_coef<false, LPA><<<nb, kFieldBlock, 0, s>>>(THP_EFLD0_ARGS);
 #undef THP_EFLD0_ARGS
   }
+}
+
+int launch_efld0_coef_on(Ctx& c, bool with_field, cudaStream_t s) {
+  if (c.n < THP_EFLD0_WARP_ATOMS)
+    launch_field_pass<32>(c, with_field, s);
+  else
+    launch_field_pass<8>(c, with_field, s);
   c.have_coef = true;
   return cuda_status(cudaGetLastError(), &c, "efld0/coef");
 }

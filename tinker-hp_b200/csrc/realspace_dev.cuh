@@ -96,6 +96,7 @@ __device__ __forceinline__ void ld_rec8(const float* p, float (&v)[8]) {
 // Partner data of the three row forms: position (in the form's own frame)
 // and the six dipole components (d xyz, p xyz) of atom k.
 struct Partner64 {  // FP64: double4 positions as given, mu [n][6] double
+  static constexpr int kNC = 6;
   const double4* __restrict__ pos;
   const double* __restrict__ mu;
   __device__ __forceinline__ void load(int k, double (&p)[3], double (&u)[6]) const {
@@ -107,6 +108,7 @@ struct Partner64 {  // FP64: double4 positions as given, mu [n][6] double
   }
 };
 struct Partner32 {  // FP32: float4 positions wrapped into the box, mu [n][6] float
+  static constexpr int kNC = 6;
   const float4* __restrict__ pos;
   const float* __restrict__ mu;
   __device__ __forceinline__ void load(int k, float (&p)[3], float (&u)[6]) const {
@@ -121,6 +123,7 @@ struct Partner32 {  // FP32: float4 positions wrapped into the box, mu [n][6] fl
 // position wrapped into the box, mpz[k] = p dipole z): two gathers per
 // partner, one of them a 256-bit load.
 struct PartnerRec {
+  static constexpr int kNC = 6;
   const float* __restrict__ rec;
   const float* __restrict__ mpz;
   __device__ __forceinline__ void load(int k, float (&p)[3], float (&u)[6]) const {
@@ -132,11 +135,56 @@ struct PartnerRec {
   }
 };
 
+// FP64 atom records (rec[k] = {x, y, z, d dipole, p dipole x, y} with the
+// position wrapped into the box, mpz[k] = p dipole z): 72 bytes per partner in
+// two 256-bit loads and one of 8 bytes, where the position and the dipoles
+// apart took five loads over three or four sectors.
+struct PartnerRec64 {
+  static constexpr int kNC = 6;
+  const double* __restrict__ rec;
+  const double* __restrict__ mpz;
+  __device__ __forceinline__ void load(int k, double (&p)[3], double (&u)[6]) const {
+    const double* q = rec + (size_t)k * 8;
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(p[0]), "=d"(p[1]), "=d"(p[2]), "=d"(u[0]) : "l"(q));
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(u[1]), "=d"(u[2]), "=d"(u[3]), "=d"(u[4]) : "l"(q + 4));
+    u[5] = __ldg(mpz + k);
+  }
+};
+
+// Records of the single-field rows (rec[k] = {x, y, z, dipole, 2 unused}).
+template <typename T>
+struct PartnerRec1 {
+  static constexpr int kNC = 3;
+  const T* __restrict__ rec;
+  __device__ __forceinline__ void load(int k, T (&p)[3], T (&u)[3]) const {
+    const T* q = rec + (size_t)k * 8;
+    if constexpr (sizeof(T) == 4) {
+      float v[8];
+      ld_rec8(q, v);
+      p[0] = v[0]; p[1] = v[1]; p[2] = v[2];
+      u[0] = v[3]; u[1] = v[4]; u[2] = v[5];
+    } else {
+      asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(p[0]), "=d"(p[1]), "=d"(p[2]), "=d"(u[0]) : "l"(q));
+      const double2 b = __ldg(reinterpret_cast<const double2*>(q + 4));
+      u[1] = b.x; u[2] = b.y;
+    }
+  }
+};
+
 // Displacement imaged into the box: FP64 by image.f's rule, FP32 by one wrap
 // of coordinates that already lie in the box.
 struct Image64 {
   Box box;
   __device__ __forceinline__ void apply(double& x, double& y, double& z) const { image3(box, x, y, z); }
+};
+// one wrap of FP64 coordinates that already lie in the box
+struct Image64In {
+  Box box;
+  __device__ __forceinline__ void apply(double& x, double& y, double& z) const {
+    x = fabs(x) > box.half[0] ? x - copysign(box.l[0], x) : x;
+    y = fabs(y) > box.half[1] ? y - copysign(box.l[1], y) : y;
+    z = fabs(z) > box.half[2] ? z - copysign(box.l[2], z) : z;
+  }
 };
 struct Image32 {
   float bx, by, bz;
@@ -187,7 +235,7 @@ __device__ __forceinline__ void stream_round(const int* pk, const typename Vec2<
 // of the box, so no pair crosses one.
 template <typename T, int U, bool NOL1, bool WRAP, typename Ld, typename Im>
 __device__ __forceinline__ void group_row_part(const PairRows& pr, const Ld& ld, const Im& im, const T (&pi)[3],
-                                               int i_safe, int j, int m, int nblk, size_t base, T (&acc)[6]) {
+                                               int i_safe, int j, int m, int nblk, size_t base, T (&acc)[Ld::kNC]) {
   using T2 = typename Vec2<T>::type;
   const int* __restrict__ pk = pr.pk + base;
   const T2* __restrict__ pc = (const T2*)pr.pcc + base;
@@ -198,7 +246,7 @@ __device__ __forceinline__ void group_row_part(const PairRows& pr, const Ld& ld,
 #pragma unroll 1
   for (int b = 0; b < nblk; b += U) {
     if (!THP_GROW_PF) stream_round<T, U, NOL1>(pk + 32 * b, pc + 32 * b, b, mj, nblk, i_safe, k, c3, c5);
-    T p[U][3], w[U][6];
+    T p[U][3], w[U][Ld::kNC];
 #pragma unroll
     for (int u = 0; u < U; ++u) ld.load(k[u], p[u], w[u]);
     int kn[U];
@@ -209,15 +257,16 @@ __device__ __forceinline__ void group_row_part(const PairRows& pr, const Ld& ld,
     for (int u = 0; u < U; ++u) {
       T xr = p[u][0] - pi[0], yr = p[u][1] - pi[1], zr = p[u][2] - pi[2];
       if (WRAP) im.apply(xr, yr, zr);
-      const T dd = xr * w[u][0] + yr * w[u][1] + zr * w[u][2];
-      const T dp = xr * w[u][3] + yr * w[u][4] + zr * w[u][5];
-      const T sd = c5[u] * dd, sp = c5[u] * dp;
+      const T sd = c5[u] * (xr * w[u][0] + yr * w[u][1] + zr * w[u][2]);
       acc[0] += c3[u] * w[u][0] - sd * xr;
       acc[1] += c3[u] * w[u][1] - sd * yr;
       acc[2] += c3[u] * w[u][2] - sd * zr;
-      acc[3] += c3[u] * w[u][3] - sp * xr;
-      acc[4] += c3[u] * w[u][4] - sp * yr;
-      acc[5] += c3[u] * w[u][5] - sp * zr;
+      if constexpr (Ld::kNC == 6) {
+        const T sp = c5[u] * (xr * w[u][3] + yr * w[u][4] + zr * w[u][5]);
+        acc[3] += c3[u] * w[u][3] - sp * xr;
+        acc[4] += c3[u] * w[u][4] - sp * yr;
+        acc[5] += c3[u] * w[u][5] - sp * zr;
+      }
     }
     if (THP_GROW_PF) {
 #pragma unroll
@@ -238,7 +287,7 @@ __device__ __forceinline__ void group_row_part(const PairRows& pr, const Ld& ld,
 // bound where that frame is not the wrapped box.
 template <typename T, int U, bool NOL1, typename Ld, typename Im>
 __device__ __forceinline__ void group_row(const PairRows& pr, const Ld& ld, const Im& im, int g, int lane,
-                                          T (&acc)[6], T interior) {
+                                          T (&acc)[Ld::kNC], T interior) {
   const int a = lane >> 3, j = lane & 7;
   const int i = 4 * g + a;
   const bool live = i < pr.n;
@@ -247,10 +296,10 @@ __device__ __forceinline__ void group_row(const PairRows& pr, const Ld& ld, cons
   mb = max(mb, __shfl_xor_sync(kFullMask, mb, 16));
   const int nblk = (mb + 7) >> 3;
   const int i_safe = live ? i : 4 * g;
-  T pi[3], wi[6];
+  T pi[3], wi[Ld::kNC];
   ld.load(i_safe, pi, wi);
 #pragma unroll
-  for (int q = 0; q < 6; ++q) acc[q] = T(0);
+  for (int q = 0; q < Ld::kNC; ++q) acc[q] = T(0);
   const bool inside = fabs(pi[0]) <= interior && fabs(pi[1]) <= interior && fabs(pi[2]) <= interior;
   const size_t base = (size_t)g * pr.cap8 * 32 + lane;
   if (__all_sync(kFullMask, inside))
@@ -260,7 +309,7 @@ __device__ __forceinline__ void group_row(const PairRows& pr, const Ld& ld, cons
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
-    for (int q = 0; q < 6; ++q) acc[q] += __shfl_xor_sync(kFullMask, acc[q], o);
+    for (int q = 0; q < Ld::kNC; ++q) acc[q] += __shfl_xor_sync(kFullMask, acc[q], o);
 }
 
 // Component j (0..5) of a six-vector held in registers, without local memory.
@@ -275,12 +324,12 @@ __device__ __forceinline__ T pick6(const T (&v)[6], int j) {
   return r;
 }
 
-// An atom's eight lanes' partial sums combined (fixed tree); every lane of
+// The partial sums of an atom's LPA lanes combined (fixed tree); every lane of
 // the atom gets the total.
-template <int NV>
-__device__ __forceinline__ void lane8_sum(double (&v)[NV]) {
+template <int LPA, int NV>
+__device__ __forceinline__ void lanes_sum(double (&v)[NV]) {
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1)
+  for (int o = LPA / 2; o > 0; o >>= 1)
 #pragma unroll
     for (int q = 0; q < NV; ++q) v[q] += __shfl_xor_sync(kFullMask, v[q], o);
 }

@@ -17,7 +17,7 @@
 // lbuffer for the atoms' drift since the sort, and the largest allowed
 // reduction shift on both sides).  The list is rebuilt after a re-sort or
 // once an atom has moved lbuffer/2 since the positions it was built from, as
-// the reference's list update does.  One thread per site evaluates each pair
+// the reference's list update does.  Eight lanes per site evaluate each pair
 // from its own end (no atomics for the pair terms): its list is dense in
 // interacting pairs, so the lanes of a warp stay together through the pair
 // arithmetic.  The site's summed force goes to the atom and its parent in
@@ -27,6 +27,7 @@
 
 #include "grad_dev.cuh"
 #include "kernels.h"
+#include "realspace_dev.cuh"
 
 namespace thp {
 
@@ -67,7 +68,7 @@ __global__ void k_vdw_sites(int n, const int* __restrict__ perm, const int* __re
   vred[s] = make_double4(x, y, z, r);
   double wx = x, wy = y, wz = z;  // wrapped into the box for the FP32 screen of the list build
   image3(box, wx, wy, wz);
-  vredf[s] = make_float4((float)wx, (float)wy, (float)wz, 0.f);
+  vredf[s] = make_float4((float)wx, (float)wy, (float)wz, __int_as_float(cls[o]));  // the class rides in w
   vinfo[s] = make_int2(cls[o], ps);
 }
 
@@ -79,7 +80,7 @@ __device__ __forceinline__ int axis_cell(int c, int nc, int w, int q) {
 
 // vlistcell (nblist.f:1148-1305) over the cell sort: every other site whose
 // reduced minimum-image distance is within vbuf (both directions)
-__global__ void __launch_bounds__(kBlock) k_vdw_list(int n, int npad, Box box, double vbuf2, int prefilter, float lo,
+__global__ void __launch_bounds__(kBlock) k_vdw_list(int n, int cap8, Box box, double vbuf2, int prefilter, float lo,
                                                      float hi, int wx, int wy, int wz, const double4* __restrict__ vred,
                                                      const float4* __restrict__ vredf, const int2* __restrict__ vinfo,
                                                      const double* __restrict__ vtab, int nclass,
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(kBlock) k_vdw_list(int n, int npad, Box box, d
           }
           if (take && __ldg(vtab + (size_t)__ldg(&vinfo[k].x) * (nclass + 1)) == 0.0) take = false;
           if (take) {
-            if (cnt < maxvnb) vnb[(size_t)cnt * npad + i] = k;
+            if (cnt < maxvnb) vnb[pair_slot(cap8, i, cnt)] = k;
             ++cnt;
           }
         }
@@ -213,118 +214,144 @@ __device__ __forceinline__ U hal_pair(U r2, U rv, U eps, const VdwConst& vc, dou
   return de / rik;
 }
 
+// special partners of a site held in registers (a longer list is searched
+// past those)
+constexpr int kSpCache = 4;
+
+// A warp takes four consecutive (cell-sorted) sites, eight lanes each: lane j
+// takes list entries j, j+8, ..., and the lanes' sums are combined in a fixed
+// shuffle tree (one thread per site left small systems with a few blocks of
+// long dependent chains).  The pair tables of up to kVdwTab classes are staged
+// in shared memory.
 // VIR: each block also writes the sum of its sites' pair virials (half of
 // each pair from each end, ehal1.f:431-446) to vpart[block][6].
+constexpr int kVdwTab = 8;
+
 template <bool MIXED, bool VIR>
-__global__ void __launch_bounds__(kBlock) k_ehal(int n, int npad, Box box, VdwConst vc,
+__global__ void __launch_bounds__(kBlock) k_ehal(int n, int cap8, Box box, VdwConst vc,
                                                  const double4* __restrict__ vred, const float4* __restrict__ vredf,
                                                  const int2* __restrict__ vinfo, const double* __restrict__ vtab,
                                                  const int* __restrict__ perm, const int* __restrict__ sp_off,
                                                  const int* __restrict__ sp_ks, const int* __restrict__ sp_c,
                                                  const int* __restrict__ vnnb, const int* __restrict__ vnb,
-                                                 unsigned long long* __restrict__ dev, double* __restrict__ epart,
+                                                 FixAcc dev, double* __restrict__ epart,
                                                  double* __restrict__ vpart) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  using U = typename std::conditional<MIXED, float, double>::type;
+  __shared__ U stab[4 * kVdwTab * kVdwTab];
+  const int nc2 = vc.nclass * vc.nclass;
+  const bool staged = vc.nclass <= kVdwTab;
+  if (staged) {
+    for (int q = threadIdx.x; q < 4 * nc2; q += blockDim.x) stab[q] = (U)vtab[q];
+    __syncthreads();
+  }
+  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, jl = threadIdx.x & 7;
+  const bool live = i0 < n;
+  const int i = live ? i0 : n - 1;  // a valid site for the loads of idle lanes
   double eacc = 0.0;
   double v6[6] = {0, 0, 0, 0, 0, 0};
-  if (i < n) {
-    const double4 ri = vred[i];
+  double gx = 0.0, gy = 0.0, gz = 0.0;
+  const double4 ri = vred[i];
+  const int2 inf = vinfo[i];
+  {
     const float4 fi = vredf[i];
     const float bx = (float)box.l[0], by = (float)box.l[1], bz = (float)box.l[2];
     const float hx = 0.5f * bx, hy = 0.5f * by, hz = 0.5f * bz;
     const float off2f = (float)vc.off2;
-    const int2 inf = vinfo[i];
     const int it = inf.x;
     const int io = perm[i];
     const int s0 = sp_off[io], s1 = sp_off[io + 1];
-    const int nc2 = vc.nclass * vc.nclass;
-    double gx = 0.0, gy = 0.0, gz = 0.0;
-    const int nn = vnnb[i];
-    int knext = nn > 0 ? __ldg(vnb + i) : 0;  // list entries fetched one pair ahead
+    int spk[kSpCache];
+#pragma unroll
+    for (int q = 0; q < kSpCache; ++q) spk[q] = s0 + q < s1 ? __ldg(sp_ks + s0 + q) : -1;
+    const int nn = live ? vnnb[i] : 0;
+    const int* __restrict__ row = vnb + pair_slot(cap8, i, jl);  // entry s: 4 (s - j) on
+    int knext = jl < nn ? __ldg(row) : i;  // list entries fetched one step ahead
 #pragma unroll 1
-    for (int s = 0; s < nn; ++s) {
+    for (int s = jl; s < nn; s += 8) {
       const int k = knext;
-      if (s + 1 < nn) knext = __ldg(vnb + (size_t)(s + 1) * npad + i);
-      double xr, yr, zr;
-      float xf = 0.f, yf = 0.f, zf = 0.f, r2f = 0.f;
-      double rik2 = 0.0;
+      if (s + 8 < nn) knext = __ldg(row + 4 * (size_t)(s + 8 - jl));
+      U xr, yr, zr, r2;
+      int kt;
       if constexpr (MIXED) {
         const float4 fk = vredf[k];
-        xf = fi.x - fk.x;
-        yf = fi.y - fk.y;
-        zf = fi.z - fk.z;
-        xf = fabsf(xf) > hx ? xf - copysignf(bx, xf) : xf;
-        yf = fabsf(yf) > hy ? yf - copysignf(by, yf) : yf;
-        zf = fabsf(zf) > hz ? zf - copysignf(bz, zf) : zf;
-        r2f = xf * xf + yf * yf + zf * zf;
-        if (r2f > off2f) continue;
+        xr = fi.x - fk.x;
+        yr = fi.y - fk.y;
+        zr = fi.z - fk.z;
+        xr = fabsf(xr) > hx ? xr - copysignf(bx, xr) : xr;
+        yr = fabsf(yr) > hy ? yr - copysignf(by, yr) : yr;
+        zr = fabsf(zr) > hz ? zr - copysignf(bz, zr) : zr;
+        r2 = xr * xr + yr * yr + zr * zr;
+        if (r2 > off2f) continue;
+        kt = __float_as_int(fk.w);
       } else {
         const double4 rk = vred[k];
+        kt = __ldg(&vinfo[k].x);
         xr = ri.x - rk.x;
         yr = ri.y - rk.y;
         zr = ri.z - rk.z;
         image3(box, xr, yr, zr);
-        rik2 = r2_exact(xr, yr, zr);
-        if (rik2 > vc.off2) continue;
+        r2 = r2_exact(xr, yr, zr);
+        if (r2 > vc.off2) continue;
       }
-      const int kt = __ldg(&vinfo[k].x);
-      double vs = 1.0;
-      bool is14 = false;
-      for (int q = s0; q < s1; ++q)
-        if (__ldg(sp_ks + q) == k) {
-          const int cls = __ldg(sp_c + q);
-          vs = cls == 0 ? vc.vscale[0] : cls == 1 ? vc.vscale[1] : cls == 2 ? vc.vscale[2]
-                                                            : cls == 3 ? vc.vscale[3] : 1.0;
-          is14 = cls == 2;
-          break;
-        }
-      const int t = kt * vc.nclass + it;
-      const double rv = __ldg(vtab + (is14 ? 2 * nc2 : 0) + t);
-      const double eps = __ldg(vtab + (is14 ? 3 * nc2 : nc2) + t) * vs;
-      double dx, dy, dz, px, py, pz;  // dE/dx of the pair and its separation
-      if constexpr (MIXED) {
-        const float de = hal_pair<float>(r2f, (float)rv, (float)eps, vc, eacc);
-        dx = (double)(de * xf);
-        dy = (double)(de * yf);
-        dz = (double)(de * zf);
-        px = xf;
-        py = yf;
-        pz = zf;
+      int sq = -1;
+#pragma unroll
+      for (int q = 0; q < kSpCache; ++q)
+        if (spk[q] == k) sq = s0 + q;
+      if (sq < 0 && s1 - s0 > kSpCache)
+        for (int q = s0 + kSpCache; q < s1; ++q)
+          if (__ldg(sp_ks + q) == k) {
+            sq = q;
+            break;
+          }
+      int t = kt * vc.nclass + it;
+      U rv, eps;
+      if (sq < 0) {
+        rv = staged ? stab[t] : (U)__ldg(vtab + t);
+        eps = staged ? stab[nc2 + t] : (U)__ldg(vtab + nc2 + t);
       } else {
-        const double de = hal_pair<double>(rik2, rv, eps, vc, eacc);
-        dx = de * xr;
-        dy = de * yr;
-        dz = de * zr;
-        px = xr;
-        py = yr;
-        pz = zr;
+        const int cls = __ldg(sp_c + sq);
+        const double vs = cls == 0 ? vc.vscale[0] : cls == 1 ? vc.vscale[1] : cls == 2 ? vc.vscale[2]
+                                                                  : cls == 3 ? vc.vscale[3] : 1.0;
+        if (cls == 2) t += 2 * nc2;
+        rv = (U)__ldg(vtab + t);
+        eps = (U)(__ldg(vtab + nc2 + t) * vs);
       }
+      const U de = hal_pair<U>(r2, rv, eps, vc, eacc);
+      const double dx = (double)(de * xr), dy = (double)(de * yr), dz = (double)(de * zr);
       gx += dx;
       gy += dy;
       gz += dz;
       if (VIR) {
-        v6[0] += 0.5 * px * dx;
-        v6[1] += 0.5 * py * dx;
-        v6[2] += 0.5 * pz * dx;
-        v6[3] += 0.5 * py * dy;
-        v6[4] += 0.5 * pz * dy;
-        v6[5] += 0.5 * pz * dz;
+        v6[0] += 0.5 * xr * dx;
+        v6[1] += 0.5 * yr * dx;
+        v6[2] += 0.5 * zr * dx;
+        v6[3] += 0.5 * yr * dy;
+        v6[4] += 0.5 * zr * dy;
+        v6[5] += 0.5 * zr * dz;
       }
     }
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    gx += __shfl_xor_sync(0xffffffffu, gx, o);
+    gy += __shfl_xor_sync(0xffffffffu, gy, o);
+    gz += __shfl_xor_sync(0xffffffffu, gz, o);
+  }
+  if (live && jl == 0) {
     // the site's force: to the atom (kred) and its parent (1 - kred)
     const int iv = inf.y;
     if (iv == i) {
-      fix_add(dev + 3 * i + 0, gx);
-      fix_add(dev + 3 * i + 1, gy);
-      fix_add(dev + 3 * i + 2, gz);
+      dev.add(3 * i + 0, gx);
+      dev.add(3 * i + 1, gy);
+      dev.add(3 * i + 2, gz);
     } else {
       const double redi = ri.w, rediv = 1.0 - redi;
-      fix_add(dev + 3 * i + 0, gx * redi);
-      fix_add(dev + 3 * i + 1, gy * redi);
-      fix_add(dev + 3 * i + 2, gz * redi);
-      fix_add(dev + 3 * iv + 0, gx * rediv);
-      fix_add(dev + 3 * iv + 1, gy * rediv);
-      fix_add(dev + 3 * iv + 2, gz * rediv);
+      dev.add(3 * i + 0, gx * redi);
+      dev.add(3 * i + 1, gy * redi);
+      dev.add(3 * i + 2, gz * redi);
+      dev.add(3 * iv + 0, gx * rediv);
+      dev.add(3 * iv + 1, gy * rediv);
+      dev.add(3 * iv + 2, gz * rediv);
     }
   }
   block_partial<kBlock>(eacc, epart);
@@ -350,9 +377,9 @@ int launch_vdw_list(Ctx& c) {
   if (!c.have_vdw) return THP_E_STATE;
   const size_t n = c.n;
   const int nb = (c.n + kBlock - 1) / kBlock;
-  if ((st = alloc_once(c, &c.d_vred, n, "alloc vdw sites"))) return st;
-  if ((st = alloc_once(c, &c.d_vinfo, n, "alloc vdw sites"))) return st;
-  if ((st = alloc_once(c, &c.d_vredf, n, "alloc vdw sites"))) return st;
+  if ((st = alloc_once(c, &c.d_vred, c.cap_n, "alloc vdw sites"))) return st;
+  if ((st = alloc_once(c, &c.d_vinfo, c.cap_n, "alloc vdw sites"))) return st;
+  if ((st = alloc_once(c, &c.d_vredf, c.cap_n, "alloc vdw sites"))) return st;
   k_vdw_sites<<<nb, kBlock, 0, c.stream>>>(c.n, c.d_perm, c.d_iperm, c.d_pos, c.d_vcls, c.d_vired, c.d_vkred, c.box,
                                            kShiftMax * kShiftMax, c.d_vred, c.d_vredf, c.d_vinfo, c.d_flags);
   if ((st = cuda_status(cudaGetLastError(), &c, "vdw sites"))) return st;
@@ -366,13 +393,13 @@ int launch_vdw_list(Ctx& c) {
   }
   if (!build) return THP_OK;
   if (!c.d_vnb) {
-    c.maxvnb = c.cfg.max_neighbors > 0 ? 2 * c.cfg.max_neighbors : kDefaultMaxVnb;
-    if ((st = cuda_status(cudaMalloc((void**)&c.d_vnb, sizeof(int) * (size_t)c.maxvnb * c.npad), &c,
+    c.maxvnb = c.cfg.max_neighbors > 0 ? (2 * c.cfg.max_neighbors + 7) / 8 * 8 : kDefaultMaxVnb;
+    if ((st = cuda_status(cudaMalloc((void**)&c.d_vnb, sizeof(int) * (size_t)c.maxvnb * ((c.cap_n + 31) / 32 * 32)), &c,
                           "alloc vdw list")))
       return st;
   }
-  if ((st = alloc_once(c, &c.d_vnnb, n, "alloc vdw list"))) return st;
-  if ((st = alloc_once(c, &c.d_vpos_built, n, "alloc vdw list"))) return st;
+  if ((st = alloc_once(c, &c.d_vnnb, c.cap_n, "alloc vdw list"))) return st;
+  if ((st = alloc_once(c, &c.d_vpos_built, c.cap_n, "alloc vdw list"))) return st;
   // cells within reach: vdwcut + lbuffer, the atoms' drift since the sort
   // (below lbuffer/2 each) and the reduction shift on each side
   const double reach = c.vdw_cut + 2.0 * c.cfg.lbuffer + 2.0 * kShiftMax;
@@ -389,7 +416,7 @@ int launch_vdw_list(Ctx& c) {
   const double dr = 1.7320508075688772 * 4.0 * lmax * 5.9604644775390625e-08;
   const double band = std::max(1e-5, 2.0 * (2.0 * vbuf * dr + dr * dr) / vbuf2);
   const float lo = (float)(vbuf2 * (1.0 - band)), hi = (float)(vbuf2 * (1.0 + band));
-  k_vdw_list<<<nb, kBlock, 0, c.stream>>>(c.n, c.npad, c.box, vbuf2, prefilter, lo, hi, w[0], w[1], w[2], c.d_vred,
+  k_vdw_list<<<nb, kBlock, 0, c.stream>>>(c.n, c.maxvnb / 8, c.box, vbuf2, prefilter, lo, hi, w[0], w[1], w[2], c.d_vred,
                                           c.d_vredf, c.d_vinfo, c.d_vtab, c.vdw_nclass, c.d_scell,
                                           c.d_cell_start, c.d_cell_count, c.nc[0], c.nc[1], c.nc[2], c.maxvnb, c.d_vnnb,
                                           c.d_vnb, c.d_flags);
@@ -405,14 +432,11 @@ int launch_vdw_list(Ctx& c) {
 int launch_ehal(Ctx& c, double* d_out) {
   int st;
   if (!c.have_vdw) return THP_E_STATE;
-  const size_t n = c.n;
-  const int nb = (c.n + kBlock - 1) / kBlock;
-  if ((st = alloc_once(c, &c.d_depfix, 3 * n, "alloc gradient"))) return st;
-  if ((st = alloc_once(c, &c.d_evpart, (size_t)nb + 1, "alloc vdw partials"))) return st;
-  c.d_ev = c.d_evpart + nb;
-  unsigned long long* dev = c.d_depfix;
-  if ((st = cuda_status(cudaMemsetAsync(dev, 0, sizeof(unsigned long long) * 3 * n, c.stream), &c, "zero dev")))
-    return st;
+  if ((st = zero_gradient(c))) return st;
+  const int nbp = (c.n + 15) / 16;  // eight lanes per site, blocks of 16 sites
+  if ((st = alloc_once(c, &c.d_evpart, c.cap_n / 16 + 2, "alloc vdw partials"))) return st;
+  c.d_ev = c.d_evpart + nbp;
+  const FixAcc dev = fix_acc(c.d_depfix, c.n, c.mixed);
   if ((st = launch_vdw_list(c))) return st;
   VdwConst vc;
   const double off = c.vdw_cut, cut = c.vdw_taper;
@@ -438,24 +462,24 @@ int launch_ehal(Ctx& c, double* d_out) {
   vc.nclass = c.vdw_nclass;
   const bool vir = c.want_virial;
   double *kpart = nullptr, *vpart = nullptr, *epart = nullptr;
-  if (vir && (st = virial_scratch(c, nb, 0, &kpart, &vpart, &epart))) return st;
+  if (vir && (st = virial_scratch(c, nbp, 0, &kpart, &vpart, &epart))) return st;
 #define THP_EHAL_ARGS                                                                                             \
-  c.n, c.npad, c.box, vc, c.d_vred, c.d_vredf, c.d_vinfo, c.d_vtab, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_c, \
+  c.n, c.maxvnb / 8, c.box, vc, c.d_vred, c.d_vredf, c.d_vinfo, c.d_vtab, c.d_perm, c.d_sp_off, c.d_sp_ks, c.d_sp_c, \
       c.d_vnnb, c.d_vnb, dev, c.d_evpart, vpart
   if (c.mixed && vir)
-    k_ehal<true, true><<<nb, kBlock, 0, c.stream>>>(THP_EHAL_ARGS);
+    k_ehal<true, true><<<nbp, kBlock, 0, c.stream>>>(THP_EHAL_ARGS);
   else if (c.mixed)
-    k_ehal<true, false><<<nb, kBlock, 0, c.stream>>>(THP_EHAL_ARGS);
+    k_ehal<true, false><<<nbp, kBlock, 0, c.stream>>>(THP_EHAL_ARGS);
   else if (vir)
-    k_ehal<false, true><<<nb, kBlock, 0, c.stream>>>(THP_EHAL_ARGS);
+    k_ehal<false, true><<<nbp, kBlock, 0, c.stream>>>(THP_EHAL_ARGS);
   else
-    k_ehal<false, false><<<nb, kBlock, 0, c.stream>>>(THP_EHAL_ARGS);
+    k_ehal<false, false><<<nbp, kBlock, 0, c.stream>>>(THP_EHAL_ARGS);
 #undef THP_EHAL_ARGS
   if ((st = cuda_status(cudaGetLastError(), &c, "ehal"))) return st;
-  k_sum_partials<<<1, 256, 0, c.stream>>>(nb, c.d_evpart, c.d_ev);
+  k_sum_partials<<<1, 256, 0, c.stream>>>(nbp, c.d_evpart, c.d_ev);
   if ((st = cuda_status(cudaGetLastError(), &c, "ehal energy"))) return st;
-  if (vir && (st = virial_total(c, 0, nb, 0, kpart, vpart, epart, c.h_vvir))) return st;
-  return launch_gradient_out(c, dev, d_out);
+  if (vir && (st = virial_total(c, 0, nbp, 0, kpart, vpart, epart, c.h_vvir))) return st;
+  return launch_gradient_out(c, d_out);
 }
 
 }  // namespace thp
