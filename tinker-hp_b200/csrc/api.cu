@@ -245,18 +245,18 @@ static int prepare_list(thp_ctx* h, bool force_rebuild, bool carry, bool* rebuil
 }
 
 // E0 = direct + reciprocal + self (newinduce_pme2.f:110-148) and the matvec
-// coefficients, after the list build when `build` is set.  A system whose CG
-// rows run on the side stream runs the list build and the direct pass there
-// too, concurrent with the spread and FFTs of the permanent multipoles on the
-// main stream; the gather that completes E0 follows the join.  Returns with
-// the main stream joined, on error as well.
+// coefficients, after the list build when `build` is set.  The list build and
+// the direct pass run on the side stream, concurrent with the spread and
+// transforms of the permanent multipoles on the main stream; the gather that
+// completes E0 follows the join.  Returns with the main stream joined, on error
+// as well.
 #ifndef THP_FRONT_OVERLAP
 #define THP_FRONT_OVERLAP 1
 #endif
 
 static int launch_fields(Ctx& c, bool build) {
   int st;
-  if (!THP_FRONT_OVERLAP || !overlap_rows(c)) {
+  if (!THP_FRONT_OVERLAP) {
     if (build && (st = launch_build_list(c))) return st;
     if ((st = launch_efld0_coef(c, true))) return st;
     return launch_efld0_recip(c);
@@ -433,9 +433,9 @@ size_t footprint_bytes(const thp_config& cfg, int* ncell_out) {
   b += n * 32 + n * 16 + 2 * n * 8 + 10 * n * 8 + n * 32 + n * 64;  // sorted data
   b += n * 4 + maxnb * npad * 4;                         // list
   b += n * 4 + maxnb * npad * (4 + 2 * (mixed ? 4 : 8));  // pairs
-  b += ngrid * (mixed ? 12 : 24);                        // grid + qfac
+  b += ngrid * (mixed ? 24 : 48);                        // grid, convolved grid and two influence functions
   b += 10 * n * 6 * 8 + 4 * n * 8 + n * 6 * 4 + n * 9 * 4 + 4 * n * 6 * 4;  // vectors, FP32 row input and CG vectors
-  b += (n / 128 + 2) * 4 * 8 + 4096;
+  b += (n / 128 + 2) * 4 * 8 + 4096 + (mixed ? 0 : 72 * n);  // reductions; FP64 row records
   b += 64 << 20;  // cuFFT work area and runtime slack
   return b;
 }
@@ -576,6 +576,7 @@ static int size_buffers(Ctx& c) {
                      item(&c.d_res, 6 * n), item(&c.d_h, 6 * n), item(&c.d_pp, 6 * n), item(&c.d_zr, 6 * n),
                      item(&c.d_dip, 6 * n), item(&c.d_tmp6, 6 * n), item(&c.d_tmp6b, 6 * n), item(&c.d_cphi, 4 * n),
                      item(&c.d_vecf, 6 * n), item(&c.d_rec, 8 * n), item(&c.d_mpz, n), item(&c.d_ef_prev, 6 * n),
+                     item(&c.d_rec64, c.mixed ? 0 : 8 * n), item(&c.d_mpz64, c.mixed ? 0 : n),
                      item(&c.d_ppf, 6 * n), item(&c.d_hf, 6 * n), item(&c.d_resf, 6 * n), item(&c.d_zrf, 6 * n),
                      item(&c.d_partials, (size_t)(c.nblk_reduce + 8) * 4)},
                     "per-atom buffers");

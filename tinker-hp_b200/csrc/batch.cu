@@ -11,9 +11,10 @@
 //   1. kb_spread: pp = zr + beta pp (the 32-byte partner records of the mixed
 //      rows beside it) and the dipole spread (grid_uind_site,
 //      pmestuff.f:280-405) into the plan's grids, zeroed just before;
-//   2. the convolution: one batched cuFFT transform per grid-size class (the
-//      classes' grids lie end to end, and the classes run as parallel
-//      branches), kb_qfac over every grid, the batched inverse transforms;
+//   2. the convolution per grid-size class (the classes' grids lie end to end,
+//      and the classes run as parallel branches): three kernels over all of a
+//      class's systems (conv_dev.cuh), or, for grids those do not cover, one
+//      batched cuFFT transform, kb_qfac, the batched inverse transform;
 //   3. kb_row: real-space rows (tmatxb_pme); kb_combine: the dipole field
 //      gathered from the grid (fphi_uind_site), h, pp.h and alpha;
 //   4. kb_update: mu, residual, preconditioned residual, beta and the stop
@@ -34,6 +35,7 @@
 #include <vector>
 
 #include "cg_dev.cuh"
+#include "conv.h"
 #include "kernels.h"
 
 namespace thp {
@@ -61,6 +63,7 @@ struct BatchSys {
   double *mu, *res, *h, *zr, *pp;
   float *rec, *mpz;  // mixed form: 32-byte partner records of pp (PartnerRec)
   void* grid;  // the system's grid in the plan's class-ordered grid array
+  void* conv;  // its convolved grid (grid itself for a cuFFT class)
   const void* qfac;
   CgScalars* cg;
   double* partials;
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(kBlock) kb_row(const BatchSys* __restrict__ sy
     const int2 w = items[it];
     const BatchSys& s = sys[w.x];
     if (s.cg->stop) continue;
-    row_block<MIXED, MIXED, GPW>(w.y, s.pr, s.box, s.pos, s.posf, s.pp, nullptr, s.rec, s.mpz, s.interior, s.h);
+    row_block<MIXED, GPW>(w.y, s.pr, s.box, s.pos, s.pp, s.rec, s.mpz, s.interior, s.h);
   }
 }
 
@@ -192,8 +195,9 @@ __global__ void __launch_bounds__(kBlock) kb_combine(const BatchSys* __restrict_
     const int2 w = items[it];
     const BatchSys& s = sys[w.x];
     if (s.cg->stop) continue;
-    cg_combine_block<MIXED ? 1 : 2, double, double>(w.y, s.nblk, s.n, nullptr, s.g, s.pos, s.grid, s.pp, s.pol,
-                                                    s.ef, s.term, 0, s.h, s.res, s.zr, s.pp, s.cg, s.partials);
+    using T = typename std::conditional<MIXED, float, double>::type;
+    cg_combine8_block<T>(w.y, s.nblk_mv[0], s.n, s.g, s.pos, s.conv, s.pp, s.pol, s.ef, s.term, 0, s.h, s.res, s.zr,
+                         s.pp, s.cg, s.partials);
   }
 }
 
@@ -297,6 +301,9 @@ struct FftClass {
   int n[3] = {0, 0, 0};
   int count = 0;
   size_t offset = 0;  // first grid point of the class in the plan's array
+  size_t points = 0;  // grid points of all its systems, padding included
+  bool conv = false;  // the three-kernel convolution (else cuFFT)
+  conv::Sys* d_sys = nullptr;
   cufftHandle plan = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
@@ -315,6 +322,7 @@ struct BatchPlan {
   int2* d_qfac_items = nullptr;  // (system, chunk of grid points)
   int n_qfac_items = 0;
   void* d_grid = nullptr;        // every system's grid, class by class
+  void* d_conv = nullptr;        // the convolved grids of the three-kernel classes, at the same places
   size_t grid_bytes = 0;
   std::vector<FftClass> classes;
   unsigned* d_loops = nullptr;
@@ -344,13 +352,19 @@ struct BatchPlan {
   BatchOut* d_out = nullptr;
 };
 
-// Every class's batched transform in one direction, as parallel branches.
+// Every class's batched transform in one direction, as parallel branches; the
+// three-kernel classes run their whole convolution on the forward call.
 static int enqueue_ffts(BatchPlan& p, int dir) {
   cudaEventRecord(p.ev_fork, p.stream);
   for (FftClass& k : p.classes) {
+    if (k.conv && dir != CUFFT_FORWARD) continue;
     cudaStreamWaitEvent(k.stream, p.ev_fork, 0);
-    cufftResult r;
-    if (p.mixed) {
+    cufftResult r = CUFFT_SUCCESS;
+    if (k.conv) {
+      const cudaError_t e = p.mixed ? launch_conv32(k.n[0], conv::Sys{}, k.d_sys, k.count, 1, k.stream)
+                                    : launch_conv64(k.n[0], conv::Sys{}, k.d_sys, k.count, 1, k.stream);
+      if (e != cudaSuccess) return THP_E_CUDA;
+    } else if (p.mixed) {
       cufftComplex* g = static_cast<cufftComplex*>(p.d_grid) + k.offset;
       r = cufftExecC2C(k.plan, g, g, dir);
     } else {
@@ -373,7 +387,10 @@ static int enqueue_body(BatchPlan& p, const BatchTune& t, cudaGraphConditionalHa
     if (events) cudaEventRecord(p.prof_ev[ke++], p.stream);
   };
   mark();
-  cudaMemsetAsync(p.d_grid, 0, p.grid_bytes, p.stream);
+  // the three-kernel classes' grids are zero already
+  const size_t csz = p.mixed ? sizeof(cufftComplex) : sizeof(cufftDoubleComplex);
+  for (const FftClass& k : p.classes)
+    if (!k.conv) cudaMemsetAsync(static_cast<char*>(p.d_grid) + k.offset * csz, 0, k.points * csz, p.stream);
   if (p.mixed)
     launch_kb_spread<true>(p.stream, p.d_sys, p.d_atom_items, p.n_atom_items, ab);
   else
@@ -382,7 +399,9 @@ static int enqueue_body(BatchPlan& p, const BatchTune& t, cudaGraphConditionalHa
   if (enqueue_ffts(p, CUFFT_FORWARD)) return THP_E_CUDA;
   mark();
   const int qb = std::max(1, std::min(p.n_qfac_items, 8 * p.sms));
-  if (p.mixed)
+  if (p.n_qfac_items == 0) {
+    // every class convolves in three kernels
+  } else if (p.mixed)
     kb_qfac<float><<<qb, 256, 0, p.stream>>>(p.d_sys, p.d_qfac_items, p.n_qfac_items);
   else
     kb_qfac<double><<<qb, 256, 0, p.stream>>>(p.d_sys, p.d_qfac_items, p.n_qfac_items);
@@ -391,18 +410,19 @@ static int enqueue_body(BatchPlan& p, const BatchTune& t, cudaGraphConditionalHa
   mark();
   const int g = t.gpw - 1;
   const int mb = std::max(1, std::min(p.n_mv_items[g], 2 * t.blocks * p.sms));
+  const int cb = std::max(1, std::min(p.n_mv_items[0], 16 * p.sms));
   if (p.mixed) {
     if (t.gpw == 1)
       kb_row<true, 1><<<mb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[g], p.n_mv_items[g]);
     else
       kb_row<true, 2><<<mb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[g], p.n_mv_items[g]);
-    kb_combine<true><<<ab, kBlock, 0, p.stream>>>(p.d_sys, p.d_atom_items, p.n_atom_items);
+    kb_combine<true><<<cb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[0], p.n_mv_items[0]);
   } else {
     if (t.gpw == 1)
       kb_row<false, 1><<<mb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[g], p.n_mv_items[g]);
     else
       kb_row<false, 2><<<mb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[g], p.n_mv_items[g]);
-    kb_combine<false><<<ab, kBlock, 0, p.stream>>>(p.d_sys, p.d_atom_items, p.n_atom_items);
+    kb_combine<false><<<cb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[0], p.n_mv_items[0]);
   }
   mark();
   kb_update<<<ab, kBlock, 0, p.stream>>>(p.d_sys, p.d_atom_items, p.n_atom_items);
@@ -458,6 +478,7 @@ void batch_plan_destroy(BatchPlan* p) {
     if (kv.second) cudaGraphExecDestroy(kv.second);
   for (FftClass& k : p->classes) {
     if (k.plan) cufftDestroy(k.plan);
+    cudaFree(k.d_sys);
     if (k.stream) cudaStreamDestroy(k.stream);
     if (k.done) cudaEventDestroy(k.done);
   }
@@ -467,6 +488,7 @@ void batch_plan_destroy(BatchPlan* p) {
   for (auto& m : p->d_mv_items) cudaFree(m);
   cudaFree(p->d_qfac_items);
   cudaFree(p->d_grid);
+  cudaFree(p->d_conv);
   cudaFree(p->d_loops);
   for (auto& e : p->prof_ev)
     if (e) cudaEventDestroy(e);
@@ -544,15 +566,19 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
   size_t off = 0;
   for (FftClass& k : p->classes) {
     k.offset = off;
-    off += (size_t)k.count * slot(k);
+    k.points = (size_t)k.count * slot(k);
+    off += k.points;
+    int r1, r2;
+    k.conv = conv_covers(k.n, p->mixed, &r1, &r2);
   }
   p->grid_bytes = off * csz;
-  ok(cudaMalloc(&p->d_grid, p->grid_bytes));
+  if (ok(cudaMalloc(&p->d_grid, p->grid_bytes))) ok(cudaMemset(p->d_grid, 0, p->grid_bytes));
+  ok(cudaMalloc(&p->d_conv, p->grid_bytes));
   for (FftClass& k : p->classes) {
     const int dims[3] = {k.n[2], k.n[1], k.n[0]};
     const int dist = (int)slot(k);
     // the storage dimensions given, so that cuFFT honours the padded distance
-    if (cufftPlanMany(&k.plan, 3, const_cast<int*>(dims), const_cast<int*>(dims), 1, dist,
+    if (!k.conv && cufftPlanMany(&k.plan, 3, const_cast<int*>(dims), const_cast<int*>(dims), 1, dist,
                       const_cast<int*>(dims), 1, dist,
                       p->mixed ? CUFFT_C2C : CUFFT_Z2Z, k.count) != CUFFT_SUCCESS && !st)
       st = THP_E_CUDA;
@@ -565,6 +591,7 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     ok(cudaHostGetDevicePointer((void**)&p->d_out, p->h_out, 0));
   std::vector<BatchSys> hs(count);
   std::vector<size_t> next(p->classes.size());
+  std::vector<std::vector<conv::Sys>> csys(p->classes.size());
   for (size_t k = 0; k < p->classes.size(); ++k) next[k] = p->classes[k].offset;
   for (int q = 0; q < count; ++q) {
     Ctx& c = *cs[q];
@@ -594,6 +621,8 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     s.rec = c.d_rec;
     s.mpz = c.d_mpz;
     s.grid = static_cast<char*>(p->d_grid) + next[cls[q]] * csz;
+    s.conv = p->classes[cls[q]].conv ? static_cast<char*>(p->d_conv) + next[cls[q]] * csz : s.grid;
+    csys[cls[q]].push_back(conv::Sys{s.grid, s.conv, c.d_qfacp, c.d_cg});
     next[cls[q]] += slot(p->classes[cls[q]]);
     s.qfac = c.d_qfac;
     s.cg = c.d_cg;
@@ -602,13 +631,20 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     p->politer_max = std::max(p->politer_max, c.cfg.politer);
     p->sig.emplace_back(c.n, c.d_pp, c.d_pk, c.d_cg);
   }
+  for (size_t k = 0; k < p->classes.size(); ++k) {
+    FftClass& f = p->classes[k];
+    if (!f.conv) continue;
+    const size_t b = sizeof(conv::Sys) * csys[k].size();
+    if (ok(cudaMalloc(&f.d_sys, b))) ok(cudaMemcpy(f.d_sys, csys[k].data(), b, cudaMemcpyHostToDevice));
+  }
   // work lists, large systems first so the round-robin ends on small items
   std::vector<int> order(count);
   for (int q = 0; q < count; ++q) order[q] = q;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cs[a]->n > cs[b]->n; });
   std::vector<int2> atom_items, mv_items[2], qfac_items;
   for (int q : order) {
-    for (int b = 0; b * kQfacChunk < hs[q].ngrid; ++b) qfac_items.push_back(make_int2(q, b));
+    if (!p->classes[cls[q]].conv)
+      for (int b = 0; b * kQfacChunk < hs[q].ngrid; ++b) qfac_items.push_back(make_int2(q, b));
     for (int b = 0; b < hs[q].nblk; ++b) atom_items.push_back(make_int2(q, b));
     for (int g = 0; g < 2; ++g)
       for (int b = 0; b < hs[q].nblk_mv[g]; ++b) mv_items[g].push_back(make_int2(q, b));
@@ -619,7 +655,7 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
   ok(cudaMalloc(&p->d_atom_items, sizeof(int2) * atom_items.size()));
   ok(cudaMemcpy(p->d_atom_items, atom_items.data(), sizeof(int2) * atom_items.size(), cudaMemcpyHostToDevice));
   p->n_qfac_items = (int)qfac_items.size();
-  ok(cudaMalloc(&p->d_qfac_items, sizeof(int2) * qfac_items.size()));
+  ok(cudaMalloc(&p->d_qfac_items, sizeof(int2) * std::max<size_t>(1, qfac_items.size())));
   ok(cudaMemcpy(p->d_qfac_items, qfac_items.data(), sizeof(int2) * qfac_items.size(), cudaMemcpyHostToDevice));
   for (int g = 0; g < 2; ++g) {
     p->n_mv_items[g] = (int)mv_items[g].size();

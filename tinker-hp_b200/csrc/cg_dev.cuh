@@ -91,137 +91,45 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double* __restrict_
 }
 
 
-// h = T_real x + x/alpha + dipfield(x) - term x  (newinduce_pme2.f:398-405, 469-475)
-// init: also res = ef - h, zr = diag res, pp = zr, ggold = sum res.zr
-// iter: gg = sum pp.h, alpha = ggold / gg
-// A block covers kBlock consecutive atoms: each warp sums the rows of eight
-// groups of four atoms (group_row) into shared memory, then every thread
-// finishes its own atom.
-// REC (mixed form): partners from the 32-byte records rec / mpz (the
-// position and the dipoles of x, PartnerRec) instead of posf and xf.
-// GPW: groups of four atoms per warp; a block of kBlock threads covers
-// 16 GPW atoms (GPW = 8: one atom per thread in the combine step; smaller
-// blocks for small systems, whose few blocks would otherwise each run a long
-// chain of group rows).
-template <bool MIXED, int GATHER, bool REC = false, int GPW = 8>
-__device__ __forceinline__ void cg_matvec_block(int blk, int nblk, const PairRows& pr, const Box& box,
-                                                const double4* __restrict__ pos, const float4* __restrict__ posf,
-                                                const double* __restrict__ dipf, const PmeGeom& pg,
-                                                const void* __restrict__ grid, const double* __restrict__ x,
-                                                const float* __restrict__ xf, const float* __restrict__ rec,
-                                                const float* __restrict__ mpz, const double* __restrict__ pol,
-                                                const double* __restrict__ ef, double term, int init,
-                                                double* __restrict__ h, double* __restrict__ res,
-                                                double* __restrict__ zr, double* __restrict__ pp, CgScalars* cg,
-                                                double* __restrict__ partials, float interior) {
-  static_assert(kBlock == 128 && GPW >= 1 && GPW <= 8, "four warps, up to eight groups each");
-  constexpr int AB = 16 * GPW;  // atoms per block
-  __shared__ double srow[AB * 6];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gw = blk * 4 * GPW + warp * GPW;  // first group of this warp
-  for (int gg = 0; gg < GPW; ++gg) {
-    const int g = gw + gg;
-    if (4 * g >= pr.n) break;  // the same for every lane of the warp
-    const int t = warp * 4 * GPW + gg * 4 + (lane >> 3), j = lane & 7;
-    if (MIXED) {
-      float a32[6];
-      const Image32 im{(float)box.l[0], (float)box.l[1], (float)box.l[2]};
-      if constexpr (REC)
-        group_row<float, THP_GROW_U32, false>(pr, PartnerRec{rec, mpz}, im, g, lane, a32, interior);
-      else
-        group_row<float, THP_GROW_U32, false>(pr, Partner32{posf, xf}, im, g, lane, a32, interior);
-      if (j < 6) srow[t * 6 + j] = (double)pick6(a32, j);
+// The end of a matvec's reduction, by thread 0 of the last block: tot = r.z
+// (init, of the start) or p.h of the d and p sets.
+__device__ __forceinline__ void cg_after_matvec(const double (&tot)[2], int init, CgScalars* cg) {
+  if (init) {
+    cg->ggold[0] = tot[0];
+    cg->ggold[1] = tot[1];
+    cg->beta[0] = 0.0;
+    cg->beta[1] = 0.0;
+  } else {
+    cg->gg[0] = tot[0];
+    cg->gg[1] = tot[1];
+    if (tot[0] == 0.0 || tot[1] == 0.0) {
+      cg->stop = 1;  // newinduce_pme2.f:505 returns on gg == 0
     } else {
-      double a64[6];
-      group_row<double, THP_GROW_U64, false>(pr, Partner64{pos, x}, Image64{box}, g, lane, a64, -1.0);
-      if (j < 6) srow[t * 6 + j] = pick6(a64, j);
-    }
-  }
-  __syncthreads();
-  const int i = blk * AB + threadIdx.x;
-  double red[2] = {0.0, 0.0};
-  if (threadIdx.x < AB && i < pr.n) {
-    double acc[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) acc[q] = srow[threadIdx.x * 6 + q];
-    double dip[6], xi[6];
-    if constexpr (GATHER == 1)
-      gather_dip<float>(pg, pos[i], reinterpret_cast<const cufftComplex*>(grid), dip);
-    else if constexpr (GATHER == 2)
-      gather_dip<double>(pg, pos[i], reinterpret_cast<const cufftDoubleComplex*>(grid), dip);
-    else
-      load6(dipf + (size_t)i * 6, dip);
-    load6(x + (size_t)i * 6, xi);
-    const double p = pol[i];
-    const double ip = (p == 0.0) ? 1.0 / kTinyPol : 1.0 / p;
-    double hv[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) hv[q] = ((acc[q] + xi[q] * ip) + dip[q]) - term * xi[q];
-    store6(h + (size_t)i * 6, hv);
-    if (init) {
-      double e6[6], r6[6], z6[6];
-      load6(ef + (size_t)i * 6, e6);
-      const double dg = diag_of(p);
-#pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        r6[q] = e6[q] - hv[q];
-        z6[q] = dg * r6[q];
-      }
-      store6(res + (size_t)i * 6, r6);
-      store6(zr + (size_t)i * 6, z6);
-      store6(pp + (size_t)i * 6, z6);
-      red[0] = r6[0] * z6[0] + r6[1] * z6[1] + r6[2] * z6[2];
-      red[1] = r6[3] * z6[3] + r6[4] * z6[4] + r6[5] * z6[5];
-    } else {
-      red[0] = xi[0] * hv[0] + xi[1] * hv[1] + xi[2] * hv[2];
-      red[1] = xi[3] * hv[3] + xi[4] * hv[4] + xi[5] * hv[5];
-    }
-  }
-  __syncthreads();  // srow is reused by the block's next item
-  double tot[2];
-  if (grid_reduce_of<2>(red, partials, &cg->counter[0], blk, nblk, tot) && threadIdx.x == 0) {
-    if (init) {
-      cg->ggold[0] = tot[0];
-      cg->ggold[1] = tot[1];
-      cg->beta[0] = 0.0;
-      cg->beta[1] = 0.0;
-    } else {
-      cg->gg[0] = tot[0];
-      cg->gg[1] = tot[1];
-      if (tot[0] == 0.0 || tot[1] == 0.0) {
-        cg->stop = 1;  // newinduce_pme2.f:505 returns on gg == 0
-      } else {
-        cg->alpha[0] = cg->ggold[0] / tot[0];
-        cg->alpha[1] = cg->ggold[1] / tot[1];
-      }
+      cg->alpha[0] = cg->ggold[0] / tot[0];
+      cg->alpha[1] = cg->ggold[1] / tot[1];
     }
   }
 }
 
-
-// h = hreal + x/alpha + dipfield(x) - term x, then the reductions of
-// k_cg_matvec (init: residual, zr, pp and ggold; iter: gg and alpha).
-// GATHER 0 reads dipfield from dipf; 1 / 2 gather it here from the
-// convolved FP32 / FP64 grid (the work of k_gather_dip, without the round
-// trip of dipfield through memory).
-template <int GATHER, typename XV, typename V>
-__device__ __forceinline__ void cg_combine_block(int blk, int nblk, int n, const double* __restrict__ dipf,
-                                                 const PmeGeom& g, const double4* __restrict__ pos,
-                                                 const void* __restrict__ grid, const XV* __restrict__ x,
-                                                 const double* __restrict__ pol, const double* __restrict__ ef,
-                                                 double term, int init, V* __restrict__ h, V* __restrict__ res,
-                                                 V* __restrict__ zr, V* __restrict__ pp, CgScalars* cg,
-                                                 double* __restrict__ partials) {
+// h = hreal + x/alpha + dipfield(x) - term x  (newinduce_pme2.f:398-405,
+// 469-475), then the reductions
+// init: also res = ef - h, zr = diag res, pp = zr, ggold = sum res.zr
+// iter: gg = sum pp.h, alpha = ggold / gg
+// The dipole field is gathered here from the convolved grid, a thread per atom
+// (a shared-memory tile per 16 atoms took twice the instructions and 1.8 times
+// as long at 288,000 atoms).
+template <typename T, typename XV, typename V>
+__device__ __forceinline__ void cg_combine_block(int blk, int nblk, int n, const PmeGeom& g,
+                                                 const double4* __restrict__ pos, const void* __restrict__ grid,
+                                                 const XV* __restrict__ x, const double* __restrict__ pol,
+                                                 const double* __restrict__ ef, double term, int init,
+                                                 V* __restrict__ h, V* __restrict__ res, V* __restrict__ zr,
+                                                 V* __restrict__ pp, CgScalars* cg, double* __restrict__ partials) {
   const int i = blk * kBlock + threadIdx.x;
   double red[2] = {0.0, 0.0};
   if (i < n) {
     double acc[6], dip[6], xi[6];
-    if constexpr (GATHER == 1)
-      gather_dip<float>(g, pos[i], reinterpret_cast<const cufftComplex*>(grid), dip);
-    else if constexpr (GATHER == 2)
-      gather_dip<double>(g, pos[i], reinterpret_cast<const cufftDoubleComplex*>(grid), dip);
-    else
-      load6(dipf + (size_t)i * 6, dip);
+    gather_dip<T>(g, pos[i], reinterpret_cast<const typename Cplx<T>::type*>(grid), dip);
     load6(h + (size_t)i * 6, acc);
     load6(x + (size_t)i * 6, xi);
     const double p = pol[i];
@@ -250,32 +158,64 @@ __device__ __forceinline__ void cg_combine_block(int blk, int nblk, int n, const
     }
   }
   double tot[2];
-  if (grid_reduce_of<2>(red, partials, &cg->counter[0], blk, nblk, tot) && threadIdx.x == 0) {
+  if (grid_reduce_of<2>(red, partials, &cg->counter[0], blk, nblk, tot) && threadIdx.x == 0)
+    cg_after_matvec(tot, init, cg);
+}
+
+// The same for 16 atoms per block, eight lanes each: the lanes share an atom's
+// 25 stencil lines, then lane j < 6 finishes component j.  A thread per atom
+// walks 125 dependent grid loads, which small systems cannot hide (648 atoms
+// are six blocks).
+template <typename T>
+__device__ __forceinline__ void cg_combine8_block(int blk, int nblk, int n, const PmeGeom& g,
+                                                  const double4* __restrict__ pos, const void* __restrict__ grid,
+                                                  const double* __restrict__ x, const double* __restrict__ pol,
+                                                  const double* __restrict__ ef, double term, int init,
+                                                  double* __restrict__ h, double* __restrict__ res,
+                                                  double* __restrict__ zr, double* __restrict__ pp, CgScalars* cg,
+                                                  double* __restrict__ partials) {
+  static_assert(kBlock == 128, "16 atoms of eight lanes");
+  __shared__ SiteWeights<T> sw[16];
+  const int a = threadIdx.x >> 3, j = threadIdx.x & 7;
+  const int i0 = blk * 16 + a;
+  const bool live = i0 < n;
+  const int i = live ? i0 : n - 1;
+  if (j < 3) stage_axis<T>(g, pos[i], j, sw[a]);
+  __syncwarp();
+  double dip[6];
+  gather_dip8<T>(g, sw[a], j, reinterpret_cast<const typename Cplx<T>::type*>(grid), dip);
+  double red[2] = {0.0, 0.0};
+  if (live && j < 6) {
+    const size_t q = (size_t)i * 6 + j;
+    const double xi = x[q], p = pol[i];
+    const double ip = (p == 0.0) ? 1.0 / kTinyPol : 1.0 / p;
+    const double hv = ((h[q] + xi * ip) + pick6(dip, j)) - term * xi;
+    h[q] = hv;
+    double v;
     if (init) {
-      cg->ggold[0] = tot[0];
-      cg->ggold[1] = tot[1];
-      cg->beta[0] = 0.0;
-      cg->beta[1] = 0.0;
+      const double r = ef[q] - hv, z = diag_of(p) * r;
+      res[q] = r;
+      zr[q] = z;
+      pp[q] = z;
+      v = r * z;
     } else {
-      cg->gg[0] = tot[0];
-      cg->gg[1] = tot[1];
-      if (tot[0] == 0.0 || tot[1] == 0.0) {
-        cg->stop = 1;  // newinduce_pme2.f:505 returns on gg == 0
-      } else {
-        cg->alpha[0] = cg->ggold[0] / tot[0];
-        cg->alpha[1] = cg->ggold[1] / tot[1];
-      }
+      v = xi * hv;
     }
+    red[0] = j < 3 ? v : 0.0;
+    red[1] = j < 3 ? 0.0 : v;
   }
+  double tot[2];
+  if (grid_reduce_of<2>(red, partials, &cg->counter[0], blk, nblk, tot) && threadIdx.x == 0)
+    cg_after_matvec(tot, init, cg);
 }
 
 // The real-space rows T_real x of the atoms of block blk (16 GPW atoms:
 // four warps of GPW groups of four), hreal[i][6] in FP64; lane j < 6 of an
-// atom writes component j.  Partners as in cg_matvec_block.
-template <bool MIXED, bool REC, int GPW>
+// atom writes component j.  Mixed form: partners from the 32-byte records rec /
+// mpz (the position and the dipoles of x).
+template <bool MIXED, int GPW>
 __device__ __forceinline__ void row_block(int blk, const PairRows& pr, const Box& box,
-                                          const double4* __restrict__ pos, const float4* __restrict__ posf,
-                                          const double* __restrict__ x, const float* __restrict__ xf,
+                                          const double4* __restrict__ pos, const double* __restrict__ x,
                                           const float* __restrict__ rec, const float* __restrict__ mpz,
                                           float interior, double* __restrict__ hreal) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -287,10 +227,7 @@ __device__ __forceinline__ void row_block(int blk, const PairRows& pr, const Box
     if (MIXED) {
       float a32[6];
       const Image32 im{(float)box.l[0], (float)box.l[1], (float)box.l[2]};
-      if constexpr (REC)
-        group_row<float, THP_GROW_U32, false>(pr, PartnerRec{rec, mpz}, im, g, lane, a32, interior);
-      else
-        group_row<float, THP_GROW_U32, false>(pr, Partner32{posf, xf}, im, g, lane, a32, interior);
+      group_row<float, THP_GROW_U32, false>(pr, PartnerRec{rec, mpz}, im, g, lane, a32, interior);
       if (j < 6 && i < pr.n) hreal[(size_t)i * 6 + j] = (double)pick6(a32, j);
     } else {
       double a64[6];
@@ -304,8 +241,9 @@ __device__ __forceinline__ void row_block(int blk, const PairRows& pr, const Box
 // diagnostic printed at each step) is formed once, after the loop, from the
 // final mu and residual (k_epol / kb_finish): the same value the last
 // iteration would give, without reading E0 on every iteration.
+// Returns true in thread 0 of the block that finished the reduction.
 template <typename V>
-__device__ __forceinline__ void cg_update_block(int blk, int nblk, int n, const double* __restrict__ pol,
+__device__ __forceinline__ bool cg_update_block(int blk, int nblk, int n, const double* __restrict__ pol,
                                                 const V* __restrict__ h, const V* __restrict__ pp,
                                                 double* __restrict__ mu, V* __restrict__ res, V* __restrict__ zr,
                                                 CgScalars* cg, double* __restrict__ partials, double poleps,
@@ -334,7 +272,8 @@ __device__ __forceinline__ void cg_update_block(int blk, int nblk, int n, const 
     for (int q = 0; q < 6; ++q) red[q < 3 ? 0 : 1] += r6[q] * z6[q];
   }
   double tot[2];
-  if (grid_reduce_of<2>(red, partials, &cg->counter[1], blk, nblk, tot) && threadIdx.x == 0) {
+  const bool last = grid_reduce_of<2>(red, partials, &cg->counter[1], blk, nblk, tot) && threadIdx.x == 0;
+  if (last) {
     const double nrm = (double)(3 * n);
     double resnrm = 0.0;
     bool bad = false;
@@ -358,6 +297,7 @@ __device__ __forceinline__ void cg_update_block(int blk, int nblk, int n, const 
       cg->stop = 1;
     }
   }
+  return last;
 }
 
 

@@ -162,6 +162,16 @@ struct Ctx {
   size_t cap_ngrid = 0;
   void* d_grid = nullptr;  // cufftDoubleComplex or cufftComplex
   void* d_qfac = nullptr;  // double or float
+  // cubic grids of the lengths of conv_dev.cuh convolve in three kernels
+  // (conv 1): d_grid is spread into and always zero between convolutions, the
+  // convolved potential is in d_conv, the influence function in the
+  // convolution's x order in d_qfacp.  Other grids (conv 0) use cuFFT in place:
+  // d_conv is d_grid, zeroed before each spread.
+  int conv = 0;
+  int conv_r[2] = {0, 0};        // the grid length's factors
+  void* d_conv = nullptr;
+  void* d_conv_buf = nullptr;
+  void* d_qfacp = nullptr;
   double a_frac[3] = {0, 0, 0};  // nfft_d * recip(d,d)
 
   // CG vectors, sorted order, [n][6] = (d xyz, p xyz)
@@ -181,6 +191,9 @@ struct Ctx {
   double* d_ef_prev = nullptr;  // [n][6]
   bool have_ef_prev = false;
   float* d_mpz = nullptr;     // [n]
+  // the same of the FP64 form: {x, y, z (wrapped), d dipole, p dipole x, y} and p dipole z
+  double* d_rec64 = nullptr;  // [n][8]
+  double* d_mpz64 = nullptr;  // [n]
   // the mixed form's overlapped CG keeps its search direction, h, residual
   // and preconditioned residual in FP32 (dot products and scalars in FP64)
   float *d_ppf = nullptr, *d_hf = nullptr, *d_resf = nullptr, *d_zrf = nullptr;  // [n][6]

@@ -645,9 +645,9 @@ int launch_fphi_mpole20(Ctx& c) {
   const int nb = (c.n + kBlock - 1) / kBlock;
   PmeGeom g = pme_geom(c);
   if (c.mixed)
-    k_fphi_mpole20<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_grid, c.d_fphirec);
+    k_fphi_mpole20<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_conv, c.d_fphirec);
   else
-    k_fphi_mpole20<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_grid,
+    k_fphi_mpole20<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_conv,
                                                         c.d_fphirec);
   return cuda_status(cudaGetLastError(), &c, "fphi mpole");
 }
@@ -733,16 +733,16 @@ int launch_forces(Ctx& c, double* d_out) {
   // dipole grid of uind (Re) / uinp (Im), convolved
   if ((st = launch_pme_dipole(c, c.d_mu, nullptr, 0))) return st;
   if (c.mixed && vir)
-    k_force_recip<float, true><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_grid,
+    k_force_recip<float, true><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_conv,
                                                             c.d_fphirec, c.d_mu, c.d_rpole, c.d_trq, dep, rpart);
   else if (c.mixed)
-    k_force_recip<float, false><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_grid,
+    k_force_recip<float, false><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_conv,
                                                              c.d_fphirec, c.d_mu, c.d_rpole, c.d_trq, dep, rpart);
   else if (vir)
-    k_force_recip<double, true><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_grid,
+    k_force_recip<double, true><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_conv,
                                                              c.d_fphirec, c.d_mu, c.d_rpole, c.d_trq, dep, rpart);
   else
-    k_force_recip<double, false><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_grid,
+    k_force_recip<double, false><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_conv,
                                                               c.d_fphirec, c.d_mu, c.d_rpole, c.d_trq, dep, rpart);
   if ((st = cuda_status(cudaGetLastError(), &c, "force recip"))) return st;
   // (rpole + uinp) x (rpole + uind) k-space virial: the grid is free again

@@ -32,12 +32,16 @@ int launch_mpole_grid_virial(Ctx& c, double* d_part, double sign);
 int launch_pair_grid_virial(Ctx& c, double* d_part);   // (rpole+uinp) x (rpole+uind) k-space virial
 int kspace_virial_blocks();
 int launch_gather_mpole(Ctx& c, double* cphi10, bool with_e0);  // cphi from the convolved grid, E0 completion
-int launch_pme_dipole_f32(Ctx& c, const float* d_vec);  // mode-2 spread of an FP32 vector + convolution
+// dipole spread and convolution of an FP32 / FP64 vector (check_stop: skipped once the CG has stopped);
+// d_out: also the gathered field
+int launch_pme_dipole_f32(Ctx& c, const float* d_vec, int check_stop);
+int launch_pme_dipole(Ctx& c, const double* d_vec, double* d_out, int check_stop);
+int launch_spread_small(Ctx& c, double* d_vec, int update);  // the small systems' CG spread, without convolution
+int launch_convolve(Ctx& c, int check_stop);
 bool overlap_rows(const Ctx& c);  // the system runs real-space passes on the side stream
-int zero_grid(Ctx& c);
+int zero_grid(Ctx& c);  // before a spread: d_grid zero (nothing to do for the three-kernel convolution)
 struct PmeGeom;
 PmeGeom pme_geom(const Ctx& c);
-int launch_pme_dipole(Ctx& c, const double* d_vec, double* d_out, int mode);
 int launch_gather_dip(Ctx& c, double* d_out, bool check_stop);
 
 // forces.cu

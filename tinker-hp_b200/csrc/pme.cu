@@ -13,6 +13,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "conv.h"
 #include "kernels.h"
 #include "pme_dev.cuh"
 
@@ -68,6 +69,38 @@ __global__ void k_spread_mpole(int n, PmeGeom g, const double4* __restrict__ pos
       }
     }
   }
+}
+
+// The same with a warp per site, lane l < 25 on stencil line (y, z) =
+// (l % 5, l / 5), for systems too small to fill the GPU with a thread per site.
+template <typename T>
+__global__ void __launch_bounds__(128) k_spread_mpole_small(int n, PmeGeom g, const double4* __restrict__ pos,
+                                                            const double* __restrict__ rp,
+                                                            typename Cplx<T>::type* __restrict__ grid) {
+  __shared__ SiteWeights<T, 3> sw[4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 4 + warp;
+  if (i >= n) return;  // the same for the whole warp
+  SiteWeights<T, 3>& s = sw[warp];
+  if (lane >= 29) stage_axis<T, 3>(g, pos[i], lane - 29, s);
+  const double* r = rp + (size_t)i * 10;
+  const T f0 = (T)r[0], f1 = (T)(g.a[0] * r[1]), f2 = (T)(g.a[1] * r[2]), f3 = (T)(g.a[2] * r[3]);
+  const T f4 = (T)(g.a[0] * g.a[0] * r[4]), f5 = (T)(g.a[1] * g.a[1] * r[7]), f6 = (T)(g.a[2] * g.a[2] * r[9]);
+  const T f7 = (T)(g.a[0] * g.a[1] * (2.0 * r[5])), f8 = (T)(g.a[0] * g.a[2] * (2.0 * r[6])),
+          f9 = (T)(g.a[1] * g.a[2] * (2.0 * r[8]));
+  __syncwarp();
+  if (lane >= kBs * kBs) return;
+  const int b = lane % kBs, c = lane / kBs;
+  const T u0 = s.w[1][3 * b], u1 = s.w[1][3 * b + 1], u2 = s.w[1][3 * b + 2];
+  const T v0 = s.w[2][3 * c], v1 = s.w[2][3 * c + 1], v2 = s.w[2][3 * c + 2];
+  const T term0 = f0 * u0 * v0 + f2 * u1 * v0 + f3 * u0 * v1 + f5 * u2 * v0 + f6 * u0 * v2 + f9 * u1 * v1;
+  const T term1 = f1 * u0 * v0 + f7 * u1 * v0 + f8 * u0 * v1;
+  const T term2 = f4 * u0 * v0;
+  const size_t row = ((size_t)wrapk(s.g0[2] + c, g.n3) * g.n2 + wrapk(s.g0[1] + b, g.n2)) * g.n1;
+#pragma unroll
+  for (int a = 0; a < kBs; ++a)
+    grid_add_re(grid, row + wrapk(s.g0[0] + a, g.n1),
+                term0 * s.w[0][3 * a] + term1 * s.w[0][3 * a + 1] + term2 * s.w[0][3 * a + 2]);
 }
 
 // grid_mpole_site for the two multipole sets of eprecip1's virial
@@ -174,12 +207,9 @@ __global__ void __launch_bounds__(256) k_kspace_virial(int n1, int n2, int n3, c
     for (int q = 0; q < 6; ++q) part[(size_t)blockIdx.x * 6 + q] = sign * v[q];
 }
 
-// The vector a site spreads: vec[i] (mode 1: zr + beta vec, written back),
-// with the FP32 copy in vecf when given.
+// The vector a site spreads.
 template <typename V>
-__device__ __forceinline__ void spread_load(int i, V* __restrict__ vec, const double* __restrict__ zr,
-                                            float* __restrict__ vecf, const CgScalars* __restrict__ cg, int mode,
-                                            double (&v)[6]) {
+__device__ __forceinline__ void spread_load(int i, const V* __restrict__ vec, double (&v)[6]) {
   if constexpr (std::is_same<V, float>::value) {
     const float2* v2 = reinterpret_cast<const float2*>(vec + (size_t)i * 6);
     const float2 a0 = v2[0], a1 = v2[1], a2 = v2[2];
@@ -189,29 +219,6 @@ __device__ __forceinline__ void spread_load(int i, V* __restrict__ vec, const do
     double2 a0 = v2[0], a1 = v2[1], a2 = v2[2];
     v[0] = a0.x; v[1] = a0.y; v[2] = a1.x; v[3] = a1.y; v[4] = a2.x; v[5] = a2.y;
   }
-  if constexpr (std::is_same<V, double>::value) {
-    if (mode == 1) {
-      const double2* z2 = reinterpret_cast<const double2*>(zr + (size_t)i * 6);
-      double2 b0 = z2[0], b1 = z2[1], b2 = z2[2];
-      double bd = cg->beta[0], bp = cg->beta[1];
-      v[0] = b0.x + bd * v[0];
-      v[1] = b0.y + bd * v[1];
-      v[2] = b1.x + bd * v[2];
-      v[3] = b1.y + bp * v[3];
-      v[4] = b2.x + bp * v[4];
-      v[5] = b2.y + bp * v[5];
-      double2* w2 = reinterpret_cast<double2*>(vec + (size_t)i * 6);
-      w2[0] = make_double2(v[0], v[1]);
-      w2[1] = make_double2(v[2], v[3]);
-      w2[2] = make_double2(v[4], v[5]);
-    }
-  }
-  if (vecf) {
-    float2* o = reinterpret_cast<float2*>(vecf + (size_t)i * 6);
-    o[0] = make_float2((float)v[0], (float)v[1]);
-    o[1] = make_float2((float)v[2], (float)v[3]);
-    o[2] = make_float2((float)v[4], (float)v[5]);
-  }
 }
 
 // grid_uind_site (pmestuff.f:280-405); d dipoles in Re, p dipoles in Im.
@@ -220,16 +227,13 @@ __device__ __forceinline__ void spread_load(int i, V* __restrict__ vec, const do
 // 1.6x slower); TA = 16: the warp sums the stencils of 16 neighbouring sites
 // at a time in a shared-memory tile first (spread_dip_warp), blocks of
 // kSpreadThreads threads with one SpreadWarp<T> per warp in dynamic shared
-// memory.  mode 1 first forms pp = zr + beta*pp (inducepcg_pme2.f:553-559) and
-// writes it back.
-// V: the stored type of vec (FP32 for the mixed form's overlapped CG, which
-// spreads in mode 2 only)
+// memory.
+// V: the stored type of vec (FP32 for the mixed form's overlapped CG)
 template <typename T, typename V = double, int TA = 0>
 __global__ void __launch_bounds__(128) k_spread_dip(int n, PmeGeom g, const double4* __restrict__ pos,
-                                                   V* __restrict__ vec, const double* __restrict__ zr,
-                                                   float* __restrict__ vecf, const CgScalars* __restrict__ cg,
-                                                   int mode, typename Cplx<T>::type* __restrict__ grid) {
-  if (mode >= 1 && cg->stop) return;
+                                                   const V* __restrict__ vec, const CgScalars* __restrict__ cg,
+                                                   int check_stop, typename Cplx<T>::type* __restrict__ grid) {
+  if (check_stop && cg->stop) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   SpreadWarp<T>* sw = nullptr;
   if constexpr (TA > 0) {
@@ -243,13 +247,60 @@ __global__ void __launch_bounds__(128) k_spread_dip(int n, PmeGeom g, const doub
   double v[6] = {0, 0, 0, 0, 0, 0};
   double4 pi = make_double4(0, 0, 0, 0);
   if (live) {
-    spread_load(i, vec, zr, vecf, cg, mode, v);
+    spread_load(i, vec, v);
     pi = pos[i];
   }
   if constexpr (TA > 0)
     spread_dip_warp<T>(g, pi, v, live, grid, *sw);
   else
     spread_dip_site<T>(g, pi, v, grid);
+}
+
+// The same with a warp per site, for systems too small to fill the GPU with a
+// thread per site: the lanes share the site's 25 stencil lines (648 atoms: 16.9
+// -> 4.4 us FP64, 9,003 atoms 15.2 -> 11.2 us FP32).  update: first pp = zr + beta pp
+// (inducepcg_pme2.f:553-559), written back.  rec (mixed form): the 32-byte
+// partner records of vec the real-space rows read (wrapped FP32 position, d
+// dipole, p dipole x, y; the p dipole z in mpz).
+template <typename T>
+__global__ void __launch_bounds__(128) k_spread_dip_small(int n, PmeGeom g, const double4* __restrict__ pos,
+                                                          double* __restrict__ vec, const double* __restrict__ zr,
+                                                          const CgScalars* __restrict__ cg, int check_stop, int update,
+                                                          const float4* __restrict__ posf, float* __restrict__ rec,
+                                                          float* __restrict__ mpz,
+                                                          typename Cplx<T>::type* __restrict__ grid) {
+  __shared__ SiteWeights<T> sw[4];
+  if (check_stop && cg->stop) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 4 + warp;
+  if (i >= n) return;  // the same for the whole warp
+  double v = 0.0;
+  if (lane < 6) {
+    const size_t q = (size_t)i * 6 + lane;
+    v = vec[q];
+    if (update) {
+      v = zr[q] + cg->beta[lane < 3 ? 0 : 1] * v;
+      vec[q] = v;
+    }
+    if (rec) {
+      if (lane < 5)
+        rec[(size_t)i * 8 + 3 + lane] = (float)v;
+      else
+        mpz[i] = (float)v;
+    }
+  } else if (lane < 9 && rec) {
+    const float4 p = posf[i];
+    rec[(size_t)i * 8 + (lane - 6)] = lane == 6 ? p.x : (lane == 7 ? p.y : p.z);
+  }
+  if (lane >= 29) stage_axis<T>(g, pos[i], lane - 29, sw[warp]);
+  __syncwarp();
+  T fd[3], fp[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    fd[d] = (T)(g.a[d] * __shfl_sync(0xffffffffu, v, d));
+    fp[d] = (T)(g.a[d] * __shfl_sync(0xffffffffu, v, 3 + d));
+  }
+  spread_dip_lines<T>(g, sw[warp], lane, fd, fp, grid);
 }
 
 template <typename C, typename T>
@@ -436,12 +487,15 @@ PmeGeom geom_of(const Ctx& c) {
   return g;
 }
 
+// cuFFT of the whole grid: forward in place, inverse into d_conv (d_grid
+// itself without the three-kernel convolution)
 int fft(Ctx& c, int dir) {
   cufftResult r;
+  void* out = dir == CUFFT_FORWARD ? c.d_grid : c.d_conv;
   if (c.mixed)
-    r = cufftExecC2C(c.plan, (cufftComplex*)c.d_grid, (cufftComplex*)c.d_grid, dir);
+    r = cufftExecC2C(c.plan, (cufftComplex*)c.d_grid, (cufftComplex*)out, dir);
   else
-    r = cufftExecZ2Z(c.plan, (cufftDoubleComplex*)c.d_grid, (cufftDoubleComplex*)c.d_grid, dir);
+    r = cufftExecZ2Z(c.plan, (cufftDoubleComplex*)c.d_grid, (cufftDoubleComplex*)out, dir);
   if (r != CUFFT_SUCCESS) {
     c.last_msg = "cuFFT exec failed";
     return THP_E_CUDA;
@@ -449,7 +503,17 @@ int fft(Ctx& c, int dir) {
   return THP_OK;
 }
 
+// d_grid -> d_conv: forward transform, influence function, inverse
+// transform.  Three kernels where the grid allows (at 120^3: 73 -> 38 us FP32,
+// 98 -> 53 us FP64 against cuFFT's six launches and the product; 60^3 34 -> 15 us), else
+// cuFFT.
 int convolve(Ctx& c, int check_stop) {
+  if (c.conv) {
+    const conv::Sys s{c.d_grid, c.d_conv, c.d_qfacp, c.d_cg};
+    const cudaError_t e = c.mixed ? launch_conv32(c.nfft[0], s, nullptr, 1, check_stop, c.stream)
+                                  : launch_conv64(c.nfft[0], s, nullptr, 1, check_stop, c.stream);
+    return cuda_status(e, &c, "convolution");
+  }
   int st = fft(c, CUFFT_FORWARD);
   if (st) return st;
   int blocks = 148 * 8;
@@ -509,9 +573,11 @@ bool plan_cached(const PlanKey& k) {
 
 // qfac(k) = exp(-pi^2 h^2 / a^2) / (pi V h^2 bsmod1 bsmod2 bsmod3), zero at
 // h = 0 and where the exponent is below -50 (newinduce_pme.f:1802-1854)
+// qp (optional): the same values with each row in the x order of the
+// three-kernel convolution for the factors f1 x f2 of n1.
 template <typename T>
 __global__ void k_qfac_init(int n1, int n2, int n3, const double* __restrict__ bsm, double r1, double r2, double r3,
-                            double pterm, double volterm, T* __restrict__ q) {
+                            double pterm, double volterm, int f1, int f2, T* __restrict__ q, T* __restrict__ qp) {
   const size_t ng = (size_t)n1 * n2 * n3;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < ng; t += (size_t)gridDim.x * blockDim.x) {
     const int k1 = (int)(t % n1), k2 = (int)((t / n1) % n2), k3 = (int)(t / ((size_t)n1 * n2));
@@ -526,10 +592,16 @@ __global__ void k_qfac_init(int n1, int n2, int n3, const double* __restrict__ b
       if (term > -50.0) v = exp(term) / (volterm * hsq * bsm[k1] * bsm[n1 + k2] * bsm[n1 + n2 + k3]);
     }
     q[t] = (T)v;
+    if (qp) qp[t - k1 + f2 * (k1 % f1) + k1 / f1] = (T)v;
   }
 }
 
 }  // namespace
+
+bool conv_covers(const int n[3], int mixed, int* r1, int* r2) {
+  if (n[0] != n[1] || n[1] != n[2]) return false;
+  return mixed ? conv_split32(n[0], r1, r2) : conv_split64(n[0], r1, r2);
+}
 
 // B-spline moduli by grid length, computed once per process (an O(K^2)
 // trigonometric sum per axis; servers re-target contexts to new grids often)
@@ -555,14 +627,20 @@ int pme_init(Ctx& c) {
   // grid buffers are kept while they are large enough (a re-targeted
   // context reuses them)
   if (c.ngrid > c.cap_ngrid) {
-    cudaFree(c.d_qfac);
-    cudaFree(c.d_grid);
-    c.d_qfac = c.d_grid = nullptr;
+    for (void** p : {&c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf}) {
+      cudaFree(*p);
+      *p = nullptr;
+    }
     c.cap_ngrid = 0;
     if (cuda_status(cudaMalloc(&c.d_qfac, esz * c.ngrid), &c, "alloc qfac")) return THP_E_CUDA;
     if (cuda_status(cudaMalloc(&c.d_grid, csz * c.ngrid), &c, "alloc grid")) return THP_E_CUDA;
+    if (cuda_status(cudaMalloc(&c.d_qfacp, esz * c.ngrid), &c, "alloc qfac")) return THP_E_CUDA;
+    if (cuda_status(cudaMalloc(&c.d_conv_buf, csz * c.ngrid), &c, "alloc grid")) return THP_E_CUDA;
     c.cap_ngrid = c.ngrid;
   }
+  c.conv_r[0] = c.conv_r[1] = 1;
+  c.conv = conv_covers(c.nfft, c.mixed, &c.conv_r[0], &c.conv_r[1]) ? 1 : 0;
+  c.d_conv = c.conv ? c.d_conv_buf : c.d_grid;
   // influence function on the device (newinduce_pme.f:1802-1854): the
   // B-spline moduli go through the front of the grid buffer
   std::vector<double> bsm(m1.begin() + 1, m1.begin() + 1 + c.nfft[0]);
@@ -576,12 +654,16 @@ int pme_init(Ctx& c) {
   const int blocks = (int)std::min<size_t>((c.ngrid + 255) / 256, 148 * 16);
   if (c.mixed)
     k_qfac_init<float><<<blocks, 256, 0, c.stream>>>(c.nfft[0], c.nfft[1], c.nfft[2], d_bsm, c.box.recip[0],
-                                                     c.box.recip[1], c.box.recip[2], pterm, volterm,
-                                                     (float*)c.d_qfac);
+                                                     c.box.recip[1], c.box.recip[2], pterm, volterm, c.conv_r[0],
+                                                     c.conv_r[1], (float*)c.d_qfac,
+                                                     c.conv ? (float*)c.d_qfacp : nullptr);
   else
     k_qfac_init<double><<<blocks, 256, 0, c.stream>>>(c.nfft[0], c.nfft[1], c.nfft[2], d_bsm, c.box.recip[0],
-                                                      c.box.recip[1], c.box.recip[2], pterm, volterm,
-                                                      (double*)c.d_qfac);
+                                                      c.box.recip[1], c.box.recip[2], pterm, volterm, c.conv_r[0],
+                                                      c.conv_r[1], (double*)c.d_qfac,
+                                                      c.conv ? (double*)c.d_qfacp : nullptr);
+  // the spread grid is zero from here on between convolutions
+  if (c.conv) cudaMemsetAsync(c.d_grid, 0, csz * c.ngrid, c.stream);
   // no host wait: the influence function is ready, stream-ordered, for the
   // context's next solve (bsm is copied out before the call returns)
   if (cuda_status(cudaGetLastError(), &c, "qfac")) return THP_E_CUDA;
@@ -622,29 +704,51 @@ int plan_prefetch(int device, const int nfft[3], int mixed) {
 void pme_free(Ctx& c) {
   if (c.have_plan) give_plan(plan_key(c), c.plan);
   c.have_plan = false;
-  cudaFree(c.d_qfac);
-  cudaFree(c.d_grid);
-  c.d_qfac = c.d_grid = nullptr;
+  for (void** p : {&c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf}) {
+    cudaFree(*p);
+    *p = nullptr;
+  }
+  c.d_conv = nullptr;
   c.cap_ngrid = 0;
 }
 
-int zero_grid(Ctx& c) {
+// d_grid to zero: what cuFFT's transforms in place leave has to go before
+// the next spread; the three-kernel convolution zeroes what it reads
+static int clear_grid(Ctx& c) {
   size_t csz = c.mixed ? sizeof(cufftComplex) : sizeof(cufftDoubleComplex);
   return cuda_status(cudaMemsetAsync(c.d_grid, 0, csz * c.ngrid, c.stream), &c, "zero grid");
+}
+
+int zero_grid(Ctx& c) { return c.conv ? THP_OK : clear_grid(c); }
+
+// systems below this many atoms spread with a warp per site
+#ifndef THP_SPREAD_WARP_ATOMS
+#define THP_SPREAD_WARP_ATOMS 20000
+#endif
+
+static int spread_mpole(Ctx& c, const PmeGeom& g) {
+  const bool small = c.n < THP_SPREAD_WARP_ATOMS;
+  const int nb = small ? (c.n + 3) / 4 : (c.n + kBlock - 1) / kBlock;
+  cufftComplex* gf = (cufftComplex*)c.d_grid;
+  cufftDoubleComplex* gd = (cufftDoubleComplex*)c.d_grid;
+  if (c.mixed && small)
+    k_spread_mpole_small<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, gf);
+  else if (c.mixed)
+    k_spread_mpole<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, gf);
+  else if (small)
+    k_spread_mpole_small<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, gd);
+  else
+    k_spread_mpole<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, gd);
+  return cuda_status(cudaGetLastError(), &c, "spread mpole");
 }
 
 // Permanent-multipole PME: d_cphi (and cphi10 when non-null) and, when
 // with_e0, completes d_ef = E_direct - cphi(2:4) + (4/3) a^3/sqrt(pi) d.
 int launch_mpole_grid(Ctx& c) {
   PmeGeom g = geom_of(c);
-  int nb = (c.n + kBlock - 1) / kBlock;
   int st = zero_grid(c);
   if (st) return st;
-  if (c.mixed)
-    k_spread_mpole<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, (cufftComplex*)c.d_grid);
-  else
-    k_spread_mpole<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, (cufftDoubleComplex*)c.d_grid);
-  if ((st = cuda_status(cudaGetLastError(), &c, "spread mpole"))) return st;
+  if ((st = spread_mpole(c, g))) return st;
   return convolve(c, 0);
 }
 
@@ -670,14 +774,9 @@ static int kspace_virial(Ctx& c, int mode, double sign, double* d_part) {
 // (epolar1.f:534-541): kspace_virial_blocks() rows of 6 into d_part.
 int launch_mpole_grid_virial(Ctx& c, double* d_part, double sign) {
   PmeGeom g = geom_of(c);
-  int nb = (c.n + kBlock - 1) / kBlock;
   int st = zero_grid(c);
   if (st) return st;
-  if (c.mixed)
-    k_spread_mpole<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, (cufftComplex*)c.d_grid);
-  else
-    k_spread_mpole<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, (cufftDoubleComplex*)c.d_grid);
-  if ((st = cuda_status(cudaGetLastError(), &c, "spread mpole"))) return st;
+  if ((st = spread_mpole(c, g))) return st;
   if ((st = fft(c, CUFFT_FORWARD))) return st;
   if ((st = kspace_virial(c, 0, sign, d_part))) return st;
   int blocks = 148 * 8;
@@ -688,7 +787,8 @@ int launch_mpole_grid_virial(Ctx& c, double* d_part, double sign) {
     k_qfac<cufftDoubleComplex, double><<<blocks, 256, 0, c.stream>>>(
         c.ngrid, (const double*)c.d_qfac, (cufftDoubleComplex*)c.d_grid, c.d_cg, 0);
   if ((st = cuda_status(cudaGetLastError(), &c, "qfac"))) return st;
-  return fft(c, CUFFT_INVERSE);
+  if ((st = fft(c, CUFFT_INVERSE))) return st;
+  return c.conv ? clear_grid(c) : THP_OK;
 }
 
 // The (rpole + uinp) x (rpole + uind) scalar-sum virial of eprecip1
@@ -706,7 +806,8 @@ int launch_pair_grid_virial(Ctx& c, double* d_part) {
                                                          (cufftDoubleComplex*)c.d_grid);
   if ((st = cuda_status(cudaGetLastError(), &c, "spread mpole pair"))) return st;
   if ((st = fft(c, CUFFT_FORWARD))) return st;
-  return kspace_virial(c, 1, 1.0, d_part);
+  if ((st = kspace_virial(c, 1, 1.0, d_part))) return st;
+  return c.conv ? clear_grid(c) : THP_OK;
 }
 
 int launch_efld0_recip_ex(Ctx& c, double* cphi10, bool with_e0) {
@@ -721,10 +822,10 @@ int launch_gather_mpole(Ctx& c, double* cphi10, bool with_e0) {
   double a = c.cfg.aewald;
   double term = (4.0 / 3.0) * a * a * a / kSqrtPi;
   if (c.mixed)
-    k_gather_mpole<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_grid, c.d_rpole,
+    k_gather_mpole<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_conv, c.d_rpole,
                                                        term, c.d_cphi, cphi10, with_e0 ? c.d_ef : nullptr);
   else
-    k_gather_mpole<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_grid,
+    k_gather_mpole<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_conv,
                                                         c.d_rpole, term, c.d_cphi, cphi10,
                                                         with_e0 ? c.d_ef : nullptr);
   return cuda_status(cudaGetLastError(), &c, "gather mpole");
@@ -732,11 +833,6 @@ int launch_gather_mpole(Ctx& c, double* cphi10, bool with_e0) {
 
 int launch_efld0_recip(Ctx& c) { return launch_efld0_recip_ex(c, nullptr, true); }
 
-// Dipole PME pass.  mode 0: spread d_vec as is (the mixed form also writes
-// its FP32 copy); mode 1: pp update first (CG loop, honours the stop flag);
-// mode 2: spread as is, no FP32 copy, honours the stop flag.  d_out (if non-null) receives the gathered
-// field gradient [n][6] (tmatxbrecip's dipfield); the CG loop passes null and
-// gathers inside its fused matvec kernel.
 // 1: the dipole spread of systems of at least THP_SPREAD_TILE_ATOMS (FP32
 // grid) / THP_SPREAD_TILE_ATOMS_F64 atoms sums the stencils of 16
 // neighbouring sites in a shared-memory tile per warp before adding them to
@@ -755,59 +851,88 @@ int launch_efld0_recip(Ctx& c) { return launch_efld0_recip_ex(c, nullptr, true);
 #endif
 
 template <typename T, typename V, int TA>
-static void spread_tiled(Ctx& c, const PmeGeom& g, V* vec, float* vf, int mode, typename Cplx<T>::type* grid) {
+static void spread_tiled(Ctx& c, const PmeGeom& g, const V* vec, int check_stop, typename Cplx<T>::type* grid) {
   constexpr size_t smem = sizeof(SpreadWarp<T>) * (kSpreadThreads / 32);
   static std::atomic<unsigned long long> limit_set{0};
   smem_limit_once(k_spread_dip<T, V, TA>, smem, limit_set);
   const int nb = (c.n + kSpreadThreads - 1) / kSpreadThreads;
-  k_spread_dip<T, V, TA><<<nb, kSpreadThreads, smem, c.stream>>>(c.n, g, c.d_pos, vec, c.d_zr, vf, c.d_cg, mode,
-                                                                  grid);
+  k_spread_dip<T, V, TA><<<nb, kSpreadThreads, smem, c.stream>>>(c.n, g, c.d_pos, vec, c.d_cg, check_stop, grid);
 }
 
 template <typename T, typename V>
-static void spread_dipoles(Ctx& c, const PmeGeom& g, V* vec, float* vf, int mode, typename Cplx<T>::type* grid) {
+static void spread_dipoles(Ctx& c, const PmeGeom& g, const V* vec, int check_stop, typename Cplx<T>::type* grid) {
   constexpr int kMin = std::is_same<T, float>::value ? THP_SPREAD_TILE_ATOMS : THP_SPREAD_TILE_ATOMS_F64;
-  if (THP_SPREAD_TILE && c.n >= kMin)
-    spread_tiled<T, V, 16>(c, g, vec, vf, mode, grid);
-  else
-    k_spread_dip<T, V, 0><<<(c.n + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, vec, c.d_zr, vf,
-                                                                             c.d_cg, mode, grid);
+  if (THP_SPREAD_TILE && c.n >= kMin) {
+    spread_tiled<T, V, 16>(c, g, vec, check_stop, grid);
+  } else if constexpr (std::is_same<V, double>::value) {
+    if (c.n < THP_SPREAD_WARP_ATOMS) {
+      k_spread_dip_small<T><<<(c.n + 3) / 4, 128, 0, c.stream>>>(c.n, g, c.d_pos, const_cast<double*>(vec), nullptr,
+                                                                c.d_cg, check_stop, 0, nullptr, nullptr, nullptr, grid);
+      return;
+    }
+    k_spread_dip<T, V, 0><<<(c.n + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, vec, c.d_cg,
+                                                                               check_stop, grid);
+  } else {
+    k_spread_dip<T, V, 0><<<(c.n + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, vec, c.d_cg,
+                                                                               check_stop, grid);
+  }
 }
 
-int launch_pme_dipole(Ctx& c, const double* d_vec, double* d_out, int mode) {
+int launch_convolve(Ctx& c, int check_stop) { return convolve(c, check_stop); }
+
+// Spread of the small systems' CG vector (warp per site): update forms
+// pp = zr + beta pp first; the mixed form also writes the partner records.
+// The convolution is the caller's.
+int launch_spread_small(Ctx& c, double* d_vec, int update) {
+  const PmeGeom g = geom_of(c);
+  int st = zero_grid(c);
+  if (st) return st;
+  const int nb = (c.n + 3) / 4;
+  if (c.mixed)
+    k_spread_dip_small<float><<<nb, 128, 0, c.stream>>>(c.n, g, c.d_pos, d_vec, c.d_zr, c.d_cg, update, update,
+                                                        c.d_posf, c.d_rec, c.d_mpz, (cufftComplex*)c.d_grid);
+  else
+    k_spread_dip_small<double><<<nb, 128, 0, c.stream>>>(c.n, g, c.d_pos, d_vec, c.d_zr, c.d_cg, update, update,
+                                                         nullptr, nullptr, nullptr, (cufftDoubleComplex*)c.d_grid);
+  return cuda_status(cudaGetLastError(), &c, "spread dip");
+}
+
+// Dipole PME pass: spread of d_vec [n][6] and the convolution.  d_out (if
+// non-null) receives the gathered field gradient [n][6] (tmatxbrecip's
+// dipfield); the CG loop passes null and gathers inside its combine kernel.
+int launch_pme_dipole(Ctx& c, const double* d_vec, double* d_out, int check_stop) {
   PmeGeom g = geom_of(c);
   int st = zero_grid(c);
   if (st) return st;
-  float* vf = (c.mixed && mode != 2) ? c.d_vecf : nullptr;
   if (c.mixed)
-    spread_dipoles<float, double>(c, g, const_cast<double*>(d_vec), vf, mode, (cufftComplex*)c.d_grid);
+    spread_dipoles<float, double>(c, g, d_vec, check_stop, (cufftComplex*)c.d_grid);
   else
-    spread_dipoles<double, double>(c, g, const_cast<double*>(d_vec), vf, mode, (cufftDoubleComplex*)c.d_grid);
+    spread_dipoles<double, double>(c, g, d_vec, check_stop, (cufftDoubleComplex*)c.d_grid);
   if ((st = cuda_status(cudaGetLastError(), &c, "spread dip"))) return st;
-  if ((st = convolve(c, mode >= 1))) return st;
+  if ((st = convolve(c, check_stop))) return st;
   if (d_out) st = launch_gather_dip(c, d_out, false);
   return st;
 }
 
-// The overlapped mixed CG's spread of its FP32 search direction (mode 2:
-// stop flag honoured, no update, no FP32 copy), then the convolution.
-int launch_pme_dipole_f32(Ctx& c, const float* d_vec) {
+// The overlapped mixed CG's spread of its FP32 search direction, then the
+// convolution.
+int launch_pme_dipole_f32(Ctx& c, const float* d_vec, int check_stop) {
   PmeGeom g = geom_of(c);
   int st = zero_grid(c);
   if (st) return st;
-  spread_dipoles<float, float>(c, g, const_cast<float*>(d_vec), nullptr, 2, (cufftComplex*)c.d_grid);
+  spread_dipoles<float, float>(c, g, d_vec, check_stop, (cufftComplex*)c.d_grid);
   if ((st = cuda_status(cudaGetLastError(), &c, "spread dip"))) return st;
-  return convolve(c, true);
+  return convolve(c, check_stop);
 }
 
 int launch_gather_dip(Ctx& c, double* d_out, bool check_stop) {
   PmeGeom g = geom_of(c);
   const int nb = (c.n + kBlock - 1) / kBlock;
   if (c.mixed)
-    k_gather_dip<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_grid, d_out, c.d_cg,
+    k_gather_dip<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_conv, d_out, c.d_cg,
                                                   check_stop ? 1 : 0);
   else
-    k_gather_dip<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_grid, d_out,
+    k_gather_dip<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_conv, d_out,
                                                    c.d_cg, check_stop ? 1 : 0);
   return cuda_status(cudaGetLastError(), &c, "gather dip");
 }

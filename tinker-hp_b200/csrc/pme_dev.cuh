@@ -217,6 +217,102 @@ __device__ __forceinline__ void spread_dip_site(const PmeGeom& g, double4 p, con
   spread_dip_stencil<T>(g, gx, gy, gz, tx, ty, tz, fd, fp, grid);
 }
 
+// One site's spline weights staged in shared memory by the lanes that share
+// the site (stage_axis): value and derivative of the five stencil points per
+// axis, and the stencil's first grid index.
+template <typename T, int LEVEL = 2>
+struct SiteWeights {
+  T w[3][LEVEL * kBs];  // value, first derivative, ... of each point
+  int g0[3];
+};
+
+// axis ax (0..2) of site p, by one lane
+template <typename T, int LEVEL = 2>
+__device__ __forceinline__ void stage_axis(const PmeGeom& g, double4 p, int ax, SiteWeights<T, LEVEL>& s) {
+  T th[kBs][LEVEL];
+  const double x = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
+  const double rc = ax == 0 ? g.recip[0] : (ax == 1 ? g.recip[1] : g.recip[2]);
+  const int nf = ax == 0 ? g.n1 : (ax == 1 ? g.n2 : g.n3);
+  s.g0[ax] = bspline_axis<LEVEL, T>(x, rc, nf, th);
+#pragma unroll
+  for (int k = 0; k < kBs; ++k)
+#pragma unroll
+    for (int l = 0; l < LEVEL; ++l) s.w[ax][LEVEL * k + l] = th[k][l];
+}
+
+// grid_uind_site for one site by one warp.  FP32: lane l < 25 adds stencil
+// line (y, z) = (l % 5, l / 5), Re and Im of a point in one reduction.  FP64,
+// whose reductions take one value: lanes 2 l and 2 l + 1 add Re and Im of line
+// l, then of line 16 + l, so that a pair of lanes shares a sector's reduction.
+// The weights are staged (s) and visible to the warp.
+template <typename T>
+__device__ __forceinline__ void spread_dip_lines(const PmeGeom& g, const SiteWeights<T>& s, int lane, const T (&fd)[3],
+                                                 const T (&fp)[3], typename Cplx<T>::type* __restrict__ grid) {
+  if constexpr (std::is_same<T, double>::value) {
+    const int d = lane & 1;
+    const T f0 = d ? fp[0] : fd[0], f1 = d ? fp[1] : fd[1], f2 = d ? fp[2] : fd[2];
+    for (int l = lane >> 1; l < kBs * kBs; l += 16) {
+      const int b = l % kBs, c = l / kBs;
+      const T u0 = s.w[1][2 * b], u1 = s.w[1][2 * b + 1], v0 = s.w[2][2 * c], v1 = s.w[2][2 * c + 1];
+      const T t0 = f1 * u1 * v0 + f2 * u0 * v1, t1 = f0 * u0 * v0;
+      const size_t row = ((size_t)wrapk(s.g0[2] + c, g.n3) * g.n2 + wrapk(s.g0[1] + b, g.n2)) * g.n1;
+#pragma unroll
+      for (int a = 0; a < kBs; ++a)
+        red_add(&grid[row + wrapk(s.g0[0] + a, g.n1)].x + d, t0 * s.w[0][2 * a] + t1 * s.w[0][2 * a + 1]);
+    }
+    return;
+  }
+  if (lane >= kBs * kBs) return;
+  const int b = lane % kBs, c = lane / kBs;
+  const T u0 = s.w[1][2 * b], u1 = s.w[1][2 * b + 1], v0 = s.w[2][2 * c], v1 = s.w[2][2 * c + 1];
+  const T t01 = fd[1] * u1 * v0 + fd[2] * u0 * v1, t11 = fd[0] * u0 * v0;
+  const T t02 = fp[1] * u1 * v0 + fp[2] * u0 * v1, t12 = fp[0] * u0 * v0;
+  const int gx = s.g0[0];
+  const size_t row = ((size_t)wrapk(s.g0[2] + c, g.n3) * g.n2 + wrapk(s.g0[1] + b, g.n2)) * g.n1;
+#pragma unroll
+  for (int a = 0; a < kBs; ++a) {
+    const T w0 = s.w[0][2 * a], w1 = s.w[0][2 * a + 1];
+    grid_add(grid, row + wrapk(gx + a, g.n1), t01 * w0 + t11 * w1, t02 * w0 + t12 * w1);
+  }
+}
+
+// fphi_uind_site's field part for one site by eight lanes (j = 0..7, lines j,
+// j+8, j+16 and 24): every lane returns the six components (gather_dip's),
+// summed in a fixed shuffle tree.  All lanes of the warp call.
+template <typename T>
+__device__ __forceinline__ void gather_dip8(const PmeGeom& g, const SiteWeights<T>& s, int j,
+                                            const typename Cplx<T>::type* __restrict__ grid, double (&out)[6]) {
+  T acc[6] = {0, 0, 0, 0, 0, 0};
+  const int gx = s.g0[0];
+  for (int q = j; q < kBs * kBs; q += 8) {
+    const int b = q % kBs, c = q / kBs;
+    const T u0 = s.w[1][2 * b], u1 = s.w[1][2 * b + 1], v0 = s.w[2][2 * c], v1 = s.w[2][2 * c + 1];
+    const size_t row = ((size_t)wrapk(s.g0[2] + c, g.n3) * g.n2 + wrapk(s.g0[1] + b, g.n2)) * g.n1;
+    T t0a = 0, t1a = 0, t0b = 0, t1b = 0;
+#pragma unroll
+    for (int a = 0; a < kBs; ++a) {
+      const auto e = grid[row + wrapk(gx + a, g.n1)];
+      const T w0 = s.w[0][2 * a], w1 = s.w[0][2 * a + 1];
+      t0a += e.x * w0;
+      t1a += e.x * w1;
+      t0b += e.y * w0;
+      t1b += e.y * w1;
+    }
+    acc[0] += t1a * u0 * v0;
+    acc[1] += t0a * u1 * v0;
+    acc[2] += t0a * u0 * v1;
+    acc[3] += t1b * u0 * v0;
+    acc[4] += t0b * u1 * v0;
+    acc[5] += t0b * u0 * v1;
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 6; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) out[q] = g.a[q % 3] * (double)acc[q];
+}
+
 // Warp-aggregated spread.  The sites of a warp are consecutive in the cell
 // order, so their stencils overlap heavily: 16 sites of the 288k water box
 // touch about 900 distinct grid points instead of 2,000.  The warp sums the

@@ -2,9 +2,8 @@
 //
 // inducepcg_pme2 (newinduce_pme2.f:285-636) with every vector and scalar on
 // the device.  Per iteration (systems of THP_OVERLAP_MIN_ATOMS atoms and
-// more; smaller ones run one fused matvec kernel after the PME branch):
-//   1. pp = zr + beta*pp (the mixed form also writes the 32-byte partner
-//      records of its FP32 real-space row);
+// more; smaller ones: matvec_small):
+//   1. pp = zr + beta*pp, with the partner records of the real-space row;
 //   2. fork: the real-space row T_real pp runs on the side stream while the
 //      main stream spreads pp on the PME grid, runs cuFFT forward, qfac and
 //      cuFFT backward;
@@ -24,9 +23,9 @@
 #include "kernels.h"
 
 // Systems of at least THP_OVERLAP_MIN_ATOMS atoms run the real-space row of
-// each CG matvec on a side stream, concurrent with the PME branch.  Smaller
-// systems are launch-bound (and overlap with each other when batched), so
-// they use one fused matvec kernel after the PME branch.
+// each CG matvec on a side stream, concurrent with the whole PME branch.
+// Smaller systems are bound by launches and latency: their spread forms the
+// search direction itself and the row runs beside the convolution.
 // 1: the CG loop runs on the device as one graph with a conditional WHILE
 // node; 0: graph-replayed chunks of kCgChunk iterations with a host check
 #ifndef THP_DEVICE_LOOP
@@ -48,9 +47,9 @@
 #define THP_OVERLAP_MIN_ATOMS 20000
 #endif
 
-// systems below this many atoms run the fused matvec in blocks of 32 atoms
-#ifndef THP_MATVEC_SMALL_ATOMS
-#define THP_MATVEC_SMALL_ATOMS 8000
+// systems below this many atoms run their rows in blocks of one warp
+#ifndef THP_ROW_SMALL_ATOMS
+#define THP_ROW_SMALL_ATOMS 8000
 #endif
 
 namespace thp {
@@ -63,33 +62,36 @@ namespace {
 
 using namespace cg;
 
-
-
-
-// h = T_real x + x/alpha + dipfield(x) - term x and the reductions of one
-// CG step (cg_matvec_block); dipfield comes from k_gather_dip.
-template <bool MIXED, int GPW>
-__global__ void __launch_bounds__(kBlock) k_cg_matvec(PairRows pr, Box box, const double4* __restrict__ pos,
-                                                      const float4* __restrict__ posf, const double* __restrict__ dipf,
-                                                      const double* __restrict__ x, const float* __restrict__ xf,
-                                                      const double* __restrict__ pol, const double* __restrict__ ef,
-                                                      double term, int init, double* __restrict__ h,
-                                                      double* __restrict__ res, double* __restrict__ zr,
-                                                      double* __restrict__ pp, CgScalars* cg,
-                                                      double* __restrict__ partials, float interior) {
-  if (cg->stop) return;
-  cg_matvec_block<MIXED, 0, false, GPW>((int)blockIdx.x, (int)gridDim.x, pr, box, pos, posf, dipf, PmeGeom{},
-                                        nullptr, x, xf, nullptr, nullptr, pol, ef, term, init, h, res, zr, pp, cg,
-                                        partials, interior);
-}
-
-// pp = zr + beta pp (newinduce_pme2.f:553-559) of the overlapped FP64 rows.
-__global__ void __launch_bounds__(256) k_pp_update(int n, const double* __restrict__ zr, double* __restrict__ x,
-                                                  const CgScalars* __restrict__ cg) {
-  if (cg->stop) return;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 6 * n) return;
-  x[t] = zr[t] + cg->beta[(t % 6) < 3 ? 0 : 1] * x[t];
+// pp = zr + beta pp (newinduce_pme2.f:553-559) of the overlapped FP64 rows,
+// with the partner records they read (rec, mpz: the wrapped position beside
+// the dipoles); one thread per atom.  update 0 only writes the records of x.
+__global__ void __launch_bounds__(256) k_pp_rec64(int n, int update, Box box, const double* __restrict__ zr,
+                                                 double* __restrict__ x, const double4* __restrict__ pos,
+                                                 double* __restrict__ rec, double* __restrict__ mpz,
+                                                 const CgScalars* __restrict__ cg) {
+  if (update && cg->stop) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double v[6];
+  load6(x + (size_t)i * 6, v);
+  double2* r = reinterpret_cast<double2*>(rec + (size_t)i * 8);
+  if (update) {
+    double z[6];
+    load6(zr + (size_t)i * 6, z);
+    const double bd = cg->beta[0], bp = cg->beta[1];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) v[q] = z[q] + (q < 3 ? bd : bp) * v[q];
+    store6(x + (size_t)i * 6, v);
+    rec[(size_t)i * 8 + 3] = v[0];
+  } else {  // the start of a solve: positions too
+    double4 p = pos[i];
+    image3(box, p.x, p.y, p.z);
+    r[0] = make_double2(p.x, p.y);
+    r[1] = make_double2(p.z, v[0]);
+  }
+  r[2] = make_double2(v[1], v[2]);
+  r[3] = make_double2(v[3], v[4]);
+  mpz[i] = v[5];
 }
 
 // The same update for the overlapped rows of the mixed form, which read the
@@ -147,41 +149,79 @@ __global__ void __launch_bounds__(kBlock, THP_ROW_MINB) k_real_row(PairRows pr, 
   }
 }
 
-// h = hreal + x/alpha + dipfield(x) - term x and the reductions of one CG
-// step (cg_combine_block); hreal comes from k_real_row.
-template <int GATHER, typename XV, typename V>
-__global__ void __launch_bounds__(kBlock) k_cg_combine(int n, const double* __restrict__ dipf, PmeGeom g,
-                                                       const double4* __restrict__ pos, const void* __restrict__ grid,
-                                                       const XV* __restrict__ x, const double* __restrict__ pol,
-                                                       const double* __restrict__ ef, double term, int init,
-                                                       V* __restrict__ h, V* __restrict__ res, V* __restrict__ zr,
-                                                       V* __restrict__ pp, CgScalars* cg,
-                                                       double* __restrict__ partials) {
-  if (cg->stop) return;
-  cg_combine_block<GATHER, XV, V>((int)blockIdx.x, (int)gridDim.x, n, dipf, g, pos, grid, x, pol, ef, term, init, h,
-                                  res, zr, pp, cg, partials);
+// the same for the FP64 form's partner records (large systems)
+template <bool NOL1>
+__global__ void __launch_bounds__(kBlock) k_real_row64(PairRows pr, Box box, const double* __restrict__ rec,
+                                                       const double* __restrict__ mpz, const CgScalars* __restrict__ cg,
+                                                       int check_stop, double interior, double* __restrict__ hreal) {
+  if (check_stop && cg->stop) return;
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (4 * g >= pr.n) return;
+  const int lane = threadIdx.x & 31;
+  const int i = 4 * g + (lane >> 3), j = lane & 7;
+  double acc[6];
+  group_row<double, THP_GROW_U64, NOL1>(pr, PartnerRec64{rec, mpz}, Image64In{box}, g, lane, acc, interior);
+  if (j < 6 && i < pr.n) hreal[(size_t)i * 6 + j] = pick6(acc, j);
 }
 
-// mu, residual and preconditioned residual of one CG step (cg_update_block)
+// h = hreal + x/alpha + dipfield(x) - term x and the reductions of one CG
+// step (cg_combine_block); hreal comes from the real-space row.
+template <typename T, typename XV, typename V>
+__global__ void __launch_bounds__(kBlock) k_cg_combine(int n, PmeGeom g, const double4* __restrict__ pos,
+                                                       const void* __restrict__ grid, const XV* __restrict__ x,
+                                                       const double* __restrict__ pol, const double* __restrict__ ef,
+                                                       double term, int init, V* __restrict__ h, V* __restrict__ res,
+                                                       V* __restrict__ zr, V* __restrict__ pp, CgScalars* cg,
+                                                       double* __restrict__ partials) {
+  if (cg->stop) return;
+  cg_combine_block<T, XV, V>((int)blockIdx.x, (int)gridDim.x, n, g, pos, grid, x, pol, ef, term, init, h, res, zr, pp,
+                             cg, partials);
+}
+
+template <typename T, typename XV, typename V>
+static void launch_combine(Ctx& c, const XV* x, double term, int init, V* h, V* res, V* zr, V* pp) {
+  k_cg_combine<T, XV, V><<<(c.n + kBlock - 1) / kBlock, kBlock, 0, c.stream>>>(
+      c.n, pme_geom(c), c.d_pos, c.d_conv, x, c.d_pol, c.d_ef, term, init, h, res, zr, pp, c.d_cg, c.d_partials);
+}
+
+// The same for small systems, eight lanes per atom (cg_combine8_block).
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k_cg_combine8(int n, PmeGeom g, const double4* __restrict__ pos,
+                                                        const void* __restrict__ grid, const double* __restrict__ x,
+                                                        const double* __restrict__ pol, const double* __restrict__ ef,
+                                                        double term, int init, double* __restrict__ h,
+                                                        double* __restrict__ res, double* __restrict__ zr,
+                                                        double* __restrict__ pp, CgScalars* cg,
+                                                        double* __restrict__ partials) {
+  if (cg->stop) return;
+  cg_combine8_block<T>((int)blockIdx.x, (int)gridDim.x, n, g, pos, grid, x, pol, ef, term, init, h, res, zr, pp, cg,
+                       partials);
+}
+
+// The loop graph's condition as the update kernel, the last of the body, sets
+// it; max_loops 0 outside the loop graph.
+struct LoopCond {
+  cudaGraphConditionalHandle handle;
+  int max_loops;
+};
+
+// mu, residual and preconditioned residual of one CG step (cg_update_block).
+// In the loop graph it also ends the loop: the condition starts at 1 and is
+// only ever cleared, by the block that finds the CG stopped, or after max_loops
+// bodies whatever the kernels before did (a hard bound, counted at entry).
 template <typename V>
 __global__ void __launch_bounds__(kBlock) k_cg_update(int n, const double* __restrict__ pol,
                                                       const V* __restrict__ h, const V* __restrict__ pp,
                                                       double* __restrict__ mu, V* __restrict__ res,
                                                       V* __restrict__ zr, CgScalars* cg, double* __restrict__ partials,
-                                                      double poleps, int politer) {
-  if (cg->stop) return;
-  cg_update_block<V>((int)blockIdx.x, (int)gridDim.x, n, pol, h, pp, mu, res, zr, cg, partials, poleps, politer);
-}
-
-// Last node of the device-side loop body: keep looping while the CG has not
-// stopped, and never more than max_loops bodies (a hard bound on the loop,
-// whatever the kernels before it did).
-__global__ void k_loop_cond(CgScalars* cg, cudaGraphConditionalHandle handle, int max_loops) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int l = ++cg->loops;
-  unsigned keep = (cg->stop == 0 && l < max_loops) ? 1u : 0u;
-  if (!keep) cg->stop = 1;
-  cudaGraphSetConditional(handle, keep);
+                                                      double poleps, int politer, LoopCond loop) {
+  const bool stopped = cg->stop;
+  if (loop.max_loops && blockIdx.x == 0 && threadIdx.x == 0 && (++cg->loops >= loop.max_loops || stopped))
+    cudaGraphSetConditional(loop.handle, 0);
+  if (stopped) return;
+  if (cg_update_block<V>((int)blockIdx.x, (int)gridDim.x, n, pol, h, pp, mu, res, zr, cg, partials, poleps, politer) &&
+      loop.max_loops && cg->stop)
+    cudaGraphSetConditional(loop.handle, 0);
 }
 
 __global__ void k_guess_direct(int n, const double* __restrict__ pol, const double* __restrict__ ef,
@@ -293,7 +333,6 @@ static bool overlapped(const Ctx& c) { return overlap_rows(c); }
 // enqueued.
 template <typename XV>
 static int matvec_overlapped(Ctx& c, const XV* x, int init) {
-  const int nb = (c.n + kBlock - 1) / kBlock;
   int st;
   cudaEventRecord(c.ev_fork, c.stream);
   cudaStreamWaitEvent(c.stream2, c.ev_fork, 0);
@@ -307,64 +346,67 @@ static int matvec_overlapped(Ctx& c, const XV* x, int init) {
   else if (c.mixed)
     k_real_row<true, false, float><<<nbr, kBlock, 0, c.stream2>>>(pr, c.box, c.d_pos, c.d_rec, nullptr, c.d_mpz,
                                                                   c.d_cg, !init, interior, c.d_hf);
-  else if constexpr (std::is_same<XV, double>::value)
-    k_real_row<false, false, double><<<nbr, kBlock, 0, c.stream2>>>(pr, c.box, c.d_pos, nullptr, x, nullptr, c.d_cg,
-                                                                    !init, -1.f, c.d_h);
+  else if (c.n >= THP_STREAM_NO_L1_ATOMS)
+    k_real_row64<true><<<nbr, kBlock, 0, c.stream2>>>(pr, c.box, c.d_rec64, c.d_mpz64, c.d_cg, !init, interior, c.d_h);
+  else
+    k_real_row64<false><<<nbr, kBlock, 0, c.stream2>>>(pr, c.box, c.d_rec64, c.d_mpz64, c.d_cg, !init, interior, c.d_h);
   prof_mark(c, c.stream2);
   if ((st = cuda_status(cudaGetLastError(), &c, "real row"))) return st;
   cudaEventRecord(c.ev_join, c.stream2);
   if constexpr (std::is_same<XV, float>::value)
-    st = launch_pme_dipole_f32(c, x);
+    st = launch_pme_dipole_f32(c, x, !init);
   else
-    st = launch_pme_dipole(c, x, nullptr, 2);
+    st = launch_pme_dipole(c, x, nullptr, !init);
   if (st) return st;
   const double a = c.cfg.aewald;
   const double term = (4.0 / 3.0) * a * a * a / kSqrtPi;
-  const PmeGeom g = pme_geom(c);
   cudaStreamWaitEvent(c.stream, c.ev_join, 0);
   if (c.mixed)
-    k_cg_combine<1, XV, float><<<nb, kBlock, 0, c.stream>>>(c.n, nullptr, g, c.d_pos, c.d_grid, x, c.d_pol, c.d_ef,
-                                                            term, init, c.d_hf, c.d_resf, c.d_zrf, c.d_ppf, c.d_cg,
-                                                            c.d_partials);
+    launch_combine<float, XV, float>(c, x, term, init, c.d_hf, c.d_resf, c.d_zrf, c.d_ppf);
   else if constexpr (std::is_same<XV, double>::value)
-    k_cg_combine<2, double, double><<<nb, kBlock, 0, c.stream>>>(c.n, nullptr, g, c.d_pos, c.d_grid, x, c.d_pol,
-                                                                 c.d_ef, term, init, c.d_h, c.d_res, c.d_zr, c.d_pp,
-                                                                 c.d_cg, c.d_partials);
+    launch_combine<double, double, double>(c, x, term, init, c.d_h, c.d_res, c.d_zr, c.d_pp);
   return cuda_status(cudaGetLastError(), &c, "cg combine");
 }
 
-static int launch_matvec(Ctx& c, const double* x, int init) {
-  int st = launch_gather_dip(c, c.d_dip, init == 0);
+// One application of the CG matrix for small systems.  The spread also forms
+// the new search direction (and the mixed form's partner records), then the
+// real-space row runs on the side stream beside the convolution.  Small blocks
+// spread a small system's groups over the SMs.
+static int matvec_small(Ctx& c, double* x, int init) {
+  int st = launch_spread_small(c, x, !init);
   if (st) return st;
-  prof_mark(c, c.stream);
-  PairRows pr = pair_rows(c);
+  cudaEventRecord(c.ev_fork, c.stream);
+  cudaStreamWaitEvent(c.stream2, c.ev_fork, 0);
+  const PairRows pr = pair_rows(c);
+  const int rb = c.n < THP_ROW_SMALL_ATOMS ? 32 : kBlock;
+  const int nbr = group_blocks(c.n, rb);
+  prof_mark(c, c.stream2);
+  if (c.mixed)
+    k_real_row<true, false, double><<<nbr, rb, 0, c.stream2>>>(pr, c.box, c.d_pos, c.d_rec, nullptr, c.d_mpz, c.d_cg,
+                                                               !init, row_interior(c), c.d_h);
+  else
+    k_real_row<false, false, double><<<nbr, rb, 0, c.stream2>>>(pr, c.box, c.d_pos, nullptr, x, nullptr, c.d_cg, !init,
+                                                                -1.f, c.d_h);
+  prof_mark(c, c.stream2);
+  st = cuda_status(cudaGetLastError(), &c, "real row");
+  cudaEventRecord(c.ev_join, c.stream2);
+  const int st2 = launch_convolve(c, !init);
+  cudaStreamWaitEvent(c.stream, c.ev_join, 0);
+  if (st || st2) return st ? st : st2;
   const double a = c.cfg.aewald;
   const double term = (4.0 / 3.0) * a * a * a / kSqrtPi;
-  const float interior = c.mixed ? row_interior(c) : -1.f;
-#define THP_MATVEC_ARGS                                                                                          \
-  pr, c.box, c.d_pos, c.d_posf, c.d_dip, x, c.d_vecf, c.d_pol, c.d_ef, term, init, c.d_h, c.d_res, c.d_zr, c.d_pp, \
-      c.d_cg, c.d_partials, interior
-  // small systems: two groups per warp (blocks of 32 atoms), so their few
-  // atoms spread over many blocks instead of long per-warp chains
-  if (c.n < THP_MATVEC_SMALL_ATOMS) {
-    const int nb = (c.n + 31) / 32;
-    if (c.mixed)
-      k_cg_matvec<true, 2><<<nb, kBlock, 0, c.stream>>>(THP_MATVEC_ARGS);
-    else
-      k_cg_matvec<false, 2><<<nb, kBlock, 0, c.stream>>>(THP_MATVEC_ARGS);
-  } else {
-    const int nb = (c.n + kBlock - 1) / kBlock;
-    if (c.mixed)
-      k_cg_matvec<true, 8><<<nb, kBlock, 0, c.stream>>>(THP_MATVEC_ARGS);
-    else
-      k_cg_matvec<false, 8><<<nb, kBlock, 0, c.stream>>>(THP_MATVEC_ARGS);
-  }
-#undef THP_MATVEC_ARGS
-  prof_mark(c, c.stream);
-  return cuda_status(cudaGetLastError(), &c, "cg matvec");
+  const PmeGeom g = pme_geom(c);
+  const int nb = (c.n + 15) / 16;
+  if (c.mixed)
+    k_cg_combine8<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_conv, x, c.d_pol, c.d_ef, term, init, c.d_h,
+                                                      c.d_res, c.d_zr, c.d_pp, c.d_cg, c.d_partials);
+  else
+    k_cg_combine8<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_conv, x, c.d_pol, c.d_ef, term, init, c.d_h,
+                                                       c.d_res, c.d_zr, c.d_pp, c.d_cg, c.d_partials);
+  return cuda_status(cudaGetLastError(), &c, "cg combine");
 }
 
-static int enqueue_iteration(Ctx& c) {
+static int enqueue_iteration(Ctx& c, const LoopCond& loop) {
   int st;
   const int nb = (c.n + kBlock - 1) / kBlock;
   if (overlapped(c) && c.mixed) {
@@ -373,19 +415,19 @@ static int enqueue_iteration(Ctx& c) {
     if ((st = cuda_status(cudaGetLastError(), &c, "pp update"))) return st;
     if ((st = matvec_overlapped<float>(c, c.d_ppf, 0))) return st;
     k_cg_update<float><<<nb, kBlock, 0, c.stream>>>(c.n, c.d_pol, c.d_hf, c.d_ppf, c.d_mu, c.d_resf,
-                                                    c.d_zrf, c.d_cg, c.d_partials, c.cfg.poleps, c.cfg.politer);
+                                                    c.d_zrf, c.d_cg, c.d_partials, c.cfg.poleps, c.cfg.politer, loop);
     return cuda_status(cudaGetLastError(), &c, "cg update");
   }
   if (overlapped(c)) {
-    k_pp_update<<<(6 * c.n + 255) / 256, 256, 0, c.stream>>>(c.n, c.d_zr, c.d_pp, c.d_cg);
+    k_pp_rec64<<<(c.n + 255) / 256, 256, 0, c.stream>>>(c.n, 1, c.box, c.d_zr, c.d_pp, c.d_pos, c.d_rec64, c.d_mpz64,
+                                                        c.d_cg);
     if ((st = cuda_status(cudaGetLastError(), &c, "pp update"))) return st;
     if ((st = matvec_overlapped<double>(c, c.d_pp, 0))) return st;
   } else {
-    if ((st = launch_pme_dipole(c, c.d_pp, nullptr, 1))) return st;
-    if ((st = launch_matvec(c, c.d_pp, 0))) return st;
+    if ((st = matvec_small(c, c.d_pp, 0))) return st;
   }
   k_cg_update<double><<<nb, kBlock, 0, c.stream>>>(c.n, c.d_pol, c.d_h, c.d_pp, c.d_mu, c.d_res, c.d_zr,
-                                                   c.d_cg, c.d_partials, c.cfg.poleps, c.cfg.politer);
+                                                   c.d_cg, c.d_partials, c.cfg.poleps, c.cfg.politer, loop);
   return cuda_status(cudaGetLastError(), &c, "cg update");
 }
 
@@ -409,18 +451,20 @@ int pcg_begin(Ctx& c, int guess) {
     if (c.mixed) {
       k_pp_rec<double><<<(c.n + 255) / 256, 256, 0, c.stream>>>(c.n, 0, nullptr, c.d_mu, c.d_posf, c.d_rec, c.d_mpz,
                                                                 c.d_cg);
-      if ((st = cuda_status(cudaGetLastError(), &c, "mu copy"))) return st;
+    } else {
+      k_pp_rec64<<<(c.n + 255) / 256, 256, 0, c.stream>>>(c.n, 0, c.box, nullptr, c.d_mu, c.d_pos, c.d_rec64, c.d_mpz64,
+                                                          c.d_cg);
     }
+    if ((st = cuda_status(cudaGetLastError(), &c, "mu copy"))) return st;
     return matvec_overlapped<double>(c, c.d_mu, 1);
   }
-  if ((st = launch_pme_dipole(c, c.d_mu, nullptr, 0))) return st;
-  return launch_matvec(c, c.d_mu, 1);
+  return matvec_small(c, c.d_mu, 1);
 }
 
 static int enqueue_chunk(Ctx& c) {
   int st;
   for (int q = 0; q < kCgChunk; ++q)
-    if ((st = enqueue_iteration(c))) return st;
+    if ((st = enqueue_iteration(c, LoopCond{}))) return st;
   return cuda_status(cudaMemcpyAsync(c.h_cg, c.d_cg, sizeof(CgScalars), cudaMemcpyDeviceToHost, c.stream), &c,
                      "cg scalars");
 }
@@ -452,7 +496,7 @@ int pcg_chunk_async(Ctx& c) {
 }
 
 // Builds the CG loop graph: a conditional WHILE node whose body is one
-// iteration plus k_loop_cond.  Returns false (and leaves the chunked graph
+// iteration.  Returns false (and leaves the chunked graph
 // in charge) when the runtime refuses any step.
 static bool build_loop_graph(Ctx& c) {
   cudaGraph_t g = nullptr;
@@ -470,8 +514,7 @@ static bool build_loop_graph(Ctx& c) {
       cudaGraph_t body = p.conditional.phGraph_out[0];
       if (cudaStreamBeginCaptureToGraph(c.stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) ==
           cudaSuccess) {
-        int st = enqueue_iteration(c);
-        if (!st) k_loop_cond<<<1, 32, 0, c.stream>>>(c.d_cg, handle, c.cfg.politer + 2);
+        const int st = enqueue_iteration(c, LoopCond{handle, c.cfg.politer + 2});
         cudaGraph_t out = nullptr;
         const cudaError_t e = cudaStreamEndCapture(c.stream, &out);
         ok = !st && e == cudaSuccess && cudaGetLastError() == cudaSuccess;
