@@ -157,7 +157,15 @@ static int reserve_special_pairs(Ctx& c) {
   return THP_OK;
 }
 
+// Whether every special pair has the same d and p scale (then E_d = E_p).
+static bool scales_agree(const Ctx& c) {
+  for (size_t q = 0; q < c.sp_k.size(); ++q)
+    if (c.sp_s[3 * q] != c.sp_s[3 * q + 1]) return false;
+  return true;
+}
+
 int upload_special_pairs(Ctx& c) {
+  c.dp_equal = scales_agree(c);
   c.have_list = false;  // sorted partner numbers are made at the next sort
   int st = reserve_special_pairs(c);
   if (st) return st;
@@ -384,6 +392,15 @@ static void pinned_give(Ctx& c) {
   c.h_flags = nullptr;
 }
 
+static void drop_loop_graphs(Ctx& c) {
+  for (int f = 0; f < 2; ++f) {
+    if (c.chunk_exec[f]) cudaGraphExecDestroy(c.chunk_exec[f]);
+    if (c.loop_exec[f]) cudaGraphExecDestroy(c.loop_exec[f]);
+    c.chunk_exec[f] = c.loop_exec[f] = nullptr;
+    c.loop_state[f] = 0;
+  }
+}
+
 void free_ctx(Ctx& c) {
   void* ptrs[] = {c.slab_cells, c.slab_atoms, c.slab_pairs, c.d_sp_off, c.d_sp_k, c.d_sp_ks, c.d_sp_s, c.d_sp_c,
                   c.d_cg, c.d_flags, c.d_fphirec, c.d_depfix, c.d_trq, c.d_frs, c.d_grad, c.d_sgrid, c.d_sscratch,
@@ -392,8 +409,7 @@ void free_ctx(Ctx& c) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   pme_free(c);
-  if (c.chunk_exec) cudaGraphExecDestroy(c.chunk_exec);
-  if (c.loop_exec) cudaGraphExecDestroy(c.loop_exec);
+  drop_loop_graphs(c);
   for (auto& row : c.front_exec)
     for (auto& ex : row)
       if (ex) cudaGraphExecDestroy(ex);
@@ -433,7 +449,7 @@ size_t footprint_bytes(const thp_config& cfg, int* ncell_out) {
   b += n * 32 + n * 16 + 2 * n * 8 + 10 * n * 8 + n * 32 + n * 64;  // sorted data
   b += n * 4 + maxnb * npad * 4;                         // list
   b += n * 4 + maxnb * npad * (4 + 2 * (mixed ? 4 : 8));  // pairs
-  b += ngrid * (mixed ? 24 : 48);                        // grid, convolved grid and two influence functions
+  b += ngrid * (mixed ? 28 : 56);                        // grids, potential and two influence functions
   b += 10 * n * 6 * 8 + 4 * n * 8 + n * 6 * 4 + n * 9 * 4 + 4 * n * 6 * 4;  // vectors, FP32 row input and CG vectors
   b += (n / 128 + 2) * 4 * 8 + 4096 + (mixed ? 0 : 72 * n);  // reductions; FP64 row records
   b += 64 << 20;  // cuFFT work area and runtime slack
@@ -666,10 +682,7 @@ int thp_ctx_reset(thp_ctx* h, const thp_config* cfg) {
   if (set_current_device(c)) return THP_E_CUDA;
   if ((st = cuda_status(cudaStreamSynchronize(c.stream), &c, "reset"))) return st;
   // graphs hold this system's sizes and launch shapes
-  if (c.chunk_exec) cudaGraphExecDestroy(c.chunk_exec);
-  if (c.loop_exec) cudaGraphExecDestroy(c.loop_exec);
-  c.chunk_exec = c.loop_exec = nullptr;
-  c.loop_state = 0;
+  drop_loop_graphs(c);
   drop_front_graphs(c);
   for (cudaEvent_t e : c.prof_events) cudaEventDestroy(e);
   c.prof_events.clear();
@@ -862,6 +875,7 @@ int image_load(thp_ctx* h, const SystemImage* img) {
   c.sp_k.assign(img->sp_k, img->sp_k + img->m);
   c.sp_s.assign(img->sp_s, img->sp_s + 3 * (size_t)img->m);
   c.sp_c.assign(img->sp_c, img->sp_c + img->m);
+  c.dp_equal = scales_agree(c);
   c.have_conn = true;
   int st = reserve_special_pairs(c);
   if (st) return st;
@@ -1163,6 +1177,7 @@ int thp_solve(thp_ctx* h, int guess, thp_solve_info* info) {
 
 static int solve_one(thp_ctx* h, int guess, thp_solve_info* info) {
   Ctx& c = h->c;
+  const int asked = guess;
   cudaEventRecord(c.ev0, c.stream);
   // one host sync per solve: the list/pair overflow bits and the CG scalars
   // are read together after Epol (the predictor's least-squares fit and the
@@ -1171,10 +1186,11 @@ static int solve_one(thp_ctx* h, int guess, thp_solve_info* info) {
   if (st) return st;
   if ((st = resolve_predict(c, &guess))) return st;
   bool pending = false;
-  if ((st = run_pcg_async(c, guess, &pending))) return st;
+  // a caller's guess may differ between the two sets of dipoles
+  if ((st = run_pcg_async(c, guess, &pending, asked != THP_GUESS_HOST && single_field(c)))) return st;
   h->guess_uploaded = false;
+  if ((st = launch_epol(c))) return st;  // also completes d_mu of a single-field solve
   if ((st = predictor_push(c))) return st;
-  if ((st = launch_epol(c))) return st;
   cudaEventRecord(c.ev1, c.stream);
   cudaMemcpyAsync(c.h_cg, c.d_cg, sizeof(CgScalars), cudaMemcpyDeviceToHost, c.stream);
   cudaMemcpyAsync(c.h_flags, c.d_flags, sizeof(int), cudaMemcpyDeviceToHost, c.stream);
@@ -1269,6 +1285,7 @@ static void front_replayed(thp_ctx* h) {
   c.have_perm = c.have_list = true;
   ++c.sort_epoch;  // the replay re-sorted the atoms: lists in the old numbering are stale
   c.have_ef_prev = true;
+  c.single = 0;
   h->pos_dirty = h->rpole_dirty = false;
   h->field_valid = true;
 }

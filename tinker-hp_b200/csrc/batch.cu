@@ -361,8 +361,8 @@ static int enqueue_ffts(BatchPlan& p, int dir) {
     cudaStreamWaitEvent(k.stream, p.ev_fork, 0);
     cufftResult r = CUFFT_SUCCESS;
     if (k.conv) {
-      const cudaError_t e = p.mixed ? launch_conv32(k.n[0], conv::Sys{}, k.d_sys, k.count, 1, k.stream)
-                                    : launch_conv64(k.n[0], conv::Sys{}, k.d_sys, k.count, 1, k.stream);
+      const cudaError_t e = p.mixed ? launch_conv32(k.n[0], conv::Sys{}, k.d_sys, k.count, 1, false, k.stream)
+                                    : launch_conv64(k.n[0], conv::Sys{}, k.d_sys, k.count, 1, false, k.stream);
       if (e != cudaSuccess) return THP_E_CUDA;
     } else if (p.mixed) {
       cufftComplex* g = static_cast<cufftComplex*>(p.d_grid) + k.offset;
@@ -622,7 +622,7 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     s.mpz = c.d_mpz;
     s.grid = static_cast<char*>(p->d_grid) + next[cls[q]] * csz;
     s.conv = p->classes[cls[q]].conv ? static_cast<char*>(p->d_conv) + next[cls[q]] * csz : s.grid;
-    csys[cls[q]].push_back(conv::Sys{s.grid, s.conv, c.d_qfacp, c.d_cg});
+    csys[cls[q]].push_back(conv::Sys{s.grid, s.conv, c.d_qfacp, c.d_cg, nullptr});
     next[cls[q]] += slot(p->classes[cls[q]]);
     s.qfac = c.d_qfac;
     s.cg = c.d_cg;

@@ -20,6 +20,14 @@
 #endif
 
 namespace thp {
+
+// The loop graph's condition as the update kernel, the last of the body, sets
+// it; max_loops 0 outside the loop graph.
+struct LoopCond {
+  cudaGraphConditionalHandle handle;
+  int max_loops;
+};
+
 namespace cg {
 
 constexpr int kBlock = 128;
@@ -81,6 +89,17 @@ __device__ __forceinline__ void store6(float* p, const double (&v)[6]) {
   q[0] = make_float2((float)v[0], (float)v[1]);
   q[1] = make_float2((float)v[2], (float)v[3]);
   q[2] = make_float2((float)v[4], (float)v[5]);
+}
+
+// Entry of the update kernel in the loop graph: counts the body and ends the
+// loop once the CG has stopped or after max_loops bodies, whatever the kernels
+// before did; returns whether the CG has stopped.  The condition starts at 1
+// and is only ever cleared.
+__device__ __forceinline__ bool loop_entry(const LoopCond& loop, CgScalars* cg) {
+  const bool stopped = cg->stop;
+  if (loop.max_loops && blockIdx.x == 0 && threadIdx.x == 0 && (++cg->loops >= loop.max_loops || stopped))
+    cudaGraphSetConditional(loop.handle, 0);
+  return stopped;
 }
 
 __device__ __forceinline__ double diag_of(double p) { return p == 0.0 ? kTinyPol : p; }
@@ -237,6 +256,33 @@ __device__ __forceinline__ void row_block(int blk, const PairRows& pr, const Box
   }
 }
 
+// The end of an update's reduction, by one thread: tot = r.z of the two sets.
+__device__ __forceinline__ void cg_after_update(const double (&tot)[2], int n, CgScalars* cg, double poleps,
+                                                int politer) {
+  const double nrm = (double)(3 * n);
+  double resnrm = 0.0;
+  bool bad = false;
+  for (int k = 0; k < 2; ++k) {
+    cg->ggnew[k] = tot[k];
+    const double gn = sqrt(tot[k] / nrm);
+    resnrm = fmax(resnrm, gn);
+    bad |= !isfinite(tot[k]);
+    cg->beta[k] = tot[k] / cg->ggold[k];
+    cg->ggold[k] = tot[k];
+  }
+  cg->resnrm = resnrm;
+  cg->niter += 1;
+  if (bad) {
+    cg->status = THP_E_NAN;
+    cg->stop = 1;
+  } else if (resnrm < poleps) {
+    cg->converged = 1;
+    cg->stop = 1;
+  } else if (cg->niter >= politer) {
+    cg->stop = 1;
+  }
+}
+
 // newinduce_pme2.f:512-572.  The reference's per-iteration energy ene (a
 // diagnostic printed at each step) is formed once, after the loop, from the
 // final mu and residual (k_epol / kb_finish): the same value the last
@@ -274,28 +320,7 @@ __device__ __forceinline__ bool cg_update_block(int blk, int nblk, int n, const 
   double tot[2];
   const bool last = grid_reduce_of<2>(red, partials, &cg->counter[1], blk, nblk, tot) && threadIdx.x == 0;
   if (last) {
-    const double nrm = (double)(3 * n);
-    double resnrm = 0.0;
-    bool bad = false;
-    for (int k = 0; k < 2; ++k) {
-      cg->ggnew[k] = tot[k];
-      const double gn = sqrt(tot[k] / nrm);
-      resnrm = fmax(resnrm, gn);
-      bad |= !isfinite(tot[k]);
-      cg->beta[k] = tot[k] / cg->ggold[k];
-      cg->ggold[k] = tot[k];
-    }
-    cg->resnrm = resnrm;
-    cg->niter += 1;
-    if (bad) {
-      cg->status = THP_E_NAN;
-      cg->stop = 1;
-    } else if (resnrm < poleps) {
-      cg->converged = 1;
-      cg->stop = 1;
-    } else if (cg->niter >= politer) {
-      cg->stop = 1;
-    }
+    cg_after_update(tot, n, cg, poleps, politer);
   }
   return last;
 }

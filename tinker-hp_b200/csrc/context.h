@@ -172,6 +172,7 @@ struct Ctx {
   void* d_conv = nullptr;
   void* d_conv_buf = nullptr;
   void* d_qfacp = nullptr;
+  void* d_pot = nullptr;         // the potential of a real convolution, one real per point
   double a_frac[3] = {0, 0, 0};  // nfft_d * recip(d,d)
 
   // CG vectors, sorted order, [n][6] = (d xyz, p xyz)
@@ -191,6 +192,12 @@ struct Ctx {
   double* d_ef_prev = nullptr;  // [n][6]
   bool have_ef_prev = false;
   float* d_mpz = nullptr;     // [n]
+  // the d and p scales of every special pair agree: the two direct fields, and
+  // so the two sets of induced dipoles, are the same (the reference's dpequal)
+  bool dp_equal = false;
+  // the solve in hand runs the single-field CG (cg_single.cu): its vectors are
+  // [n][3] in the front of the two-field buffers, its dipoles in d_dip
+  int single = 0;
   // the same of the FP64 form: {x, y, z (wrapped), d dipole, p dipole x, y} and p dipole z
   double* d_rec64 = nullptr;  // [n][8]
   double* d_mpz64 = nullptr;  // [n]
@@ -254,11 +261,12 @@ struct Ctx {
   double* bqgrid = nullptr;  // pme::qgrid2in_2d(2,n1,n2,n3), read by fphi_uind_site_
 
   // CUDA graph of one CG chunk (captured on first use)
-  cudaGraphExec_t chunk_exec = nullptr;
+  // (the two graphs of each form: [0] d and p dipoles, [1] single field)
+  cudaGraphExec_t chunk_exec[2] = {};
   // the whole CG loop as one graph (conditional WHILE node); loop_state:
   // 0 not built yet, 1 built, -1 not available (the chunked graph is used)
-  cudaGraphExec_t loop_exec = nullptr;
-  int loop_state = 0;
+  cudaGraphExec_t loop_exec[2] = {};
+  int loop_state[2] = {0, 0};
   // front of a batched solve per guess mode and dipole carry (api.cu)
   cudaGraphExec_t front_exec[3][2] = {};
   bool front_failed = false;

@@ -11,9 +11,9 @@ namespace thp {
 
 bool conv_split64(int n, int* r1, int* r2) { return conv::split_of<double>(n, r1, r2); }
 
-cudaError_t launch_conv64(int n, const conv::Sys& one, const conv::Sys* many, int count, int check_stop,
+cudaError_t launch_conv64(int n, const conv::Sys& one, const conv::Sys* many, int count, int check_stop, bool real,
                           cudaStream_t st) {
-  return conv::launch_length<double>(n, one, many, count, check_stop, st);
+  return conv::launch_length<double>(n, one, many, count, check_stop, real, st);
 }
 
 }  // namespace thp

@@ -188,11 +188,11 @@ constexpr size_t plane_bytes() {
 // exp(-2 pi i m / N), m < N
 template <typename T, int N>
 struct RootTable {
-  T c[N], s[N];
-  constexpr RootTable() : c(), s() {
+  alignas(2 * sizeof(T)) T v[2 * N];  // (cos, sin) pairs, one load each
+  constexpr RootTable() : v() {
     for (int m = 0; m < N; ++m) {
-      c[m] = (T)root_cos(m, N);
-      s[m] = (T)-root_sin(m, N);
+      v[2 * m] = (T)root_cos(m, N);
+      v[2 * m + 1] = (T)-root_sin(m, N);
     }
   }
 };
@@ -209,9 +209,8 @@ THP_CONV_LENGTHS(THP_ROOTS)
 
 template <typename T, int N, bool INV, typename C>
 __device__ __forceinline__ C mul_table(C v, int m) {
-  const T c = __ldg(&roots<T, N>().c[m]);
-  T s = __ldg(&roots<T, N>().s[m]);
-  if (INV) s = -s;
+  const C w = __ldg(reinterpret_cast<const C*>(&roots<T, N>().v[2 * m]));
+  const T c = w.x, s = INV ? -w.y : w.y;
   return C{v.x * c - v.y * s, v.x * s + v.y * c};
 }
 
@@ -229,7 +228,7 @@ constexpr int plane_threads() {  // a thread per DFT of the wider stage, within 
   return want < most ? want : most;
 }
 
-template <typename T, int N, int R1, int R2, int TH>
+template <typename T, int N, int R1, int R2, int TH, bool REAL>
 __global__ void __launch_bounds__(TH) k_conv_xy(Sys one, const Sys* __restrict__ many, int check_stop) {
   using C = typename Cplx<T>::type;
   extern __shared__ __align__(16) unsigned char conv_smem[];
@@ -238,14 +237,22 @@ __global__ void __launch_bounds__(TH) k_conv_xy(Sys one, const Sys* __restrict__
   if (check_stop && s.cg->stop) return;
   constexpr int LD = N + 1;
   C* __restrict__ in = static_cast<C*>(s.in) + (size_t)blockIdx.x * N * N;
+  T* __restrict__ rin = static_cast<T*>(s.in) + (size_t)blockIdx.x * N * N;
   C* __restrict__ out = static_cast<C*>(s.out) + (size_t)blockIdx.x * N * N;
   for (int b = threadIdx.x; b < N * R2; b += TH) {
     const int row = b / R2, n2 = b - row * R2;
     C v[R1];
+    if constexpr (REAL) {
 #pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1) v[n1] = in[row * N + R2 * n1 + n2];
+      for (int n1 = 0; n1 < R1; ++n1) v[n1] = C{rin[row * N + R2 * n1 + n2], T(0)};
 #pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1) in[row * N + R2 * n1 + n2] = C{T(0), T(0)};
+      for (int n1 = 0; n1 < R1; ++n1) rin[row * N + R2 * n1 + n2] = T(0);
+    } else {
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) v[n1] = in[row * N + R2 * n1 + n2];
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) in[row * N + R2 * n1 + n2] = C{T(0), T(0)};
+    }
     dft<R1, false>(v);
 #pragma unroll
     for (int k1 = 0; k1 < R1; ++k1)
@@ -286,7 +293,7 @@ __global__ void __launch_bounds__(TH) k_conv_xy(Sys one, const Sys* __restrict__
   }
 }
 
-template <typename T, int N, int R1, int R2, int TH>
+template <typename T, int N, int R1, int R2, int TH, bool REAL>
 __global__ void __launch_bounds__(TH) k_conv_yx(Sys one, const Sys* __restrict__ many, int check_stop) {
   using C = typename Cplx<T>::type;
   extern __shared__ __align__(16) unsigned char conv_smem[];
@@ -295,6 +302,7 @@ __global__ void __launch_bounds__(TH) k_conv_yx(Sys one, const Sys* __restrict__
   if (check_stop && s.cg->stop) return;
   constexpr int LD = N + 1;
   C* __restrict__ out = static_cast<C*>(s.out) + (size_t)blockIdx.x * N * N;
+  T* __restrict__ pot = static_cast<T*>(s.pot) + (size_t)blockIdx.x * N * N;
   for (int b = threadIdx.x; b < N * R1; b += TH) {
     const int k1 = b / N, col = b - k1 * N;
     C v[R2];
@@ -336,7 +344,12 @@ __global__ void __launch_bounds__(TH) k_conv_yx(Sys one, const Sys* __restrict__
     for (int k1 = 0; k1 < R1; ++k1) v[k1] = q[R2 * k1];
     dft<R1, true>(v);
 #pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1) out[row * N + R2 * n1 + n2] = v[n1];
+    for (int n1 = 0; n1 < R1; ++n1) {
+      if constexpr (REAL)
+        pot[row * N + R2 * n1 + n2] = v[n1].x;
+      else
+        out[row * N + R2 * n1 + n2] = v[n1];
+    }
   }
 }
 
@@ -394,19 +407,19 @@ __global__ void __launch_bounds__(kZCols<T>*(R1 > R2 ? R1 : R2)) k_conv_z(Sys on
 
 // The three launches for one system (many null) or for count systems of one
 // grid length.
-template <typename T, int N, int R1, int R2>
+template <typename T, int N, int R1, int R2, bool REAL>
 cudaError_t launch(const Sys& one, const Sys* many, int count, int check_stop, cudaStream_t st) {
   constexpr int TH = plane_threads<T, N, (R1 > R2 ? R1 : R2)>();
   constexpr size_t smem = plane_bytes<T, N>();
   constexpr int W = kZCols<T>;
   static std::atomic<unsigned long long> set_xy{0}, set_yx{0};
   if (smem > 48 * 1024) {
-    smem_limit_once(k_conv_xy<T, N, R1, R2, TH>, smem, set_xy);
-    smem_limit_once(k_conv_yx<T, N, R1, R2, TH>, smem, set_yx);
+    smem_limit_once(k_conv_xy<T, N, R1, R2, TH, REAL>, smem, set_xy);
+    smem_limit_once(k_conv_yx<T, N, R1, R2, TH, REAL>, smem, set_yx);
   }
-  k_conv_xy<T, N, R1, R2, TH><<<dim3(N, count), TH, smem, st>>>(one, many, check_stop);
+  k_conv_xy<T, N, R1, R2, TH, REAL><<<dim3(N, count), TH, smem, st>>>(one, many, check_stop);
   k_conv_z<T, N, R1, R2><<<dim3((N * N + W - 1) / W, count), W*(R1 > R2 ? R1 : R2), 0, st>>>(one, many, check_stop);
-  k_conv_yx<T, N, R1, R2, TH><<<dim3(N, count), TH, smem, st>>>(one, many, check_stop);
+  k_conv_yx<T, N, R1, R2, TH, REAL><<<dim3(N, count), TH, smem, st>>>(one, many, check_stop);
   return cudaGetLastError();
 }
 
@@ -427,10 +440,13 @@ bool split_of(int n, int* r1, int* r2) {
 }
 
 template <typename T>
-cudaError_t launch_length(int n, const Sys& one, const Sys* many, int count, int check_stop, cudaStream_t st) {
+cudaError_t launch_length(int n, const Sys& one, const Sys* many, int count, int check_stop, bool real,
+                          cudaStream_t st) {
 #define THP_CASE(N, A, B)                        \
   if constexpr (plane_bytes<T, N>() <= kMaxSmem) \
-    if (n == N) return launch<T, N, A, B>(one, many, count, check_stop, st);
+    if (n == N)                                  \
+      return real ? launch<T, N, A, B, true>(one, many, count, check_stop, st) \
+                  : launch<T, N, A, B, false>(one, many, count, check_stop, st);
   THP_CONV_LENGTHS(THP_CASE)
 #undef THP_CASE
   return cudaErrorInvalidValue;

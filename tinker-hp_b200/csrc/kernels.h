@@ -37,7 +37,7 @@ int launch_gather_mpole(Ctx& c, double* cphi10, bool with_e0);  // cphi from the
 int launch_pme_dipole_f32(Ctx& c, const float* d_vec, int check_stop);
 int launch_pme_dipole(Ctx& c, const double* d_vec, double* d_out, int check_stop);
 int launch_spread_small(Ctx& c, double* d_vec, int update);  // the small systems' CG spread, without convolution
-int launch_convolve(Ctx& c, int check_stop);
+int launch_convolve(Ctx& c, int check_stop, bool real = false);  // real: conv.h
 bool overlap_rows(const Ctx& c);  // the system runs real-space passes on the side stream
 int zero_grid(Ctx& c);  // before a spread: d_grid zero (nothing to do for the three-kernel convolution)
 struct PmeGeom;
@@ -83,13 +83,21 @@ int launch_ekin(Ctx& c, const double* d_mass, const double* d_vel, double* d_scr
 
 // solver.cu
 int run_pcg(Ctx& c, int guess);
-int run_pcg_async(Ctx& c, int guess, bool* pending);  // see solver.cu
+int run_pcg_async(Ctx& c, int guess, bool* pending, bool single);  // see solver.cu
 int pcg_status(Ctx& c);
-int pcg_begin(Ctx& c, int guess);
+int pcg_begin(Ctx& c, int guess, bool single = false);
 int pcg_chunk_async(Ctx& c);
 int pcg_loop_async(Ctx& c);  // whole CG loop in one graph launch; -1 when unavailable
 int pcg_status(Ctx& c);
 int launch_epol(Ctx& c);
+
+// cg_single.cu: the CG when the d and p dipoles are the same
+struct LoopCond;
+bool single_field(const Ctx& c);  // whether the system and its grid qualify
+int single_begin(Ctx& c);         // from the guess in d_mu: initial residual
+int single_iteration(Ctx& c, const LoopCond& loop);
+int single_epol(Ctx& c);          // Epol, ene, and both sets of dipoles into d_mu
+void prof_mark(Ctx& c, cudaStream_t s);  // solver.cu
 
 // reorder helpers (solver.cu)
 int launch_to_sorted6(Ctx& c, const double* d_orig, double* d_sorted, int nrhs);

@@ -506,12 +506,13 @@ int fft(Ctx& c, int dir) {
 // d_grid -> d_conv: forward transform, influence function, inverse
 // transform.  Three kernels where the grid allows (at 120^3: 73 -> 38 us FP32,
 // 98 -> 53 us FP64 against cuFFT's six launches and the product; 60^3 34 -> 15 us), else
-// cuFFT.
-int convolve(Ctx& c, int check_stop) {
+// cuFFT.  real (three-kernel form only): one real per point in the front of
+// d_grid, the result in d_pot.
+int convolve(Ctx& c, int check_stop, bool real = false) {
   if (c.conv) {
-    const conv::Sys s{c.d_grid, c.d_conv, c.d_qfacp, c.d_cg};
-    const cudaError_t e = c.mixed ? launch_conv32(c.nfft[0], s, nullptr, 1, check_stop, c.stream)
-                                  : launch_conv64(c.nfft[0], s, nullptr, 1, check_stop, c.stream);
+    const conv::Sys s{c.d_grid, c.d_conv, c.d_qfacp, c.d_cg, c.d_pot};
+    const cudaError_t e = c.mixed ? launch_conv32(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream)
+                                  : launch_conv64(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream);
     return cuda_status(e, &c, "convolution");
   }
   int st = fft(c, CUFFT_FORWARD);
@@ -627,7 +628,7 @@ int pme_init(Ctx& c) {
   // grid buffers are kept while they are large enough (a re-targeted
   // context reuses them)
   if (c.ngrid > c.cap_ngrid) {
-    for (void** p : {&c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf}) {
+    for (void** p : {&c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf, &c.d_pot}) {
       cudaFree(*p);
       *p = nullptr;
     }
@@ -636,6 +637,7 @@ int pme_init(Ctx& c) {
     if (cuda_status(cudaMalloc(&c.d_grid, csz * c.ngrid), &c, "alloc grid")) return THP_E_CUDA;
     if (cuda_status(cudaMalloc(&c.d_qfacp, esz * c.ngrid), &c, "alloc qfac")) return THP_E_CUDA;
     if (cuda_status(cudaMalloc(&c.d_conv_buf, csz * c.ngrid), &c, "alloc grid")) return THP_E_CUDA;
+    if (cuda_status(cudaMalloc(&c.d_pot, esz * c.ngrid), &c, "alloc grid")) return THP_E_CUDA;
     c.cap_ngrid = c.ngrid;
   }
   c.conv_r[0] = c.conv_r[1] = 1;
@@ -704,7 +706,7 @@ int plan_prefetch(int device, const int nfft[3], int mixed) {
 void pme_free(Ctx& c) {
   if (c.have_plan) give_plan(plan_key(c), c.plan);
   c.have_plan = false;
-  for (void** p : {&c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf}) {
+  for (void** p : {&c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf, &c.d_pot}) {
     cudaFree(*p);
     *p = nullptr;
   }
@@ -878,7 +880,7 @@ static void spread_dipoles(Ctx& c, const PmeGeom& g, const V* vec, int check_sto
   }
 }
 
-int launch_convolve(Ctx& c, int check_stop) { return convolve(c, check_stop); }
+int launch_convolve(Ctx& c, int check_stop, bool real) { return convolve(c, check_stop, real); }
 
 // Spread of the small systems' CG vector (warp per site): update forms
 // pp = zr + beta pp first; the mixed form also writes the partner records.

@@ -198,13 +198,6 @@ __global__ void __launch_bounds__(kBlock) k_cg_combine8(int n, PmeGeom g, const 
                        partials);
 }
 
-// The loop graph's condition as the update kernel, the last of the body, sets
-// it; max_loops 0 outside the loop graph.
-struct LoopCond {
-  cudaGraphConditionalHandle handle;
-  int max_loops;
-};
-
 // mu, residual and preconditioned residual of one CG step (cg_update_block).
 // In the loop graph it also ends the loop: the condition starts at 1 and is
 // only ever cleared, by the block that finds the CG stopped, or after max_loops
@@ -215,10 +208,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_update(int n, const double* __res
                                                       double* __restrict__ mu, V* __restrict__ res,
                                                       V* __restrict__ zr, CgScalars* cg, double* __restrict__ partials,
                                                       double poleps, int politer, LoopCond loop) {
-  const bool stopped = cg->stop;
-  if (loop.max_loops && blockIdx.x == 0 && threadIdx.x == 0 && (++cg->loops >= loop.max_loops || stopped))
-    cudaGraphSetConditional(loop.handle, 0);
-  if (stopped) return;
+  if (cg::loop_entry(loop, cg)) return;
   if (cg_update_block<V>((int)blockIdx.x, (int)gridDim.x, n, pol, h, pp, mu, res, zr, cg, partials, poleps, politer) &&
       loop.max_loops && cg->stop)
     cudaGraphSetConditional(loop.handle, 0);
@@ -316,7 +306,7 @@ int launch_to_orig6(Ctx& c, const double* d_sorted, double* d_orig, int nrhs) {
   return cuda_status(cudaGetLastError(), &c, "to orig");
 }
 
-static void prof_mark(Ctx& c, cudaStream_t s) {
+void prof_mark(Ctx& c, cudaStream_t s) {
   if (!c.profiling) return;
   cudaEvent_t e;
   cudaEventCreate(&e);
@@ -407,6 +397,7 @@ static int matvec_small(Ctx& c, double* x, int init) {
 }
 
 static int enqueue_iteration(Ctx& c, const LoopCond& loop) {
+  if (c.single) return single_iteration(c, loop);
   int st;
   const int nb = (c.n + kBlock - 1) / kBlock;
   if (overlapped(c) && c.mixed) {
@@ -432,8 +423,9 @@ static int enqueue_iteration(Ctx& c, const LoopCond& loop) {
 }
 
 // Initial residual on the guess (newinduce_pme2.f:161-200, 398-417), async.
-int pcg_begin(Ctx& c, int guess) {
+int pcg_begin(Ctx& c, int guess, bool single) {
   int st;
+  c.single = single;
   cudaMemsetAsync(c.d_cg, 0, sizeof(CgScalars), c.stream);
   if (guess == THP_GUESS_DIRECT) {
     k_guess_direct<<<(c.n * 6 + 255) / 256, 256, 0, c.stream>>>(c.n, c.d_pol, c.d_ef, c.d_mu);
@@ -447,6 +439,7 @@ int pcg_begin(Ctx& c, int guess) {
     cudaMemcpyAsync(c.d_ef_prev, c.d_ef, sizeof(double) * 6 * c.n, cudaMemcpyDeviceToDevice, c.stream);
   c.have_ef_prev = true;
   if ((st = cuda_status(cudaGetLastError(), &c, "cg start"))) return st;
+  if (c.single) return single_begin(c);
   if (overlapped(c)) {
     if (c.mixed) {
       k_pp_rec<double><<<(c.n + 255) / 256, 256, 0, c.stream>>>(c.n, 0, nullptr, c.d_mu, c.d_posf, c.d_rec, c.d_mpz,
@@ -475,7 +468,8 @@ static int enqueue_chunk(Ctx& c) {
 int pcg_chunk_async(Ctx& c) {
   // no capture while profiling, nor on the legacy default stream
   if (c.profiling || c.stream == nullptr) return enqueue_chunk(c);
-  if (!c.chunk_exec) {
+  cudaGraphExec_t& exec = c.chunk_exec[c.single];
+  if (!exec) {
     cudaGraph_t g = nullptr;
     int st = cuda_status(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal), &c, "capture");
     if (st) return st;
@@ -485,14 +479,14 @@ int pcg_chunk_async(Ctx& c) {
       if (g) cudaGraphDestroy(g);
       return st_enq ? st_enq : st;
     }
-    st = cuda_status(cudaGraphInstantiate(&c.chunk_exec, g, 0), &c, "instantiate");
+    st = cuda_status(cudaGraphInstantiate(&exec, g, 0), &c, "instantiate");
     cudaGraphDestroy(g);
     if (st) {
-      c.chunk_exec = nullptr;
+      exec = nullptr;
       return st;
     }
   }
-  return cuda_status(cudaGraphLaunch(c.chunk_exec, c.stream), &c, "graph launch");
+  return cuda_status(cudaGraphLaunch(exec, c.stream), &c, "graph launch");
 }
 
 // Builds the CG loop graph: a conditional WHILE node whose body is one
@@ -521,9 +515,9 @@ static bool build_loop_graph(Ctx& c) {
       }
     }
   }
-  if (ok) ok = cudaGraphInstantiate(&c.loop_exec, g, 0) == cudaSuccess;
+  if (ok) ok = cudaGraphInstantiate(&c.loop_exec[c.single], g, 0) == cudaSuccess;
   if (!ok) {
-    c.loop_exec = nullptr;
+    c.loop_exec[c.single] = nullptr;
     cudaGetLastError();  // clear a refused step so later status checks see only their own errors
   }
   cudaGraphDestroy(g);
@@ -535,9 +529,10 @@ static bool build_loop_graph(Ctx& c) {
 // without waiting.  -1 when the loop graph is not available.
 int pcg_loop_async(Ctx& c) {
   if (!THP_DEVICE_LOOP || c.profiling || c.stream == nullptr) return -1;
-  if (c.loop_state == 0) c.loop_state = build_loop_graph(c) ? 1 : -1;
-  if (c.loop_state < 0) return -1;
-  int st = cuda_status(cudaGraphLaunch(c.loop_exec, c.stream), &c, "loop graph launch");
+  int& state = c.loop_state[c.single];
+  if (state == 0) state = build_loop_graph(c) ? 1 : -1;
+  if (state < 0) return -1;
+  int st = cuda_status(cudaGraphLaunch(c.loop_exec[c.single], c.stream), &c, "loop graph launch");
   if (st) return st;
   return cuda_status(cudaMemcpyAsync(c.h_cg, c.d_cg, sizeof(CgScalars), cudaMemcpyDeviceToHost, c.stream), &c,
                      "cg scalars");
@@ -555,9 +550,9 @@ int pcg_status(Ctx& c) {
 // Like run_pcg, but with the device loop available it only enqueues the CG
 // and the copy of its scalars (*pending = true); the caller synchronises and
 // then reads pcg_status.
-int run_pcg_async(Ctx& c, int guess, bool* pending) {
+int run_pcg_async(Ctx& c, int guess, bool* pending, bool single) {
   *pending = false;
-  int st = pcg_begin(c, guess);
+  int st = pcg_begin(c, guess, single);
   if (st) return st;
   st = pcg_loop_async(c);
   if (st >= 0) {
@@ -596,6 +591,7 @@ int run_pcg(Ctx& c, int guess) {
 }
 
 int launch_epol(Ctx& c) {
+  if (c.single) return single_epol(c);
   const int nb = (c.n + kBlock - 1) / kBlock;
   if (overlapped(c) && c.mixed)
     k_epol<float><<<nb, kBlock, 0, c.stream>>>(c.n, c.d_mu, c.d_ef, c.d_resf, c.d_cg, c.d_partials);
