@@ -187,7 +187,10 @@ __global__ void __launch_bounds__(kBlock) kb_row(const BatchSys* __restrict__ sy
 }
 
 // h = T_real pp + pp/alpha + dipfield(pp) - self term, the dipole field
-// gathered from the convolved grid (fphi_uind_site), pp.h and alpha
+// gathered from the convolved grid (fphi_uind_site), pp.h and alpha.  A thread
+// per atom: with every system's atoms in flight the gathers' instructions
+// count, not their latency (18 us a batched iteration of 32 boxes; eight lanes
+// per atom, which serve a single small system, 40).
 template <bool MIXED>
 __global__ void __launch_bounds__(kBlock) kb_combine(const BatchSys* __restrict__ sys, const int2* __restrict__ items,
                                                      int nitems) {
@@ -196,8 +199,8 @@ __global__ void __launch_bounds__(kBlock) kb_combine(const BatchSys* __restrict_
     const BatchSys& s = sys[w.x];
     if (s.cg->stop) continue;
     using T = typename std::conditional<MIXED, float, double>::type;
-    cg_combine8_block<T>(w.y, s.nblk_mv[0], s.n, s.g, s.pos, s.conv, s.pp, s.pol, s.ef, s.term, 0, s.h, s.res, s.zr,
-                         s.pp, s.cg, s.partials);
+    cg_combine_block<T, double, double>(w.y, s.nblk, s.n, s.g, s.pos, s.conv, s.pp, s.pol, s.ef, s.term, 0, s.h, s.res,
+                                        s.zr, s.pp, s.cg, s.partials);
   }
 }
 
@@ -410,19 +413,18 @@ static int enqueue_body(BatchPlan& p, const BatchTune& t, cudaGraphConditionalHa
   mark();
   const int g = t.gpw - 1;
   const int mb = std::max(1, std::min(p.n_mv_items[g], 2 * t.blocks * p.sms));
-  const int cb = std::max(1, std::min(p.n_mv_items[0], 16 * p.sms));
   if (p.mixed) {
     if (t.gpw == 1)
       kb_row<true, 1><<<mb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[g], p.n_mv_items[g]);
     else
       kb_row<true, 2><<<mb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[g], p.n_mv_items[g]);
-    kb_combine<true><<<cb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[0], p.n_mv_items[0]);
+    kb_combine<true><<<ab, kBlock, 0, p.stream>>>(p.d_sys, p.d_atom_items, p.n_atom_items);
   } else {
     if (t.gpw == 1)
       kb_row<false, 1><<<mb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[g], p.n_mv_items[g]);
     else
       kb_row<false, 2><<<mb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[g], p.n_mv_items[g]);
-    kb_combine<false><<<cb, kBlock, 0, p.stream>>>(p.d_sys, p.d_mv_items[0], p.n_mv_items[0]);
+    kb_combine<false><<<ab, kBlock, 0, p.stream>>>(p.d_sys, p.d_atom_items, p.n_atom_items);
   }
   mark();
   kb_update<<<ab, kBlock, 0, p.stream>>>(p.d_sys, p.d_atom_items, p.n_atom_items);

@@ -340,8 +340,11 @@ __global__ void __launch_bounds__(256) k1_rec(int n, int update, Box box, const 
   store3(r + 3, v);
 }
 
+// One block of pair-stream entries a round in FP64 (64 registers: 250 us at
+// 288,000 atoms; two blocks 261, three 274) and four in FP32, both compiled for
+// 8 blocks per SM (FP32: 120 us; at the compiler's 66 registers and 7 blocks 129).
 #ifndef THP_GROW1_U64
-#define THP_GROW1_U64 2
+#define THP_GROW1_U64 1
 #endif
 #ifndef THP_GROW1_U32
 #define THP_GROW1_U32 4
@@ -349,8 +352,11 @@ __global__ void __launch_bounds__(256) k1_rec(int n, int update, Box box, const 
 
 // T_real x without the diagonal (tmatxb_pme, newinduce_pme.f:1392-1668); lane
 // j < 3 of an atom writes component j
+#ifndef THP_ROW1_MINB
+#define THP_ROW1_MINB 8
+#endif
 template <typename T, bool NOL1, typename HV>
-__global__ void __launch_bounds__(kBlock) k1_row(PairRows pr, Box box, const T* __restrict__ rec,
+__global__ void __launch_bounds__(kBlock, THP_ROW1_MINB) k1_row(PairRows pr, Box box, const T* __restrict__ rec,
                                                  const CgScalars* __restrict__ cg, int check_stop, float interior,
                                                  HV* __restrict__ hreal) {
   if (check_stop && cg->stop) return;
