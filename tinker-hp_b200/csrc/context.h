@@ -158,6 +158,7 @@ struct Ctx {
   size_t ngrid = 0;
   cufftHandle plan = 0;
   bool have_plan = false;
+  void* d_grids = nullptr;  // the allocation of the grid arrays below
   int plan_dims[3] = {0, 0, 0};
   size_t cap_ngrid = 0;
   void* d_grid = nullptr;  // cufftDoubleComplex or cufftComplex

@@ -487,48 +487,6 @@ PmeGeom geom_of(const Ctx& c) {
   return g;
 }
 
-// cuFFT of the whole grid: forward in place, inverse into d_conv (d_grid
-// itself without the three-kernel convolution)
-int fft(Ctx& c, int dir) {
-  cufftResult r;
-  void* out = dir == CUFFT_FORWARD ? c.d_grid : c.d_conv;
-  if (c.mixed)
-    r = cufftExecC2C(c.plan, (cufftComplex*)c.d_grid, (cufftComplex*)out, dir);
-  else
-    r = cufftExecZ2Z(c.plan, (cufftDoubleComplex*)c.d_grid, (cufftDoubleComplex*)out, dir);
-  if (r != CUFFT_SUCCESS) {
-    c.last_msg = "cuFFT exec failed";
-    return THP_E_CUDA;
-  }
-  return THP_OK;
-}
-
-// d_grid -> d_conv: forward transform, influence function, inverse
-// transform.  Three kernels where the grid allows (at 120^3: 73 -> 38 us FP32,
-// 98 -> 53 us FP64 against cuFFT's six launches and the product; 60^3 34 -> 15 us), else
-// cuFFT.  real (three-kernel form only): one real per point in the front of
-// d_grid, the result in d_pot.
-int convolve(Ctx& c, int check_stop, bool real = false) {
-  if (c.conv) {
-    const conv::Sys s{c.d_grid, c.d_conv, c.d_qfacp, c.d_cg, c.d_pot};
-    const cudaError_t e = c.mixed ? launch_conv32(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream)
-                                  : launch_conv64(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream);
-    return cuda_status(e, &c, "convolution");
-  }
-  int st = fft(c, CUFFT_FORWARD);
-  if (st) return st;
-  int blocks = 148 * 8;
-  if (c.mixed)
-    k_qfac<cufftComplex, float><<<blocks, 256, 0, c.stream>>>(c.ngrid, (const float*)c.d_qfac,
-                                                             (cufftComplex*)c.d_grid, c.d_cg, check_stop);
-  else
-    k_qfac<cufftDoubleComplex, double><<<blocks, 256, 0, c.stream>>>(
-        c.ngrid, (const double*)c.d_qfac, (cufftDoubleComplex*)c.d_grid, c.d_cg, check_stop);
-  st = cuda_status(cudaGetLastError(), &c, "qfac");
-  if (st) return st;
-  return fft(c, CUFFT_INVERSE);
-}
-
 // Process-wide cache of cuFFT plans by device, dimensions and type: a
 // context that is destroyed or re-targeted to another grid gives its plan
 // back, and the next context of that shape takes it instead of planning
@@ -570,6 +528,64 @@ bool plan_cached(const PlanKey& k) {
   for (const auto& p : g_plans)
     if (p.first == k) return true;
   return false;
+}
+
+// the context's plan of its grid (cuFFT dims: slowest first; data [n3][n2][n1]),
+// from the cache or new; not under capture
+int make_plan(Ctx& c) {
+  if (!take_plan(plan_key(c), &c.plan) &&
+      cufftPlan3d(&c.plan, c.nfft[2], c.nfft[1], c.nfft[0], c.mixed ? CUFFT_C2C : CUFFT_Z2Z) != CUFFT_SUCCESS) {
+    c.last_msg = "cufftPlan3d failed";
+    return THP_E_CUDA;
+  }
+  c.have_plan = true;
+  cufftSetStream(c.plan, c.stream);
+  return THP_OK;
+}
+
+// cuFFT of the whole grid: forward in place, inverse into d_conv (d_grid
+// itself without the three-kernel convolution)
+int fft(Ctx& c, int dir) {
+  if (!c.have_plan) {
+    if (int st = make_plan(c)) return st;
+  }
+  cufftResult r;
+  void* out = dir == CUFFT_FORWARD ? c.d_grid : c.d_conv;
+  if (c.mixed)
+    r = cufftExecC2C(c.plan, (cufftComplex*)c.d_grid, (cufftComplex*)out, dir);
+  else
+    r = cufftExecZ2Z(c.plan, (cufftDoubleComplex*)c.d_grid, (cufftDoubleComplex*)out, dir);
+  if (r != CUFFT_SUCCESS) {
+    c.last_msg = "cuFFT exec failed";
+    return THP_E_CUDA;
+  }
+  return THP_OK;
+}
+
+// d_grid -> d_conv: forward transform, influence function, inverse
+// transform.  Three kernels where the grid allows (at 120^3: 73 -> 38 us FP32,
+// 98 -> 53 us FP64 against cuFFT's six launches and the product; 60^3 34 -> 15 us), else
+// cuFFT.  real (three-kernel form only): one real per point in the front of
+// d_grid, the result in d_pot.
+int convolve(Ctx& c, int check_stop, bool real = false) {
+  if (c.conv) {
+    const conv::Sys s{c.d_grid, c.d_conv, c.d_qfacp, c.d_cg, c.d_pot};
+    const cudaError_t e = c.mixed ? launch_conv32(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream)
+                                  : launch_conv64(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream);
+    return cuda_status(e, &c, "convolution");
+  }
+  int st = fft(c, CUFFT_FORWARD);
+  if (st) return st;
+  int blocks = 148 * 8;
+  if (c.mixed)
+    k_qfac<cufftComplex, float><<<blocks, 256, 0, c.stream>>>(c.ngrid, (const float*)c.d_qfac,
+                                                             (cufftComplex*)c.d_grid, c.d_cg, check_stop);
+  else
+    k_qfac<cufftDoubleComplex, double><<<blocks, 256, 0, c.stream>>>(
+        c.ngrid, (const double*)c.d_qfac, (cufftDoubleComplex*)c.d_grid, c.d_cg, check_stop);
+  st = cuda_status(cudaGetLastError(), &c, "qfac");
+  if (st) return st;
+  return fft(c, CUFFT_INVERSE);
 }
 
 // qfac(k) = exp(-pi^2 h^2 / a^2) / (pi V h^2 bsmod1 bsmod2 bsmod3), zero at
@@ -615,6 +631,12 @@ static const std::vector<double>& dftmod_cached(int nfft) {
   return it->second;  // map nodes are stable: the reference outlives the lock
 }
 
+static void free_grids(Ctx& c) {
+  cudaFree(c.d_grids);
+  for (void** p : {&c.d_grids, &c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf, &c.d_pot}) *p = nullptr;
+  c.cap_ngrid = 0;
+}
+
 int pme_init(Ctx& c) {
   for (int d = 0; d < 3; ++d) c.nfft[d] = c.cfg.nfft[d];
   c.ngrid = (size_t)c.nfft[0] * c.nfft[1] * c.nfft[2];
@@ -628,16 +650,21 @@ int pme_init(Ctx& c) {
   // grid buffers are kept while they are large enough (a re-targeted
   // context reuses them)
   if (c.ngrid > c.cap_ngrid) {
-    for (void** p : {&c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf, &c.d_pot}) {
-      cudaFree(*p);
-      *p = nullptr;
+    free_grids(c);
+    // one allocation, each array on a 256-byte boundary
+    const struct {
+      void** p;
+      size_t bytes;
+    } grids[] = {{&c.d_grid, csz * c.ngrid},   {&c.d_conv_buf, csz * c.ngrid}, {&c.d_qfac, esz * c.ngrid},
+                 {&c.d_qfacp, esz * c.ngrid}, {&c.d_pot, esz * c.ngrid}};
+    size_t total = 0;
+    for (const auto& g : grids) total += (g.bytes + 255) / 256 * 256;
+    if (cuda_status(cudaMalloc(&c.d_grids, total), &c, "alloc grid")) return THP_E_CUDA;
+    char* at = static_cast<char*>(c.d_grids);
+    for (const auto& g : grids) {
+      *g.p = at;
+      at += (g.bytes + 255) / 256 * 256;
     }
-    c.cap_ngrid = 0;
-    if (cuda_status(cudaMalloc(&c.d_qfac, esz * c.ngrid), &c, "alloc qfac")) return THP_E_CUDA;
-    if (cuda_status(cudaMalloc(&c.d_grid, csz * c.ngrid), &c, "alloc grid")) return THP_E_CUDA;
-    if (cuda_status(cudaMalloc(&c.d_qfacp, esz * c.ngrid), &c, "alloc qfac")) return THP_E_CUDA;
-    if (cuda_status(cudaMalloc(&c.d_conv_buf, csz * c.ngrid), &c, "alloc grid")) return THP_E_CUDA;
-    if (cuda_status(cudaMalloc(&c.d_pot, esz * c.ngrid), &c, "alloc grid")) return THP_E_CUDA;
     c.cap_ngrid = c.ngrid;
   }
   c.conv_r[0] = c.conv_r[1] = 1;
@@ -669,24 +696,18 @@ int pme_init(Ctx& c) {
   // no host wait: the influence function is ready, stream-ordered, for the
   // context's next solve (bsm is copied out before the call returns)
   if (cuda_status(cudaGetLastError(), &c, "qfac")) return THP_E_CUDA;
-  // cuFFT dims: slowest first; data [n3][n2][n1]; the plan is kept when the
-  // grid dimensions are unchanged
-  const bool same = c.have_plan && c.plan_dims[0] == c.nfft[0] && c.plan_dims[1] == c.nfft[1] &&
-                    c.plan_dims[2] == c.nfft[2];
+  // the plan is kept when the grid dimensions are unchanged; a grid that the
+  // three-kernel convolution covers gets one when a virial first asks for it
+  const bool same = c.plan_dims[0] == c.nfft[0] && c.plan_dims[1] == c.nfft[1] && c.plan_dims[2] == c.nfft[2];
   if (!same) {
     if (c.have_plan) give_plan(plan_key(c), c.plan);
     c.have_plan = false;
     for (int d = 0; d < 3; ++d) c.plan_dims[d] = c.nfft[d];
-    if (!take_plan(plan_key(c), &c.plan)) {
-      cufftResult r = cufftPlan3d(&c.plan, c.nfft[2], c.nfft[1], c.nfft[0], c.mixed ? CUFFT_C2C : CUFFT_Z2Z);
-      if (r != CUFFT_SUCCESS) {
-        c.last_msg = "cufftPlan3d failed";
-        return THP_E_CUDA;
-      }
-    }
-    c.have_plan = true;
   }
-  cufftSetStream(c.plan, c.stream);
+  if (!c.conv && !c.have_plan) {
+    if (int st = make_plan(c)) return st;
+  }
+  if (c.have_plan) cufftSetStream(c.plan, c.stream);
   return cuda_status(cudaGetLastError(), &c, "pme init");
 }
 
@@ -694,7 +715,8 @@ int pme_init(Ctx& c) {
 // registered, so the first request of a new shape does not wait for it).
 int plan_prefetch(int device, const int nfft[3], int mixed) {
   const PlanKey k{device, nfft[0], nfft[1], nfft[2], mixed};
-  if (plan_cached(k)) return THP_OK;
+  int r1, r2;
+  if (conv_covers(nfft, mixed, &r1, &r2) || plan_cached(k)) return THP_OK;
   if (cudaSetDevice(device) != cudaSuccess) return THP_E_CUDA;
   cufftHandle plan;
   if (cufftPlan3d(&plan, nfft[2], nfft[1], nfft[0], mixed ? CUFFT_C2C : CUFFT_Z2Z) != CUFFT_SUCCESS)
@@ -706,12 +728,8 @@ int plan_prefetch(int device, const int nfft[3], int mixed) {
 void pme_free(Ctx& c) {
   if (c.have_plan) give_plan(plan_key(c), c.plan);
   c.have_plan = false;
-  for (void** p : {&c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf, &c.d_pot}) {
-    cudaFree(*p);
-    *p = nullptr;
-  }
+  free_grids(c);
   c.d_conv = nullptr;
-  c.cap_ngrid = 0;
 }
 
 // d_grid to zero: what cuFFT's transforms in place leave has to go before
