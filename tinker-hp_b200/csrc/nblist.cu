@@ -337,15 +337,11 @@ __device__ __forceinline__ int axis_cells(int c, int nc, int q) {
 #define THP_LIST_WARP_ATOMS 20000
 #endif
 
-// candidates loaded together by the per-row-shift list build
-#ifndef THP_LIST_BATCH
-#define THP_LIST_BATCH 8
-#endif
-
-// 1: larger systems with at least 7 cells per axis screen their candidates
-// with one periodic shift per candidate row (list_row_shifted)
-#ifndef THP_LIST_SHIFTED
-#define THP_LIST_SHIFTED 1
+// systems of at least this many atoms (and 7 cells per axis) build theirs with
+// k_build_list_split; below, a warp per atom has more threads in flight (4,113
+// atoms 28 against 37 us, 6,300 atoms 44 against 36)
+#ifndef THP_LIST_SPLIT_ATOMS
+#define THP_LIST_SPLIT_ATOMS 5000
 #endif
 
 // The list decision for candidate k of atom i: the FP32 screen accepts below
@@ -380,6 +376,13 @@ struct ListTest {
     }
     return exact(pi, k, pos);
   }
+};
+
+// The cell grid: counts, edges, and the square of the list radius with what
+// the FP32 positions and cell faces can be off by.
+struct ListCells {
+  int nx, ny, nz;
+  float ey, ez, ivx, reach2;
 };
 
 // The list row of atom i, its candidates read from global memory.
@@ -424,80 +427,166 @@ __device__ __forceinline__ void list_row_global(int i, int cap8, const ListTest&
   if (cnt > maxnb) atomicOr(flags, DEV_LIST_OVERFLOW);
 }
 
-// The same row with one periodic shift per candidate row instead of a wrap
-// per candidate: with at least 7 cells along every axis, every candidate of
-// the +-2 window lies within 3 cells (< half a box) of the atom once the
-// rows past a face are shifted by one box length, so the FP32 screen is
-// fi - shift - fk with no per-candidate image.  The screen's error bound is
-// the same (two roundings per coordinate); the exact FP64 test still images
-// each undecided pair itself.
-__device__ __forceinline__ void list_row_shifted(int i, int cap8, const ListTest& lt, int ncx, int ncy, int ncz,
-                                                 const double4* __restrict__ pos, const float4* __restrict__ posf,
-                                                 const int* __restrict__ scell, const int* __restrict__ cell_start,
-                                                 const int* __restrict__ cell_count, int maxnb,
-                                                 int* __restrict__ nnb, int* __restrict__ nb,
-                                                 int* __restrict__ flags) {
-  const double4 pi = pos[i];
-  const float4 fi = posf[i];
-  const int c = scell[i];
-  const int cx = c % ncx, cy = (c / ncx) % ncy, cz = c / (ncx * ncy);
-  int a0, a1, b0, b1;
-  row_ranges(cx, ncx, a0, a1, b0, b1);
-  // part b lies past the lower face (cx - 2 < 0) or the upper one
-  const float fxb = cx < 2 ? fi.x + lt.bx : fi.x - lt.bx;
-  int* __restrict__ row = nb + pair_slot(cap8, i, 0);  // entry s: row[s + 3 (s & ~7)]
-  int cnt = 0;
-  for (int qz = 0; qz < 5; ++qz) {
-    const int zr = cz + qz - 2;
-    const int z = zr < 0 ? zr + ncz : (zr >= ncz ? zr - ncz : zr);
-    const float fz = zr < 0 ? fi.z + lt.bz : (zr >= ncz ? fi.z - lt.bz : fi.z);
-    for (int qy = 0; qy < 5; ++qy) {
-      const int yr = cy + qy - 2;
-      const int y = yr < 0 ? yr + ncy : (yr >= ncy ? yr - ncy : yr);
-      const float fy = yr < 0 ? fi.y + lt.by : (yr >= ncy ? fi.y - lt.by : fi.y);
-      const int rowbase = (z * ncy + y) * ncx;
-#pragma unroll
-      for (int part = 0; part < 2; ++part) {
-        const int x0 = part ? b0 : a0, x1 = part ? b1 : a1;
-        if (x0 > x1) continue;
-        const float fx = part ? fxb : fi.x;
-        const int k0 = cell_start[rowbase + x0];
-        const int k1 = cell_start[rowbase + x1] + cell_count[rowbase + x1];
-        // candidates in batches of THP_LIST_BATCH, all loads of a batch
-        // issued before its tests (a slot past the range reads as far away)
-        for (int kb = k0; kb < k1; kb += THP_LIST_BATCH) {
-          float4 fk[THP_LIST_BATCH];
-#pragma unroll
-          for (int u = 0; u < THP_LIST_BATCH; ++u)
-            fk[u] = kb + u < k1 ? __ldg(posf + kb + u) : make_float4(3.0e18f, 3.0e18f, 3.0e18f, 0.f);
-#pragma unroll
-          for (int u = 0; u < THP_LIST_BATCH; ++u) {
-            const int k = kb + u;
-            const float dx = fx - fk[u].x, dy = fy - fk[u].y, dz = fz - fk[u].z;
-            const float r2f = dx * dx + dy * dy + dz * dz;
-            if (r2f > lt.hi || k == i) continue;
-            if (r2f >= lt.lo && !lt.exact(pi, k, pos)) continue;
-            if (cnt < maxnb) row[cnt + 3 * (cnt & ~7)] = k;
-            ++cnt;
-          }
-        }
-      }
-    }
-  }
-  nnb[i] = cnt;
-  if (cnt > maxnb) atomicOr(flags, DEV_LIST_OVERFLOW);
+// Five warps build the rows of 32 consecutive atoms: lane = atom, warp w the
+// rows of cells (qy, qz) with qy = (w + 2 qz) mod 5, one per z layer, so that
+// the rows near the atom, which hold most of its partners, fall on different
+// warps.  For boxes of at least 7 cells per axis (and the FP32 screen):
+//   * one periodic shift per candidate row instead of a wrap per candidate:
+//     every candidate of the +-2 window lies within 3 cells (< half a box) of
+//     the atom once the rows past a face are shifted by one box length.  The
+//     screen's error bound is the same (two roundings per coordinate); the
+//     exact FP64 test images each undecided pair itself;
+//   * a row is walked only over the cells the list sphere reaches in it
+//     (445 candidates per atom in water at a cell edge of 3.76 A and 497 at
+//     4.28 A; the whole windows hold 668 and 982);
+//   * accepted partners wait in shared memory; a row's warps then write it
+//     together, 8 consecutive slots per atom at a time.  A lane with more than
+//     kListBuf partners (water: 30 to 37, at most 64) walks its rows again once
+//     its first slot is known and writes them itself.
+// What bounds it is issue and, in smaller systems, the chain of loads: a
+// thread per atom leaves a 32,000-atom system two warps per scheduler.
+// 288,000 atoms: 404 us (a thread per atom 490), 32,000: 76 (123), 9,003: 43 (a
+// warp per atom 56).  Buffers of 48 entries send a few lanes around again
+// (657 us at 288,000 atoms); batches of 2, 3, 4 and 8 candidates take 434, 404,
+// 431 and 535 us: a row holds 18 on average.
+constexpr int kListWarps = 5;
+#ifndef THP_LIST_BUF
+#define THP_LIST_BUF 64
+#endif
+constexpr int kListBuf = THP_LIST_BUF;
+// candidates loaded together
+#ifndef THP_LIST_BATCH
+#define THP_LIST_BATCH 3
+#endif
+
+// cells lo..hi of the +-2 window around cell c, c among them, that lie within
+// ext of coordinate f (from the box's lower face), cell edges 1/inv
+__device__ __forceinline__ void reached_cells(int c, float f, float ext, float inv, int& lo, int& hi) {
+  lo = min(c, max(c - 2, (int)floorf((f - ext) * inv)));
+  hi = max(c, min(c + 2, (int)floorf((f + ext) * inv)));
 }
 
-__global__ void __launch_bounds__(128, THP_LIST_MINB) k_build_list_shifted(int n, int cap8, ListTest lt, int ncx,
-                                                    int ncy, int ncz, const double4* __restrict__ pos,
-                                                    const float4* __restrict__ posf, const int* __restrict__ scell,
-                                                    const int* __restrict__ cell_start,
-                                                    const int* __restrict__ cell_count, int maxnb,
-                                                    int* __restrict__ nnb, int* __restrict__ nb,
-                                                    int* __restrict__ flags) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  list_row_shifted(i, cap8, lt, ncx, ncy, ncz, pos, posf, scell, cell_start, cell_count, maxnb, nnb, nb, flags);
+// distance from f to cell q of edge e
+__device__ __forceinline__ float cell_gap(float f, int q, float e) {
+  return fmaxf(0.f, fmaxf(q * e - f, f - (q + 1) * e));
+}
+
+template <typename Add>
+__device__ __forceinline__ void scan_rows(int i, int w, const ListTest& lt, const ListCells& lc,
+                                          const double4* __restrict__ pos, const float4* __restrict__ posf,
+                                          const int* __restrict__ scell, const int* __restrict__ cell_start,
+                                          const int* __restrict__ cell_count, Add&& add) {
+  const float4 fi = posf[i];
+  const int c = scell[i];
+  const int cx = c % lc.nx, cy = (c / lc.nx) % lc.ny, cz = c / (lc.nx * lc.ny);
+  const float rx = fi.x + lt.hx, ry = fi.y + lt.hy, rz = fi.z + lt.hz;
+  int lo = 0, hi = -1, base = 0, k0 = 0, k1 = 0;  // of the row after the current one
+  float sy = 0.f, sz = 0.f;
+  auto next = [&](int qz) {
+    const int qy = (w + 2 * qz) % kListWarps;
+    const int zr = cz + qz - 2, yr = cy + qy - 2;
+    const float gz = cell_gap(rz, zr, lc.ez), gy = cell_gap(ry, yr, lc.ey);
+    const float e2 = lc.reach2 - gz * gz - gy * gy;
+    lo = 0;
+    hi = -1;
+    k0 = k1 = 0;
+    if (e2 < 0.f) return;
+    reached_cells(cx, rx, sqrtf(e2), lc.ivx, lo, hi);
+    const int z = zr < 0 ? zr + lc.nz : (zr >= lc.nz ? zr - lc.nz : zr);
+    const int y = yr < 0 ? yr + lc.ny : (yr >= lc.ny ? yr - lc.ny : yr);
+    sz = zr < 0 ? fi.z + lt.bz : (zr >= lc.nz ? fi.z - lt.bz : fi.z);
+    sy = yr < 0 ? fi.y + lt.by : (yr >= lc.ny ? fi.y - lt.by : fi.y);
+    base = (z * lc.ny + y) * lc.nx;
+    const int x1 = base + min(hi, lc.nx - 1);
+    k0 = cell_start[base + max(lo, 0)];
+    k1 = cell_start[x1] + cell_count[x1];
+  };
+  auto walk = [&](int ka, int ke, float fx, float fy, float fz) {
+    for (int kb = ka; kb < ke; kb += THP_LIST_BATCH) {
+      // all loads of a batch before its tests (a slot past the range reads as far away)
+      float4 fk[THP_LIST_BATCH];
+#pragma unroll
+      for (int u = 0; u < THP_LIST_BATCH; ++u)
+        fk[u] = kb + u < ke ? __ldg(posf + kb + u) : make_float4(3.0e18f, 3.0e18f, 3.0e18f, 0.f);
+#pragma unroll
+      for (int u = 0; u < THP_LIST_BATCH; ++u) {
+        const int k = kb + u;
+        const float dx = fx - fk[u].x, dy = fy - fk[u].y, dz = fz - fk[u].z;
+        const float r2f = dx * dx + dy * dy + dz * dz;
+        if (r2f > lt.hi || k == i) continue;
+        if (r2f >= lt.lo && !lt.exact(pos[i], k, pos)) continue;
+        add(k);
+      }
+    }
+  };
+  next(0);
+#pragma unroll 1
+  for (int qz = 0; qz < 5; ++qz) {
+    const int a = k0, b = k1, l = lo, h = hi, rb = base;
+    const float fy = sy, fz = sz;
+    if (qz < 4) next(qz + 1);
+    walk(a, b, fi.x, fy, fz);
+    if (l < 0) {  // the part past the lower face
+      const int x1 = rb + lc.nx - 1;
+      walk(cell_start[rb + l + lc.nx], cell_start[x1] + cell_count[x1], fi.x + lt.bx, fy, fz);
+    } else if (h >= lc.nx) {  // past the upper face
+      const int x1 = rb + h - lc.nx;
+      walk(cell_start[rb], cell_start[x1] + cell_count[x1], fi.x - lt.bx, fy, fz);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(32 * kListWarps, THP_LIST_MINB) k_build_list_split(
+    int n, int cap8, ListTest lt, ListCells lc, const double4* __restrict__ pos, const float4* __restrict__ posf,
+    const int* __restrict__ scell, const int* __restrict__ cell_start, const int* __restrict__ cell_count, int maxnb,
+    int* __restrict__ nnb, int* __restrict__ nb, int* __restrict__ flags) {
+  __shared__ int buf[kListBuf][kListWarps][32];
+  __shared__ int part[kListWarps][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i0 = blockIdx.x * 32, i = i0 + lane;
+  int cnt = 0;
+  if (i < n)
+    scan_rows(i, w, lt, lc, pos, posf, scell, cell_start, cell_count, [&](int k) {
+      if (cnt < kListBuf) buf[cnt][w][lane] = k;
+      ++cnt;
+    });
+  part[w][lane] = cnt;
+  __syncthreads();
+  if (cnt > kListBuf) {
+    int s = 0;
+    for (int v = 0; v < w; ++v) s += part[v][lane];
+    int* __restrict__ row = nb + pair_slot(cap8, i, 0);  // entry s: row[s + 3 (s & ~7)]
+    scan_rows(i, w, lt, lc, pos, posf, scell, cell_start, cell_count, [&](int k) {
+      if (s < maxnb) row[s + 3 * (s & ~7)] = k;
+      ++s;
+    });
+  }
+  // eight lanes per atom, a group of four atoms per warp: consecutive slots
+  const int a = lane >> 3, j = lane & 7;
+  for (int g = w; g < 8; g += kListWarps) {
+    const int q = 4 * g + a;
+    if (i0 + q >= n) continue;
+    int* __restrict__ row = nb + pair_slot(cap8, i0 + q, 0);
+    int end[kListWarps];
+    int run = 0;
+#pragma unroll
+    for (int v = 0; v < kListWarps; ++v) end[v] = run += part[v][q];
+    if (j == 0) {
+      nnb[i0 + q] = run;
+      if (run > maxnb) atomicOr(flags, DEV_LIST_OVERFLOW);
+    }
+    const int top = min(run, maxnb);
+    for (int s = j; s < top; s += 8) {
+      int v = 0, first = 0;
+#pragma unroll
+      for (int u = 0; u < kListWarps - 1; ++u)
+        if (s >= end[u]) {
+          v = u + 1;
+          first = end[u];
+        }
+      if (part[v][q] <= kListBuf) row[s + 3 * (s & ~7)] = buf[s - first][v][q];
+    }
+  }
 }
 
 __global__ void __launch_bounds__(128, THP_LIST_MINB) k_build_list(int n, int cap8, ListTest lt, int ncx,
@@ -795,15 +884,24 @@ int launch_build_list_on(Ctx& c, cudaStream_t s) {
   lt.hx = 0.5f * lt.bx;
   lt.hy = 0.5f * lt.by;
   lt.hz = 0.5f * lt.bz;
+  ListCells lc;
+  lc.nx = c.nc[0];
+  lc.ny = c.nc[1];
+  lc.nz = c.nc[2];
+  lc.ey = (float)(c.box.l[1] / lc.ny);
+  lc.ez = (float)(c.box.l[2] / lc.nz);
+  lc.ivx = (float)(lc.nx / c.box.l[0]);
+  const double reach = sqrt(mbuf2 * (1.0 + band)) + 16.0 * dr + 1e-3;
+  lc.reach2 = (float)(reach * reach);
   const int cap8 = c.maxpr / 8;
-  if (n < THP_LIST_WARP_ATOMS)
+  if (prefilter && n >= THP_LIST_SPLIT_ATOMS && c.nc[0] >= 7 && c.nc[1] >= 7 && c.nc[2] >= 7)
+    k_build_list_split<<<(n + 31) / 32, 32 * kListWarps, 0, s>>>(n, cap8, lt, lc, c.d_pos, c.d_posf, c.d_scell,
+                                                                 c.d_cell_start, c.d_cell_count, c.maxnb, c.d_nnb,
+                                                                 c.d_nb, c.d_flags);
+  else if (n < THP_LIST_WARP_ATOMS)
     k_build_list_warp<<<(n + 3) / 4, 128, 0, s>>>(n, cap8, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos, c.d_posf,
                                                   c.d_scell, c.d_cell_start, c.d_cell_count, c.maxnb, c.d_nnb,
                                                   c.d_nb, c.d_flags);
-  else if (THP_LIST_SHIFTED && prefilter && c.nc[0] >= 7 && c.nc[1] >= 7 && c.nc[2] >= 7)
-    k_build_list_shifted<<<(n + 127) / 128, 128, 0, s>>>(n, cap8, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos,
-                                                         c.d_posf, c.d_scell, c.d_cell_start, c.d_cell_count,
-                                                         c.maxnb, c.d_nnb, c.d_nb, c.d_flags);
   else
     k_build_list<<<(n + 127) / 128, 128, 0, s>>>(n, cap8, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos, c.d_posf,
                                                  c.d_scell, c.d_cell_start, c.d_cell_count, c.maxnb, c.d_nnb,
