@@ -444,7 +444,7 @@ size_t footprint_bytes(const thp_config& cfg, int* ncell_out) {
   const bool mixed = cfg.precision == THP_MIXED;
   const size_t ngrid = (size_t)cfg.nfft[0] * cfg.nfft[1] * cfg.nfft[2];
   size_t b = 0;
-  b += 3 * ncell * 4 + 2 * n * 4 + 2 * n * 4;          // cells, perm
+  b += 2 * ncell * 4 + 2 * n * 4 + 2 * n * 4;          // cells, perm
   b += (3 + 3 + 13 + 13) * n * 8 + 3 * n * 4;            // staging
   b += n * 32 + n * 16 + 2 * n * 8 + 10 * n * 8 + n * 32 + n * 64;  // sorted data
   b += n * 4 + maxnb * npad * 4;                         // list
@@ -567,7 +567,7 @@ static int size_buffers(Ctx& c) {
     c.slab_cells = nullptr;
     c.cap_ncell = 0;
     const size_t m = c.ncell;
-    st = alloc_slab(c, &c.slab_cells, {item(&c.d_cell_count, m), item(&c.d_cell_start, m), item(&c.d_cell_fill, m)},
+    st = alloc_slab(c, &c.slab_cells, {item(&c.d_cell_count, m), item(&c.d_cell_start, m)},
                     "cells");
     if (!st) c.cap_ncell = c.ncell;
   }

@@ -79,7 +79,6 @@ struct Ctx {
   int ncell = 1;
   int* d_cell_count = nullptr;
   int* d_cell_start = nullptr;
-  int* d_cell_fill = nullptr;
   int* d_atom_cell = nullptr;   // original order
   int* d_scell = nullptr;       // cell of sorted atom
 

@@ -34,12 +34,12 @@ __device__ __forceinline__ int cell_of(const Box& box, int ncx, int ncy, int ncz
 }
 
 __global__ void k_cell_count(int n, Box box, int ncx, int ncy, int ncz, const double* __restrict__ xyz,
-                             int* __restrict__ atom_cell, int* __restrict__ cell_count) {
+                             int* __restrict__ atom_cell, int* __restrict__ cell_count, int* __restrict__ arrival) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int cell = cell_of(box, ncx, ncy, ncz, xyz[i], xyz[n + i], xyz[2 * n + i]);
   atom_cell[i] = cell;
-  atomicAdd(&cell_count[cell], 1);
+  arrival[i] = atomicAdd(&cell_count[cell], 1);
 }
 
 // exclusive scan of m ints by one block of 1024 threads
@@ -66,8 +66,8 @@ __global__ void k_scan_single(int m, const int* __restrict__ in, int* __restrict
 }
 
 // The same scan over many blocks: each block scans 1024 cells (k_scan_tiles,
-// writing its total), one block scans the totals (k_scan_totals), and every
-// block adds its offset (k_scan_offsets).  Used up to 1024 x 1024 cells.
+// writing its total), and every block of k_scan_offsets adds the totals of the
+// tiles before its own.  Used up to 1024 x 1024 cells.
 __device__ __forceinline__ int block_excl_scan_1024(int v, int* s_warp, int* total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int x = v;
@@ -104,52 +104,42 @@ __global__ void __launch_bounds__(1024) k_scan_tiles(int m, const int* __restric
   if (threadIdx.x == 0) tile_sum[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_totals(int nt, int* __restrict__ tile_sum) {
+__global__ void __launch_bounds__(1024) k_scan_offsets(int m, int* __restrict__ out, const int* __restrict__ tile_sum) {
   __shared__ int s_warp[32];
-  const int v = threadIdx.x < nt ? tile_sum[threadIdx.x] : 0;
   int total;
-  const int e = block_excl_scan_1024(v, s_warp, &total);
-  if (threadIdx.x < nt) tile_sum[threadIdx.x] = e;
+  block_excl_scan_1024(threadIdx.x < blockIdx.x ? tile_sum[threadIdx.x] : 0, s_warp, &total);
+  const int i = blockIdx.x * 1024 + threadIdx.x;
+  if (i < m) out[i] += total;
 }
 
-__global__ void k_scan_offsets(int m, int* __restrict__ out, const int* __restrict__ tile_sum) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < m) out[i] += tile_sum[i >> 10];
-}
-
+// an atom's arrival in its cell (arrival[i], from the count) places it; the
+// order inside a cell is whatever the count's atomics made it
 __global__ void k_cell_fill(int n, const int* __restrict__ atom_cell, const int* __restrict__ cell_start,
-                            int* __restrict__ cell_fill, int* __restrict__ perm) {
+                            const int* __restrict__ arrival, int* __restrict__ filled) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int c = atom_cell[i];
-  int p = cell_start[c] + atomicAdd(&cell_fill[c], 1);
-  perm[p] = i;
+  if (i < n) filled[cell_start[atom_cell[i]] + arrival[i]] = i;
 }
 
-// deterministic order inside a cell: ascending original index
-__global__ void k_cell_sort(int ncell, const int* __restrict__ cell_start, const int* __restrict__ cell_count,
+// deterministic order inside a cell, ascending original index: one thread per
+// atom counts the smaller indices of its cell (32,400 atoms: 4 us; one thread
+// sorting each cell in place 18)
+__global__ void k_cell_rank(int n, const int* __restrict__ atom_cell, const int* __restrict__ cell_start,
+                            const int* __restrict__ cell_count, const int* __restrict__ filled,
                             int* __restrict__ perm, int* __restrict__ iperm, int* __restrict__ scell) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
-  int b = cell_start[c], m = cell_count[c];
-  for (int a = 1; a < m; ++a) {
-    int v = perm[b + a];
-    int q = a - 1;
-    while (q >= 0 && perm[b + q] > v) {
-      perm[b + q + 1] = perm[b + q];
-      --q;
-    }
-    perm[b + q + 1] = v;
-  }
-  for (int a = 0; a < m; ++a) {
-    iperm[perm[b + a]] = b + a;
-    scell[b + a] = c;
-  }
+  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const int i = filled[p], c = atom_cell[i];
+  const int b = cell_start[c], m = cell_count[c];
+  int s = b;
+  for (int a = 0; a < m; ++a) s += filled[b + a] < i;
+  perm[s] = i;
+  iperm[i] = s;
+  scell[s] = c;
 }
 
 // The whole cell sort of a small system in one block: cells, counts, scan,
 // fill and the order inside each cell in shared memory, then the special
-// partners in the new numbering.  The seven launches of the general form take
+// partners in the new numbering.  The six launches of the general form take
 // about 3 us each whatever the size; one block keeps up with them to
 // kSortSmallAtoms atoms.
 constexpr int kSortSmallAtoms = 8192, kSortSmallCells = 4096;
@@ -820,23 +810,23 @@ int launch_sort_atoms(Ctx& c, bool carry) {
     return st;
   }
   cudaMemsetAsync(c.d_cell_count, 0, sizeof(int) * c.ncell, s);
-  cudaMemsetAsync(c.d_cell_fill, 0, sizeof(int) * c.ncell, s);
   k_cell_count<<<nb, kBlock, 0, s>>>(n, c.box, c.nc[0], c.nc[1], c.nc[2], c.d_xyz_orig, c.d_atom_cell,
-                                     c.d_cell_count);
+                                     c.d_cell_count, c.d_iperm);
   const int ntile = (c.ncell + 1023) / 1024;
   // the tile totals live in the reduction partials (free outside the CG),
   // which hold 8 ints per 128 atoms plus 64
   if (ntile <= 1024 && (size_t)ntile <= 8 * ((size_t)c.nblk_reduce + 8)) {
     int* tile_sum = reinterpret_cast<int*>(c.d_partials);
     k_scan_tiles<<<ntile, 1024, 0, s>>>(c.ncell, c.d_cell_count, c.d_cell_start, tile_sum);
-    k_scan_totals<<<1, 1024, 0, s>>>(ntile, tile_sum);
-    k_scan_offsets<<<(c.ncell + 255) / 256, 256, 0, s>>>(c.ncell, c.d_cell_start, tile_sum);
+    k_scan_offsets<<<ntile, 1024, 0, s>>>(c.ncell, c.d_cell_start, tile_sum);
   } else {
     k_scan_single<<<1, 1024, 0, s>>>(c.ncell, c.d_cell_count, c.d_cell_start);
   }
-  k_cell_fill<<<nb, kBlock, 0, s>>>(n, c.d_atom_cell, c.d_cell_start, c.d_cell_fill, c.d_perm);
-  k_cell_sort<<<(c.ncell + kBlock - 1) / kBlock, kBlock, 0, s>>>(c.ncell, c.d_cell_start, c.d_cell_count,
-                                                                 c.d_perm, c.d_iperm, c.d_scell);
+  // d_iperm holds the arrivals until the ranks are known; d_nnb is free: the
+  // list of the old order is gone, and every re-sort is followed by a build
+  k_cell_fill<<<nb, kBlock, 0, s>>>(n, c.d_atom_cell, c.d_cell_start, c.d_iperm, c.d_nnb);
+  k_cell_rank<<<nb, kBlock, 0, s>>>(n, c.d_atom_cell, c.d_cell_start, c.d_cell_count, c.d_nnb, c.d_perm, c.d_iperm,
+                                    c.d_scell);
   c.have_perm = true;
   if (m > 0) k_sp_to_sorted<<<(m + 255) / 256, 256, 0, s>>>(m, c.d_iperm, c.d_sp_k, c.d_sp_ks);
   int st = cuda_status(cudaGetLastError(), &c, "sort atoms");
