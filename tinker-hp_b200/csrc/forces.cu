@@ -17,6 +17,7 @@
 // add their contributions does not change the sums.
 #include <type_traits>
 
+#include "damp_dev.cuh"
 #include "grad_dev.cuh"
 #include "kernels.h"
 #include "pme_dev.cuh"
@@ -446,12 +447,13 @@ __global__ void __launch_bounds__(kBlock, MIXED ? THP_FORCE_MINB : 1) k_force_re
     if constexpr (MIXED)
       rinv = rsqrtf(r2);
     else
-      rinv = T(1) / sqrt(r2);
+      rinv = rsqrt(r2);
     const T rr = r2 * rinv, r2inv = rinv * rinv;
     PairRadial<T> p;
     const T ra = (T)ew.a * rr;
-    const T ex = exp(-ra * ra);
-    const T b0 = erfc(ra) * rinv;
+    T ex, er;
+    screen(ra, ex, er);
+    const T b0 = er * rinv;
     const T b1 = (b0 + (T)ew.f1 * ex) * r2inv;
     const T b2 = (T(3) * b1 + (T)ew.f2 * ex) * r2inv;
     const T b3 = (T(5) * b2 + (T)ew.f3 * ex) * r2inv;

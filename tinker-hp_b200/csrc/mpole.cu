@@ -19,6 +19,7 @@
 // by per-block partials summed in block order, so both are deterministic.
 #include <type_traits>
 
+#include "damp_dev.cuh"
 #include "grad_dev.cuh"
 #include "kernels.h"
 #include "pme_dev.cuh"
@@ -62,7 +63,7 @@ __device__ __forceinline__ void mpole_pair(U xr, U yr, U zr, U r2, U scalek, con
   if constexpr (std::is_same<U, float>::value)
     rinv = rsqrtf(r2);
   else
-    rinv = U(1) / sqrt(r2);
+    rinv = rsqrt(r2);
   const U r = r2 * rinv;
   const U r2inv = rinv * rinv;
   // intermediates involving moments and separation distance
@@ -82,8 +83,9 @@ __device__ __forceinline__ void mpole_pair(U xr, U yr, U zr, U r2, U scalek, con
   // reciprocal distance terms with the Ewald damping to order 11
   // (damping.f:17-55); the bare terms only for scaled pairs
   const U ra = (U)ew.a * r;
-  const U ex = exp(-ra * ra);
-  const U b0 = erfc(ra) * rinv;
+  U ex, er;
+  screen(ra, ex, er);
+  const U b0 = er * rinv;
   const U b1 = (b0 + (U)ew.f[0] * ex) * r2inv;
   const U b2 = (U(3) * b1 + (U)ew.f[1] * ex) * r2inv;
   const U b3 = (U(5) * b2 + (U)ew.f[2] * ex) * r2inv;
