@@ -691,11 +691,12 @@ def main():
 
     peaks, peak_kind = measured_peaks()
     # roofline of the real-space row of the mixed CG matvec (the PME branch runs beside it on
-    # another stream; the combine is its own kernel): algorithmic bytes per launch, the FP64 a3 figure 136 N + 4 L with per-atom data
-    # halved in the mixed form: 68 N (positions, polarity, mu in, field out) + 4 L (half list,
-    # 88.4 entries per atom at 7.5 A)
+    # another stream; the combine is its own kernel): algorithmic bytes per launch, the FP64 a3 figure 136 N + 4 L less the second
+    # field's mu and result (48 N, the d and p scales of water agree), per-atom data halved in the
+    # mixed form: 44 N (positions, polarity, mu in, field out) + 4 L (half list, 88.4 entries per
+    # atom at 7.5 A)
     L_entries = 88.4 * n
-    alg_bytes = 68.0 * n + 4.0 * L_entries
+    alg_bytes = 44.0 * n + 4.0 * L_entries
     avg_ms = mv_ms / max(mv_launches, 1)
     achieved = alg_bytes / (avg_ms * 1e-3) / 1e9
     # DRAM bytes per launch (read + write) from one ncu capture of this kernel on the 96,000-atom
@@ -703,7 +704,7 @@ def main():
     # (index and two FP32 coefficients, 12 B per directed pair) plus per-atom data, both
     # proportional to n
     traffic = 182.1e6 * n / 96000.0
-    roof = {"bound": "hbm", "kernel": "k_real_row<mixed> (real-space row of the CG matvec)",
+    roof = {"bound": "hbm", "kernel": "k1_row<mixed> (real-space row of the CG matvec)",
             "limiter": "L1 data pipe (73 % of cycles) and the latency of the dependent stream and partner "
                        "loads; DRAM at 40 % (ncu, 96k-atom capture)",
             "achieved": achieved, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
@@ -801,20 +802,19 @@ def main():
         sv = extras["serving"]
         line["serving"] = {k: sv[k] for k in ("solves_per_s", "p50_ms", "p99_ms", "requests", "rate_req_per_s",
                                               "mean_setup_ms", "mean_solve_ms", "completed", "failed")}
-    # kernels of this library per timed step (cuFFT's not counted; the
-    # positions do not move, so rotpole does not run):
-    #   re-sort 11: dipoles and last E0 out of sorted order (2), cell count,
-    #     scan (3), fill, sort, special pairs to sorted numbering, dipoles and
-    #     last E0 back (2);
+    # kernels of this library per timed step (the positions do not move, so
+    # rotpole does not run; a cold start carries no dipoles through the sort):
+    #   re-sort 6: cell count, scan (2), fill, rank, special pairs to sorted
+    #     numbering;
     #   sorted gather 1; list 1; E_direct + pair stream 1; multipole spread,
-    #     qfac, multipole gather 3;
-    #   CG start 6: direct guess, row records, real row, dipole spread, qfac,
-    #     combine;
-    #   7 per iteration (device-side loop): row records, real row, dipole
-    #     spread, qfac, combine, update, loop condition;
+    #     convolution (3), multipole gather 5;
+    #   CG start 9: direct guess, one field taken, row records, row, dipole
+    #     spread, convolution (3), combine;
+    #   8 per iteration (device-side loop): row records, row, dipole spread,
+    #     convolution (3), combine, update;
     #   Epol 1.
     it = int(np.median(niter))
-    per_step = 11 + 1 + 1 + 1 + 3 + 6 + 7 * it + 1
+    per_step = 6 + 1 + 1 + 1 + 5 + 9 + 8 * it + 1
     line["gpu_launches"] = per_step * steps
     if rank == 0:
         print(json.dumps(line), flush=True)

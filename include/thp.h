@@ -101,7 +101,7 @@ typedef struct thp_ctx thp_ctx;
 int thp_ctx_create(const thp_config* cfg, thp_ctx** out);
 int thp_ctx_destroy(thp_ctx* ctx);
 /* Re-target a context to another system (same precision and device): every
- * device buffer that is large enough and the cuFFT plan of an unchanged grid
+ * device buffer that is large enough and any cuFFT plan of an unchanged grid
  * are kept, so no device memory is freed or allocated unless the new system
  * is larger.  All system state is cleared (parameters, connectivity,
  * positions, multipoles, list, dipoles, bindings), as after thp_ctx_create. */
@@ -160,7 +160,7 @@ int thp_solve_batch(thp_ctx** ctxs, int count, int guess, thp_solve_info* infos)
  * contexts on one device in one precision, each below 20,000 atoms, and runs
  * the CG iterations of all of them as batched persistent kernels: one launch
  * per kernel per iteration walks a device work list of (system, tile) items,
- * the convolution runs as one batched cuFFT transform per grid shape, and the
+ * the convolution runs over all systems of a grid shape at once, and the
  * loop is a conditional WHILE node that runs until every system has stopped.
  * A solve whose systems all take the same start (guess DIRECT, PREVIOUS or
  * HOST after resolution, and the same dipole carry) runs as one graph launch:
