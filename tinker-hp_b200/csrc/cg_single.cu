@@ -473,23 +473,47 @@ __global__ void __launch_bounds__(kBlock) k1_combine8(int n, PmeGeom g, const do
   SiteWeights<T>& s = sw[a8];
   if (j < 3) stage_axis<T>(g, pos[i], j, s);
   __syncwarp();
-  T acc[3] = {0, 0, 0};
   const int gx = s.g0[0];
-  for (int q = j; q < kBs * kBs; q += 8) {
+  auto line = [&](int q) {
+    const int b = q % kBs, c = q / kBs;
+    return ((size_t)wrapk(s.g0[2] + c, g.n3) * g.n2 + wrapk(s.g0[1] + b, g.n2)) * g.n1;
+  };
+  // lines j, j + 8 and j + 16 whole, one point of the last line each, all loads
+  // before the sums: the chain of loads is what bounds this kernel (a solve of
+  // 648 atoms 519 -> 494 us against a loop over the lane's lines)
+  T e[3][kBs];
+#pragma unroll
+  for (int l = 0; l < 3; ++l) {
+    const size_t row = line(j + 8 * l);
+#pragma unroll
+    for (int a = 0; a < kBs; ++a) e[l][a] = __ldg(pot + row + wrapk(gx + a, g.n1));
+  }
+  const T last = j < kBs ? __ldg(pot + line(kBs * kBs - 1) + wrapk(gx + j, g.n1)) : T(0);
+  double xi = 0.0, hi = 0.0, p = 0.0;
+  if (live && j < 3) {
+    xi = x[(size_t)i * 3 + j];
+    hi = h[(size_t)i * 3 + j];
+    p = pol[i];
+  }
+  T acc[3] = {0, 0, 0};
+  auto add = [&](int q, T t0, T t1) {
     const int b = q % kBs, c = q / kBs;
     const T u0 = s.w[1][2 * b], u1 = s.w[1][2 * b + 1], v0 = s.w[2][2 * c], v1 = s.w[2][2 * c + 1];
-    const size_t row = ((size_t)wrapk(s.g0[2] + c, g.n3) * g.n2 + wrapk(s.g0[1] + b, g.n2)) * g.n1;
-    T t0 = 0, t1 = 0;
-#pragma unroll
-    for (int a = 0; a < kBs; ++a) {
-      const T e = __ldg(pot + row + wrapk(gx + a, g.n1));
-      t0 += e * s.w[0][2 * a];
-      t1 += e * s.w[0][2 * a + 1];
-    }
     acc[0] += t1 * u0 * v0;
     acc[1] += t0 * u1 * v0;
     acc[2] += t0 * u0 * v1;
+  };
+#pragma unroll
+  for (int l = 0; l < 3; ++l) {
+    T t0 = 0, t1 = 0;
+#pragma unroll
+    for (int a = 0; a < kBs; ++a) {
+      t0 += e[l][a] * s.w[0][2 * a];
+      t1 += e[l][a] * s.w[0][2 * a + 1];
+    }
+    add(j + 8 * l, t0, t1);
   }
+  if (j < kBs) add(kBs * kBs - 1, last * s.w[0][2 * j], last * s.w[0][2 * j + 1]);
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
@@ -499,9 +523,8 @@ __global__ void __launch_bounds__(kBlock) k1_combine8(int n, PmeGeom g, const do
     const size_t q = (size_t)i * 3 + j;
     const double dip = (j == 0 ? g.a[0] : (j == 1 ? g.a[1] : g.a[2])) *
                        (double)(j == 0 ? acc[0] : (j == 1 ? acc[1] : acc[2]));
-    const double xi = x[q], p = pol[i];
     const double ip = (p == 0.0) ? 1.0 / kTinyPol : 1.0 / p;
-    const double hv = ((h[q] + xi * ip) + dip) - term * xi;
+    const double hv = ((hi + xi * ip) + dip) - term * xi;
     h[q] = hv;
     if (init) {
       const double r = ef[(size_t)i * 6 + j] - hv, z = diag_of(p) * r;
