@@ -700,13 +700,13 @@ def main():
     avg_ms = mv_ms / max(mv_launches, 1)
     achieved = alg_bytes / (avg_ms * 1e-3) / 1e9
     # DRAM bytes per launch (read + write) from one ncu capture of this kernel on the 96,000-atom
-    # box (182.1 MB per launch), scaled by the atom count: the traffic is the streamed pair entries
+    # box (180.9 MB per launch), scaled by the atom count: the traffic is the streamed pair entries
     # (index and two FP32 coefficients, 12 B per directed pair) plus per-atom data, both
     # proportional to n
-    traffic = 182.1e6 * n / 96000.0
+    traffic = 180.9e6 * n / 96000.0
     roof = {"bound": "hbm", "kernel": "k1_row<mixed> (real-space row of the CG matvec)",
-            "limiter": "L1 data pipe (73 % of cycles) and the latency of the dependent stream and partner "
-                       "loads; DRAM at 40 % (ncu, 96k-atom capture)",
+            "limiter": "L1 (73 % of cycles) and the latency of the dependent stream and partner "
+                       "loads; DRAM at 47 % (ncu, 96k-atom capture)",
             "achieved": achieved, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
             "frac": achieved / peaks.get("hbm_gbs"), "peak_kind": peak_kind, "traffic": traffic,
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, 96k-atom capture scaled by n",
