@@ -664,7 +664,7 @@ int matvec_large(Ctx& c, XV* x, int init) {
   const int spw = c.n < THP_SPREAD1_HALF_ATOMS ? 16 : 32, spb = spw * (kSpreadThreads / 32);
   k1_spread<T, XV><<<(c.n + spb - 1) / spb, kSpreadThreads, smem, c.stream>>>(c.n, pme_geom(c), c.d_pos, x, c.d_cg,
                                                                              !init, spw, (T*)c.d_grid);
-  int st2 = cuda_status(cudaGetLastError(), &c, "spread dip");
+  int st2 = spread_status(c, cuda_status(cudaGetLastError(), &c, "spread dip"));
   if (!st2) st2 = launch_convolve(c, !init, true);
   cudaStreamWaitEvent(c.stream, c.ev_join, 0);
   if (st || st2) return st ? st : st2;
@@ -679,7 +679,7 @@ int matvec_small(Ctx& c, double* x, int init) {
   const Vecs<double> v = vecs(c, 0.0);
   k1_spread_small<T><<<(c.n + 3) / 4, 128, 0, c.stream>>>(c.n, pme_geom(c), c.box, c.d_pos, c.d_posf, x, v.zr, c.d_cg,
                                                          !init, records<T>(c), (T*)c.d_grid);
-  int st = cuda_status(cudaGetLastError(), &c, "spread dip");
+  int st = spread_status(c, cuda_status(cudaGetLastError(), &c, "spread dip"));
   if (st) return st;
   cudaEventRecord(c.ev_fork, c.stream);
   cudaStreamWaitEvent(c.stream2, c.ev_fork, 0);

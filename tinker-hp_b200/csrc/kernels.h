@@ -40,6 +40,7 @@ int launch_spread_small(Ctx& c, double* d_vec, int update);  // the small system
 int launch_convolve(Ctx& c, int check_stop, bool real = false);  // real: conv.h
 bool overlap_rows(const Ctx& c);  // the system runs real-space passes on the side stream
 int zero_grid(Ctx& c);  // before a spread: d_grid zero (nothing to do for the three-kernel convolution)
+int spread_status(Ctx& c, int st);  // after a spread that no convolution will follow: d_grid zero again
 struct PmeGeom;
 PmeGeom pme_geom(const Ctx& c);
 int launch_gather_dip(Ctx& c, double* d_out, bool check_stop);

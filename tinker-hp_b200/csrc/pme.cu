@@ -535,6 +535,7 @@ bool plan_cached(const PlanKey& k) {
 int make_plan(Ctx& c) {
   if (!take_plan(plan_key(c), &c.plan) &&
       cufftPlan3d(&c.plan, c.nfft[2], c.nfft[1], c.nfft[0], c.mixed ? CUFFT_C2C : CUFFT_Z2Z) != CUFFT_SUCCESS) {
+    cudaGetLastError();  // the allocation cuFFT was refused: reported here, not by the next launch's check
     c.last_msg = "cufftPlan3d failed";
     return THP_E_CUDA;
   }
@@ -543,12 +544,13 @@ int make_plan(Ctx& c) {
   return THP_OK;
 }
 
+// the context's grid has a plan (a grid that the three-kernel convolution
+// covers is made without one)
+int ensure_plan(Ctx& c) { return c.have_plan ? THP_OK : make_plan(c); }
+
 // cuFFT of the whole grid: forward in place, inverse into d_conv (d_grid
 // itself without the three-kernel convolution)
 int fft(Ctx& c, int dir) {
-  if (!c.have_plan) {
-    if (int st = make_plan(c)) return st;
-  }
   cufftResult r;
   void* out = dir == CUFFT_FORWARD ? c.d_grid : c.d_conv;
   if (c.mixed)
@@ -562,6 +564,13 @@ int fft(Ctx& c, int dir) {
   return THP_OK;
 }
 
+// d_grid to zero: what cuFFT's transforms in place leave has to go before
+// the next spread; the three-kernel convolution zeroes what it reads
+int clear_grid(Ctx& c) {
+  size_t csz = c.mixed ? sizeof(cufftComplex) : sizeof(cufftDoubleComplex);
+  return cuda_status(cudaMemsetAsync(c.d_grid, 0, csz * c.ngrid, c.stream), &c, "zero grid");
+}
+
 // d_grid -> d_conv: forward transform, influence function, inverse
 // transform.  Three kernels where the grid allows (at 120^3: 73 -> 38 us FP32,
 // 98 -> 53 us FP64 against cuFFT's six launches and the product; 60^3 34 -> 15 us), else
@@ -572,7 +581,7 @@ int convolve(Ctx& c, int check_stop, bool real = false) {
     const conv::Sys s{c.d_grid, c.d_conv, c.d_qfacp, c.d_cg, c.d_pot};
     const cudaError_t e = c.mixed ? launch_conv32(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream)
                                   : launch_conv64(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream);
-    return cuda_status(e, &c, "convolution");
+    return spread_status(c, cuda_status(e, &c, "convolution"));
   }
   int st = fft(c, CUFFT_FORWARD);
   if (st) return st;
@@ -732,14 +741,15 @@ void pme_free(Ctx& c) {
   c.d_conv = nullptr;
 }
 
-// d_grid to zero: what cuFFT's transforms in place leave has to go before
-// the next spread; the three-kernel convolution zeroes what it reads
-static int clear_grid(Ctx& c) {
-  size_t csz = c.mixed ? sizeof(cufftComplex) : sizeof(cufftDoubleComplex);
-  return cuda_status(cudaMemsetAsync(c.d_grid, 0, csz * c.ngrid, c.stream), &c, "zero grid");
-}
-
 int zero_grid(Ctx& c) { return c.conv ? THP_OK : clear_grid(c); }
+
+// Status st of a step between a spread and the end of its convolution.  After a
+// failure no convolution will zero the charges, so they are cleared here: the
+// next spread into a covered grid does not.
+int spread_status(Ctx& c, int st) {
+  if (st && c.conv) clear_grid(c);
+  return st;
+}
 
 // systems below this many atoms spread with a warp per site
 #ifndef THP_SPREAD_WARP_ATOMS
@@ -759,7 +769,7 @@ static int spread_mpole(Ctx& c, const PmeGeom& g) {
     k_spread_mpole_small<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, gd);
   else
     k_spread_mpole<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, gd);
-  return cuda_status(cudaGetLastError(), &c, "spread mpole");
+  return spread_status(c, cuda_status(cudaGetLastError(), &c, "spread mpole"));
 }
 
 // Permanent-multipole PME: d_cphi (and cphi10 when non-null) and, when
@@ -794,11 +804,12 @@ static int kspace_virial(Ctx& c, int mode, double sign, double* d_part) {
 // (epolar1.f:534-541): kspace_virial_blocks() rows of 6 into d_part.
 int launch_mpole_grid_virial(Ctx& c, double* d_part, double sign) {
   PmeGeom g = geom_of(c);
-  int st = zero_grid(c);
+  int st = ensure_plan(c);
   if (st) return st;
+  if ((st = zero_grid(c))) return st;
   if ((st = spread_mpole(c, g))) return st;
-  if ((st = fft(c, CUFFT_FORWARD))) return st;
-  if ((st = kspace_virial(c, 0, sign, d_part))) return st;
+  if ((st = fft(c, CUFFT_FORWARD))) return spread_status(c, st);
+  if ((st = kspace_virial(c, 0, sign, d_part))) return spread_status(c, st);
   int blocks = 148 * 8;
   if (c.mixed)
     k_qfac<cufftComplex, float><<<blocks, 256, 0, c.stream>>>(c.ngrid, (const float*)c.d_qfac,
@@ -806,8 +817,8 @@ int launch_mpole_grid_virial(Ctx& c, double* d_part, double sign) {
   else
     k_qfac<cufftDoubleComplex, double><<<blocks, 256, 0, c.stream>>>(
         c.ngrid, (const double*)c.d_qfac, (cufftDoubleComplex*)c.d_grid, c.d_cg, 0);
-  if ((st = cuda_status(cudaGetLastError(), &c, "qfac"))) return st;
-  if ((st = fft(c, CUFFT_INVERSE))) return st;
+  if ((st = cuda_status(cudaGetLastError(), &c, "qfac"))) return spread_status(c, st);
+  if ((st = fft(c, CUFFT_INVERSE))) return spread_status(c, st);
   return c.conv ? clear_grid(c) : THP_OK;
 }
 
@@ -817,16 +828,17 @@ int launch_mpole_grid_virial(Ctx& c, double* d_part, double sign) {
 int launch_pair_grid_virial(Ctx& c, double* d_part) {
   PmeGeom g = geom_of(c);
   int nb = (c.n + kBlock - 1) / kBlock;
-  int st = zero_grid(c);
+  int st = ensure_plan(c);
   if (st) return st;
+  if ((st = zero_grid(c))) return st;
   if (c.mixed)
     k_spread_mpole2<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, c.d_mu, (cufftComplex*)c.d_grid);
   else
     k_spread_mpole2<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, c.d_rpole, c.d_mu,
                                                          (cufftDoubleComplex*)c.d_grid);
-  if ((st = cuda_status(cudaGetLastError(), &c, "spread mpole pair"))) return st;
-  if ((st = fft(c, CUFFT_FORWARD))) return st;
-  if ((st = kspace_virial(c, 1, 1.0, d_part))) return st;
+  if ((st = cuda_status(cudaGetLastError(), &c, "spread mpole pair"))) return spread_status(c, st);
+  if ((st = fft(c, CUFFT_FORWARD))) return spread_status(c, st);
+  if ((st = kspace_virial(c, 1, 1.0, d_part))) return spread_status(c, st);
   return c.conv ? clear_grid(c) : THP_OK;
 }
 
@@ -914,7 +926,7 @@ int launch_spread_small(Ctx& c, double* d_vec, int update) {
   else
     k_spread_dip_small<double><<<nb, 128, 0, c.stream>>>(c.n, g, c.d_pos, d_vec, c.d_zr, c.d_cg, update, update,
                                                          nullptr, nullptr, nullptr, (cufftDoubleComplex*)c.d_grid);
-  return cuda_status(cudaGetLastError(), &c, "spread dip");
+  return spread_status(c, cuda_status(cudaGetLastError(), &c, "spread dip"));
 }
 
 // Dipole PME pass: spread of d_vec [n][6] and the convolution.  d_out (if
@@ -928,7 +940,7 @@ int launch_pme_dipole(Ctx& c, const double* d_vec, double* d_out, int check_stop
     spread_dipoles<float, double>(c, g, d_vec, check_stop, (cufftComplex*)c.d_grid);
   else
     spread_dipoles<double, double>(c, g, d_vec, check_stop, (cufftDoubleComplex*)c.d_grid);
-  if ((st = cuda_status(cudaGetLastError(), &c, "spread dip"))) return st;
+  if ((st = cuda_status(cudaGetLastError(), &c, "spread dip"))) return spread_status(c, st);
   if ((st = convolve(c, check_stop))) return st;
   if (d_out) st = launch_gather_dip(c, d_out, false);
   return st;
@@ -941,7 +953,7 @@ int launch_pme_dipole_f32(Ctx& c, const float* d_vec, int check_stop) {
   int st = zero_grid(c);
   if (st) return st;
   spread_dipoles<float, float>(c, g, d_vec, check_stop, (cufftComplex*)c.d_grid);
-  if ((st = cuda_status(cudaGetLastError(), &c, "spread dip"))) return st;
+  if ((st = cuda_status(cudaGetLastError(), &c, "spread dip"))) return spread_status(c, st);
   return convolve(c, check_stop);
 }
 
