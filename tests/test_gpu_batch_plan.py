@@ -145,3 +145,27 @@ def test_plan_with_an_odd_grid_ahead(lib, boxes, precision):
         d = max(rms(uind, ua), rms(uinp, pa))
         assert d < (1e-9 if prec == lib.FP64 else 5e-6), (q, d)
     plan.close()
+
+
+@pytest.mark.parametrize("change", ["grid", "box", "nothing"])
+def test_plan_refuses_a_retargeted_context(lib, thp, change):
+    # same atom count and list capacity, so the per-atom buffers stay where the
+    # plan has them; a longer grid moves the grid arrays, another box only the
+    # constants in the plan's descriptors
+    base = thp.water.make_water_box(216, cfg=0)
+    other = {"grid": dataclasses.replace(base, nfft=(48, 48, 48)),
+             "box": thp.water.make_water_box(216, edge=1.1 * base.box[0], cfg=0), "nothing": base}[change]
+    ctxs = [lib.Context(base, precision=lib.MIXED), lib.Context(thp.water.make_water_box(300, cfg=1), precision=lib.MIXED)]
+    plan = lib.Batch(ctxs)
+    plan.solve()
+    ctxs[0].retarget(other)
+    with pytest.raises(lib.ThpError) as e:
+        plan.solve()
+    assert e.value.status == lib.THP_E_STATE
+    plan.close()
+    # a plan made now serves the new system
+    plan = lib.Batch(ctxs)
+    plan.solve()
+    _, (ua, _) = solve_alone(lib, other, lib.MIXED)
+    assert rms(ctxs[0].dipoles()[0], ua) < 5e-6
+    plan.close()

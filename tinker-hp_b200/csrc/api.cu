@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -494,8 +495,14 @@ static int check_config(const thp_config& k) {
   return THP_OK;
 }
 
+static unsigned long long next_system_id() {
+  static std::atomic<unsigned long long> last{0};
+  return ++last;
+}
+
 // System geometry and sizes from a configuration (no device work).
 static void apply_config(Ctx& c, const thp_config& k) {
+  c.system_id = next_system_id();
   c.cfg = k;
   c.n = k.n;
   c.npad = (k.n + 31) / 32 * 32;

@@ -329,9 +329,10 @@ struct BatchPlan {
   size_t grid_bytes = 0;
   std::vector<FftClass> classes;
   unsigned* d_loops = nullptr;
-  // the buffers each system's descriptor points at, checked before every
-  // solve (a context re-targeted since the plan was made invalidates it)
-  std::vector<std::tuple<int, const void*, const void*, const void*>> sig;
+  // each context's system_id, checked before every solve: the descriptors hold
+  // its buffers, box and grid, which a re-target may change even where the
+  // sizes and the addresses of the per-atom buffers stay
+  std::vector<unsigned long long> sig;
   cudaGraphExec_t exec[kNumCandidates] = {};
   float best_ms[kNumCandidates];
   int tried = 0;    // candidates measured so far (online tuning)
@@ -631,7 +632,7 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     s.partials = c.d_partials;
     s.flags = c.d_flags;
     p->politer_max = std::max(p->politer_max, c.cfg.politer);
-    p->sig.emplace_back(c.n, c.d_pp, c.d_pk, c.d_cg);
+    p->sig.push_back(c.system_id);
   }
   for (size_t k = 0; k < p->classes.size(); ++k) {
     FftClass& f = p->classes[k];
@@ -681,11 +682,8 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
 }
 
 int batch_plan_check(const BatchPlan& p, Ctx* const* cs) {
-  for (int q = 0; q < p.count; ++q) {
-    const Ctx& c = *cs[q];
-    if (p.sig[q] != std::make_tuple(c.n, (const void*)c.d_pp, (const void*)c.d_pk, (const void*)c.d_cg))
-      return THP_E_STATE;
-  }
+  for (int q = 0; q < p.count; ++q)
+    if (p.sig[q] != cs[q]->system_id) return THP_E_STATE;
   return THP_OK;
 }
 

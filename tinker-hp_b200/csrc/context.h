@@ -61,6 +61,10 @@ struct Ctx {
   cudaStream_t stream2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 
+  // number of the system's sizes, box and buffers: drawn anew (next_system_id)
+  // by every create and reset, so that whatever holds them can tell
+  unsigned long long system_id = 0;
+
   // host copies (original atom order)
   std::vector<double> h_polarity, h_thole, h_pdamp;
   bool have_params = false, have_pos = false, have_rpole = false, have_conn = false;
