@@ -169,3 +169,41 @@ def test_plan_refuses_a_retargeted_context(lib, thp, change):
     _, (ua, _) = solve_alone(lib, other, lib.MIXED)
     assert rms(ctxs[0].dipoles()[0], ua) < 5e-6
     plan.close()
+
+
+@pytest.mark.parametrize("change", ["rpole", "connectivity"])
+def test_plan_follows_changed_inputs(lib, thp, change):
+    # the whole-solve graph holds the fronts as they were captured: multipoles
+    # given instead of rotated, and a longer table of special pairs (which moves
+    # its buffers), reach the next solve of the plan
+    base = thp.water.make_water_box(216, cfg=0)
+    ctxs = [lib.Context(base, precision=lib.FP64), lib.Context(thp.water.make_water_box(300, cfg=1), precision=lib.FP64)]
+    plan = lib.Batch(ctxs)
+    while plan.tuning() is None:
+        plan.solve()
+    for _ in range(2):  # the kept shape's graph, captured and replayed
+        plan.solve()
+    before = ctxs[0].dipoles()
+    alone = lib.Context(base, precision=lib.FP64)
+    if change == "rpole":
+        rp = np.random.default_rng(3).normal(0.0, 0.05, (base.n, 13))
+        for c in (ctxs[0], alone):
+            c.set_rpole(rp)
+    else:
+        # 1-4 partners for every atom: the same two atoms of the next molecule
+        n, idx = base.n, [[(3 * (i // 3 + 1) + q) % base.n for q in range(2)] for i in range(base.n)]
+        idx = [sorted(set(idx[i]) | {k for k in range(n) if i in idx[k]}) for i in range(n)]
+        off = np.cumsum([0] + [len(r) for r in idx]).astype(np.int32)
+        conn = dict(base.conn)
+        conn["i14"] = (off, np.concatenate(idx).astype(np.int32))
+        scales = dict(base.scales)
+        scales["p_scale"] = [0.0, 0.0, 0.5, 1.0]
+        moved = dataclasses.replace(base, conn=conn, scales=scales)
+        for c in (ctxs[0], alone):
+            c._setup(moved, True, None)
+    plan.solve()
+    alone.solve()
+    got, ref = ctxs[0].dipoles(), alone.dipoles()
+    assert max(rms(ref[0], before[0]), rms(ref[1], before[1])) > 1e-3  # the change matters
+    assert rms(got[0], ref[0]) < 1e-9 and rms(got[1], ref[1]) < 1e-9
+    plan.close()

@@ -424,8 +424,9 @@ void free_ctx(Ctx& c) {
 }
 
 // graphs that hold a system's structure (rotpole on/off, special pairs,
-// sizes) are dropped when it changes
+// sizes) are dropped when it changes; a batch plan drops its own
 static void drop_front_graphs(Ctx& c) {
+  ++c.structure;
   for (auto& row : c.front_exec)
     for (auto& ex : row)
       if (ex) {
@@ -1496,6 +1497,7 @@ static int batch_solve_graph(thp_batch* b, int guess, thp_solve_info* infos) {
     carry0 = carry;
   }
   const int cand = batch_plan_candidate(p);
+  batch_plan_drop_stale(p, b->cs.data());
   cudaGraphExec_t ex = batch_plan_solve_exec(p, g0, carry0, cand);
   if (!ex) {
     // capture every front (the host state moves as it is enqueued) and build

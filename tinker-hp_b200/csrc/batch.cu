@@ -352,6 +352,7 @@ struct BatchPlan {
   // whole-solve graphs (fronts, loop, results) per (guess, dipole carry,
   // candidate), and the mapped host records their last kernel writes
   std::map<std::tuple<int, int, int>, cudaGraphExec_t> solve_exec;
+  std::vector<unsigned> structure;  // of each context when they were captured
   BatchOut* h_out = nullptr;
   BatchOut* d_out = nullptr;
 };
@@ -788,6 +789,18 @@ int batch_plan_profile(BatchPlan& p, int enable, double* ms, int* iterations) {
   for (auto& m : p.prof_ms) m = 0.0;
   p.prof_iterations = 0;
   return THP_OK;
+}
+
+// The whole-solve graphs hold every front as it was captured; once a context's
+// structure has changed (its multipoles, frames or connectivity were set) they
+// go, and the next solve captures it anew.
+void batch_plan_drop_stale(BatchPlan& p, Ctx* const* cs) {
+  std::vector<unsigned> now(p.count);
+  for (int q = 0; q < p.count; ++q) now[q] = cs[q]->structure;
+  if (now == p.structure) return;
+  for (auto& kv : p.solve_exec) cudaGraphExecDestroy(kv.second);
+  p.solve_exec.clear();
+  p.structure = std::move(now);
 }
 
 cudaGraphExec_t batch_plan_solve_exec(const BatchPlan& p, int guess, int carry, int cand) {

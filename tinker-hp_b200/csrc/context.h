@@ -64,6 +64,9 @@ struct Ctx {
   // number of the system's sizes, box and buffers: drawn anew (next_system_id)
   // by every create and reset, so that whatever holds them can tell
   unsigned long long system_id = 0;
+  // counts the changes of what a captured front holds: multipoles rotated or
+  // given, frames, the special pairs' number and buffers
+  unsigned structure = 0;
 
   // host copies (original atom order)
   std::vector<double> h_polarity, h_thole, h_pdamp;

@@ -128,6 +128,7 @@ int batch_plan_profile(BatchPlan& p, int enable, double* ms, int* iterations);
 int batch_plan_candidate(const BatchPlan& p);  // the launch shape the next solve uses
 bool batch_plan_profiling(const BatchPlan& p);
 // whole-solve graphs: every system's front, the batched loop and the results
+void batch_plan_drop_stale(BatchPlan& p, Ctx* const* cs);  // whole-solve graphs of fronts that changed
 cudaGraphExec_t batch_plan_solve_exec(const BatchPlan& p, int guess, int carry, int cand);
 int batch_plan_make_solve_exec(BatchPlan& p, const std::vector<cudaGraph_t>& fronts, int guess, int carry, int cand);
 int batch_plan_run_solve(BatchPlan& p, cudaGraphExec_t ex, const CgScalars** cg_out, const int** flags_out,
