@@ -542,6 +542,12 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
   ok(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
   for (cudaEvent_t* e : {&p->ev_start, &p->ev_loop, &p->ev_done}) ok(cudaEventCreate(e));
   ok(cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming));
+  // everything the plan's kernels read is filled on the plan's own stream (a
+  // non-blocking one, which the default stream does not order) and is in place
+  // before the call returns
+  auto upload = [&](void* dst, const void* src, size_t bytes) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, p->stream);
+  };
   const size_t csz = p->mixed ? sizeof(cufftComplex) : sizeof(cufftDoubleComplex);
   long atoms = 0;
   for (int q = 0; q < count; ++q) atoms += cs[q]->n;
@@ -576,7 +582,7 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     k.conv = conv_covers(k.n, p->mixed, &r1, &r2);
   }
   p->grid_bytes = off * csz;
-  if (ok(cudaMalloc(&p->d_grid, p->grid_bytes))) ok(cudaMemset(p->d_grid, 0, p->grid_bytes));
+  if (ok(cudaMalloc(&p->d_grid, p->grid_bytes))) ok(cudaMemsetAsync(p->d_grid, 0, p->grid_bytes, p->stream));
   ok(cudaMalloc(&p->d_conv, p->grid_bytes));
   for (FftClass& k : p->classes) {
     const int dims[3] = {k.n[2], k.n[1], k.n[0]};
@@ -639,7 +645,7 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     FftClass& f = p->classes[k];
     if (!f.conv) continue;
     const size_t b = sizeof(conv::Sys) * csys[k].size();
-    if (ok(cudaMalloc(&f.d_sys, b))) ok(cudaMemcpy(f.d_sys, csys[k].data(), b, cudaMemcpyHostToDevice));
+    if (ok(cudaMalloc(&f.d_sys, b))) ok(upload(f.d_sys, csys[k].data(), b));
   }
   // work lists, large systems first so the round-robin ends on small items
   std::vector<int> order(count);
@@ -654,17 +660,17 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
       for (int b = 0; b < hs[q].nblk_mv[g]; ++b) mv_items[g].push_back(make_int2(q, b));
   }
   ok(cudaMalloc(&p->d_sys, sizeof(BatchSys) * count));
-  ok(cudaMemcpy(p->d_sys, hs.data(), sizeof(BatchSys) * count, cudaMemcpyHostToDevice));
+  ok(upload(p->d_sys, hs.data(), sizeof(BatchSys) * count));
   p->n_atom_items = (int)atom_items.size();
   ok(cudaMalloc(&p->d_atom_items, sizeof(int2) * atom_items.size()));
-  ok(cudaMemcpy(p->d_atom_items, atom_items.data(), sizeof(int2) * atom_items.size(), cudaMemcpyHostToDevice));
+  ok(upload(p->d_atom_items, atom_items.data(), sizeof(int2) * atom_items.size()));
   p->n_qfac_items = (int)qfac_items.size();
   ok(cudaMalloc(&p->d_qfac_items, sizeof(int2) * std::max<size_t>(1, qfac_items.size())));
-  ok(cudaMemcpy(p->d_qfac_items, qfac_items.data(), sizeof(int2) * qfac_items.size(), cudaMemcpyHostToDevice));
+  ok(upload(p->d_qfac_items, qfac_items.data(), sizeof(int2) * qfac_items.size()));
   for (int g = 0; g < 2; ++g) {
     p->n_mv_items[g] = (int)mv_items[g].size();
     ok(cudaMalloc(&p->d_mv_items[g], sizeof(int2) * mv_items[g].size()));
-    ok(cudaMemcpy(p->d_mv_items[g], mv_items[g].data(), sizeof(int2) * mv_items[g].size(), cudaMemcpyHostToDevice));
+    ok(upload(p->d_mv_items[g], mv_items[g].data(), sizeof(int2) * mv_items[g].size()));
   }
   p->key = TuneKey(p->mixed, log2i(atoms), log2i(count));
   {
@@ -673,6 +679,7 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     if (f != g_tuned.end()) p->chosen = f->second;
   }
   for (auto& m : p->best_ms) m = 1e30f;
+  if (p->stream) ok(cudaStreamSynchronize(p->stream));
   if (st) {
     if (msg) *msg = "batch: device allocation, copy or FFT plan failed";
     batch_plan_destroy(p);
