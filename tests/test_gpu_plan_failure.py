@@ -110,3 +110,28 @@ def test_solve_after_a_failed_virial_call(tmp_path, precision):
                 assert fail_exec.value == 0
                 same(f"transform {k}")
     """)
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED"])
+def test_batch_after_a_failed_profiled_solve(tmp_path, precision):
+    # the profiled loop runs eagerly: the cuFFT class fails after both classes
+    # have spread and before the other class convolves
+    run_child(tmp_path, precision, """
+        import dataclasses
+        base = thp.water.make_water_box(216, cfg=0)
+        boxes = [dataclasses.replace(base, nfft=g) for g in ((20, 24, 20), (20, 20, 20))]
+        ctxs = [lib.Context(b, precision=getattr(lib, precision)) for b in boxes]
+        alone = []
+        for c in ctxs:
+            c.solve()
+            alone.append(c.dipoles()[0])
+        plan = lib.Batch(ctxs)
+        plan.profile(True)
+        fail_exec.value = 5  # after the two convolutions of the first context's front
+        refused(plan.solve)
+        assert fail_exec.value == 0
+        plan.profile(False)
+        plan.solve()
+        for c, ref in zip(ctxs, alone):
+            assert np.abs(c.dipoles()[0] - ref).max() < (1e-10 if precision == "FP64" else 2e-6) * np.abs(ref).max()
+    """)

@@ -718,7 +718,12 @@ int batch_plan_loop(BatchPlan& p, Ctx* const* cs) {
     // eager iterations with a host check of the running systems after each
     const BatchTune& t = kCandidates[cand];
     for (int it = 0; it < p.politer_max + 2; ++it) {
-      if (enqueue_body(p, t, cudaGraphConditionalHandle{}, true)) return THP_E_CUDA;
+      if (enqueue_body(p, t, cudaGraphConditionalHandle{}, true)) {
+        // charges already spread may be left without a convolution to zero them
+        for (FftClass& k : p.classes) cudaStreamSynchronize(k.stream);
+        cudaMemsetAsync(p.d_grid, 0, p.grid_bytes, p.stream);
+        return THP_E_CUDA;
+      }
       kb_running<<<1, 32, 0, p.stream>>>(p.d_sys, p.count, p.d_running);
       cudaMemcpyAsync(p.h_running, p.d_running, sizeof(int), cudaMemcpyDeviceToHost, p.stream);
       if (cudaStreamSynchronize(p.stream) != cudaSuccess) return THP_E_CUDA;
