@@ -50,6 +50,21 @@ def test_footprint_scales_with_size(thp):
     assert 0 < a < b
 
 
+def test_footprint_of_the_grid(thp):
+    """A grid point counts for the spread grid and the influence function, 12
+    bytes (24 in the FP64 form), whichever convolution serves the grid; the
+    allowance for cuFFT's work area covers the own convolution's second grid and potential."""
+    import dataclasses
+    from tinker_hp_b200 import lib as L
+    ws = thp.water.make_water_box(216)
+    for precision, per_point in ((L.MIXED, 12), (L.FP64, 24)):
+        def at(*nfft):
+            return L.footprint(dataclasses.replace(ws, nfft=nfft), precision)
+        base = at(20, 20, 20)
+        for nfft in ((20, 24, 20), (120, 120, 120), (160, 160, 160), (162, 162, 162)):
+            assert at(*nfft) - base == per_point * (nfft[0] * nfft[1] * nfft[2] - 8000), nfft
+
+
 def test_fortran_shim_binds_declared_noncolliding_symbols():
     # The shim reaches the library only through names that no Tinker-HP
     # object defines (thp_*), each declared in include/thp.h; the

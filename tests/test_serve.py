@@ -137,6 +137,43 @@ def test_server_reuses_contexts_under_a_tight_budget(thp):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["FP64", "MIXED"])
+@pytest.mark.parametrize("nfft", [120, 160, 162])
+def test_context_fits_its_footprint(thp, nfft, precision):
+    # what admission counts covers what a context allocates, on grids of the own
+    # convolution and of cuFFT (with its work area)
+    import dataclasses
+    import torch
+    from tinker_hp_b200 import lib
+    prec = getattr(lib, precision)
+    small = thp.water.make_water_box(216, cfg=0)
+    lib.Context(small, precision=prec).solve()  # modules and libraries are loaded
+    ws = dataclasses.replace(thp.water.make_water_box(400, cfg=0), nfft=(nfft,) * 3)
+    free = torch.cuda.mem_get_info()[0]
+    ctx = lib.Context(ws, precision=prec)
+    ctx.solve()
+    used = free - torch.cuda.mem_get_info()[0]
+    assert 0 < used <= lib.footprint(ws, prec), (used, lib.footprint(ws, prec))
+
+
+@pytest.mark.gpu
+def test_context_moves_between_kinds_of_grid(thp):
+    # re-targets from a grid of the own convolution to one of cuFFT, larger, and
+    # back: the second grid is allocated when the first such grid needs it
+    import dataclasses
+    from tinker_hp_b200 import lib
+    base = thp.water.make_water_box(216, cfg=0)
+    ctx = lib.Context(dataclasses.replace(base, nfft=(20, 24, 20)), precision=lib.FP64)
+    for nfft in ((20, 24, 20), (20, 20, 20), (25, 25, 25), (24, 24, 24), (30, 24, 20), (18, 18, 18)):
+        ws = dataclasses.replace(base, nfft=nfft)
+        ctx.retarget(ws)
+        alone = lib.Context(ws, precision=lib.FP64)
+        assert abs(ctx.solve()["epol"] - alone.solve()["epol"]) < 1e-12 * abs(ctx.solve()["epol"]), nfft
+        u, ua = ctx.dipoles()[0], alone.dipoles()[0]
+        assert np.abs(u - ua).max() < 1e-12 * np.abs(ua).max(), nfft
+
+
+@pytest.mark.gpu
 def test_context_retarget_matches_fresh_context(thp):
     # one context serves a small, a larger and another small system in turn
     # (thp_ctx_reset grows buffers and re-plans the FFT only when needed)

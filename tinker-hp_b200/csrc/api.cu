@@ -447,10 +447,12 @@ size_t footprint_bytes(const thp_config& cfg, int* ncell_out) {
   b += n * 32 + n * 16 + 2 * n * 8 + 10 * n * 8 + n * 32 + n * 64;  // sorted data
   b += n * 4 + maxnb * npad * 4;                         // list
   b += n * 4 + maxnb * npad * (4 + 2 * (mixed ? 4 : 8));  // pairs
-  b += ngrid * (mixed ? 28 : 56);                        // grids, potential and two influence functions
+  b += ngrid * (mixed ? 12 : 24);                        // grid and influence function
   b += 10 * n * 6 * 8 + 4 * n * 8 + n * 6 * 4 + n * 9 * 4 + 4 * n * 6 * 4;  // vectors, FP32 row input and CG vectors
   b += (n / 128 + 2) * 4 * 8 + 4096 + (mixed ? 0 : 72 * n);  // reductions; FP64 row records
-  b += 64 << 20;  // cuFFT work area and runtime slack
+  // cuFFT's work area, or on the grids that convolve without it the second grid
+  // and the real potential (at most 49 MB, 160^3 FP32), and runtime slack
+  b += 64 << 20;
   return b;
 }
 

@@ -632,7 +632,7 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     s.mpz = c.d_mpz;
     s.grid = static_cast<char*>(p->d_grid) + next[cls[q]] * csz;
     s.conv = p->classes[cls[q]].conv ? static_cast<char*>(p->d_conv) + next[cls[q]] * csz : s.grid;
-    csys[cls[q]].push_back(conv::Sys{s.grid, s.conv, c.d_qfacp, c.d_cg, nullptr});
+    csys[cls[q]].push_back(conv::Sys{s.grid, s.conv, c.d_qfac, c.d_cg, nullptr});
     next[cls[q]] += slot(p->classes[cls[q]]);
     s.qfac = c.d_qfac;
     s.cg = c.d_cg;

@@ -166,20 +166,22 @@ struct Ctx {
   bool have_plan = false;
   void* d_grids = nullptr;  // the allocation of the grid arrays below
   int plan_dims[3] = {0, 0, 0};
-  size_t cap_ngrid = 0;
+  size_t cap_ngrid = 0, cap_conv = 0;  // points of d_grid and d_qfac, of d_conv_buf and d_pot
   void* d_grid = nullptr;  // cufftDoubleComplex or cufftComplex
-  void* d_qfac = nullptr;  // double or float
+  // influence function, double or float: rows in the x order of the
+  // three-kernel convolution (x_slot with the factors conv_r)
+  void* d_qfac = nullptr;
   // cubic grids of the lengths of conv_dev.cuh convolve in three kernels
   // (conv 1): d_grid is spread into and always zero between convolutions, the
-  // convolved potential is in d_conv, the influence function in the
-  // convolution's x order in d_qfacp.  Other grids (conv 0) use cuFFT in place:
+  // convolved potential is in d_conv (of a real convolution, one real per point,
+  // in d_pot: in the front of d_conv's planes instead, a 32,000-atom FP32 solve
+  // took 1.050 ms against 1.037).  Other grids (conv 0) use cuFFT in place:
   // d_conv is d_grid, zeroed before each spread.
   int conv = 0;
-  int conv_r[2] = {0, 0};        // the grid length's factors
+  int conv_r[2] = {1, 1};        // the grid length's factors (conv 0: 1, 1)
   void* d_conv = nullptr;
-  void* d_conv_buf = nullptr;
-  void* d_qfacp = nullptr;
-  void* d_pot = nullptr;         // the potential of a real convolution, one real per point
+  void* d_conv_buf = nullptr;    // with d_pot, in contexts that have served a conv 1 grid
+  void* d_pot = nullptr;
   double a_frac[3] = {0, 0, 0};  // nfft_d * recip(d,d)
 
   // CG vectors, sorted order, [n][6] = (d xyz, p xyz)

@@ -158,6 +158,13 @@ __global__ void k_spread_mpole2(int n, PmeGeom g, const double4* __restrict__ po
   }
 }
 
+// Where a row of the influence function holds x frequency k, n1 = f1 f2 (conv.h;
+// f1 = f2 = 1: at k, the order of cuFFT's grids).
+struct XOrder {
+  int f1, f2;
+  __device__ __forceinline__ int slot(int k) const { return f2 * (k % f1) + k / f1; }
+};
+
 // Sum over the reciprocal lattice (all k but 0 with qfac > 0) of the PME
 // virial terms h h vterm - eterm (eterm = 0.5 f qfac struc2, vterm =
 // (2/h^2)(1 + pterm h^2) eterm; emrecip1 / eprecip1, epolar1.f:1041-1091)
@@ -167,7 +174,7 @@ __global__ void k_spread_mpole2(int n, PmeGeom g, const double4* __restrict__ po
 // A = (G(k) + conj G(-k)) / 2, B = (G(k) - conj G(-k)) / 2i.  Each block
 // writes its 6 sums (xx, xy, xz, yy, yz, zz) to part[block].
 template <typename C, typename Q>
-__global__ void __launch_bounds__(256) k_kspace_virial(int n1, int n2, int n3, const C* __restrict__ grid,
+__global__ void __launch_bounds__(256) k_kspace_virial(int n1, int n2, int n3, XOrder xo, const C* __restrict__ grid,
                                                        const Q* __restrict__ qfac, double r1, double r2, double r3,
                                                        double pterm, double f, int mode, double sign,
                                                        double* __restrict__ part) {
@@ -175,9 +182,10 @@ __global__ void __launch_bounds__(256) k_kspace_virial(int n1, int n2, int n3, c
   const long ng = (long)n1 * n2 * n3;
   const int nf1 = (n1 + 1) / 2, nf2 = (n2 + 1) / 2, nf3 = (n3 + 1) / 2;
   for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < ng; idx += (long)gridDim.x * blockDim.x) {
-    const double qf = (double)qfac[idx];
+    const int k1 = (int)(idx % n1);
+    const double qf = (double)qfac[idx - k1 + xo.slot(k1)];
     if (qf == 0.0) continue;
-    const int k1 = (int)(idx % n1), k2 = (int)((idx / n1) % n2), k3 = (int)(idx / ((long)n1 * n2));
+    const int k2 = (int)((idx / n1) % n2), k3 = (int)(idx / ((long)n1 * n2));
     const int m1 = k1 + 1 > nf1 ? k1 - n1 : k1, m2 = k2 + 1 > nf2 ? k2 - n2 : k2, m3 = k3 + 1 > nf3 ? k3 - n3 : k3;
     const C gk = grid[idx];
     double struc2;
@@ -304,13 +312,14 @@ __global__ void __launch_bounds__(128) k_spread_dip_small(int n, PmeGeom g, cons
 }
 
 template <typename C, typename T>
-__global__ void k_qfac(size_t ng, const T* __restrict__ qfac, C* __restrict__ grid, const CgScalars* __restrict__ cg,
-                       int check_stop) {
+__global__ void k_qfac(size_t ng, int n1, XOrder xo, const T* __restrict__ qfac, C* __restrict__ grid,
+                       const CgScalars* __restrict__ cg, int check_stop) {
   if (check_stop && cg->stop) return;
   size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (; q < ng; q += stride) {
-    T f = qfac[q];
+    const int k1 = xo.f1 == 1 ? 0 : (int)(q % n1);
+    T f = qfac[q - k1 + xo.slot(k1)];
     C v = grid[q];
     v.x *= f;
     v.y *= f;
@@ -578,20 +587,21 @@ int clear_grid(Ctx& c) {
 // d_grid, the result in d_pot.
 int convolve(Ctx& c, int check_stop, bool real = false) {
   if (c.conv) {
-    const conv::Sys s{c.d_grid, c.d_conv, c.d_qfacp, c.d_cg, c.d_pot};
+    const conv::Sys s{c.d_grid, c.d_conv, c.d_qfac, c.d_cg, c.d_pot};
     const cudaError_t e = c.mixed ? launch_conv32(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream)
                                   : launch_conv64(c.nfft[0], s, nullptr, 1, check_stop, real, c.stream);
     return spread_status(c, cuda_status(e, &c, "convolution"));
   }
   int st = fft(c, CUFFT_FORWARD);
   if (st) return st;
-  int blocks = 148 * 8;
+  const int blocks = 148 * 8;
+  const XOrder xo{c.conv_r[0], c.conv_r[1]};
   if (c.mixed)
-    k_qfac<cufftComplex, float><<<blocks, 256, 0, c.stream>>>(c.ngrid, (const float*)c.d_qfac,
+    k_qfac<cufftComplex, float><<<blocks, 256, 0, c.stream>>>(c.ngrid, c.nfft[0], xo, (const float*)c.d_qfac,
                                                              (cufftComplex*)c.d_grid, c.d_cg, check_stop);
   else
     k_qfac<cufftDoubleComplex, double><<<blocks, 256, 0, c.stream>>>(
-        c.ngrid, (const double*)c.d_qfac, (cufftDoubleComplex*)c.d_grid, c.d_cg, check_stop);
+        c.ngrid, c.nfft[0], xo, (const double*)c.d_qfac, (cufftDoubleComplex*)c.d_grid, c.d_cg, check_stop);
   st = cuda_status(cudaGetLastError(), &c, "qfac");
   if (st) return st;
   return fft(c, CUFFT_INVERSE);
@@ -599,11 +609,9 @@ int convolve(Ctx& c, int check_stop, bool real = false) {
 
 // qfac(k) = exp(-pi^2 h^2 / a^2) / (pi V h^2 bsmod1 bsmod2 bsmod3), zero at
 // h = 0 and where the exponent is below -50 (newinduce_pme.f:1802-1854)
-// qp (optional): the same values with each row in the x order of the
-// three-kernel convolution for the factors f1 x f2 of n1.
 template <typename T>
 __global__ void k_qfac_init(int n1, int n2, int n3, const double* __restrict__ bsm, double r1, double r2, double r3,
-                            double pterm, double volterm, int f1, int f2, T* __restrict__ q, T* __restrict__ qp) {
+                            double pterm, double volterm, XOrder xo, T* __restrict__ q) {
   const size_t ng = (size_t)n1 * n2 * n3;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < ng; t += (size_t)gridDim.x * blockDim.x) {
     const int k1 = (int)(t % n1), k2 = (int)((t / n1) % n2), k3 = (int)(t / ((size_t)n1 * n2));
@@ -617,8 +625,7 @@ __global__ void k_qfac_init(int n1, int n2, int n3, const double* __restrict__ b
       const double term = -pterm * hsq;
       if (term > -50.0) v = exp(term) / (volterm * hsq * bsm[k1] * bsm[n1 + k2] * bsm[n1 + n2 + k3]);
     }
-    q[t] = (T)v;
-    if (qp) qp[t - k1 + f2 * (k1 % f1) + k1 / f1] = (T)v;
+    q[t - k1 + xo.slot(k1)] = (T)v;
   }
 }
 
@@ -642,8 +649,8 @@ static const std::vector<double>& dftmod_cached(int nfft) {
 
 static void free_grids(Ctx& c) {
   cudaFree(c.d_grids);
-  for (void** p : {&c.d_grids, &c.d_qfac, &c.d_grid, &c.d_qfacp, &c.d_conv_buf, &c.d_pot}) *p = nullptr;
-  c.cap_ngrid = 0;
+  for (void** p : {&c.d_grids, &c.d_qfac, &c.d_grid, &c.d_conv_buf, &c.d_pot}) *p = nullptr;
+  c.cap_ngrid = c.cap_conv = 0;
 }
 
 int pme_init(Ctx& c) {
@@ -656,16 +663,20 @@ int pme_init(Ctx& c) {
   const std::vector<double>& m3 = dftmod_cached(c.nfft[2]);
   size_t esz = c.mixed ? sizeof(float) : sizeof(double);
   size_t csz = c.mixed ? sizeof(cufftComplex) : sizeof(cufftDoubleComplex);
+  c.conv_r[0] = c.conv_r[1] = 1;
+  c.conv = conv_covers(c.nfft, c.mixed, &c.conv_r[0], &c.conv_r[1]) ? 1 : 0;
+  const XOrder xo{c.conv_r[0], c.conv_r[1]};
   // grid buffers are kept while they are large enough (a re-targeted
-  // context reuses them)
-  if (c.ngrid > c.cap_ngrid) {
+  // context reuses them); only the three-kernel convolution needs a second grid and a potential
+  const size_t nconv = c.conv ? c.ngrid : 0;
+  if (c.ngrid > c.cap_ngrid || nconv > c.cap_conv) {
+    const size_t m = std::max(c.ngrid, c.cap_ngrid), mc = std::max(nconv, c.cap_conv);
     free_grids(c);
     // one allocation, each array on a 256-byte boundary
     const struct {
       void** p;
       size_t bytes;
-    } grids[] = {{&c.d_grid, csz * c.ngrid},   {&c.d_conv_buf, csz * c.ngrid}, {&c.d_qfac, esz * c.ngrid},
-                 {&c.d_qfacp, esz * c.ngrid}, {&c.d_pot, esz * c.ngrid}};
+    } grids[] = {{&c.d_grid, csz * m}, {&c.d_qfac, esz * m}, {&c.d_conv_buf, csz * mc}, {&c.d_pot, esz * mc}};
     size_t total = 0;
     for (const auto& g : grids) total += (g.bytes + 255) / 256 * 256;
     if (cuda_status(cudaMalloc(&c.d_grids, total), &c, "alloc grid")) return THP_E_CUDA;
@@ -674,10 +685,9 @@ int pme_init(Ctx& c) {
       *g.p = at;
       at += (g.bytes + 255) / 256 * 256;
     }
-    c.cap_ngrid = c.ngrid;
+    c.cap_ngrid = m;
+    c.cap_conv = mc;
   }
-  c.conv_r[0] = c.conv_r[1] = 1;
-  c.conv = conv_covers(c.nfft, c.mixed, &c.conv_r[0], &c.conv_r[1]) ? 1 : 0;
   c.d_conv = c.conv ? c.d_conv_buf : c.d_grid;
   // influence function on the device (newinduce_pme.f:1802-1854): the
   // B-spline moduli go through the front of the grid buffer
@@ -692,14 +702,12 @@ int pme_init(Ctx& c) {
   const int blocks = (int)std::min<size_t>((c.ngrid + 255) / 256, 148 * 16);
   if (c.mixed)
     k_qfac_init<float><<<blocks, 256, 0, c.stream>>>(c.nfft[0], c.nfft[1], c.nfft[2], d_bsm, c.box.recip[0],
-                                                     c.box.recip[1], c.box.recip[2], pterm, volterm, c.conv_r[0],
-                                                     c.conv_r[1], (float*)c.d_qfac,
-                                                     c.conv ? (float*)c.d_qfacp : nullptr);
+                                                     c.box.recip[1], c.box.recip[2], pterm, volterm, xo,
+                                                     (float*)c.d_qfac);
   else
     k_qfac_init<double><<<blocks, 256, 0, c.stream>>>(c.nfft[0], c.nfft[1], c.nfft[2], d_bsm, c.box.recip[0],
-                                                      c.box.recip[1], c.box.recip[2], pterm, volterm, c.conv_r[0],
-                                                      c.conv_r[1], (double*)c.d_qfac,
-                                                      c.conv ? (double*)c.d_qfacp : nullptr);
+                                                      c.box.recip[1], c.box.recip[2], pterm, volterm, xo,
+                                                      (double*)c.d_qfac);
   // the spread grid is zero from here on between convolutions
   if (c.conv) cudaMemsetAsync(c.d_grid, 0, csz * c.ngrid, c.stream);
   // no host wait: the influence function is ready, stream-ordered, for the
@@ -788,13 +796,14 @@ int kspace_virial_blocks() { return 148 * 2; }
 static int kspace_virial(Ctx& c, int mode, double sign, double* d_part) {
   const double pterm = (kPi / c.cfg.aewald) * (kPi / c.cfg.aewald);
   const PmeGeom g = geom_of(c);
+  const XOrder xo{c.conv_r[0], c.conv_r[1]};
   if (c.mixed)
     k_kspace_virial<cufftComplex, float><<<kspace_virial_blocks(), 256, 0, c.stream>>>(
-        g.n1, g.n2, g.n3, (const cufftComplex*)c.d_grid, (const float*)c.d_qfac, g.recip[0], g.recip[1], g.recip[2],
-        pterm, kElectric, mode, sign, d_part);
+        g.n1, g.n2, g.n3, xo, (const cufftComplex*)c.d_grid, (const float*)c.d_qfac, g.recip[0], g.recip[1],
+        g.recip[2], pterm, kElectric, mode, sign, d_part);
   else
     k_kspace_virial<cufftDoubleComplex, double><<<kspace_virial_blocks(), 256, 0, c.stream>>>(
-        g.n1, g.n2, g.n3, (const cufftDoubleComplex*)c.d_grid, (const double*)c.d_qfac, g.recip[0], g.recip[1],
+        g.n1, g.n2, g.n3, xo, (const cufftDoubleComplex*)c.d_grid, (const double*)c.d_qfac, g.recip[0], g.recip[1],
         g.recip[2], pterm, kElectric, mode, sign, d_part);
   return cuda_status(cudaGetLastError(), &c, "k-space virial");
 }
@@ -810,13 +819,14 @@ int launch_mpole_grid_virial(Ctx& c, double* d_part, double sign) {
   if ((st = spread_mpole(c, g))) return st;
   if ((st = fft(c, CUFFT_FORWARD))) return spread_status(c, st);
   if ((st = kspace_virial(c, 0, sign, d_part))) return spread_status(c, st);
-  int blocks = 148 * 8;
+  const int blocks = 148 * 8;
+  const XOrder xo{c.conv_r[0], c.conv_r[1]};
   if (c.mixed)
-    k_qfac<cufftComplex, float><<<blocks, 256, 0, c.stream>>>(c.ngrid, (const float*)c.d_qfac,
+    k_qfac<cufftComplex, float><<<blocks, 256, 0, c.stream>>>(c.ngrid, c.nfft[0], xo, (const float*)c.d_qfac,
                                                              (cufftComplex*)c.d_grid, c.d_cg, 0);
   else
     k_qfac<cufftDoubleComplex, double><<<blocks, 256, 0, c.stream>>>(
-        c.ngrid, (const double*)c.d_qfac, (cufftDoubleComplex*)c.d_grid, c.d_cg, 0);
+        c.ngrid, c.nfft[0], xo, (const double*)c.d_qfac, (cufftDoubleComplex*)c.d_grid, c.d_cg, 0);
   if ((st = cuda_status(cudaGetLastError(), &c, "qfac"))) return spread_status(c, st);
   if ((st = fft(c, CUFFT_INVERSE))) return spread_status(c, st);
   return c.conv ? clear_grid(c) : THP_OK;
