@@ -65,6 +65,23 @@ def test_footprint_of_the_grid(thp):
             assert at(*nfft) - base == per_point * (nfft[0] * nfft[1] * nfft[2] - 8000), nfft
 
 
+def test_footprint_of_an_atom(thp):
+    """Past the pair buffers (12 to 24 bytes a list slot) an atom of the FP64 form
+    takes no more than one of the mixed form: the FP32 rows' arrays belong to one
+    form, the FP64 row records to the other."""
+    import dataclasses
+    from tinker_hp_b200 import lib as L
+    ws = thp.water.make_water_box(1000)
+
+    def per_atom(precision, slots):
+        a, b = (L.config_for(dataclasses.replace(ws, n=n), precision, max_neighbors=slots) for n in (32_000, 64_000))
+        return (L.load().thp_footprint(C.byref(b)) - L.load().thp_footprint(C.byref(a))) / 32_000
+    # the slots' share by difference: list 4 bytes, pair stream 4 + 2 reals
+    fp64 = per_atom(L.FP64, 160) - 160 * (per_atom(L.FP64, 168) - per_atom(L.FP64, 160)) / 8
+    mixed = per_atom(L.MIXED, 160) - 160 * (per_atom(L.MIXED, 168) - per_atom(L.MIXED, 160)) / 8
+    assert fp64 < mixed, (fp64, mixed)
+
+
 def test_fortran_shim_binds_declared_noncolliding_symbols():
     # The shim reaches the library only through names that no Tinker-HP
     # object defines (thp_*), each declared in include/thp.h; the

@@ -448,8 +448,9 @@ size_t footprint_bytes(const thp_config& cfg, int* ncell_out) {
   b += n * 4 + maxnb * npad * 4;                         // list
   b += n * 4 + maxnb * npad * (4 + 2 * (mixed ? 4 : 8));  // pairs
   b += ngrid * (mixed ? 12 : 24);                        // grid and influence function
-  b += 10 * n * 6 * 8 + 4 * n * 8 + n * 6 * 4 + n * 9 * 4 + 4 * n * 6 * 4;  // vectors, FP32 row input and CG vectors
-  b += (n / 128 + 2) * 4 * 8 + 4096 + (mixed ? 0 : 72 * n);  // reductions; FP64 row records
+  b += 10 * n * 6 * 8 + 4 * n * 8;                       // vectors
+  b += n * (mixed ? 6 * 4 + 9 * 4 + 4 * 6 * 4 : 9 * 8);  // FP32 row input, records and CG vectors; FP64 row records
+  b += (n / 128 + 2) * 4 * 8 + 4096;                     // reductions
   // cuFFT's work area, or on the grids that convolve without it the second grid
   // and the real potential (at most 49 MB, 160^3 FP32), and runtime slack
   b += 64 << 20;
@@ -568,6 +569,7 @@ static int size_buffers(Ctx& c) {
   int st = THP_OK;
   const size_t n = c.n, npad = c.npad;
   const size_t esz = c.mixed ? 4 : 8;
+  const size_t n32 = c.mixed ? n : 0, n64 = c.mixed ? 0 : n;  // of the arrays only one form uses
   if ((size_t)c.ncell > c.cap_ncell) {
     cudaFree(c.slab_cells);
     c.slab_cells = nullptr;
@@ -593,13 +595,13 @@ static int size_buffers(Ctx& c) {
                      item(&c.d_xyz_orig, 3 * n), item(&c.d_par_orig, 3 * n), item(&c.d_rpole_orig, 13 * n),
                      item(&c.d_pole_local, 13 * n), item(&c.d_frames, 3 * n), item(&c.d_pos, n),
                      item(&c.d_posf, n), item(&c.d_thole, n), item(&c.d_pol, n), item(&c.d_rpole, 10 * n),
-                     item(&c.d_mrec, 12 * n), item(&c.d_mrecf, 12 * n), item(&c.d_erec, 16 * n), item(&c.d_pos_built, n),
+                     item(&c.d_mrec, 12 * n), item(&c.d_mrecf, 12 * n32), item(&c.d_erec, 16 * n32), item(&c.d_pos_built, n),
                      item(&c.d_nnb, n), item(&c.d_npr, n), item(&c.d_ef, 6 * n), item(&c.d_mu, 6 * n),
                      item(&c.d_res, 6 * n), item(&c.d_h, 6 * n), item(&c.d_pp, 6 * n), item(&c.d_zr, 6 * n),
                      item(&c.d_dip, 6 * n), item(&c.d_tmp6, 6 * n), item(&c.d_tmp6b, 6 * n), item(&c.d_cphi, 4 * n),
-                     item(&c.d_vecf, 6 * n), item(&c.d_rec, 8 * n), item(&c.d_mpz, n), item(&c.d_ef_prev, 6 * n),
-                     item(&c.d_rec64, c.mixed ? 0 : 8 * n), item(&c.d_mpz64, c.mixed ? 0 : n),
-                     item(&c.d_ppf, 6 * n), item(&c.d_hf, 6 * n), item(&c.d_resf, 6 * n), item(&c.d_zrf, 6 * n),
+                     item(&c.d_vecf, 6 * n32), item(&c.d_rec, 8 * n32), item(&c.d_mpz, n32), item(&c.d_ef_prev, 6 * n),
+                     item(&c.d_rec64, 8 * n64), item(&c.d_mpz64, n64),
+                     item(&c.d_ppf, 6 * n32), item(&c.d_hf, 6 * n32), item(&c.d_resf, 6 * n32), item(&c.d_zrf, 6 * n32),
                      item(&c.d_partials, (size_t)(c.nblk_reduce + 8) * 4)},
                     "per-atom buffers");
     if (!st) c.cap_n = n;
