@@ -207,3 +207,20 @@ def test_plan_follows_changed_inputs(lib, thp, change):
     assert max(rms(ref[0], before[0]), rms(ref[1], before[1])) > 1e-3  # the change matters
     assert rms(got[0], ref[0]) < 1e-9 and rms(got[1], ref[1]) < 1e-9
     plan.close()
+
+
+def test_plan_of_cufft_grids_has_one_grid_each(lib, boxes):
+    # the second grid belongs to the own convolution: a plan whose grids cuFFT
+    # transforms in place takes one complex grid per system (8 bytes a point) and
+    # little besides, one of covered grids two
+    import torch
+    taken = {}
+    for edge in (80, 84):  # the own convolution, cuFFT; six grids are a few MB of tables and rounding above
+        ctxs = [lib.Context(dataclasses.replace(ws, nfft=(edge,) * 3), precision=lib.MIXED) for ws in boxes[:6]]
+        lib.Batch(ctxs).close()  # libraries and plans of the shape are loaded
+        free = torch.cuda.mem_get_info()[0]
+        plan = lib.Batch(ctxs)
+        taken[edge] = (free - torch.cuda.mem_get_info()[0]) / (6 * edge ** 3)
+        plan.close()
+        del plan, ctxs
+    assert taken[80] < 18 and taken[84] < 10, taken

@@ -304,6 +304,7 @@ struct FftClass {
   int n[3] = {0, 0, 0};
   int count = 0;
   size_t offset = 0;  // first grid point of the class in the plan's array
+  size_t conv_offset = 0;  // in the array of the convolved grids (conv)
   size_t points = 0;  // grid points of all its systems, padding included
   bool conv = false;  // the three-kernel convolution (else cuFFT)
   conv::Sys* d_sys = nullptr;
@@ -325,7 +326,7 @@ struct BatchPlan {
   int2* d_qfac_items = nullptr;  // (system, chunk of grid points)
   int n_qfac_items = 0;
   void* d_grid = nullptr;        // every system's grid, class by class
-  void* d_conv = nullptr;        // the convolved grids of the three-kernel classes, at the same places
+  void* d_conv = nullptr;        // the convolved grids of the three-kernel classes, end to end
   size_t grid_bytes = 0;
   std::vector<FftClass> classes;
   unsigned* d_loops = nullptr;
@@ -573,17 +574,21 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     const size_t pts = (size_t)k.n[0] * k.n[1] * k.n[2];
     return pts + (pts & 1);
   };
-  size_t off = 0;
+  size_t off = 0, conv_points = 0;
   for (FftClass& k : p->classes) {
     k.offset = off;
     k.points = (size_t)k.count * slot(k);
     off += k.points;
     int r1, r2;
     k.conv = conv_covers(k.n, p->mixed, &r1, &r2);
+    if (k.conv) {
+      k.conv_offset = conv_points;
+      conv_points += k.points;
+    }
   }
   p->grid_bytes = off * csz;
   if (ok(cudaMalloc(&p->d_grid, p->grid_bytes))) ok(cudaMemsetAsync(p->d_grid, 0, p->grid_bytes, p->stream));
-  ok(cudaMalloc(&p->d_conv, p->grid_bytes));
+  if (conv_points) ok(cudaMalloc(&p->d_conv, conv_points * csz));
   for (FftClass& k : p->classes) {
     const int dims[3] = {k.n[2], k.n[1], k.n[0]};
     const int dist = (int)slot(k);
@@ -631,7 +636,8 @@ int batch_plan_create(Ctx* const* cs, int count, BatchPlan** out, std::string* m
     s.rec = c.d_rec;
     s.mpz = c.d_mpz;
     s.grid = static_cast<char*>(p->d_grid) + next[cls[q]] * csz;
-    s.conv = p->classes[cls[q]].conv ? static_cast<char*>(p->d_conv) + next[cls[q]] * csz : s.grid;
+    const FftClass& k = p->classes[cls[q]];
+    s.conv = k.conv ? static_cast<char*>(p->d_conv) + (k.conv_offset + next[cls[q]] - k.offset) * csz : s.grid;
     csys[cls[q]].push_back(conv::Sys{s.grid, s.conv, c.d_qfac, c.d_cg, nullptr});
     next[cls[q]] += slot(p->classes[cls[q]]);
     s.qfac = c.d_qfac;
