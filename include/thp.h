@@ -209,7 +209,9 @@ int thp_get_gradient_device(thp_ctx* ctx, double* d_dep);
  * lattice ((rpole+uinp) x (rpole+uind) minus the permanent-only sum,
  * :534-541, :932-1091), epreal1c's pair terms (:2326-2342) and the frame-atom
  * terms of its torques (:2460-2486).  It costs one more grid spread and
- * forward transform and two passes over the grid per call. */
+ * forward transform and two passes over the grid per call.  Switching it on
+ * plans the grid for cuFFT (milliseconds and device memory, once per context
+ * and grid; THP_E_CUDA and still off when that fails). */
 int thp_set_virial(thp_ctx* ctx, int on);
 /* vir [3][3] (kcal/mol, symmetric) of the last gradient call made with the
  * virial on (THP_E_STATE otherwise).  form 0: as the reference accumulates
@@ -415,7 +417,8 @@ int thp_last_error(void);
 /* bind deriv::dep(3,n), written by epolar1_ */
 int thp_bind_gradient(thp_ctx* ctx, double* dep);
 /* bind virial::vir(3,3) (may be NULL): epolar1_ adds the polarization virial
- * into it (form 0 of thp_get_virial), as epolar1c adds into vir */
+ * into it (form 0 of thp_get_virial), as epolar1c adds into vir.  Plans the
+ * grid as thp_set_virial does */
 int thp_bind_virial(thp_ctx* ctx, double* vir);
 /* bind neigh::nvlst(n) and vlst(maxvlst,n), filled by vlistcell_ */
 int thp_bind_vlist(thp_ctx* ctx, int* nvlst, int* vlst, int maxvlst);

@@ -112,6 +112,37 @@ def test_solve_after_a_failed_virial_call(tmp_path, precision):
     """)
 
 
+def test_plan_is_made_when_the_virial_is_switched_on(tmp_path):
+    # on a grid of the own convolution, which has none before; the calls with
+    # virials, and a re-target that keeps them on, make none themselves
+    run_child(tmp_path, "FP64", """
+        import dataclasses
+        ws = thp.water.make_water_box(216, cfg=0)
+        ctx = lib.Context(ws)
+        ctx.solve()
+        assert plans.value == 0
+        ctx.set_virial(True)
+        assert plans.value == 1
+        ctx.solve()
+        ctx.gradient()
+        ctx.empole1()
+        ctx.set_virial(False)
+        ctx.set_virial(True)
+        assert plans.value == 1
+        ctx.retarget(dataclasses.replace(ws, nfft=(24, 24, 24)))
+        assert plans.value == 2
+        ctx.solve()
+        ctx.gradient()
+        assert plans.value == 2
+        # bound as the reference's virial: planned by the binding
+        other = lib.Context(dataclasses.replace(ws, nfft=(30, 30, 30)))
+        vir = np.zeros(9)
+        fail_plan.value = 1
+        assert lib.load().thp_bind_virial(other.h, lib._p(vir)) == lib.THP_E_CUDA
+        assert lib.load().thp_bind_virial(other.h, lib._p(vir)) == lib.THP_OK and plans.value == 3
+    """)
+
+
 @pytest.mark.parametrize("precision", ["FP64", "MIXED"])
 def test_batch_after_a_failed_profiled_solve(tmp_path, precision):
     # the profiled loop runs eagerly: the cuFFT class fails after both classes

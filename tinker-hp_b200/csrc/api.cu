@@ -1675,8 +1675,18 @@ int thp_get_ehal_virial(thp_ctx* h, double* vir) {
   return THP_OK;
 }
 
+// The virial's transforms run through cuFFT, for which a grid of the own
+// convolution has no plan yet: it is made here, not inside the first gradient.
+static int virial_plan(Ctx& c) {
+  if (set_current_device(c)) return THP_E_CUDA;
+  return ensure_plan(c);
+}
+
 int thp_set_virial(thp_ctx* h, int on) {
   if (!h) return THP_E_INVALID;
+  if (on) {
+    if (int st = virial_plan(h->c)) return st;
+  }
   h->c.want_virial = on != 0;
   return THP_OK;
 }
@@ -1979,6 +1989,9 @@ int thp_bind_grid(thp_ctx* h, double* qgrid) {
 
 int thp_bind_virial(thp_ctx* h, double* vir) {
   if (!h) return THP_E_INVALID;
+  if (vir) {
+    if (int st = virial_plan(h->c)) return st;
+  }
   h->c.bvir = vir;
   return THP_OK;
 }

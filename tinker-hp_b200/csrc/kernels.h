@@ -39,6 +39,7 @@ int launch_pme_dipole(Ctx& c, const double* d_vec, double* d_out, int check_stop
 int launch_spread_small(Ctx& c, double* d_vec, int update);  // the small systems' CG spread, without convolution
 int launch_convolve(Ctx& c, int check_stop, bool real = false);  // real: conv.h
 bool overlap_rows(const Ctx& c);  // the system runs real-space passes on the side stream
+int ensure_plan(Ctx& c);  // a cuFFT plan of the grid, which the virial's transforms need (not under capture)
 int zero_grid(Ctx& c);  // before a spread: d_grid zero (nothing to do for the three-kernel convolution)
 int spread_status(Ctx& c, int st);  // after a spread that no convolution will follow: d_grid zero again
 struct PmeGeom;

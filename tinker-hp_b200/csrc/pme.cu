@@ -553,10 +553,6 @@ int make_plan(Ctx& c) {
   return THP_OK;
 }
 
-// the context's grid has a plan (a grid that the three-kernel convolution
-// covers is made without one)
-int ensure_plan(Ctx& c) { return c.have_plan ? THP_OK : make_plan(c); }
-
 // cuFFT of the whole grid: forward in place, inverse into d_conv (d_grid
 // itself without the three-kernel convolution)
 int fft(Ctx& c, int dir) {
@@ -630,6 +626,10 @@ __global__ void k_qfac_init(int n1, int n2, int n3, const double* __restrict__ b
 }
 
 }  // namespace
+
+// the context's grid has a plan (a grid that the three-kernel convolution
+// covers is made without one)
+int ensure_plan(Ctx& c) { return c.have_plan ? THP_OK : make_plan(c); }
 
 bool conv_covers(const int n[3], int mixed, int* r1, int* r2) {
   if (n[0] != n[1] || n[1] != n[2]) return false;
@@ -714,15 +714,15 @@ int pme_init(Ctx& c) {
   // context's next solve (bsm is copied out before the call returns)
   if (cuda_status(cudaGetLastError(), &c, "qfac")) return THP_E_CUDA;
   // the plan is kept when the grid dimensions are unchanged; a grid that the
-  // three-kernel convolution covers gets one when a virial first asks for it
+  // three-kernel convolution covers gets one when the virial is switched on
   const bool same = c.plan_dims[0] == c.nfft[0] && c.plan_dims[1] == c.nfft[1] && c.plan_dims[2] == c.nfft[2];
   if (!same) {
     if (c.have_plan) give_plan(plan_key(c), c.plan);
     c.have_plan = false;
     for (int d = 0; d < 3; ++d) c.plan_dims[d] = c.nfft[d];
   }
-  if (!c.conv && !c.have_plan) {
-    if (int st = make_plan(c)) return st;
+  if (!c.conv || c.want_virial) {
+    if (int st = ensure_plan(c)) return st;
   }
   if (c.have_plan) cufftSetStream(c.plan, c.stream);
   return cuda_status(cudaGetLastError(), &c, "pme init");
