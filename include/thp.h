@@ -184,8 +184,9 @@ int thp_batch_tuning(thp_batch* b, int* blocks_per_sm, int* matvec_atoms, double
  * the loop eagerly, one host-checked iteration at a time, with events around
  * each step (the accumulators restart); 0: back to the graph; -1: only read.
  * ms[6] receives the accumulated ms of the spread, the forward FFTs, the
- * influence function, the inverse FFTs, the matvec and the update;
- * iterations the batched iterations timed. */
+ * influence function, the inverse FFTs, the matvec and the update (grids of the
+ * own convolution run all of it in the place of the forward FFTs); iterations
+ * the batched iterations timed. */
 int thp_batch_profile(thp_batch* b, int enable, double* ms, int* iterations);
 int thp_batch_destroy(thp_batch* b);
 /* Gradient of the polarization energy, epolar1c (epolar1.f:57-372): eprecip1

@@ -10,7 +10,8 @@
 // single-system kernels (cg_dev.cuh) on the item's system.  Per iteration:
 //   1. kb_spread: pp = zr + beta pp (the 32-byte partner records of the mixed
 //      rows beside it) and the dipole spread (grid_uind_site,
-//      pmestuff.f:280-405) into the plan's grids, zeroed just before;
+//      pmestuff.f:280-405) into the plan's grids, which are zero: a three-kernel
+//      convolution zeroes what it reads, a cuFFT class's grids are cleared first;
 //   2. the convolution per grid-size class (the classes' grids lie end to end,
 //      and the classes run as parallel branches): three kernels over all of a
 //      class's systems (conv_dev.cuh), or, for grids those do not cover, one

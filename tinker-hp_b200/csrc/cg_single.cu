@@ -11,7 +11,7 @@
 // records without a side array.
 //
 // The kernels are those of solver.cu with three components; per iteration:
-//   n >= kSingleLarge: pp and records; row beside tiled spread + convolution;
+//   n >= kLargeAtoms: pp and records; row beside tiled spread + convolution;
 //                      combine; update
 //   smaller:           spread (forms pp and the records, a warp per site); row
 //                      beside the convolution; combine (8 lanes per atom); update
@@ -26,10 +26,6 @@ int group_blocks(int n, int block);
 namespace {
 
 using namespace cg;
-
-constexpr int kSingleLarge = 20000;       // as THP_OVERLAP_MIN_ATOMS of the two-field form
-constexpr int kSingleStreamAtoms = 80000; // pair stream far beyond L2: not kept in L1
-constexpr int kSingleRowSmall = 8000;     // rows in blocks of one warp
 
 template <typename V>
 __device__ __forceinline__ void load3(const V* __restrict__ p, double (&v)[3]) {
@@ -160,7 +156,10 @@ __device__ __forceinline__ bool spread_tile_pass1(const PmeGeom& g, unsigned mk,
   return true;
 }
 
-// systems below this many atoms give a warp 16 sites (one tile) instead of 32
+// Systems below this many atoms give a warp 16 sites (one tile) instead of 32: a
+// cold solve (FP64 / mixed) of 60,000 atoms 2073 / 1303 us (32 sites 2108 / 1314),
+// 96,000 2931 / 1712 (2943 / 1730), 135,000 3764 / 2199 (3755 / 2206), 240,000
+// 6313 / 3490 (6303 / 3475).
 #ifndef THP_SPREAD1_HALF_ATOMS
 #define THP_SPREAD1_HALF_ATOMS 100000
 #endif
@@ -634,10 +633,10 @@ template <typename T, typename HV>
 int launch_row(Ctx& c, int check_stop, HV* h) {
   const PairRows pr = pair_rows(c);
   const float interior = row_interior(c);
-  const int rb = c.n < kSingleRowSmall ? 32 : kBlock;
+  const int rb = c.n < kRowSmallAtoms ? 32 : kBlock;
   const int nb = group_blocks(c.n, rb);
   prof_mark(c, c.stream2);
-  if (c.n >= kSingleStreamAtoms)
+  if (c.n >= kStreamAtoms)
     k1_row<T, true, HV><<<nb, rb, 0, c.stream2>>>(pr, c.box, records<T>(c), c.d_cg, check_stop, interior, h);
   else
     k1_row<T, false, HV><<<nb, rb, 0, c.stream2>>>(pr, c.box, records<T>(c), c.d_cg, check_stop, interior, h);
@@ -694,7 +693,7 @@ int matvec_small(Ctx& c, double* x, int init) {
   return cuda_status(cudaGetLastError(), &c, "cg combine");
 }
 
-bool float_vectors(const Ctx& c) { return c.mixed && c.n >= kSingleLarge; }
+bool float_vectors(const Ctx& c) { return c.mixed && c.n >= kLargeAtoms; }
 
 }  // namespace
 
@@ -705,7 +704,7 @@ int single_begin(Ctx& c) {
   k1_take<<<(3 * c.n + 255) / 256, 256, 0, c.stream>>>(c.n, c.d_mu, mu);
   int st = cuda_status(cudaGetLastError(), &c, "cg start");
   if (st) return st;
-  if (c.n < kSingleLarge) return c.mixed ? matvec_small<float>(c, mu, 1) : matvec_small<double>(c, mu, 1);
+  if (c.n < kLargeAtoms) return c.mixed ? matvec_small<float>(c, mu, 1) : matvec_small<double>(c, mu, 1);
   return c.mixed ? matvec_large<float, double, float>(c, mu, 1) : matvec_large<double, double, double>(c, mu, 1);
 }
 
@@ -718,7 +717,7 @@ int single_iteration(Ctx& c, const LoopCond& loop) {
                                                   c.d_partials, c.cfg.poleps, c.cfg.politer, loop);
     return cuda_status(cudaGetLastError(), &c, "cg update");
   }
-  if (c.n >= kSingleLarge)
+  if (c.n >= kLargeAtoms)
     st = matvec_large<double, double, double>(c, c.d_pp, 0);
   else
     st = c.mixed ? matvec_small<float>(c, c.d_pp, 0) : matvec_small<double>(c, c.d_pp, 0);

@@ -207,7 +207,8 @@ struct Ctx {
   // the solve in hand runs the single-field CG (cg_single.cu): its vectors are
   // [n][3] in the front of the two-field buffers, its dipoles in d_dip
   int single = 0;
-  // the same of the FP64 form: {x, y, z (wrapped), d dipole, p dipole x, y} and p dipole z
+  // the FP64 form's partner records, as d_rec and d_mpz: {x, y, z (wrapped), d dipole,
+  // p dipole x, y} and p dipole z; of the single-field CG {x, y, z, dipole}
   double* d_rec64 = nullptr;  // [n][8]
   double* d_mpz64 = nullptr;  // [n]
   // the mixed form's overlapped CG keeps its search direction, h, residual

@@ -3,7 +3,7 @@
 // Restates epolar1c (epolar1.f:57-372) for a converged solve:
 //   * eprecip1 (epolar1.f:397-1213): the dipole grid of uind (Re) / uinp (Im)
 //     gathered to all 20 potential derivatives (fphi_uind_site), combined with
-//     the permanent-multipole potential fphirec kept from the field pass;
+//     the permanent-multipole potential fphirec (its grid convolved again);
 //   * epreal1c (epolar1.f:1215-2540, Thole branch): per pair the gradient of
 //     the d- and p-scaled permanent field on uinp / uind and of the mutual
 //     tensor (uscale) on uind x uinp, plus the induced field and its gradient
@@ -13,8 +13,9 @@
 // Eight lanes own atom i over its interacting pairs (each pair is evaluated
 // from both ends, the i-side terms only).  The three torques of a site are
 // summed before one torque distribution.  Gradients are accumulated in 64-bit
-// fixed point with 2^-34 kcal/mol/A resolution, so the order in which threads
-// add their contributions does not change the sums.
+// fixed point with 2^-34 kcal/mol/A resolution (in the FP64 form with a second
+// word for the remainders, FixAcc), so the order in which threads add their
+// contributions does not change the sums.
 #include <type_traits>
 
 #include "damp_dev.cuh"

@@ -5,6 +5,22 @@
 
 namespace thp {
 
+// Sizes (atoms) at which the per-system forms of several files change together,
+// with the device time of a cold water solve (FP64 / mixed, us) on either side.
+//
+// The CG of large systems, whose row runs beside the whole PME branch, and a
+// thread per site in the spreads; below, launches and latency bound a solve: its
+// spread forms the search direction itself and the row runs beside the
+// convolution.  13,500 atoms 892 / 679 (small form 848 / 632), 19,500 1016 / 754
+// (1026 / 748), 21,300 1099 / 780 (1069 / 780), 28,500 1287 / 876 (1380 / 927).
+constexpr int kLargeAtoms = 20000;
+// the pair stream (1.7 kB an atom) is far beyond L2: rows read it without allocating in L1
+constexpr int kStreamAtoms = 80000;
+// Below, real-space rows in blocks of one warp, which spread a small system over
+// the SMs: 4,800 atoms 565 / 493 (blocks of four 562 / 492), 7,800 689 / 565
+// (682 / 564), 9,003 697 / 569 (685 / 568), 13,500 854 / 656 (841 / 648).
+constexpr int kRowSmallAtoms = 8000;
+
 // nblist.cu
 int launch_sort_atoms(Ctx& c, bool carry = true);  // cell sort and permutation; the last dipoles and E0 follow
 int launch_gather_sorted(Ctx& c);       // positions/params/rpole into sorted order
@@ -44,7 +60,7 @@ int zero_grid(Ctx& c);  // before a spread: d_grid zero (nothing to do for the t
 int spread_status(Ctx& c, int st);  // after a spread that no convolution will follow: d_grid zero again
 struct PmeGeom;
 PmeGeom pme_geom(const Ctx& c);
-int launch_gather_dip(Ctx& c, double* d_out, bool check_stop);
+int launch_gather_dip(Ctx& c, double* d_out);
 
 // forces.cu
 int launch_forces(Ctx& c, double* d_out);  // dE/dx [n][3], original order, for the dipoles in d_mu

@@ -3,8 +3,9 @@
 // efld0_recip (newinduce_pme.f:1671-1917) and tmatxbrecip (:1919-2128):
 // B-splines recomputed per pass from positions (bsplgen, pmestuff.f:64),
 // spread with global atomics into one complex grid (d dipoles in Re, p in Im,
-// as qgrid2in_2d), cuFFT forward / influence function qfac / cuFFT backward
-// (unnormalised, fft_mpi.f90:65,115), and a gather of the potential
+// as qgrid2in_2d), the convolution with the influence function qfac (three
+// kernels, conv_dev.cuh, on the cubic grids they cover, else cuFFT forward, qfac,
+// cuFFT backward; unnormalised, fft_mpi.f90:65,115), and a gather of the potential
 // derivatives (fphi_mpole_site :453, fphi_uind_site :746).  Orthogonal boxes:
 // the fractional <-> Cartesian matrices reduce to a_d = nfft_d * recip(d,d).
 #include <vector>
@@ -420,9 +421,7 @@ namespace {
 template <typename T>
 __global__ void __launch_bounds__(128) k_gather_dip(int n, PmeGeom g, const double4* __restrict__ pos,
                                                     const typename Cplx<T>::type* __restrict__ grid,
-                                                    double* __restrict__ out, const CgScalars* __restrict__ cg,
-                                                    int check_stop) {
-  if (check_stop && cg->stop) return;
+                                                    double* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double o[6];
@@ -759,13 +758,8 @@ int spread_status(Ctx& c, int st) {
   return st;
 }
 
-// systems below this many atoms spread with a warp per site
-#ifndef THP_SPREAD_WARP_ATOMS
-#define THP_SPREAD_WARP_ATOMS 20000
-#endif
-
 static int spread_mpole(Ctx& c, const PmeGeom& g) {
-  const bool small = c.n < THP_SPREAD_WARP_ATOMS;
+  const bool small = c.n < kLargeAtoms;
   const int nb = small ? (c.n + 3) / 4 : (c.n + kBlock - 1) / kBlock;
   cufftComplex* gf = (cufftComplex*)c.d_grid;
   cufftDoubleComplex* gd = (cufftDoubleComplex*)c.d_grid;
@@ -907,7 +901,7 @@ static void spread_dipoles(Ctx& c, const PmeGeom& g, const V* vec, int check_sto
   if (THP_SPREAD_TILE && c.n >= kMin) {
     spread_tiled<T, V, 16>(c, g, vec, check_stop, grid);
   } else if constexpr (std::is_same<V, double>::value) {
-    if (c.n < THP_SPREAD_WARP_ATOMS) {
+    if (c.n < kLargeAtoms) {
       k_spread_dip_small<T><<<(c.n + 3) / 4, 128, 0, c.stream>>>(c.n, g, c.d_pos, const_cast<double*>(vec), nullptr,
                                                                 c.d_cg, check_stop, 0, nullptr, nullptr, nullptr, grid);
       return;
@@ -952,7 +946,7 @@ int launch_pme_dipole(Ctx& c, const double* d_vec, double* d_out, int check_stop
     spread_dipoles<double, double>(c, g, d_vec, check_stop, (cufftDoubleComplex*)c.d_grid);
   if ((st = cuda_status(cudaGetLastError(), &c, "spread dip"))) return spread_status(c, st);
   if ((st = convolve(c, check_stop))) return st;
-  if (d_out) st = launch_gather_dip(c, d_out, false);
+  if (d_out) st = launch_gather_dip(c, d_out);
   return st;
 }
 
@@ -967,15 +961,13 @@ int launch_pme_dipole_f32(Ctx& c, const float* d_vec, int check_stop) {
   return convolve(c, check_stop);
 }
 
-int launch_gather_dip(Ctx& c, double* d_out, bool check_stop) {
+int launch_gather_dip(Ctx& c, double* d_out) {
   PmeGeom g = geom_of(c);
   const int nb = (c.n + kBlock - 1) / kBlock;
   if (c.mixed)
-    k_gather_dip<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_conv, d_out, c.d_cg,
-                                                  check_stop ? 1 : 0);
+    k_gather_dip<float><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftComplex*)c.d_conv, d_out);
   else
-    k_gather_dip<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_conv, d_out,
-                                                   c.d_cg, check_stop ? 1 : 0);
+    k_gather_dip<double><<<nb, kBlock, 0, c.stream>>>(c.n, g, c.d_pos, (const cufftDoubleComplex*)c.d_conv, d_out);
   return cuda_status(cudaGetLastError(), &c, "gather dip");
 }
 

@@ -1,12 +1,13 @@
 // solver.cu -- device-resident preconditioned conjugate gradient.
 //
 // inducepcg_pme2 (newinduce_pme2.f:285-636) with every vector and scalar on
-// the device.  Per iteration (systems of THP_OVERLAP_MIN_ATOMS atoms and
-// more; smaller ones: matvec_small):
+// the device.  Systems whose two dipole sets are the same run cg_single.cu
+// instead.  Per iteration (systems of kLargeAtoms atoms and more; smaller ones:
+// matvec_small):
 //   1. pp = zr + beta*pp, with the partner records of the real-space row;
 //   2. fork: the real-space row T_real pp runs on the side stream while the
-//      main stream spreads pp on the PME grid, runs cuFFT forward, qfac and
-//      cuFFT backward;
+//      main stream spreads pp on the PME grid and convolves it (conv_dev.cuh,
+//      or cuFFT and qfac for grids that does not cover);
 //   3. join, then the combine kernel gathers the dipole field from the grid
 //      and forms h = T_real pp + pp/alpha + dipfield - self term; partial
 //      pp.h; the last block forms gg and alpha;
@@ -22,10 +23,6 @@
 #include "cg_dev.cuh"
 #include "kernels.h"
 
-// Systems of at least THP_OVERLAP_MIN_ATOMS atoms run the real-space row of
-// each CG matvec on a side stream, concurrent with the whole PME branch.
-// Smaller systems are bound by launches and latency: their spread forms the
-// search direction itself and the row runs beside the convolution.
 // 1: the CG loop runs on the device as one graph with a conditional WHILE
 // node; 0: graph-replayed chunks of kCgChunk iterations with a host check
 #ifndef THP_DEVICE_LOOP
@@ -35,21 +32,6 @@
 // minimum resident blocks per SM asked of the compiler for the real-space row
 #ifndef THP_ROW_MINB
 #define THP_ROW_MINB 0
-#endif
-
-// systems of at least this many atoms read the mixed row's pair stream
-// (~1.7 kB per atom, far beyond L2 from here on) without allocating in L1
-#ifndef THP_STREAM_NO_L1_ATOMS
-#define THP_STREAM_NO_L1_ATOMS 80000
-#endif
-
-#ifndef THP_OVERLAP_MIN_ATOMS
-#define THP_OVERLAP_MIN_ATOMS 20000
-#endif
-
-// systems below this many atoms run their rows in blocks of one warp
-#ifndef THP_ROW_SMALL_ATOMS
-#define THP_ROW_SMALL_ATOMS 8000
 #endif
 
 namespace thp {
@@ -314,7 +296,7 @@ void prof_mark(Ctx& c, cudaStream_t s) {
   c.prof_events.push_back(e);
 }
 
-bool overlap_rows(const Ctx& c) { return c.n >= THP_OVERLAP_MIN_ATOMS; }
+bool overlap_rows(const Ctx& c) { return c.n >= kLargeAtoms; }
 static bool overlapped(const Ctx& c) { return overlap_rows(c); }
 
 // One application of the CG matrix with the real-space row on the side
@@ -330,13 +312,13 @@ static int matvec_overlapped(Ctx& c, const XV* x, int init) {
   const int nbr = group_blocks(c.n, kBlock);  // one warp per group of four atoms
   const float interior = row_interior(c);
   prof_mark(c, c.stream2);
-  if (c.mixed && c.n >= THP_STREAM_NO_L1_ATOMS)
+  if (c.mixed && c.n >= kStreamAtoms)
     k_real_row<true, true, float><<<nbr, kBlock, 0, c.stream2>>>(pr, c.box, c.d_pos, c.d_rec, nullptr, c.d_mpz, c.d_cg,
                                                                  !init, interior, c.d_hf);
   else if (c.mixed)
     k_real_row<true, false, float><<<nbr, kBlock, 0, c.stream2>>>(pr, c.box, c.d_pos, c.d_rec, nullptr, c.d_mpz,
                                                                   c.d_cg, !init, interior, c.d_hf);
-  else if (c.n >= THP_STREAM_NO_L1_ATOMS)
+  else if (c.n >= kStreamAtoms)
     k_real_row64<true><<<nbr, kBlock, 0, c.stream2>>>(pr, c.box, c.d_rec64, c.d_mpz64, c.d_cg, !init, interior, c.d_h);
   else
     k_real_row64<false><<<nbr, kBlock, 0, c.stream2>>>(pr, c.box, c.d_rec64, c.d_mpz64, c.d_cg, !init, interior, c.d_h);
@@ -368,7 +350,7 @@ static int matvec_small(Ctx& c, double* x, int init) {
   cudaEventRecord(c.ev_fork, c.stream);
   cudaStreamWaitEvent(c.stream2, c.ev_fork, 0);
   const PairRows pr = pair_rows(c);
-  const int rb = c.n < THP_ROW_SMALL_ATOMS ? 32 : kBlock;
+  const int rb = c.n < kRowSmallAtoms ? 32 : kBlock;
   const int nbr = group_blocks(c.n, rb);
   prof_mark(c, c.stream2);
   if (c.mixed)

@@ -281,7 +281,8 @@ class Batch:
     def profile(self, enable=None):
         """enable True/False switches the eager, per-kernel-timed loop on/off
         (resetting the accumulators); returns the accumulated ms per kernel
-        and the iterations timed so far."""
+        and the iterations timed so far.  Grids of the own convolution run all
+        of it in "fft_forward"; "qfac" and "fft_inverse" are those of cuFFT."""
         ms = (C.c_double * len(self.KERNELS))()
         it = C.c_int()
         mode = -1 if enable is None else (1 if enable else 0)
