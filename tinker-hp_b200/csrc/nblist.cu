@@ -139,10 +139,12 @@ __global__ void k_cell_rank(int n, const int* __restrict__ atom_cell, const int*
 
 // The whole cell sort of a small system in one block: cells, counts, scan,
 // fill and the order inside each cell in shared memory, then the special
-// partners in the new numbering.  The six launches of the general form take
-// about 3 us each whatever the size; one block keeps up with them to
-// kSortSmallAtoms atoms.
-constexpr int kSortSmallAtoms = 8192, kSortSmallCells = 4096;
+// partners in the new numbering.  The launches of the general form take about
+// 3 us each whatever the size; one block, which sorts each cell with one thread,
+// keeps up with them to kSortSmallAtoms atoms: a cold solve (FP64 / mixed) of 648
+// atoms 411 / 354 us (general sort 428 / 370), 4,113 554 / 476 (562 / 487), 6,000
+// 648 / 535 (655 / 537), 8,100 678 / 548 (669 / 546).
+constexpr int kSortSmallAtoms = 7168, kSortSmallCells = 4096;
 constexpr size_t kSortSmallSmem =
     sizeof(int) * (kSortSmallAtoms + 2 * kSortSmallCells) + sizeof(unsigned short) * kSortSmallAtoms;
 
