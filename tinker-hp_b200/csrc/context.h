@@ -165,6 +165,7 @@ struct Ctx {
   cufftHandle plan = 0;
   bool have_plan = false;
   void* d_grids = nullptr;  // the allocation of the grid arrays below
+  void* d_convs = nullptr;  // of d_conv_buf and d_pot, where they came later
   int plan_dims[3] = {0, 0, 0};
   size_t cap_ngrid = 0, cap_conv = 0;  // points of d_grid and d_qfac, of d_conv_buf and d_pot
   void* d_grid = nullptr;  // cufftDoubleComplex or cufftComplex

@@ -648,8 +648,50 @@ static const std::vector<double>& dftmod_cached(int nfft) {
 
 static void free_grids(Ctx& c) {
   cudaFree(c.d_grids);
-  for (void** p : {&c.d_grids, &c.d_qfac, &c.d_grid, &c.d_conv_buf, &c.d_pot}) *p = nullptr;
+  cudaFree(c.d_convs);
+  for (void** p : {&c.d_grids, &c.d_convs, &c.d_qfac, &c.d_grid, &c.d_conv_buf, &c.d_pot}) *p = nullptr;
   c.cap_ngrid = c.cap_conv = 0;
+}
+
+// The grid arrays in one allocation, each on a 256-byte boundary.  They are kept
+// while they are large enough (a re-targeted context reuses them).  Only the
+// three-kernel convolution needs the second grid and the potential: a context
+// made for another grid gets them, apart, when it first serves one, and nothing
+// is freed (cudaFree would stall the other contexts of a server).
+static int size_grids(Ctx& c) {
+  const size_t esz = c.mixed ? sizeof(float) : sizeof(double);
+  const size_t csz = c.mixed ? sizeof(cufftComplex) : sizeof(cufftDoubleComplex);
+  struct Array {
+    void** p;
+    size_t bytes;
+  };
+  auto take = [&](void** base, std::initializer_list<Array> arrays) {
+    size_t total = 0;
+    for (const Array& g : arrays) total += (g.bytes + 255) / 256 * 256;
+    if (cuda_status(cudaMalloc(base, total), &c, "alloc grid")) return false;
+    char* at = static_cast<char*>(*base);
+    for (const Array& g : arrays) {
+      *g.p = at;
+      at += (g.bytes + 255) / 256 * 256;
+    }
+    return true;
+  };
+  const size_t n = c.ngrid, nconv = c.conv ? n : 0;
+  if (n > c.cap_ngrid) {
+    const size_t mc = std::max(nconv, c.cap_conv);
+    free_grids(c);
+    if (!take(&c.d_grids, {{&c.d_grid, csz * n}, {&c.d_qfac, esz * n}, {&c.d_conv_buf, csz * mc}, {&c.d_pot, esz * mc}}))
+      return THP_E_CUDA;
+    c.cap_ngrid = n;
+    c.cap_conv = mc;
+  } else if (nconv > c.cap_conv) {
+    cudaFree(c.d_convs);
+    c.d_convs = nullptr;
+    c.cap_conv = 0;
+    if (!take(&c.d_convs, {{&c.d_conv_buf, csz * nconv}, {&c.d_pot, esz * nconv}})) return THP_E_CUDA;
+    c.cap_conv = nconv;
+  }
+  return THP_OK;
 }
 
 int pme_init(Ctx& c) {
@@ -660,33 +702,11 @@ int pme_init(Ctx& c) {
   const std::vector<double>& m1 = dftmod_cached(c.nfft[0]);
   const std::vector<double>& m2 = dftmod_cached(c.nfft[1]);
   const std::vector<double>& m3 = dftmod_cached(c.nfft[2]);
-  size_t esz = c.mixed ? sizeof(float) : sizeof(double);
-  size_t csz = c.mixed ? sizeof(cufftComplex) : sizeof(cufftDoubleComplex);
+  const size_t csz = c.mixed ? sizeof(cufftComplex) : sizeof(cufftDoubleComplex);
   c.conv_r[0] = c.conv_r[1] = 1;
   c.conv = conv_covers(c.nfft, c.mixed, &c.conv_r[0], &c.conv_r[1]) ? 1 : 0;
   const XOrder xo{c.conv_r[0], c.conv_r[1]};
-  // grid buffers are kept while they are large enough (a re-targeted
-  // context reuses them); only the three-kernel convolution needs a second grid and a potential
-  const size_t nconv = c.conv ? c.ngrid : 0;
-  if (c.ngrid > c.cap_ngrid || nconv > c.cap_conv) {
-    const size_t m = std::max(c.ngrid, c.cap_ngrid), mc = std::max(nconv, c.cap_conv);
-    free_grids(c);
-    // one allocation, each array on a 256-byte boundary
-    const struct {
-      void** p;
-      size_t bytes;
-    } grids[] = {{&c.d_grid, csz * m}, {&c.d_qfac, esz * m}, {&c.d_conv_buf, csz * mc}, {&c.d_pot, esz * mc}};
-    size_t total = 0;
-    for (const auto& g : grids) total += (g.bytes + 255) / 256 * 256;
-    if (cuda_status(cudaMalloc(&c.d_grids, total), &c, "alloc grid")) return THP_E_CUDA;
-    char* at = static_cast<char*>(c.d_grids);
-    for (const auto& g : grids) {
-      *g.p = at;
-      at += (g.bytes + 255) / 256 * 256;
-    }
-    c.cap_ngrid = m;
-    c.cap_conv = mc;
-  }
+  if (int st = size_grids(c)) return st;
   c.d_conv = c.conv ? c.d_conv_buf : c.d_grid;
   // influence function on the device (newinduce_pme.f:1802-1854): the
   // B-spline moduli go through the front of the grid buffer
