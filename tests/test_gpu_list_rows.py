@@ -1,7 +1,10 @@
 """Neighbour lists of boxes with at least seven cells per axis and 5,000 atoms,
 pair for pair against a k-d tree in FP64: unequal edges and cell edges from the smallest to
 nearly the largest, atom counts that leave a short last block, atoms outside the
-box, and a clump so dense that a lane's share of a row does not fit its buffer.
+box, a clump so dense that a lane's share of a row does not fit its buffer, and
+cutoffs at which some lanes' shares or nearly all do not (each size of buffer), so
+that a row is finished from the middle, or at which a smaller system's rows go to
+a warp per atom.
 Pairs within 1e-9 A of the list radius may be on either side.
 """
 import dataclasses
@@ -45,3 +48,19 @@ def test_rows_match_tree(thp, nw, stretch, clump, precision):
     assert np.isin(got, keys(reference(pos, box, r + 1e-9), ws.n)).all()
     if clump < 1.0:
         assert 2 * len(got) > 5 * 64 * ws.n  # on average more than the five lanes' buffers hold
+
+
+@pytest.mark.parametrize("nw,cut", [(3001, 7.5), (3001, 8.5), (7001, 8.0), (7001, 9.0), (7001, 9.5),
+                                    (7001, 11.0)])
+def test_rows_past_the_buffer_match_tree(thp, nw, cut):
+    from tinker_hp_b200 import lib
+    ws = dataclasses.replace(thp.water.make_water_box(nw, cfg=0), ewaldcut=cut, vdw=None)
+    ctx = lib.Context(ws, precision=lib.FP64, max_neighbors=1000)
+    assert all(e >= 7 * (0.5 * (cut + ws.lbuffer) + 1e-6) for e in ws.box)
+    ctx.nblist()
+    r, box = cut + ws.lbuffer, np.array(ws.box)
+    pairs = ctx.pairs(1000)
+    got = keys(pairs, ws.n)
+    assert len(np.unique(got)) == len(got)
+    assert np.isin(keys(reference(ws.positions(), box, r - 1e-9), ws.n), got).all()
+    assert np.isin(got, keys(reference(ws.positions(), box, r + 1e-9), ws.n)).all()

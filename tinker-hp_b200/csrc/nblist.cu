@@ -336,6 +336,13 @@ __device__ __forceinline__ int axis_cells(int c, int nc, int q) {
 #define THP_LIST_SPLIT_ATOMS 5000
 #endif
 
+// Below THP_LIST_WARP_ATOMS the long rows of a large cutoff go to a warp per atom
+// as well: k_build_list_split has too few lanes in flight for them.  Water, lists
+// alone (us, split / warp per atom): 5,103 atoms 108 / 96 at an 8 A cutoff (258
+// partners), 164 / 107 at 9 A (360); 9,003 atoms 111 / 114 at 7.5 A (215), 122 /
+// 114 at 8 A; 19,500 atoms 174 / 187 at 8.5 A (306), 223 / 204 at 10 A (486).
+constexpr double kListWarpPartners = 160.0;
+
 // The list decision for candidate k of atom i: the FP32 screen accepts below
 // lo and rejects above hi; between them (and for every candidate when the
 // screen is off) the exact FP64 r^2 of the reference decides.
@@ -433,19 +440,17 @@ __device__ __forceinline__ void list_row_global(int i, int cap8, const ListTest&
 //     4.28 A; the whole windows hold 668 and 982);
 //   * accepted partners wait in shared memory; a row's warps then write it
 //     together, 8 consecutive slots per atom at a time.  A lane with more than
-//     kListBuf partners (water: 30 to 37, at most 64) walks its rows again once
-//     its first slot is known and writes them itself.
+//     BUF partners (water at 7.5 A: 30 to 37, at most 64) walks its rows again
+//     from the one that filled its buffer, once its first slot is known, and
+//     writes the partners from there on itself.
 // What bounds it is issue and, in smaller systems, the chain of loads: a
 // thread per atom leaves a 32,000-atom system two warps per scheduler.
 // 288,000 atoms: 404 us (a thread per atom 490), 32,000: 76 (123), 9,003: 43 (a
-// warp per atom 56).  Buffers of 48 entries send a few lanes around again
-// (657 us at 288,000 atoms); batches of 2, 3, 4 and 8 candidates take 434, 404,
-// 431 and 535 us: a row holds 18 on average.
+// warp per atom 56).  Batches of 2, 3, 4 and 8 candidates take 434, 404, 431 and
+// 535 us: a row holds 18 on average.  BUF: see list_buffer.
 constexpr int kListWarps = 5;
-#ifndef THP_LIST_BUF
-#define THP_LIST_BUF 64
-#endif
-constexpr int kListBuf = THP_LIST_BUF;
+template <int BUF>
+constexpr size_t kListSmem = sizeof(int) * BUF * kListWarps * 32;
 // candidates loaded together
 #ifndef THP_LIST_BATCH
 #define THP_LIST_BATCH 3
@@ -463,11 +468,13 @@ __device__ __forceinline__ float cell_gap(float f, int q, float e) {
   return fmaxf(0.f, fmaxf(q * e - f, f - (q + 1) * e));
 }
 
-template <typename Add>
-__device__ __forceinline__ void scan_rows(int i, int w, const ListTest& lt, const ListCells& lc,
+// The rows of warp w from the q0-th on (a lane's own): begin(qz) before each
+// row, add(k) for each partner.
+template <typename Begin, typename Add>
+__device__ __forceinline__ void scan_rows(int i, int w, int q0, const ListTest& lt, const ListCells& lc,
                                           const double4* __restrict__ pos, const float4* __restrict__ posf,
                                           const int* __restrict__ scell, const int* __restrict__ cell_start,
-                                          const int* __restrict__ cell_count, Add&& add) {
+                                          const int* __restrict__ cell_count, Begin&& begin, Add&& add) {
   const float4 fi = posf[i];
   const int c = scell[i];
   const int cx = c % lc.nx, cy = (c / lc.nx) % lc.ny, cz = c / (lc.nx * lc.ny);
@@ -482,7 +489,7 @@ __device__ __forceinline__ void scan_rows(int i, int w, const ListTest& lt, cons
     lo = 0;
     hi = -1;
     k0 = k1 = 0;
-    if (e2 < 0.f) return;
+    if (e2 < 0.f || qz < q0) return;
     reached_cells(cx, rx, sqrtf(e2), lc.ivx, lo, hi);
     const int z = zr < 0 ? zr + lc.nz : (zr >= lc.nz ? zr - lc.nz : zr);
     const int y = yr < 0 ? yr + lc.ny : (yr >= lc.ny ? yr - lc.ny : yr);
@@ -517,6 +524,7 @@ __device__ __forceinline__ void scan_rows(int i, int w, const ListTest& lt, cons
     const int a = k0, b = k1, l = lo, h = hi, rb = base;
     const float fy = sy, fz = sz;
     if (qz < 4) next(qz + 1);
+    begin(qz);
     walk(a, b, fi.x, fy, fz);
     if (l < 0) {  // the part past the lower face
       const int x1 = rb + lc.nx - 1;
@@ -528,30 +536,44 @@ __device__ __forceinline__ void scan_rows(int i, int w, const ListTest& lt, cons
   }
 }
 
-__global__ void __launch_bounds__(32 * kListWarps, THP_LIST_MINB) k_build_list_split(
+template <int BUF>
+__global__ void __launch_bounds__(32 * kListWarps, 5) k_build_list_split(
     int n, int cap8, ListTest lt, ListCells lc, const double4* __restrict__ pos, const float4* __restrict__ posf,
     const int* __restrict__ scell, const int* __restrict__ cell_start, const int* __restrict__ cell_count, int maxnb,
     int* __restrict__ nnb, int* __restrict__ nb, int* __restrict__ flags) {
-  __shared__ int buf[kListBuf][kListWarps][32];
-  __shared__ int part[kListWarps][32];
+  extern __shared__ int list_smem[];
+  int(*buf)[kListWarps][32] = reinterpret_cast<int(*)[kListWarps][32]>(list_smem);  // [BUF]
+  __shared__ int part[kListWarps][32], kept[kListWarps][32];  // partners, and those of them taken from buf
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i0 = blockIdx.x * 32, i = i0 + lane;
   int cnt = 0;
+  int full = 0, before = 0;  // the row that filled the buffer, and the partners before it
   if (i < n)
-    scan_rows(i, w, lt, lc, pos, posf, scell, cell_start, cell_count, [&](int k) {
-      if (cnt < kListBuf) buf[cnt][w][lane] = k;
-      ++cnt;
-    });
+    scan_rows(
+        i, w, 0, lt, lc, pos, posf, scell, cell_start, cell_count,
+        [&](int qz) {
+          if (cnt <= BUF) {
+            full = qz;
+            before = cnt;
+          }
+        },
+        [&](int k) {
+          if (cnt < BUF) buf[cnt][w][lane] = k;
+          ++cnt;
+        });
   part[w][lane] = cnt;
+  kept[w][lane] = cnt > BUF ? before : cnt;
   __syncthreads();
-  if (cnt > kListBuf) {
-    int s = 0;
+  if (cnt > BUF) {
+    int s = before;
     for (int v = 0; v < w; ++v) s += part[v][lane];
     int* __restrict__ row = nb + pair_slot(cap8, i, 0);  // entry s: row[s + 3 (s & ~7)]
-    scan_rows(i, w, lt, lc, pos, posf, scell, cell_start, cell_count, [&](int k) {
-      if (s < maxnb) row[s + 3 * (s & ~7)] = k;
-      ++s;
-    });
+    scan_rows(
+        i, w, full, lt, lc, pos, posf, scell, cell_start, cell_count, [](int) {},
+        [&](int k) {
+          if (s < maxnb) row[s + 3 * (s & ~7)] = k;
+          ++s;
+        });
   }
   // eight lanes per atom, a group of four atoms per warp: consecutive slots
   const int a = lane >> 3, j = lane & 7;
@@ -576,7 +598,7 @@ __global__ void __launch_bounds__(32 * kListWarps, THP_LIST_MINB) k_build_list_s
           v = u + 1;
           first = end[u];
         }
-      if (part[v][q] <= kListBuf) row[s + 3 * (s & ~7)] = buf[s - first][v][q];
+      if (s - first < kept[v][q]) row[s + 3 * (s & ~7)] = buf[s - first][v][q];
     }
   }
 }
@@ -852,6 +874,33 @@ int launch_gather_sorted(Ctx& c) {
 
 int launch_build_list(Ctx& c) { return launch_build_list_on(c, c.stream); }
 
+template <int BUF>
+static void launch_list_buf(Ctx& c, int cap8, const ListTest& lt, const ListCells& lc, cudaStream_t s) {
+  static std::atomic<unsigned long long> limit_set{0};
+  if (kListSmem<BUF> > 40 * 1024) smem_limit_once(k_build_list_split<BUF>, kListSmem<BUF>, limit_set);
+  k_build_list_split<BUF><<<(c.n + 31) / 32, 32 * kListWarps, kListSmem<BUF>, s>>>(
+      c.n, cap8, lt, lc, c.d_pos, c.d_posf, c.d_scell, c.d_cell_start, c.d_cell_count, c.maxnb, c.d_nnb, c.d_nb,
+      c.d_flags);
+}
+
+// The lanes' buffers by the partners an atom expects, a fifth of them a lane's:
+// what spares the second walk against the blocks an SM holds (64 entries: five
+// blocks, 80: four, 112: three).  Lists of 288,000 / 32,400 water atoms alone, us,
+// with 64 entries and with those taken here: at an 8 A cutoff (258 partners) 769 /
+// 185 and 707 / 154, at 8.5 A (306) 987 / 220 and 892 / 190, at 9 A (360) 1220 /
+// 260 and 1077 / 214.  On the other sides 64 are the faster: at 7.5 A (215) 634
+// against 695 with 80, at 10 A (486) 1702 against 1837 with 112 (288,000 atoms,
+// a number of entries fixed at run time).
+static void launch_list_split(Ctx& c, double partners, int cap8, const ListTest& lt, const ListCells& lc,
+                              cudaStream_t s) {
+  if (partners > 230.0 && partners <= 330.0)
+    launch_list_buf<80>(c, cap8, lt, lc, s);
+  else if (partners > 330.0 && partners <= 430.0)
+    launch_list_buf<112>(c, cap8, lt, lc, s);
+  else
+    launch_list_buf<64>(c, cap8, lt, lc, s);
+}
+
 int launch_build_list_on(Ctx& c, cudaStream_t s) {
   const int n = c.n;
   const double rl = c.cfg.ewaldcut + c.cfg.lbuffer;
@@ -886,10 +935,12 @@ int launch_build_list_on(Ctx& c, cudaStream_t s) {
   const double reach = sqrt(mbuf2 * (1.0 + band)) + 16.0 * dr + 1e-3;
   lc.reach2 = (float)(reach * reach);
   const int cap8 = c.maxpr / 8;
-  if (prefilter && n >= THP_LIST_SPLIT_ATOMS && c.nc[0] >= 7 && c.nc[1] >= 7 && c.nc[2] >= 7)
-    k_build_list_split<<<(n + 31) / 32, 32 * kListWarps, 0, s>>>(n, cap8, lt, lc, c.d_pos, c.d_posf, c.d_scell,
-                                                                 c.d_cell_start, c.d_cell_count, c.maxnb, c.d_nnb,
-                                                                 c.d_nb, c.d_flags);
+  // expected partners of an atom
+  const double partners = n / (c.box.l[0] * c.box.l[1] * c.box.l[2]) * (4.0 / 3.0) * kPi * rl * rl * rl;
+  const bool split = prefilter && c.nc[0] >= 7 && c.nc[1] >= 7 && c.nc[2] >= 7 && n >= THP_LIST_SPLIT_ATOMS &&
+                     (n >= THP_LIST_WARP_ATOMS || partners <= kListWarpPartners + 0.01 * n);
+  if (split)
+    launch_list_split(c, partners, cap8, lt, lc, s);
   else if (n < THP_LIST_WARP_ATOMS)
     k_build_list_warp<<<(n + 3) / 4, 128, 0, s>>>(n, cap8, lt, c.nc[0], c.nc[1], c.nc[2], c.d_pos, c.d_posf,
                                                   c.d_scell, c.d_cell_start, c.d_cell_count, c.maxnb, c.d_nnb,
