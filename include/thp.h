@@ -104,7 +104,9 @@ int thp_ctx_destroy(thp_ctx* ctx);
  * device buffer that is large enough and any cuFFT plan of an unchanged grid
  * are kept, so no device memory is freed or allocated unless the new system
  * is larger.  All system state is cleared (parameters, connectivity,
- * positions, multipoles, list, dipoles, bindings), as after thp_ctx_create. */
+ * positions, multipoles, list, dipoles, bindings), as after thp_ctx_create.
+ * When the new system's memory cannot be allocated (THP_E_CUDA) the context
+ * serves none: calls return THP_E_STATE until another reset succeeds. */
 int thp_ctx_reset(thp_ctx* ctx, const thp_config* cfg);
 /* device bytes the context holds at its current capacity */
 size_t thp_ctx_footprint(thp_ctx* ctx);

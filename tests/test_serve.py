@@ -174,6 +174,31 @@ def test_context_moves_between_kinds_of_grid(thp):
 
 
 @pytest.mark.gpu
+def test_context_refuses_calls_after_a_failed_retarget(thp):
+    # a grid larger than the device: its allocation fails, and with it the old
+    # grid is gone; the context answers every call with a status until it is
+    # re-targeted again
+    import dataclasses
+    from tinker_hp_b200 import lib
+    ws = thp.water.make_water_box(216, cfg=0)
+    ctx = lib.Context(ws)
+    ref = ctx.solve()["epol"]
+    with pytest.raises(lib.ThpError) as e:
+        ctx.retarget(dataclasses.replace(ws, nfft=(3000, 3000, 3000)))
+    assert e.value.status == lib.THP_E_CUDA
+    for call in (ctx.solve, ctx.gradient, ctx.empole1, ctx.ehal1, ctx.nblist, ctx.field, ctx.dipoles, ctx.pairs,
+                 lambda: ctx.tmatxb(np.zeros((ws.n, 2, 3))), lambda: ctx.tmatxbrecip(np.zeros((ws.n, 2, 3))),
+                 lambda: ctx.set_guess(np.zeros((ws.n, 2, 3))), lambda: ctx.set_positions(ws.x, ws.y, ws.z),
+                 lambda: ctx.set_rpole(np.zeros((ws.n, 13))), lambda: ctx.set_vdw(ws.vdw),
+                 lambda: ctx.set_virial(True), lambda: ctx._setup(ws, True, None)):
+        with pytest.raises(lib.ThpError) as e:
+            call()
+        assert e.value.status == lib.THP_E_STATE
+    ctx.retarget(ws)
+    assert abs(ctx.solve()["epol"] - ref) < 1e-12 * abs(ref)
+
+
+@pytest.mark.gpu
 def test_context_retarget_matches_fresh_context(thp):
     # one context serves a small, a larger and another small system in turn
     # (thp_ctx_reset grows buffers and re-plans the FFT only when needed)

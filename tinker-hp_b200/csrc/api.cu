@@ -30,6 +30,7 @@ struct thp_ctx {
 namespace thp {
 int cuda_status(cudaError_t e, Ctx* c, const char* what) {
   if (e == cudaSuccess) return THP_OK;
+  cudaGetLastError();  // reported here, not again by the next launch's check
   if (c) {
     c->last_msg = std::string(what) + ": " + cudaGetErrorString(e);
   }
@@ -622,10 +623,9 @@ static int size_buffers(Ctx& c) {
   return st;
 }
 
-// Clears everything that belongs to the system a context serves, after
-// apply_config/size_buffers/pme_init: no parameters, positions,
-// multipoles, list or dipoles; no special pairs.
-static int clear_system_state(thp_ctx* h) {
+// Everything the host knows of the system a context serves: no parameters,
+// positions, multipoles, list or dipoles.
+static void forget_system(thp_ctx* h) {
   Ctx& c = h->c;
   c.have_params = c.have_pos = c.have_rpole = c.have_conn = c.have_frames = c.have_axes = false;
   c.have_perm = c.have_list = c.have_coef = c.have_dipoles = c.have_ef_prev = false;
@@ -642,6 +642,12 @@ static int clear_system_state(thp_ctx* h) {
   c.mscale[2] = c.mscale[3] = 1.0;
   c.bnelst = c.belst = nullptr;
   c.bmaxelst = 0;
+}
+
+// forget_system, and no special pairs, after apply_config/size_buffers/pme_init.
+static int clear_system_state(thp_ctx* h) {
+  Ctx& c = h->c;
+  forget_system(h);
   cudaMemsetAsync(c.d_flags, 0, sizeof(int), c.stream);
   cudaMemsetAsync(c.d_cg, 0, sizeof(CgScalars), c.stream);
   cudaMemsetAsync(c.d_mu, 0, sizeof(double) * 6 * c.n, c.stream);
@@ -670,6 +676,7 @@ int thp_ctx_create(const thp_config* cfg, thp_ctx** out) {
   if (!st) st = cuda_status(cudaEventCreate(&c.ev1), &c, "event");
   if (!st) st = size_buffers(c);
   if (!st) st = pme_init(c);
+  c.sized = !st;
   if (!st) st = clear_system_state(h);
   if (st) {
     fprintf(stderr, "thp_ctx_create: %s\n", c.last_msg.c_str());
@@ -696,14 +703,19 @@ int thp_ctx_reset(thp_ctx* h, const thp_config* cfg) {
   c.prof_events.clear();
   c.profiling = false;
   const size_t old_ngrid = c.ngrid;
+  // first: if an allocation below fails, the context has no system and takes
+  // none until another reset (some of its buffers may be gone)
+  forget_system(h);
+  c.sized = false;
+  if (g_current == h) g_current = nullptr;
   apply_config(c, *cfg);
   if ((st = size_buffers(c))) return st;
   if ((st = pme_init(c))) return st;
+  c.sized = true;
   if (c.ngrid > old_ngrid && c.d_sgrid) {
     cudaFree(c.d_sgrid);
     c.d_sgrid = nullptr;
   }
-  if (g_current == h) g_current = nullptr;
   return clear_system_state(h);
 }
 
@@ -742,6 +754,7 @@ int thp_set_stream(thp_ctx* h, void* stream) {
 int thp_set_params(thp_ctx* h, const double* polarity, const double* thole, const double* pdamp) {
   if (!h || !polarity || !thole || !pdamp) return THP_E_INVALID;
   Ctx& c = h->c;
+  if (!c.sized) return THP_E_STATE;
   if (set_current_device(c)) return THP_E_CUDA;
   const size_t n = c.n;
   c.h_polarity.assign(polarity, polarity + n);
@@ -761,6 +774,7 @@ int thp_set_params(thp_ctx* h, const double* polarity, const double* thole, cons
 int thp_set_connectivity(thp_ctx* h, const int* const* off, const int* const* idx, const double* scales) {
   if (!h || !scales) return THP_E_INVALID;
   Ctx& c = h->c;
+  if (!c.sized) return THP_E_STATE;
   drop_front_graphs(c);
   if (set_current_device(c)) return THP_E_CUDA;
   std::memcpy(c.scales, scales, sizeof(c.scales));
@@ -870,6 +884,7 @@ int image_load(thp_ctx* h, const SystemImage* img) {
   if (!h || !img) return THP_E_INVALID;
   Ctx& c = h->c;
   if (img->n != c.n) return THP_E_INVALID;
+  if (!c.sized) return THP_E_STATE;
   drop_front_graphs(c);
   if (set_current_device(c)) return THP_E_CUDA;
   const size_t n = c.n;
@@ -923,6 +938,7 @@ static bool all_finite(const double* v, size_t n) {
 int upload_positions(thp_ctx* h, const double* x, const double* y, const double* z, bool host_check) {
   if (!h || !x || !y || !z) return THP_E_INVALID;
   Ctx& c = h->c;
+  if (!c.sized) return THP_E_STATE;
   if (set_current_device(c)) return THP_E_CUDA;
   const size_t n = c.n;
   if (host_check && (!all_finite(x, n) || !all_finite(y, n) || !all_finite(z, n))) return THP_E_INVALID;
@@ -947,6 +963,7 @@ int thp_set_positions(thp_ctx* h, const double* x, const double* y, const double
 int thp_set_rpole(thp_ctx* h, const double* rpole) {
   if (!h || !rpole) return THP_E_INVALID;
   Ctx& c = h->c;
+  if (!c.sized) return THP_E_STATE;
   drop_front_graphs(c);
   if (set_current_device(c)) return THP_E_CUDA;
   cudaMemcpyAsync(c.d_rpole_orig, rpole, sizeof(double) * 13 * c.n, cudaMemcpyHostToDevice, c.stream);
@@ -960,6 +977,7 @@ int thp_set_rpole(thp_ctx* h, const double* rpole) {
 int thp_set_frames(thp_ctx* h, const double* pole, const int* zaxis, const int* xaxis, const int* axt) {
   if (!h || !pole || !zaxis || !xaxis || !axt) return THP_E_INVALID;
   Ctx& c = h->c;
+  if (!c.sized) return THP_E_STATE;
   drop_front_graphs(c);
   if (set_current_device(c)) return THP_E_CUDA;
   const int n = c.n;
@@ -1067,6 +1085,7 @@ int thp_set_vdw(thp_ctx* h, const int* cls, int nclass, const double* tables, co
                 const double* kred, const double* vscale, double vdwcut, double vdwtaper, double ghal, double dhal) {
   if (!h || !cls || !tables || !ired || !kred || !vscale || nclass <= 0 || nclass > 4096) return THP_E_INVALID;
   Ctx& c = h->c;
+  if (!c.sized) return THP_E_STATE;
   const int n = c.n;
   if (!(vdwcut > 0.0) || !(vdwtaper > 0.0) || !std::isfinite(ghal) || !std::isfinite(dhal)) return THP_E_INVALID;
   for (int i = 0; i < n; ++i)
@@ -1678,6 +1697,7 @@ int thp_get_ehal_virial(thp_ctx* h, double* vir) {
 // The virial's transforms run through cuFFT, for which a grid of the own
 // convolution has no plan yet: it is made here, not inside the first gradient.
 static int virial_plan(Ctx& c) {
+  if (!c.sized) return THP_E_STATE;
   if (set_current_device(c)) return THP_E_CUDA;
   return ensure_plan(c);
 }

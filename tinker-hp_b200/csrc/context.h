@@ -64,6 +64,7 @@ struct Ctx {
   // number of the system's sizes, box and buffers: drawn anew (next_system_id)
   // by every create and reset, so that whatever holds them can tell
   unsigned long long system_id = 0;
+  bool sized = false;  // the buffers are those of cfg (not after a reset that could not allocate them)
   // counts the changes of what a captured front holds: multipoles rotated or
   // given, frames, the special pairs' number and buffers
   unsigned structure = 0;
