@@ -93,6 +93,23 @@ def test_virial_state_and_dropin(lib, case):
     assert np.abs((vir - 2.0) - vir_ref).max() < 1e-9 * np.abs(vir_ref).max()
 
 
+def test_retarget_drops_the_bound_virial(lib, case):
+    # the caller's vir(3,3) of the system before may be gone
+    ws, orc = case
+    ctx = lib.Context(ws)
+    L, P = lib.load(), lambda a: a.ctypes.data_as(C.POINTER(C.c_double))
+    vir = np.full((3, 3), 2.0)
+    assert L.thp_bind_virial(ctx.h, P(vir)) == 0
+    ctx.retarget(ws)
+    xyz = [np.ascontiguousarray(a) for a in (ws.x, ws.y, ws.z)]
+    rp, u, p, dep, ep = np.ascontiguousarray(orc.rpole), np.zeros((ws.n, 3)), np.zeros((ws.n, 3)), np.zeros((ws.n, 3)), np.zeros(1)
+    assert L.thp_bind_state(ctx.h, *[P(a) for a in xyz], P(rp), P(u), P(p), None, None, 0, P(ep)) == 0
+    assert L.thp_bind_gradient(ctx.h, P(dep)) == 0
+    L.epolar1_()
+    assert L.thp_last_error() == 0 and np.abs(dep).max() > 0.0
+    assert np.array_equal(vir, np.full((3, 3), 2.0))
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_empole_virial_matches_oracle(lib, case, precision):
     # empole1c's virial (emrecip1's site terms and scalar sum, emreal1c's pair

@@ -634,7 +634,7 @@ static void forget_system(thp_ctx* h) {
   h->rpole_current = false;
   h->field_valid = h->guess_uploaded = h->solved_once = false;
   c.bx = c.by = c.bz = c.brpole = c.buind = c.buinp = c.bep = c.bdep = c.bqgrid = nullptr;
-  c.bem = c.bdem = c.bev = c.bdev = nullptr;
+  c.bem = c.bdem = c.bev = c.bdev = c.bvir = nullptr;
   c.bnvlst = c.bvlst = nullptr;
   c.bmaxvlst = 0;
   c.have_vdw = false;
